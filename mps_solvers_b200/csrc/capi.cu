@@ -184,13 +184,10 @@ static void mark(mps_handle* h, int tag) {
 // The merge rebuild (cellsort.cuh) when at most MERGE_SMEM_CAP particles can
 // change cell between two rebuilds (fluid and moving walls) and the current
 // order is a sorted one; else the full radix sort.  Both give the same order.
-// The compact PPE layout on or off; with the learned preconditioner the
-// compact solver applies S' by compact columns (the 8-byte solver by
-// particle columns).
+// The compact PPE layout on or off.
 static void set_compact(mps_handle* h, bool on) {
     h->ppe.c16 = on && h->ppe.c16_ready;
-    h->ppe.c16_learned = h->ppe.c16 && h->opt.precond == MPS_PRECOND_LEARNED && h->ppe.sp_ent != nullptr &&
-                         h->ppe.cr2 != nullptr;
+    h->ppe.c16_learned = h->ppe.c16 && h->opt.precond == MPS_PRECOND_LEARNED && h->ppe.c16_spfirst != nullptr;
 }
 
 static bool use_merge(const mps_handle* h) {
@@ -588,13 +585,10 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         h->ppe.c16_smem_chunks = h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
         h->ppe.precond_every = h->opt.precond_every > 0 ? h->opt.precond_every : 40;
         h->ppe.index_of_id = h->index_of_id;
-        if (h->opt.ppe_layout == 0 && !h->nscenes) {
-            e = ppe_c16_enable(h->ppe, &h->err);
+        if (h->opt.ppe_layout == 0 && !h->nscenes && ppe_c16_takes(h->cap, h->g)) {
+            e = ppe_c16_enable(h->ppe, h->g, &h->err);
+            if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
-            if (h->opt.precond == MPS_PRECOND_LEARNED) {
-                e = ppe_c16_learned_enable(h->ppe, &h->err);
-                if (e != MPS_OK) return (mps_status)e;
-            }
             set_compact(h, true);
         }
         if (h->opt.visc_implicit) {
@@ -1358,7 +1352,7 @@ extern "C" mps_status mps_get_scalars(mps_handle* h, double* o) {
     o[15] = -1.0;
     if (h->opt.method == MPS_METHOD_SEMI_IMPLICIT && h->ppe.c16) {
         uint32_t esc = 0;
-        CK(cudaMemcpyAsync(&esc, h->ppe.c16_esc, sizeof esc, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaMemcpyAsync(&esc, h->ppe.c16_stats, sizeof esc, cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
         o[15] = esc;
     }
@@ -1643,7 +1637,7 @@ extern "C" mps_status mps_autotune(mps_handle* h, int steps, mps_tune_report* re
                 r.ppe_ms[c] = -1.f;
                 continue;
             }
-            if (form == 3 && !compact_ok) continue;
+            if (form == 3 && (!compact_ok || c % 3 != 0)) continue;  // the compact solver has one shape
             const bool pipe = form == 2;
             const int threads = ppe_cand[c % 3];
             if (ppe_set_threads(h->ppe, threads) != MPS_OK) {
@@ -1698,7 +1692,7 @@ extern "C" mps_status mps_apply_tuning(mps_handle* h, const mps_tune_report* r) 
                 h->err = "the compact PPE layout is for single scenes";
                 return MPS_ERR_INVALID;
             }
-            int e = ppe_c16_enable(h->ppe, &h->err);
+            int e = ppe_c16_enable(h->ppe, h->g, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
         }

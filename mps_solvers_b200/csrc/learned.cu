@@ -317,9 +317,11 @@ __global__ void __launch_bounds__(256) k_lp_ahat(LpSystem S, const float* __rest
     const uint32_t i = __ldg(S.rowlist + k);
     const uint32_t len = __ldg(S.rlen + i);
     const float4 pi = __ldg(S.pos + i);
+    const uint32_t* ac = S.acols + (size_t)(S.acols_by_row ? k : i) * PPE_W;
     float s = 0.f;
     for (uint32_t t = lane; t < len; t += 32) {
-        const uint32_t j = __ldg(S.acols + (size_t)i * PPE_W + t);
+        uint32_t j = __ldg(ac + t);
+        if (S.acols_by_row) j = __ldg(S.rowlist + j);
         const float4 pj = __ldg(S.pos + j);
         const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
         const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);

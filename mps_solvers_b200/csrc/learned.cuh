@@ -125,6 +125,7 @@ struct LpSystem {            // the assembled PPE system the network works on
     const uint32_t* rowlist; // non-Dirichlet rows
     const uint32_t* nrows;
     const uint32_t* acols;   // rlap stencil, row-major stride PPE_W
+    bool acols_by_row = false;  // by row, its columns row numbers (rowlist), instead of by particle
     const uint32_t* cell;    // cell of each particle
     const uint32_t* cell_start;
     Grid g;

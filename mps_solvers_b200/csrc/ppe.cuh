@@ -86,35 +86,46 @@ struct PpeWork {
     int* scene_iters = nullptr;
     int* scene_outer = nullptr;
     double* scene_relres = nullptr;
-    // compact layout (ppe_compact.cu): rows numbered 0..R-1 in row-list
-    // order, slices of 4 rows with 8 lanes per row, 16-bit column codes
-    // relative to the slice, FP32 weights; single scenes, diagonal scaling
+    // compact layout (ppe_compact.cu): rows numbered along a Hilbert curve
+    // over the linked cells, tiles of consecutive rows with a column list
+    // each, 16-bit codes into it beside FP32 weights; single scenes
     bool c16 = false;                  // the solve uses this layout
     bool c16_ready = false;            // its buffers exist
     int c16_smem_chunks = 8;           // chunks per warp held in shared memory across iterations
-    size_t c16_cap_chunks = 0;
+    uint32_t c16_nsuper = 0;           // linked cells, in curve order
+    uint32_t* c16_cells = nullptr;     // the up to 4 cells of the sorted grid of each
+    uint32_t* c16_nbr = nullptr;       // the 27 linked cells around each
+    uint32_t* c16_base = nullptr;      // its rows (counts, then scanned: its first row)
     uint32_t* cpos = nullptr;          // compact row of each particle (rows only)
-    uint32_t* c16_width = nullptr;     // chunks per slice, then (scanned) the slices' first chunk
-    uint16_t* c16_codes = nullptr;     // 128 codes per chunk (column - 4 * slice + 32768; 65535: escaped)
-    float* c16_w = nullptr;            // 128 weights per chunk
-    uint32_t* c16_side = nullptr;      // compact column of an escaped entry (same layout)
-    uint32_t* c16_esc = nullptr;       // escaped entries of the last pack
+    uint32_t* clen = nullptr;          // off-diagonal entries of each compact row
+    uint32_t* c16_off = nullptr;       // chunks per slice, then (scanned) the slices' first chunk
+    unsigned char* c16_ent = nullptr;  // chunks: 128 weights and 128 codes, 768 bytes each
+    uint32_t* c16_side = nullptr;      // compact column of an escaped entry (by entry)
+    uint32_t* c16_tile = nullptr;      // tile descriptors
+    uint32_t* c16_collist = nullptr;   // the tiles' columns
+    uint32_t* c16_stats = nullptr;     // [0] entries past a 16-bit offset from their slice, [1] most columns of a tile
     double *cb64 = nullptr, *cx64 = nullptr, *cdiag64 = nullptr;
-    float *cdiag32 = nullptr, *cinv_diag = nullptr, *cr = nullptr, *cq = nullptr;
-    float2* czp[2] = {nullptr, nullptr};
+    float *cdiag32 = nullptr, *cinv_diag = nullptr, *cr = nullptr, *cp = nullptr;
+    float* cdsq = nullptr;             // 1 / sqrt(-diagonal)
+    float4* cpub[2] = {nullptr, nullptr};  // what the other blocks read of a row, two buffers
+    ulonglong2* c16_slots = nullptr;   // the solver's grid sums
+    unsigned long long* c16_epoch = nullptr;  // and the epochs its launches have used
+    // the learned S' in the tiles' codes (code << 16 | BF16 value): the
+    // tiles' slices, the entries, the columns of escaped ones
+    uint32_t* c16_spfirst = nullptr;
+    uint32_t* c16_spent = nullptr;
+    uint32_t* c16_spside = nullptr;
     // the learned preconditioner: S' = D^-1/2 S D^-1/2 (S the symmetric form
     // in LearnedWork, kept by GEO index, rebuilt every precond_every steps)
     // packed for the current rows every step (layout: ppe_device.cuh), one
     // product fused into the residual update of every PCG iteration; its
-    // columns are compact positions for the compact solver and particle
-    // indices for the 8-byte and batch solvers
+    // columns are particle indices
     bool c16_learned = false;          // the compact solve applies S'
     int precond_every = 40;            // steps between network evaluations
     uint32_t* sp_off = nullptr;        // first entry of every 32-row slice (widths, then scanned)
     uint32_t* sp_ent = nullptr;        // off-diagonal entries: column - own column (16 bits) << 16 | BF16 value
     float* sp_diag = nullptr;          // the diagonal, per row position
-    float* cr2 = nullptr;              // second residual buffer of the compact solver's fused update
-    float2* rq[2] = {nullptr, nullptr};  // the 8-byte and batch solvers' (r, q) pairs, current and next
+    float2* rq[2] = {nullptr, nullptr};  // its solvers' (r, q) pairs by particle, current and next
     size_t sp_cap_chunks = 0;
     const uint32_t* index_of_id = nullptr;  // the handle's GEO index -> sorted position
     bool build_net = true;             // this step evaluates the network (learned preconditioner)
@@ -153,21 +164,23 @@ void ppe_free(PpeWork& w);
 int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint32_t* cols, float* wts,
                        uint64_t max_entries, uint64_t* nnz, cudaStream_t st);
 // The compact 16-bit layout and its persistent solver (ppe_compact.cu):
-// buffers, the pack after the row list, the solve with p = max(x, 0), the
+// whether it takes a grid and capacity, buffers, the pack after the assembly, the solve with p = max(x, 0), the
 // escaped-entry count of the last pack, and the stencil export.
-int ppe_c16_enable(PpeWork& w, std::string* err);
+bool ppe_c16_takes(uint32_t cap, const Grid& grid);
+int ppe_c16_enable(PpeWork& w, const Grid& grid, std::string* err);
+// the row numbers, before the assembly (bthr = beta n0; a batch uses its
+// scenes' own)
+int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st);
+int ppe_c16_learned_enable(PpeWork& w, std::string* err);
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st);
 int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, uint32_t cap, cudaStream_t st);
 int ppe_c16_export(const PpeWork& w, uint32_t np, const uint32_t* d_row_start, uint32_t* d_cols, float* d_w,
                    cudaStream_t st);
 void ppe_c16_free(PpeWork& w);
-// the learned S': its buffers (ppe_sp_enable; the compact solver's second
-// residual buffer too with ppe_c16_learned_enable), and its per-step pack
-// from the symmetric form kept by GEO index, after the row list (and, for
-// the compact columns, after ppe_c16_enqueue_pack)
+// the learned S': its buffers, and its per-step pack from the symmetric form
+// kept by GEO index, after the row list
 int ppe_sp_enable(PpeWork& w, std::string* err);
-int ppe_c16_learned_enable(PpeWork& w, std::string* err);
-int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st, bool by_particle);
+int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st);
 // the persistent solver's block size (256, 512 or 1024; 1024 threads per SM
 // either way); MPS_ERR_INVALID when the device cannot hold that shape
 int ppe_set_threads(PpeWork& w, int threads);

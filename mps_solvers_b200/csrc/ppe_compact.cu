@@ -3,26 +3,33 @@
 //
 // Same system as ppe.cu (MPS_CPU::buildPoisson, MPS_CAL_v4.0/MPS_CPU.cpp:619-710,
 // solved as MPS_CPU::DoCG's CG, :829-888, with diagonal scaling and FP64
-// defect correction), stored for fewer bytes per CG iteration:
+// defect correction).  The layout is built around tiles:
 //
-//  * unknowns are the R non-Dirichlet rows, numbered 0..R-1 in row-list
-//    (ascending particle) order; every solver vector is indexed that way, so
-//    the neighbour gathers touch a dense 8-byte-per-row vector;
-//  * slices of 4 rows; a warp takes a slice with 8 lanes per row, lane
-//    8 r + l holding entries 32 t + l, + 8, + 16 and + 24 of row r in chunk t
-//    (rows padded to a multiple of 32 entries with weight 0), so the lanes
-//    of a row gather 8 consecutive entries per instruction;
-//  * a column is stored as 16 bits, column - 4 * slice + 32768 (the rows a
-//    row couples to lie within a few cell layers of it in this numbering);
-//    a column out of that range is stored as 65535 and its full value is
-//    read from a side array with the same layout (escaped entries);
-//  * weights FP32, beside the codes: 6 bytes per entry instead of 8.
+//  * the R non-Dirichlet rows are numbered 0..R-1 along a Hilbert curve over
+//    the reference's linked cells (edge max(r0, rlap); the fast arithmetic's
+//    halved cells are grouped back into them), so a run of consecutive rows
+//    is a compact lump of the fluid;
+//  * a tile is such a run, one per block of the solver up to C16_TILE_ROWS
+//    rows on average, cut where the tiles carry equal shares of the matrix.
+//    Its rows couple to few distinct columns (the lump and a shell of one
+//    kernel radius around it: 2,900 columns for 920 rows of the 310,912-
+//    particle dam break, 6,100 for 1,840 rows of a 1.6 M-particle scene; the
+//    same runs in cell order have 5,200 and 11,800), which the tile lists;
+//  * an entry is the column's position in its tile's list, times 4, in 16
+//    bits, beside its FP32 weight: 6 bytes.  Slices of 8 rows, a warp takes
+//    one with 4 lanes per row; lane L = 8 q + r holds, in every chunk of 16
+//    entries of row r, entries 4 q to 4 q + 3.  A chunk is 768 contiguous
+//    bytes: 512 of weights, then 256 of codes;
+//  * a column past the tile's list (C16_COLS columns) is coded 65535 and its
+//    number kept in a side array; only rows with far more neighbours than a
+//    lattice has get there.
 //
-// Per chunk a warp reads 256 contiguous bytes of codes and 512 of weights.
-// The slices are dealt to warps round-robin; the same deal holds for the
-// whole solve, so each warp keeps the last few chunks of its share in shared
-// memory across all iterations, the matrix's head is read with an L2
-// evict_last policy and the rest streams as evict_first.
+// In every product a block first brings the tile's columns of the vector
+// into shared memory, in coalesced runs, and then reads each entry's operand
+// from there: the product streams the matrix, and its gathers never leave
+// the SM.  Before, each entry gathered 8 bytes through L1 from a vector the
+// whole grid reads, and the wait for those gathers set the pace.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -38,141 +45,511 @@ namespace {
 
 inline uint32_t cblocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
-constexpr uint32_t C16_ROWS = 4;      // rows per slice
-constexpr uint32_t C16_CHUNK = 128;   // entries per chunk (4 rows x 32)
-constexpr uint32_t C16_ESC = 0xffffu; // escaped code
-constexpr int C16_BIAS = 32768;
+constexpr uint32_t C16_ROWS = 8;            // rows per slice
+constexpr uint32_t C16_CHUNK = 128;         // entries per chunk (8 rows x 16)
+constexpr uint32_t C16_CHUNK_BYTES = 768;   // 128 weights, then 128 codes
+constexpr uint32_t C16_ESC = 0xffffu;       // escaped code
+// Rows of a tile on average, and a slice's cost beside its chunks (1 to 32 of
+// them) when tiles are cut: a tile then has at most 37 / 5 of the average,
+// 11,904 rows, which fit its column list, and the list as doubles and the
+// row sums fit a block's shared memory.
+constexpr uint32_t C16_TILE_ROWS = 1600;
+constexpr uint32_t C16_SLICE_COST = 5;
+constexpr uint32_t C16_COLS = 12288;        // columns a tile lists (4 x 12,287 is below the escape code)
+constexpr uint32_t C16_PAGE = 256;          // rows per page of the tile's column set
+constexpr uint32_t C16_PAGES = 512;         // pages a tile's column set holds
+constexpr uint32_t C16_NONE = 0xffffffffu;
+constexpr int C16_THREADS = 512;            // a solver block
+constexpr int C16_PACK_THREADS = 1024;
+constexpr int C16_BATCH = 4;                // chunks a warp loads at a time, twice buffered
+constexpr int C16_BATCH64 = 3;              // (6 of them: 5 % slower; 768 threads with 3: 2 to 10 % slower)
+constexpr uint32_t C16_STATS = 4;
+constexpr uint32_t C16_SP_SLICES = C16_COLS / 32 + 1;  // S' slices (32 rows) a tile can have, and one
 
-// Compact numbering of the rows, the rows' vectors in that numbering, and
-// the chunk count of every slice (the longest of its 4 rows).  Thread k
-// takes compact row k; 4 consecutive lanes form a slice.
-__global__ void __launch_bounds__(256) k_c16_rows(const uint32_t* __restrict__ rowlist,
-                                                  const uint32_t* __restrict__ nrows, const uint32_t* __restrict__ rlen,
-                                                  const double* __restrict__ b64, const double* __restrict__ x64,
-                                                  const double* __restrict__ diag64, const float* __restrict__ diag32,
-                                                  const float* __restrict__ inv_diag, uint32_t* __restrict__ cpos,
-                                                  double* __restrict__ cb64, double* __restrict__ cx64,
-                                                  double* __restrict__ cdiag64, float* __restrict__ cdiag32,
-                                                  float* __restrict__ cinv_diag, uint32_t* __restrict__ width,
-                                                  uint32_t maxslices) {
-    const uint32_t R = *nrows;
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t len = 0;
-    if (k < R) {
-        const uint32_t i = rowlist[k];
-        cpos[i] = k;
-        cb64[k] = b64[i];
-        cx64[k] = x64[i];
-        cdiag64[k] = diag64[i];
-        cdiag32[k] = diag32[i];
-        cinv_diag[k] = inv_diag[i];
-        len = rlen[i];
-    }
-    len = max(len, __shfl_xor_sync(0xffffffffu, len, 1));
-    len = max(len, __shfl_xor_sync(0xffffffffu, len, 2));
-    const uint32_t s = k / C16_ROWS;
-    if ((k & 3u) == 0 && s <= maxslices) width[s] = (len + 31u) / 32u;
+// One tile: slices [s0, s1), its columns (its own rows first, then the others
+// in ascending order), whether entries are escaped, and its longest slice.
+struct C16Tile {
+    uint32_t s0, s1, ncol, esc, wmax, pad[3];
+};
+
+// Tiles of R rows for G solver blocks: the same number for every block.
+__host__ __device__ __forceinline__ uint32_t c16_tiles(uint32_t R, uint32_t G) {
+    const uint32_t per = G * C16_TILE_ROWS;
+    const uint32_t k = (R + per - 1) / per;
+    return G * (k > 0 ? k : 1u);
 }
 
-// One warp per slice: the assembly's row-major columns (particle indices)
-// and weights, recoded.  Lane L = 8 r + l writes, per chunk, its 4 codes as
-// one 8-byte store and its 4 weights as one 16-byte store.
-__global__ void __launch_bounds__(256) k_c16_pack(const uint32_t* __restrict__ cols_rm, const float* __restrict__ w_rm,
-                                                  const uint32_t* __restrict__ rlen, const uint32_t* __restrict__ rowlist,
-                                                  const uint32_t* __restrict__ nrows, const uint32_t* __restrict__ off,
-                                                  const uint32_t* __restrict__ cpos, uint16_t* __restrict__ codes,
-                                                  float* __restrict__ wts, uint32_t* __restrict__ side,
-                                                  uint32_t* __restrict__ esc_count) {
-    const uint32_t R = *nrows;
-    const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31, r = lane >> 3, l = lane & 7;
-    if (slice >= (R + C16_ROWS - 1) / C16_ROWS) return;
-    const uint32_t g0 = off[slice];
-    const uint32_t T = off[slice + 1] - g0;
-    const uint32_t k = slice * C16_ROWS + r;
-    const bool has = k < R;
-    const uint32_t i = has ? rowlist[k] : 0u;
-    const uint32_t len = has ? rlen[i] : 0u;
-    const int base = (int)(slice * C16_ROWS) - C16_BIAS;
-    const uint32_t pad = r + (uint32_t)C16_BIAS;  // the row itself, weight 0
-    uint32_t nesc = 0;
-    for (uint32_t t = 0; t < T; t++) {
-        // lane 8 r + l holds entries l, l + 8, l + 16, l + 24 of the row's 32
-        // in this chunk, so that one gather instruction of the solver reads
-        // 8 consecutive entries of each row (neighbouring columns)
-        const uint32_t e = 32u * t + l;
-        uint32_t c[4] = {pad, pad, pad, pad};
-        float w[4] = {0.f, 0.f, 0.f, 0.f};
-        const size_t at = (size_t)(g0 + t) * C16_CHUNK + 4u * lane;
+// ---------------------------------------------------------------- row order
+// Whether particle i has a row (is not Dirichlet), as the assembly's test:
+// n < beta n0 in double exactly when n < the least float >= beta n0.
+struct C16Flag {
+    const float4* pos;
+    const float* n;
+    const uint32_t* id;
+    const uint32_t* sid_of_id;  // batch: the scene of each particle id
+    const PpeScene* scenes;
+    double bthr;
+};
+
+__device__ __forceinline__ bool c16_is_row(const C16Flag& F, uint32_t i) {
+    double b = F.bthr;
+    if (F.scenes) {
+        const PpeScene& s = F.scenes[F.sid_of_id[F.id[i]]];
+        b = s.beta * s.n0;
+    }
+    return ptype(F.pos[i]) != T_DUMMY && !((double)F.n[i] < b);
+}
+
+// Rows of linked cell h (its up to 4 cells of the sorted grid).
+__global__ void __launch_bounds__(256) k_c16_count(C16Flag F, const uint32_t* __restrict__ cells, uint32_t nsuper,
+                                                   const uint32_t* __restrict__ cs, uint32_t* __restrict__ base,
+                                                   uint32_t* __restrict__ stats) {
+    const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x < C16_STATS) stats[threadIdx.x] = 0u;
+    if (h > nsuper) return;
+    uint32_t n = 0;
+    if (h < nsuper) {
+        const uint4 c4 = *reinterpret_cast<const uint4*>(cells + 4 * (size_t)h);
+        const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const uint32_t eu = e + 8u * u;
-            if (eu < len) {
-                const uint32_t col = cpos[cols_rm[(size_t)i * PPE_W + eu]];
-                const int code = (int)col - base;
-                if (code >= 0 && code < (int)C16_ESC) {
-                    c[u] = (uint32_t)code;
-                } else {
-                    c[u] = C16_ESC;
-                    side[at + u] = col;
-                    nesc++;
-                }
-                w[u] = w_rm[(size_t)i * PPE_W + eu];
+            if (c[u] == C16_NONE) continue;
+            const uint32_t lo = cs[c[u]], hi = cs[c[u] + 1];
+            for (uint32_t i = lo + lane; i < hi; i += 32) n += c16_is_row(F, i) ? 1u : 0u;
+        }
+        n = __reduce_add_sync(0xffffffffu, n);
+    }
+    if (lane == 0) base[h] = n;  // base[nsuper] = 0: the scan leaves R there
+}
+
+// After the scan: row numbers and the row list.  A particle without a row
+// gets the identity row of the particle-indexed arrays.
+__global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, const uint32_t* __restrict__ cells, uint32_t nsuper,
+                                                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ base,
+                                                  uint32_t* __restrict__ cpos, uint32_t* __restrict__ rowlist,
+                                                  uint32_t* __restrict__ nrows, uint32_t* __restrict__ rlen,
+                                                  double* __restrict__ diag64) {
+    const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    if (h >= nsuper) return;
+    uint32_t at = base[h];
+    const uint4 c4 = *reinterpret_cast<const uint4*>(cells + 4 * (size_t)h);
+    const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+    if (h == nsuper - 1 && lane == 0) *nrows = base[nsuper];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        if (c[u] == C16_NONE) continue;
+        const uint32_t lo = cs[c[u]], hi = cs[c[u] + 1];
+        for (uint32_t i0 = lo; i0 < hi; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const bool f = i < hi && c16_is_row(F, i);
+            const uint32_t m = __ballot_sync(0xffffffffu, f);
+            if (f) {
+                const uint32_t k = at + __popc(m & lt);
+                cpos[i] = k;
+                rowlist[k] = i;
+            } else if (i < hi) {
+                cpos[i] = C16_NONE;
+                rlen[i] = PPE_DIRICHLET;
+                diag64[i] = 1.0;
+            }
+            at += __popc(m);
+        }
+    }
+}
+
+// Chunks of every slice (the longest of its 8 rows), then scanned.
+__global__ void __launch_bounds__(256) k_c16_width(const uint32_t* __restrict__ clen, const uint32_t* __restrict__ nrows,
+                                                   uint32_t* __restrict__ width, uint32_t maxslices) {
+    const uint32_t R = *nrows;
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t len = k < R ? clen[k] : 0u;
+#pragma unroll
+    for (int o = 1; o < (int)C16_ROWS; o <<= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
+    const uint32_t s = k / C16_ROWS;
+    if (k % C16_ROWS == 0 && s <= maxslices) width[s] = (len + 15u) / 16u;
+}
+
+// ---------------------------------------------------------------- pack
+// smallest x in [0, n] with x == n or f(x) >= v, f ascending; a whole warp
+// probes 32 places a round
+template <class F>
+__device__ __forceinline__ uint32_t warp_lower(uint32_t n, uint64_t v, F f) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t x = lo + lane * step;
+        const uint32_t below = __popc(__ballot_sync(0xffffffffu, x < hi && f(x) < v));
+        if (below == 0) break;
+        hi = min(hi, lo + below * step);
+        lo += (below - 1) * step + 1;
+    }
+    return lo;
+}
+
+struct C16PackArgs {
+    const uint32_t* cols_rm;  // row numbers of the columns, row-major by row
+    const float* w_rm;
+    const uint32_t* clen;
+    const uint32_t* nrows;
+    const uint32_t* off;
+    const uint32_t* base;     // first row of every linked cell
+    const uint32_t* nbr;      // 27 linked cells around each (C16_NONE: outside)
+    uint32_t nsuper, blocks;
+    C16Tile* tiles;
+    uint32_t* collist;        // C16_COLS per tile
+    unsigned char* ent;
+    uint32_t* side;
+    uint32_t* stats;          // [0] entries beyond a 16-bit offset from their slice, [1] most columns, [2] most rows,
+                              // [3] fours of S' given out
+    // learned S' (LRN)
+    const uint32_t* rowlist;
+    const uint32_t* cpos;
+    const uint32_t* idv;      // GEO index of each particle
+    const uint32_t* index_of_id;
+    const float* dsq;         // 1 / sqrt(-diagonal) by row
+    const uint32_t* s_cnt;
+    const uint32_t* s_col;
+    const float* s_val;
+    const float* s_diag;
+    uint32_t np;
+    const Scalars* sc;
+    uint32_t* sp_first;       // C16_SP_SLICES per tile
+    uint32_t* sp_ent;
+    uint32_t* sp_side;
+    float* sp_diag;
+};
+
+// exclusive scan of one value per thread over the block; *total the sum
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* ws, uint32_t* total) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+        if ((int)lane >= o) x += t;
+    }
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    uint32_t w = lane < nw ? ws[lane] : 0u;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
+        if ((int)lane >= o) w += t;
+    }
+    const uint32_t prev = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0u);
+    *total = __shfl_sync(0xffffffffu, w, 31);
+    __syncthreads();
+    return (warp ? prev : 0u) + x - v;
+}
+
+__device__ __forceinline__ uint32_t sp_bf16_bits(float v) {
+    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+
+// S' of a tile: 32-row slices of its rows, each as wide as its longest row,
+// in fours of words; four f of local row k is at first[k / 32] + 32 f + k % 32.
+// One block per tile.  The rows its entries can name are those of the linked
+// cells around its own ones; their 256-row pages get consecutive slots, the
+// columns in use (other than its own rows) a bit each in their page's slot,
+// and a column's position in the tile's list is the number of bits before
+// it.  With the learned preconditioner the columns of S' are marked too, and
+// S' is coded the same way, one thread per row.
+template <bool LRN>
+__global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
+    extern __shared__ uint16_t page_slot[];  // slot of every page of rows (0xffff: none)
+    __shared__ uint2 bits[C16_PAGES * 8];    // columns in use, and those before the word
+    __shared__ uint32_t slot_page[C16_PAGES];
+    __shared__ uint32_t ws[32], found[4];
+    const uint32_t R = *A.nrows;
+    const uint32_t nsl = (R + C16_ROWS - 1) / C16_ROWS;
+    const uint32_t T = c16_tiles(R, A.blocks);
+    const uint32_t t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
+    const uint32_t lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+    if (t >= T) return;
+    // equal shares of the chunks, a slice counting C16_SLICE_COST more
+    const uint64_t W = (uint64_t)A.off[nsl] + (uint64_t)C16_SLICE_COST * nsl;
+    if (warp < 2) {
+        const uint32_t s = warp_lower(nsl, W * (t + warp) / T, [&](uint32_t x) {
+            return (uint64_t)__ldg(A.off + x) + (uint64_t)C16_SLICE_COST * x;
+        });
+        if (lane == 0) found[warp] = t + warp == T ? nsl : s;
+    }
+    const uint32_t npages = (R + C16_PAGE - 1) / C16_PAGE;
+    for (uint32_t p = tid; p < npages; p += nthr) page_slot[p] = 0;
+    __syncthreads();
+    const uint32_t s0 = found[0], s1 = found[1];
+    if (s0 >= s1) {
+        if (tid == 0) A.tiles[t] = C16Tile{s0, s0, 0u, 0u, 0u, {0u, 0u, 0u}};
+        return;
+    }
+    const uint32_t r0 = s0 * C16_ROWS, r1 = min(s1 * C16_ROWS, R), rows = r1 - r0;
+    if (warp < 2) {  // the linked cells of the first and the last row
+        const uint32_t k = warp ? r1 - 1 : r0;
+        const uint32_t h = warp_lower(A.nsuper, (uint64_t)k + 1, [&](uint32_t x) { return (uint64_t)__ldg(A.base + x); });
+        if (lane == 0) found[2 + warp] = h - 1;
+    }
+    __syncthreads();
+    const uint32_t h0 = found[2], h1 = found[3];
+    for (uint32_t x = tid; x < (h1 - h0 + 1) * 27u; x += nthr) {
+        const uint32_t nb = __ldg(A.nbr + (size_t)h0 * 27 + x);
+        if (nb == C16_NONE) continue;
+        const uint32_t lo = __ldg(A.base + nb), hi = __ldg(A.base + nb + 1);
+        if (lo < hi)
+            for (uint32_t p = lo / C16_PAGE; p <= (hi - 1) / C16_PAGE; p++) page_slot[p] = 1;
+    }
+    __syncthreads();
+    // slots in page order
+    uint32_t nslots;
+    {
+        const uint32_t per = (npages + nthr - 1) / nthr;
+        const uint32_t p0 = min(tid * per, npages), p1 = min(p0 + per, npages);
+        uint32_t c = 0;
+        for (uint32_t p = p0; p < p1; p++) c += page_slot[p];
+        uint32_t slot = block_scan(c, ws, &nslots);
+        for (uint32_t p = p0; p < p1; p++) {
+            if (page_slot[p] && slot < C16_PAGES) {
+                slot_page[slot] = p;
+                page_slot[p] = (uint16_t)slot++;
+            } else {
+                page_slot[p] = 0xffffu;
             }
         }
-        *reinterpret_cast<uint2*>(codes + at) = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
-        *reinterpret_cast<float4*>(wts + at) = make_float4(w[0], w[1], w[2], w[3]);
+        nslots = min(nslots, C16_PAGES);
     }
-    nesc = __reduce_add_sync(0xffffffffu, nesc);
-    if (lane == 0 && nesc) atomicAdd(esc_count, nesc);
+    const uint32_t words = nslots * 8;
+    for (uint32_t w = tid; w < words; w += nthr) bits[w].x = 0u;
+    __syncthreads();
+    auto mark = [&](uint32_t col) {
+        if (col - r0 < rows) return;
+        const uint32_t s = page_slot[col / C16_PAGE];
+        if (s == 0xffffu) return;
+        uint32_t* w = &bits[s * 8 + ((col / 32) & 7u)].x;
+        const uint32_t b = 1u << (col & 31u);
+        if (!(*(volatile uint32_t*)w & b)) atomicOr(w, b);
+    };
+    // a warp per row, eight of a lane's entries at a time
+    for (uint32_t k = r0 + warp; k < r1; k += nwarps) {
+        const uint32_t* rc = A.cols_rm + (size_t)k * PPE_W;
+        const uint32_t len = __ldg(A.clen + k);
+        for (uint32_t e0 = lane; e0 < len; e0 += 256) {
+            uint32_t col[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) col[u] = e0 + 32u * u < len ? __ldg(rc + e0 + 32u * u) : r0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) mark(col[u]);
+        }
+    }
+    // the row of stored neighbour u of a row with GEO index id (C16_NONE: none now)
+    auto sp_row_of = [&](uint32_t id, uint32_t u) -> uint32_t {
+        const uint32_t j = __ldg(A.index_of_id + __ldg(A.s_col + (size_t)id * LP_GW + u));
+        return j < A.sc->np ? __ldg(A.cpos + j) : C16_NONE;
+    };
+    if (LRN) {
+        for (uint32_t x = tid; x < rows * 8u; x += nthr) {  // eight threads a row
+            const uint32_t id = __ldg(A.idv + __ldg(A.rowlist + r0 + x / 8u));
+            const uint32_t n = __ldg(A.s_cnt + id);
+            for (uint32_t u = x & 7u; u < n; u += 8) {
+                const uint32_t col = sp_row_of(id, u);
+                if (col != C16_NONE) mark(col);
+            }
+        }
+    }
+    __syncthreads();
+    // the columns before every word, the list
+    uint32_t* list = A.collist + (size_t)t * C16_COLS;
+    for (uint32_t k = tid; k < rows; k += nthr) list[k] = r0 + k;
+    const uint32_t wper = (words + nthr - 1) / nthr;
+    const uint32_t w0 = min(tid * wper, words), w1 = min(w0 + wper, words);
+    uint32_t c = 0, ncol;
+    for (uint32_t w = w0; w < w1; w++) c += __popc(bits[w].x);
+    uint32_t at = rows + block_scan(c, ws, &ncol);
+    for (uint32_t w = w0; w < w1; w++) {
+        bits[w].y = at;
+        uint32_t m = bits[w].x;
+        const uint32_t c0 = slot_page[w >> 3] * C16_PAGE + (w & 7u) * 32u;
+        while (m) {
+            const uint32_t b = __ffs(m) - 1;
+            m &= m - 1;
+            if (at < C16_COLS) list[at] = c0 + b;
+            at++;
+        }
+    }
+    ncol = min(ncol + rows, C16_COLS);
+    __syncthreads();
+    // position of a column in the list, C16_NONE when it is not there
+    auto local_of = [&](uint32_t col) -> uint32_t {
+        if (col - r0 < rows) return col - r0;
+        const uint32_t s = page_slot[col / C16_PAGE];
+        if (s == 0xffffu) return C16_NONE;
+        const uint2 b = bits[s * 8 + ((col / 32) & 7u)];
+        const uint32_t p = b.y + __popc(b.x & ((1u << (col & 31u)) - 1u));
+        return p < C16_COLS ? p : C16_NONE;
+    };
+    uint32_t far = 0, nesc = 0, wmax = 0;
+    for (uint32_t s = s0 + warp; s < s1; s += nwarps) {
+        const uint32_t r = lane & 7u, q = lane >> 3;
+        const uint32_t g0 = __ldg(A.off + s), nch = __ldg(A.off + s + 1) - g0;
+        wmax = max(wmax, nch);
+        const uint32_t k = s * C16_ROWS + r;
+        const uint32_t len = k < R ? __ldg(A.clen + k) : 0u;
+        const uint4* rc = reinterpret_cast<const uint4*>(A.cols_rm + (size_t)min(k, R - 1) * PPE_W);
+        const float4* rw = reinterpret_cast<const float4*>(A.w_rm + (size_t)min(k, R - 1) * PPE_W);
+        const uint32_t padcode = 4u * min(k - r0, rows - 1);  // the row itself, weight 0
+#pragma unroll 2
+        for (uint32_t x = 0; x < nch; x++) {
+            const uint32_t e = 16u * x + 4u * q;
+            uint4 cv = make_uint4(0, 0, 0, 0);
+            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (e < len) {
+                cv = __ldg(rc + 4u * x + q);
+                w = __ldg(rw + 4u * x + q);
+            }
+            const uint32_t cc[4] = {cv.x, cv.y, cv.z, cv.w};
+            const size_t ch = (size_t)(g0 + x);
+            uint32_t code[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                code[u] = padcode;
+                if (e + u >= len) continue;
+                const uint32_t p = local_of(cc[u]);
+                const int d = (int)cc[u] - (int)(s * C16_ROWS) + 32768;
+                if (d < 0 || d >= (int)C16_ESC) far++;
+                if (p == C16_NONE) {
+                    code[u] = C16_ESC;
+                    A.side[ch * C16_CHUNK + 4u * lane + u] = cc[u];
+                    nesc++;
+                } else {
+                    code[u] = 4u * p;
+                }
+            }
+            if (e + 1 >= len) w.y = 0.f;
+            if (e + 2 >= len) w.z = 0.f;
+            if (e + 3 >= len) w.w = 0.f;
+            unsigned char* dst = A.ent + ch * C16_CHUNK_BYTES;
+            *reinterpret_cast<float4*>(dst + 16u * lane) = w;
+            *reinterpret_cast<uint2*>(dst + 512u + 8u * lane) =
+                make_uint2(code[0] | (code[1] << 16), code[2] | (code[3] << 16));
+        }
+    }
+    if (LRN) {
+        // the widths from the stored counts (rows' kept entries are at most
+        // those; the rest are zeros), then the tile's place in the array
+        __shared__ uint32_t first[C16_SP_SLICES + 1];
+        const uint32_t nsp = (rows + SP_SLICE - 1) / SP_SLICE;
+        for (uint32_t j = warp; j < nsp; j += nwarps) {
+            const uint32_t k = j * SP_SLICE + lane;
+            const uint32_t n =
+                k < rows ? (__ldg(A.s_cnt + __ldg(A.idv + __ldg(A.rowlist + r0 + k))) + 3u) / 4u : 0u;
+            const uint32_t w = __reduce_max_sync(0xffffffffu, n);
+            if (lane == 0) first[j + 1] = w * SP_SLICE;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            uint32_t n = 0;
+            for (uint32_t j = 0; j < nsp; j++) n += first[j + 1];
+            first[0] = atomicAdd(A.stats + 3, n);
+            for (uint32_t j = 0; j < nsp; j++) first[j + 1] += first[j];
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j <= nsp; j += nthr) A.sp_first[(size_t)t * C16_SP_SLICES + j] = first[j];
+        // a pair without a row now is left out (of both its rows), which
+        // keeps S' symmetric and diagonally dominant
+        for (uint32_t k = tid; k < rows; k += nthr) {
+            const uint32_t id = __ldg(A.idv + __ldg(A.rowlist + r0 + k));
+            const uint32_t n = __ldg(A.s_cnt + id);
+            const float di = __ldg(A.dsq + r0 + k);
+            A.sp_diag[r0 + k] = __ldg(A.s_diag + id) * (di * di);
+            const uint32_t f0 = first[k / SP_SLICE], words = (first[k / SP_SLICE + 1] - f0) / SP_SLICE * 4u;
+            auto place = [&](uint32_t w) { return ((size_t)f0 + w / 4u * SP_SLICE + k % SP_SLICE) * 4u + (w & 3u); };
+            uint32_t m = 0;
+            for (uint32_t u0 = 0; u0 < n; u0 += 8) {
+                uint32_t col[8];
+#pragma unroll
+                for (uint32_t b = 0; b < 8; b++) col[b] = u0 + b < n ? sp_row_of(id, u0 + b) : C16_NONE;
+                float v[8];
+#pragma unroll
+                for (uint32_t b = 0; b < 8; b++)
+                    v[b] = col[b] == C16_NONE
+                               ? 0.f
+                               : __ldg(A.s_val + (size_t)id * LP_GW + u0 + b) * (di * __ldg(A.dsq + col[b]));
+#pragma unroll
+                for (uint32_t b = 0; b < 8; b++) {
+                    if (col[b] == C16_NONE) continue;
+                    const uint32_t p = local_of(col[b]);
+                    if (p == C16_NONE) {
+                        A.sp_side[place(m)] = col[b];
+                        nesc++;
+                    }
+                    A.sp_ent[place(m)] = ((p == C16_NONE ? C16_ESC : 4u * p) << 16) | sp_bf16_bits(v[b]);
+                    m++;
+                }
+            }
+            for (; m < words; m++) A.sp_ent[place(m)] = 0u;
+        }
+    }
+    far = __reduce_add_sync(0xffffffffu, far);
+    if (lane == 0 && far) atomicAdd(A.stats, far);
+    if (lane == 0) ws[warp] = wmax;
+    const int any = __syncthreads_or((int)nesc);
+    if (tid == 0) {
+        for (uint32_t w = 0; w < nwarps; w++) wmax = max(wmax, ws[w]);
+        A.tiles[t] = C16Tile{s0, s1, ncol, any ? 1u : 0u, wmax, {0u, 0u, 0u}};
+        atomicMax(A.stats + 1, ncol);
+        atomicMax(A.stats + 2, rows);
+    }
 }
 
 // p = max(x, 0) for the rows, 0 for Dirichlet particles (pressCorr,
 // MPS_CAL_v4.0/MPS_CPU.cpp:734-743).
-__global__ void __launch_bounds__(256) k_c16_finish(const double* __restrict__ cx64, const uint32_t* __restrict__ rlen,
-                                                    const uint32_t* __restrict__ cpos, float* __restrict__ press,
-                                                    const Scalars* __restrict__ sc) {
+__global__ void __launch_bounds__(256) k_c16_finish(const double* __restrict__ cx64, const uint32_t* __restrict__ cpos,
+                                                    float* __restrict__ press, const Scalars* __restrict__ sc) {
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float p = 0.f;
-    if (rlen[i] != PPE_DIRICHLET) {
-        p = (float)cx64[cpos[i]];
+    const uint32_t k = cpos[i];
+    if (k != C16_NONE) {
+        p = (float)cx64[k];
         if (p < 0.f) p = 0.f;
     }
     press[i] = p;
 }
 
 // Export: the stored entries of every row as particle indices, at
-// row_start[i] (the particle's list) in stored order.
-__global__ void __launch_bounds__(256) k_c16_export(const uint32_t* __restrict__ rlen,
+// row_start[i] (the particle's list) in stored order.  One block per tile.
+__global__ void __launch_bounds__(256) k_c16_export(const C16Tile* __restrict__ tiles,
+                                                    const uint32_t* __restrict__ collist, uint32_t blocks,
+                                                    const uint32_t* __restrict__ clen,
                                                     const uint32_t* __restrict__ rowlist,
                                                     const uint32_t* __restrict__ nrows, const uint32_t* __restrict__ off,
-                                                    const uint16_t* __restrict__ codes, const float* __restrict__ wts,
+                                                    const unsigned char* __restrict__ ent,
                                                     const uint32_t* __restrict__ side,
                                                     const uint32_t* __restrict__ row_start, uint32_t* __restrict__ cols,
                                                     float* __restrict__ out_w) {
     const uint32_t R = *nrows;
-    const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31, r = lane >> 3, l = lane & 7;
-    if (slice >= (R + C16_ROWS - 1) / C16_ROWS) return;
-    const uint32_t k = slice * C16_ROWS + r;
-    if (k >= R) return;
-    const uint32_t g0 = off[slice], T = off[slice + 1] - g0;
-    const uint32_t i = rowlist[k];
-    const uint32_t len = rlen[i];
-    const uint32_t o = row_start[i];
-    const int base = (int)(slice * C16_ROWS) - C16_BIAS;
-    for (uint32_t t = 0; t < T; t++)
-        for (uint32_t u = 0; u < 4; u++) {
-            const uint32_t e = 32u * t + l + 8u * u;  // the pack's order (k_c16_pack)
-            if (e >= len) continue;
-            const size_t at = (size_t)(g0 + t) * C16_CHUNK + 4u * lane + u;
-            const uint32_t c = codes[at];
-            const uint32_t col = c == C16_ESC ? side[at] : (uint32_t)(base + (int)c);
-            cols[o + e] = rowlist[col];
-            out_w[o + e] = wts[at];
-        }
+    if (blockIdx.x >= c16_tiles(R, blocks)) return;
+    const C16Tile ti = tiles[blockIdx.x];
+    const uint32_t lane = threadIdx.x & 31, r = lane & 7u, q = lane >> 3;
+    for (uint32_t s = ti.s0 + (threadIdx.x >> 5); s < ti.s1; s += blockDim.x >> 5) {
+        const uint32_t k = s * C16_ROWS + r;
+        if (k >= R) continue;
+        const uint32_t g0 = off[s], W = off[s + 1] - g0;
+        const uint32_t o = row_start[rowlist[k]], len = clen[k];
+        for (uint32_t x = 0; x < W; x++)
+            for (uint32_t u = 0; u < 4; u++) {
+                const uint32_t e = 16u * x + 4u * q + u;  // the pack's order (k_c16_pack)
+                if (e >= len) continue;
+                const unsigned char* src = ent + (size_t)(g0 + x) * C16_CHUNK_BYTES;
+                const uint32_t c = reinterpret_cast<const uint16_t*>(src + 512)[4u * lane + u];
+                const uint32_t col = c == C16_ESC ? side[(size_t)(g0 + x) * C16_CHUNK + 4u * lane + u]
+                                                  : collist[(size_t)blockIdx.x * C16_COLS + c / 4u];
+                cols[o + e] = rowlist[col];
+                out_w[o + e] = reinterpret_cast<const float*>(src)[4u * lane + u];
+            }
+    }
 }
 
 // ---------------------------------------------------------------- learned S'
@@ -181,16 +558,14 @@ __global__ void __launch_bounds__(256) k_c16_export(const uint32_t* __restrict__
 // neighbours that are rows now.  A pair whose columns lie farther apart than
 // 32,767 is left out from both its rows, which keeps S' symmetric and
 // diagonally dominant (S is built dominant with a 1 % margin, more than BF16
-// rounding of the entries takes away, so S' stays SPD).  PART selects the
-// columns: particle indices (the particle-indexed solvers) or compact
-// positions (the compact solver).
+// rounding of the entries takes away, so S' stays SPD).  Columns are particle
+// indices in every solver.
 struct SpArgs {
     const uint32_t* rowlist;
     const uint32_t* nrows;
     const uint32_t* idv;       // GEO index of each particle
     const uint32_t* index_of_id;
     const uint32_t* rlen;
-    const uint32_t* cpos;
     const double* diag64;      // particle-indexed diagonal of A
     const uint32_t* s_cnt;
     const uint32_t* s_col;
@@ -206,13 +581,12 @@ struct SpArgs {
 // The pack takes a thread per row (lane = row of the 32-row slice, so the
 // packed words leave as coalesced 128-byte rows) and eight of its stored
 // neighbours at a time, their loads issued together: the chain s_col ->
-// index_of_id -> rlen, cpos, diag64 costs three dependent rounds per eight
+// index_of_id -> rlen, diag64 costs three dependent rounds per eight
 // entries instead of per entry.
 constexpr uint32_t SP_BATCH = 8;
 
 // the batch [u0, u0 + 8) of the stored neighbours of a row with own column
 // c: kept or not, the column offset and the neighbour's particle index
-template <bool PART>
 __device__ __forceinline__ void sp_batch(const SpArgs& A, uint32_t id, uint32_t n, uint32_t u0, uint32_t np,
                                          uint32_t c, bool (&ok)[SP_BATCH], int (&d)[SP_BATCH],
                                          uint32_t (&j)[SP_BATCH]) {
@@ -222,16 +596,14 @@ __device__ __forceinline__ void sp_batch(const SpArgs& A, uint32_t id, uint32_t 
         jd[b] = u0 + b < n ? __ldg(A.s_col + (size_t)id * LP_GW + u0 + b) : 0u;
 #pragma unroll
     for (uint32_t b = 0; b < SP_BATCH; b++) j[b] = u0 + b < n ? __ldg(A.index_of_id + jd[b]) : np;
-    uint32_t len[SP_BATCH], cp[SP_BATCH];
+    uint32_t len[SP_BATCH];
 #pragma unroll
     for (uint32_t b = 0; b < SP_BATCH; b++) {
-        const bool live = j[b] < np;
-        len[b] = live ? __ldg(A.rlen + j[b]) : PPE_DIRICHLET;
-        cp[b] = PART ? j[b] : (live ? __ldg(A.cpos + j[b]) : 0u);
+        len[b] = j[b] < np ? __ldg(A.rlen + j[b]) : PPE_DIRICHLET;
     }
 #pragma unroll
     for (uint32_t b = 0; b < SP_BATCH; b++) {
-        d[b] = (int)cp[b] - (int)c;
+        d[b] = (int)j[b] - (int)c;
         ok[b] = len[b] != PPE_DIRICHLET && d[b] >= -32767 && d[b] <= 32767;
     }
 }
@@ -252,13 +624,8 @@ __global__ void __launch_bounds__(256) k_sp_width(SpArgs A) {
     if ((threadIdx.x & 31) == 0 && s <= A.maxslices) A.off[s] = cnt * SP_SLICE;
 }
 
-__device__ __forceinline__ uint32_t sp_bf16_bits(float v) {
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
-}
-
 // Pass 2 (after the scan of off): the kept entries of row k in stored order,
 // then zeros up to the slice's width.
-template <bool PART>
 __global__ void __launch_bounds__(256) k_sp_pack(SpArgs A) {
     const uint32_t R = *A.nrows, np = A.sc->np;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -276,7 +643,7 @@ __global__ void __launch_bounds__(256) k_sp_pack(SpArgs A) {
             bool ok[SP_BATCH];
             int d[SP_BATCH];
             uint32_t j[SP_BATCH];
-            sp_batch<PART>(A, id, n, u0, np, PART ? i : k, ok, d, j);
+            sp_batch(A, id, n, u0, np, i, ok, d, j);
             double dg[SP_BATCH];
             float sv[SP_BATCH];
 #pragma unroll
@@ -300,54 +667,34 @@ __global__ void __launch_bounds__(256) k_sp_pack(SpArgs A) {
 // ---------------------------------------------------------------- solve
 struct C16Args {
     const uint32_t* nrows;
-    const uint32_t* off;       // first chunk of every slice
-    const uint16_t* codes;
-    const float* wts;
+    const uint32_t* off;        // first chunk of every slice
+    const unsigned char* ent;
     const uint32_t* side;
+    const C16Tile* tiles;
+    const uint32_t* collist;
+    const uint32_t* stats;      // [1] most columns and [2] most rows of a tile
     const double* b64;
     const double* diag64;
     const float* diag32;
     const float* inv_diag;
     double* x64;
-    float* r;
-    float2* zp0;               // (z, p) per row: current and next
-    float2* zp1;
-    float* q;
-    double* part;
-    double* result;
-    unsigned* bar;
+    float *p, *r;               // direction and residual (a block of several tiles keeps them here)
+    float4* pub0;               // what other blocks read of a row, current and next
+    float4* pub1;
+    ulonglong2* slots;          // grid sums: the blocks' inboxes, twice
+    unsigned long long* epoch;  // epochs used by the launches so far
     Scalars* sc;
     double tol, eta_min;
-    uint32_t keep;             // chunks read as evict_last
+    uint32_t keep;              // chunks read as evict_last, over all tiles
     int max_iter, inner_cap, max_outer;
-    int smem_chunks;           // chunks per warp held in shared memory
-    // learned S' (LRN): slices of the same 4 rows, the second residual buffer
-    const uint32_t* sp_off;
+    uint32_t smem_chunks;       // most chunks a block holds in shared memory
+    uint32_t smem_bytes;        // its dynamic shared memory
+    // learned S' (LRN): codes into the tile's columns, by row
+    const uint32_t* sp_first;
     const uint32_t* sp_ent;
+    const uint32_t* sp_side;
     const float* sp_diag;
-    float* r2;
 };
-
-// Row k of S' x on the compact rows (own column k).
-template <class X>
-__device__ __forceinline__ float sp_row(const C16Args& S, uint32_t k, X x) {
-    return sp_row_at(S.sp_off, S.sp_ent, S.sp_diag, k, k, x);
-}
-
-// The four columns of a lane's chunk entries.
-__device__ __forceinline__ void c16_cols(const uint2 cw, int base, const uint32_t* __restrict__ side, size_t at,
-                                         uint32_t (&col)[4]) {
-    col[0] = (uint32_t)(base + (int)(cw.x & 0xffffu));
-    col[1] = (uint32_t)(base + (int)(cw.x >> 16));
-    col[2] = (uint32_t)(base + (int)(cw.y & 0xffffu));
-    col[3] = (uint32_t)(base + (int)(cw.y >> 16));
-    if ((__vcmpeq2(cw.x, 0xffffffffu) | __vcmpeq2(cw.y, 0xffffffffu)) != 0u) {
-        if ((cw.x & 0xffffu) == C16_ESC) col[0] = __ldg(side + at);
-        if ((cw.x >> 16) == C16_ESC) col[1] = __ldg(side + at + 1);
-        if ((cw.y & 0xffffu) == C16_ESC) col[2] = __ldg(side + at + 2);
-        if ((cw.y >> 16) == C16_ESC) col[3] = __ldg(side + at + 3);
-    }
-}
 
 __device__ __forceinline__ uint2 ld_codes(const uint2* p, uint64_t pol) {
     uint2 v;
@@ -357,230 +704,802 @@ __device__ __forceinline__ uint2 ld_codes(const uint2* p, uint64_t pol) {
     return v;
 }
 
-__device__ __forceinline__ uint64_t c16_policy(uint32_t chunk, uint32_t keep) { return mat_policy(chunk, keep); }
+// Grid-wide sum of K doubles fused with a grid barrier, in one crossing of
+// the chip: every block has an inbox with a place for each block, a block
+// writes its sums into all inboxes as (value, epoch) pairs, single 16-byte
+// accesses, and waits for its own inbox to fill.  No place is read by more
+// than one block: with one shared place per block, 148 readers polling each
+// delayed the writes to 11 us.  The sums are added in block order by a fixed
+// tree, so they are the same in every block and every run.  Two inboxes: a
+// block writes those of epoch e + 2 only after every block has read those of
+// epoch e.  The wait is bounded: after the budget (1 s) it sets
+// ERR_DEVICE_TIMEOUT and returns false.
+struct C16Sync {
+    ulonglong2* slots;
+    unsigned long long epoch;
+    Scalars* sc;
+};
+constexpr uint32_t C16_SUMS = 3;
 
-// LRN: the learned preconditioner z = S' r instead of z = D^-1 r; S' is
-// applied in the residual update (the neighbours' new residuals formed from
-// r and q on the fly), so an iteration keeps two grid-wide reductions.
-template <bool EX, bool LRN>
-__global__ void __launch_bounds__(PPE_THREADS) k_ppe_solve_c16(C16Args S) {
-    extern __shared__ __align__(16) unsigned char c16_sm[];
-    const uint32_t R = *S.nrows;
-    const uint32_t nsl = (R + C16_ROWS - 1) / C16_ROWS;
-    const uint32_t lane = threadIdx.x & 31, rr = lane >> 3, l = lane & 7;
-    const uint32_t wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t C = (uint32_t)S.smem_chunks;
-    uint2* smc = reinterpret_cast<uint2*>(c16_sm) + (size_t)wib * C * 32;
-    float4* smw = reinterpret_cast<float4*>(c16_sm + (size_t)wpb * C * 32 * sizeof(uint2)) + (size_t)wib * C * 32;
-    const uint2* __restrict__ gcodes = reinterpret_cast<const uint2*>(S.codes);
-    const float4* __restrict__ gw4 = reinterpret_cast<const float4*>(S.wts);
-
-    // this warp's chunks, in the order it visits them; the last C of them
-    // stay in shared memory for the whole solve
-    uint32_t U = 0;
-    for (uint32_t sl = gw; sl < nsl; sl += nw) U += __ldg(S.off + sl + 1) - __ldg(S.off + sl);
-    const uint32_t u0 = U > C ? U - C : 0u;
-    {
-        uint32_t u = 0;
-        for (uint32_t sl = gw; sl < nsl; sl += nw) {
-            const uint32_t g0 = __ldg(S.off + sl), T = __ldg(S.off + sl + 1) - g0;
-            for (uint32_t t = (u0 > u ? min(T, u0 - u) : 0u); t < T; t++) {
-                const size_t g = (size_t)(g0 + t) * 32 + lane;
-                smc[(u + t - u0) * 32 + lane] = __ldg(gcodes + g);
-                smw[(u + t - u0) * 32 + lane] = __ldg(gw4 + g);
+template <int K>
+__device__ __forceinline__ bool c16_sum(const double (&v)[K], C16Sync& sy, double* got, double (&out)[K]) {
+    __shared__ double part[C16_SUMS][32];
+    __shared__ double tot[C16_SUMS];
+    __shared__ int bad;
+    const uint32_t G = gridDim.x, tid = threadIdx.x;
+    const uint32_t lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    sy.epoch++;
+    ulonglong2* buf = sy.slots + (size_t)(sy.epoch & 1ull) * G * G * C16_SUMS;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const double t = warp_sum_d(v[k]);
+        if (lane == 0) part[k][warp] = t;
+    }
+    if (tid == 0) bad = 0;
+    __syncthreads();
+    if (warp < K) {
+        const double t = warp_sum_d(lane < nw ? part[warp][lane] : 0.0);
+        if (lane == 0) tot[warp] = t;
+    }
+    __syncthreads();
+    if (tid < G * K) __threadfence();  // this block's writes before its sums
+    for (uint32_t x = tid; x < G * K; x += blockDim.x)
+        asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(
+                         buf + ((size_t)(x / K) * G + blockIdx.x) * C16_SUMS + x % K),
+                     "l"(__double_as_longlong(tot[x % K])), "l"(sy.epoch)
+                     : "memory");
+    for (uint32_t x = tid; x < G * K; x += blockDim.x) {
+        const ulonglong2* at = buf + ((size_t)blockIdx.x * G + x / K) * C16_SUMS + x % K;
+        uint64_t t0 = 0;
+        for (;;) {
+            long long val;
+            unsigned long long ep;
+            asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                         : "=l"(val), "=l"(ep)
+                         : "l"(at)
+                         : "memory");
+            if (ep == sy.epoch) {
+                got[x] = __longlong_as_double(val);
+                break;
             }
-            u += T;
+            uint64_t t1;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+            if (t0 == 0) t0 = t1;
+            if (t1 - t0 > wait_budget_ns(sy.sc)) {
+                atomicOr(&sy.sc->err, ERR_DEVICE_TIMEOUT);
+                bad = 1;
+                break;
+            }
         }
     }
-    __syncwarp();
+    if (tid < G * K) __threadfence();  // the other blocks' writes after their sums
+    __syncthreads();
+    if (warp < K) {
+        double t = 0.0;
+        for (uint32_t b = lane; b < G; b += 32) t += got[b * K + warp];
+        t = warp_sum_d(t);
+        if (lane == 0) tot[warp] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; k++) out[k] = tot[k];
+    return bad == 0;
+}
 
-    int total = 0, outers = 0;
-    double relres = 0.0;
-    bool converged = false;
-    float2* zc = S.zp0;
-    float2* zn = S.zp1;
-    float* rc = S.r;   // residual read by this iteration
-    float* ra = S.r2;  // and the buffer its update writes (LRN)
-    for (int outer = 0; outer < S.max_outer; outer++) {
-        // ---- true residual r64 = b - A x64 (FP64); z = D^-1 r, p = 0
-        double acc[3] = {0.0, 0.0, 0.0};
-        uint32_t u = 0;
-        for (uint32_t sl = gw; sl < nsl; sl += nw) {
-            const uint32_t g0 = __ldg(S.off + sl), T = __ldg(S.off + sl + 1) - g0;
-            const uint32_t ts = u0 > u ? min(T, u0 - u) : 0u;
-            const int base = (int)(sl * C16_ROWS) - C16_BIAS;
-            double s = 0.0;
-            for (uint32_t t = 0; t < T; t++) {
-                uint2 cw;
-                float4 w;
-                if (t < ts) {
-                    const uint64_t pol = c16_policy(g0 + t, S.keep);
-                    cw = ld_codes(gcodes + (size_t)(g0 + t) * 32 + lane, pol);
-                    w = ld_mat(gw4 + (size_t)(g0 + t) * 32 + lane, pol);
-                } else {
-                    cw = smc[(u + t - u0) * 32 + lane];
-                    w = smw[(u + t - u0) * 32 + lane];
-                }
-                uint32_t col[4];
-                c16_cols(cw, base, S.side, (size_t)(g0 + t) * C16_CHUNK + 4u * lane, col);
-                s += (double)w.x * S.x64[col[0]] + (double)w.y * S.x64[col[1]] + (double)w.z * S.x64[col[2]] +
-                     (double)w.w * S.x64[col[3]];
-            }
-            u += T;
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            const uint32_t k = sl * C16_ROWS + rr;
-            if (l == 0 && k < R) {
-                const double bi = S.b64[k];
-                const double ri = bi - (S.diag64[k] * S.x64[k] + s);
-                const float rf = (float)ri;
-                rc[k] = rf;
-                if (!LRN) {
-                    const float zf = rf * S.inv_diag[k];
-                    zc[k] = make_float2(zf, 0.f);
-                    acc[2] += (double)rf * (double)zf;
-                }
-                acc[0] += ri * ri;
-                acc[1] += bi * bi;
+// What a block needs of one of its tiles (uniform over the block).
+struct C16View {
+    uint32_t s0, r0, rows, ns, ncol, c0, nch;
+    uint32_t cpw;     // chunks per warp: the tile's chunks in equal contiguous shares
+    uint32_t nseg;    // most pieces this cuts a slice into
+    // of a warp's share, the last resw chunks are resident in shared memory
+    // and the first keepw are read as evict_last (mat_policy; 0xFFFFFFFF:
+    // default policy), so that every warp has the same mix of near and far
+    uint32_t resw, keepw;
+    uint32_t esc;
+    const uint32_t* cl;
+    const uint32_t* spf;  // its S' slices (k_c16_pack)
+};
+
+constexpr uint32_t C16_SEGS = 4;  // most pieces a slice's chunks are cut into
+
+__device__ __forceinline__ uint32_t c16_align(uint32_t v) { return (v + 15u) & ~15u; }
+
+__device__ __forceinline__ C16View c16_view(const C16Args& S, uint32_t t, uint32_t R, uint32_t C, uint32_t nwarps) {
+    const C16Tile ti = S.tiles[t];
+    C16View v;
+    v.s0 = ti.s0;
+    v.ns = ti.s1 - ti.s0;
+    v.r0 = ti.s0 * C16_ROWS;
+    v.rows = min(ti.s1 * C16_ROWS, R) - min(v.r0, R);
+    v.ncol = ti.ncol;
+    v.esc = ti.esc;
+    v.c0 = __ldg(S.off + ti.s0);
+    const uint32_t c1 = __ldg(S.off + ti.s1);
+    v.nch = c1 - v.c0;
+    // no slice in more than C16_SEGS pieces
+    v.cpw = max((v.nch + nwarps - 1) / nwarps, (ti.wmax + C16_SEGS - 2) / (C16_SEGS - 1));
+    v.cpw = max(v.cpw, 1u);
+    v.nseg = ti.wmax ? (ti.wmax + v.cpw - 2) / v.cpw + 1 : 1u;
+    v.resw = 0;
+    v.keepw = S.keep == 0xffffffffu ? S.keep : (uint32_t)((uint64_t)v.cpw * min(S.keep, C) / C);
+    v.cl = S.collist + (size_t)t * C16_COLS;
+    v.spf = S.sp_first + (size_t)t * C16_SP_SLICES;
+    return v;
+}
+
+// Slice offsets of the tile, from its first chunk, and the pieces of each.
+__device__ __forceinline__ void c16_slices(const C16Args& S, const C16View& v, uint32_t* soff, unsigned char* sseg) {
+    for (uint32_t s = threadIdx.x; s <= v.ns; s += blockDim.x) {
+        const uint32_t a = __ldg(S.off + v.s0 + s) - v.c0;
+        soff[s] = a;
+        if (s < v.ns) {
+            const uint32_t b = __ldg(S.off + v.s0 + s + 1) - v.c0;
+            sseg[s] = (unsigned char)(b > a ? (b - 1) / v.cpw - a / v.cpw + 1 : 0u);
+        }
+    }
+}
+
+// The row sums of a tile's product over the staged vector (at vecb): warp w
+// takes chunks [w cpw, (w + 1) cpw) whichever slices they belong to, four
+// chunks' loads in flight at a time, and leaves each slice's sums (or its
+// piece's) in q[piece * rs + row].  REMOTE gives the operand of a column that
+// is not in the tile's list.
+template <class T, bool ESC, class REMOTE>
+__device__ __forceinline__ void c16_product(const C16Args& S, const C16View& v, const unsigned char* vecb,
+                                            const uint32_t* soff, T* q, uint32_t rs, const unsigned char* res,
+                                            REMOTE remote) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = warp * v.cpw;
+    const uint32_t x1 = min(x + v.cpw, v.nch);
+    if (x >= x1) return;
+    uint32_t s = 0;  // the slice of chunk x: the last one that starts at or before it
+    {
+        uint32_t hi = v.ns;
+        while (hi - s > 1) {
+            const uint32_t mid = (s + hi) >> 1;
+            if (soff[mid] <= x) s = mid;
+            else hi = mid;
+        }
+    }
+    uint32_t seg = warp - soff[s] / v.cpw, send = soff[s + 1];
+    T a0 = 0, a1 = 0;
+    auto add = [&](const uint2 cw, const float4 w, uint32_t at) {
+        T o[4];
+        const uint32_t c[4] = {cw.x & 0xffffu, cw.x >> 16, cw.y & 0xffffu, cw.y >> 16};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (ESC && c[u] == C16_ESC)
+                o[u] = remote(__ldg(S.side + (size_t)(v.c0 + at) * C16_CHUNK + 4u * lane + u));
+            else
+                o[u] = *reinterpret_cast<const T*>(vecb + c[u] * (sizeof(T) / 4));
+        }
+        a0 += (T)w.x * o[0];
+        a1 += (T)w.y * o[1];
+        a0 += (T)w.z * o[2];
+        a1 += (T)w.w * o[3];
+        if (at + 1 == send) {  // the slice ends here
+            T t = a0 + a1;
+            t += __shfl_xor_sync(0xffffffffu, t, 8);
+            t += __shfl_xor_sync(0xffffffffu, t, 16);
+            if (lane < C16_ROWS) q[seg * rs + s * C16_ROWS + lane] = t;
+            a0 = 0;
+            a1 = 0;
+            seg = 0;
+            if (at + 1 < x1) {
+                do s++;
+                while (soff[s + 1] == at + 1);
+                send = soff[s + 1];
             }
         }
-        double tot[3];
-        if (!grid_reduce<3>(acc, S.part, S.result, S.bar, S.sc, tot)) return;
+    };
+    const uint32_t nres = min(v.resw, x1 - x), xs = x1 - nres;
+    const uint32_t xk = v.keepw == 0xffffffffu ? v.keepw : x + v.keepw;
+    // streamed chunks, in two batches of registers: one is consumed while the
+    // other is on its way
+    constexpr int UN = sizeof(T) == 4 ? C16_BATCH : C16_BATCH64;
+    const unsigned char* src = S.ent + (size_t)(v.c0 + x) * C16_CHUNK_BYTES + 16u * lane;
+    const unsigned char* srcc = src + 512u - 8u * lane;
+    const uint64_t near = mat_policy(0u, xk == 0xffffffffu ? xk : 1u), far = mat_policy(1u, xk == 0xffffffffu ? xk : 0u);
+    float4 wa[UN], wb[UN];
+    uint2 ca[UN], cb[UN];
+    auto load = [&](float4 (&w)[UN], uint2 (&c)[UN], uint32_t at) {
+        const uint64_t pol = at < xk ? near : far;
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            w[u] = ld_mat(reinterpret_cast<const float4*>(src + u * C16_CHUNK_BYTES), pol);
+            c[u] = ld_codes(reinterpret_cast<const uint2*>(srcc + u * C16_CHUNK_BYTES), pol);
+        }
+        src += UN * C16_CHUNK_BYTES;
+        srcc += UN * C16_CHUNK_BYTES;
+    };
+    auto use = [&](const float4 (&w)[UN], const uint2 (&c)[UN], uint32_t at) {
+#pragma unroll
+        for (int u = 0; u < UN; u++) add(c[u], w[u], at + u);
+    };
+    uint32_t nb = (xs - x) / UN;  // whole batches
+    if (nb) {
+        load(wa, ca, x);
+        for (; nb > 2; nb -= 2) {
+            load(wb, cb, x + UN);
+            use(wa, ca, x);
+            load(wa, ca, x + 2 * UN);
+            use(wb, cb, x + UN);
+            x += 2 * UN;
+        }
+        if (nb == 2) {
+            load(wb, cb, x + UN);
+            use(wa, ca, x);
+            use(wb, cb, x + UN);
+        } else {
+            use(wa, ca, x);
+        }
+        x += nb * UN;
+    }
+    for (; x < xs; x++) {  // and the chunks left
+        const uint64_t pol = x < xk ? near : far;
+        const float4 w = ld_mat(reinterpret_cast<const float4*>(src), pol);
+        const uint2 c = ld_codes(reinterpret_cast<const uint2*>(srcc), pol);
+        src += C16_CHUNK_BYTES;
+        srcc += C16_CHUNK_BYTES;
+        add(c, w, x);
+    }
+#pragma unroll 2
+    for (; x < x1; x++) {
+        const unsigned char* ch = res + (size_t)(warp * v.resw + (x - xs)) * C16_CHUNK_BYTES;
+        const float4 w = *reinterpret_cast<const float4*>(ch + 16u * lane);
+        const uint2 cw = *reinterpret_cast<const uint2*>(ch + 512u + 8u * lane);
+        add(cw, w, x);
+    }
+    if (x1 < send) {  // the share ends inside its last slice
+        T t = a0 + a1;
+        t += __shfl_xor_sync(0xffffffffu, t, 8);
+        t += __shfl_xor_sync(0xffffffffu, t, 16);
+        if (lane < C16_ROWS) q[seg * rs + s * C16_ROWS + lane] = t;
+    }
+}
+
+// row sum of the tile's row k (its slice's pieces in order)
+template <class T>
+__device__ __forceinline__ T c16_rowsum(const T* q, uint32_t rs, const unsigned char* sseg, uint32_t k) {
+    const uint32_t n = sseg[k / C16_ROWS];
+    T t = 0;
+    for (uint32_t g = 0; g < n; g++) t += q[g * rs + k];
+    return t;
+}
+
+// vec[c] = op(column c's number) for the tile's columns, four at a time so
+// that op's loads overlap
+template <class T, class OP>
+__device__ __forceinline__ void c16_stage(T* vec, const uint32_t* cl, uint32_t ncol, OP op) {
+    const uint32_t nthr = blockDim.x;
+    for (uint32_t c = threadIdx.x; c < ncol; c += 4 * nthr) {
+        uint32_t j[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) j[u] = cl[min(c + u * nthr, ncol - 1)];
+        T v[4];
+        op(j, v);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (c + u * nthr < ncol) vec[c + u * nthr] = v[u];
+    }
+}
+
+// A block's shared memory for tiles of at most ncol columns and rows rows in
+// nseg pieces a slice: the staged vector (at 0; doubles in the FP64 pass),
+// the row sums, the tile's slice offsets, the inbox read by the grid sums,
+// and, in a block of one tile
+// (single), its column list and its rows' state, which then never leave the
+// SM.  The rest holds chunks of the matrix.
+struct C16Plan {
+    uint32_t q, soff, sseg, got, views, cl, row, res;  // byte offsets
+    uint32_t rs;                           // row stride of the sums and the state
+};
+constexpr uint32_t C16_ROW_BYTES = 32;     // x in double; r, w, s, 1 / diagonal, p, diagonal
+
+__device__ __forceinline__ C16Plan c16_plan(uint32_t ncol, uint32_t rows, uint32_t nseg, uint32_t ntiles, bool single) {
+    C16Plan p;
+    const uint32_t ns = (rows + C16_ROWS - 1) / C16_ROWS;
+    p.rs = ns * C16_ROWS;
+    p.q = c16_align(max(ncol, 1u) * 8u);
+    p.soff = p.q + c16_align(p.rs * nseg * 8u);
+    p.sseg = p.soff + c16_align((ns + 1) * 4u);
+    p.got = p.sseg + c16_align(ns);
+    p.views = p.got + c16_align(gridDim.x * C16_SUMS * 8u);
+    p.cl = p.views + c16_align(single ? 0u : ntiles * (uint32_t)sizeof(C16View));
+    p.row = p.cl + (single ? c16_align(ncol * 4u) : 0u);
+    p.res = c16_align(p.row + (single ? p.rs * C16_ROW_BYTES : 0u));
+    return p;
+}
+
+// [p, p + bytes) towards L2, spread over the block
+__device__ __forceinline__ void c16_ahead(const void* p, uint32_t bytes) {
+    const unsigned char* a = reinterpret_cast<const unsigned char*>(p);
+    for (uint32_t x = threadIdx.x * 128u; x < bytes; x += blockDim.x * 128u)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a + x));
+}
+
+// One block of a solver: its tiles, its shared memory and, when it has one
+// tile, that tile's view.  Rows' state is in shared memory (single) or in
+// the global arrays.
+struct C16Block {
+    const C16Args& S;
+    unsigned char* sm;
+    uint32_t R, C, G, ntiles;
+    bool single, whole;
+    bool sp_res;       // S' of the block's rows is in shared memory
+    uint32_t sp_at, sp_words;  // its diagonal and first four of each 32 rows, and its entries
+    C16Plan pl;
+    C16View v;
+
+    __device__ __forceinline__ C16Block(const C16Args& S_, unsigned char* sm_, bool learned) : S(S_), sm(sm_) {
+        R = *S.nrows;
+        G = gridDim.x;
+        ntiles = c16_tiles(R, G) / G;
+        C = max(__ldg(S.off + (R + C16_ROWS - 1) / C16_ROWS), 1u);
+        v = c16_view(S, blockIdx.x + G * (ntiles - 1), R, C, blockDim.x >> 5);
+        single = false;
+        whole = false;
+        if (ntiles == 1) {
+            pl = c16_plan(v.ncol, v.rows, v.nseg, 1u, true);
+            single = pl.res <= S.smem_bytes;
+        }
+        if (!single) {
+            // a tile with so many rows and columns that the pieces do not fit
+            // is done by one warp, slices whole: slow, but right
+            pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), C16_SEGS, ntiles, false);
+            whole = pl.res > S.smem_bytes;
+            if (whole) pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), 1u, ntiles, false);
+        }
+        if (whole) v.cpw = max(v.nch, 1u);
+        sp_res = false;
+        if (learned && single) resident_sp();
+        // the end of every warp's share of the last tile stays in shared memory
+        const uint32_t nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        v.resw = min((S.smem_bytes - pl.res) / C16_CHUNK_BYTES, S.smem_chunks) / nw;
+        v.resw = min(v.resw, v.cpw);
+        {
+            const uint32_t x0 = min(warp * v.cpw, v.nch), x1 = min(x0 + v.cpw, v.nch), n = min(v.resw, x1 - x0);
+            const uint4* src = reinterpret_cast<const uint4*>(S.ent + (size_t)(v.c0 + x1 - n) * C16_CHUNK_BYTES);
+            uint4* dst = reinterpret_cast<uint4*>(sm + pl.res + (size_t)warp * v.resw * C16_CHUNK_BYTES);
+            for (uint32_t x = lane; x < n * (C16_CHUNK_BYTES / 16); x += 32) dst[x] = __ldg(src + x);
+        }
+        if (!single) {
+            C16View* views = reinterpret_cast<C16View*>(sm + pl.views);
+            for (uint32_t m = threadIdx.x; m < ntiles; m += blockDim.x) {
+                C16View t = c16_view(S, blockIdx.x + G * m, R, C, nw);
+                if (whole) t.cpw = max(t.nch, 1u);
+                if (m == ntiles - 1) t.resw = v.resw;
+                views[m] = t;
+            }
+        }
+        if (single) {
+            c16_slices(S, v, soff(), sseg());
+            uint32_t* cl = reinterpret_cast<uint32_t*>(sm + pl.cl);
+            for (uint32_t c = threadIdx.x; c < v.ncol; c += blockDim.x) cl[c] = __ldg(v.cl + c);
+            v.cl = cl;
+            for (uint32_t k = threadIdx.x; k < v.rows; k += blockDim.x) {
+                rx()[k] = S.x64[v.r0 + k];
+                rf(C16_INV)[k] = S.inv_diag[v.r0 + k];
+                rf(C16_DG)[k] = S.diag32[v.r0 + k];
+            }
+        }
+        __syncthreads();
+    }
+    // S' of the rows into shared memory, 32-row interleaved, when it fits: it
+    // is read once an iteration by one thread a row, and the wait for those
+    // few loads cost more than the chunks it displaces
+    __device__ __forceinline__ void resident_sp() {
+        const uint32_t nsp = (v.rows + SP_SLICE - 1) / SP_SLICE;
+        const uint32_t f0 = __ldg(v.spf), n = __ldg(v.spf + nsp) - f0;
+        const uint32_t head = c16_align(pl.res + (nsp * (SP_SLICE + 1) + 1) * 4u);
+        if (head + n * 16u > S.smem_bytes) return;
+        float* diag = reinterpret_cast<float*>(sm + pl.res);
+        uint32_t* first = reinterpret_cast<uint32_t*>(diag + nsp * SP_SLICE);
+        for (uint32_t j = threadIdx.x; j <= nsp; j += blockDim.x) first[j] = __ldg(v.spf + j) - f0;
+        for (uint32_t k = threadIdx.x; k < v.rows; k += blockDim.x) diag[k] = __ldg(S.sp_diag + v.r0 + k);
+        const uint4* src = reinterpret_cast<const uint4*>(S.sp_ent) + f0;
+        uint4* w = reinterpret_cast<uint4*>(sm + head);
+        for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) w[x] = __ldg(src + x);
+        sp_res = true;
+        sp_at = pl.res;
+        sp_words = head;
+        pl.res = head + n * 16u;
+    }
+    __device__ __forceinline__ uint32_t* soff() const { return reinterpret_cast<uint32_t*>(sm + pl.soff); }
+    __device__ __forceinline__ unsigned char* sseg() const { return sm + pl.sseg; }
+    __device__ __forceinline__ double* got() const { return reinterpret_cast<double*>(sm + pl.got); }
+    __device__ __forceinline__ double* rx() const { return reinterpret_cast<double*>(sm + pl.row); }
+    __device__ __forceinline__ float* rf(uint32_t f) const {
+        return reinterpret_cast<float*>(sm + pl.row + pl.rs * 8u) + f * pl.rs;
+    }
+    enum : uint32_t { C16_R = 0, C16_W, C16_S, C16_INV, C16_P, C16_DG };
+
+    // body(view) for each of the block's tiles; the slice offsets are loaded
+    // (the body's first barrier publishes them).  While a tile is worked on,
+    // ahead(view) brings what the next one reads once into L2.
+    template <class F, class P>
+    __device__ __forceinline__ void tiles(P ahead, F body) const {
+        if (single) {
+            body(v);
+            return;
+        }
+        const C16View* views = reinterpret_cast<const C16View*>(sm + pl.views);
+        for (uint32_t m = 0; m < ntiles; m++) {
+            const C16View t = views[m];
+            __syncthreads();
+            c16_slices(S, t, soff(), sseg());
+            if (m + 1 < ntiles) {
+                const C16View& n = views[m + 1];
+                c16_ahead(n.cl, n.ncol * 4u);
+                c16_ahead(S.off + n.s0, (n.ns + 1) * 4u);
+                ahead(n);
+            }
+            body(t);
+        }
+    }
+    // the tile's products over the staged vector, barriers included; row k's
+    // sum is then rowsum<T>(k)
+    template <class T, class REMOTE>
+    __device__ __forceinline__ void product(const C16View& t, REMOTE remote) const {
+        __syncthreads();
+        T* q = reinterpret_cast<T*>(sm + pl.q);
+        if (t.esc) c16_product<T, true>(S, t, sm, soff(), q, pl.rs, sm + pl.res, remote);
+        else c16_product<T, false>(S, t, sm, soff(), q, pl.rs, sm + pl.res, remote);
+        __syncthreads();
+    }
+    template <class T>
+    __device__ __forceinline__ T rowsum(uint32_t k) const {
+        return c16_rowsum(reinterpret_cast<const T*>(sm + pl.q), pl.rs, sseg(), k);
+    }
+    // r64 = b - A x64 of every row in FP64; body(view, k, r64, x)
+    template <class F>
+    __device__ __forceinline__ void residual(double (&acc)[2], F body) const {
+        tiles(
+            [&](const C16View& n) {
+                c16_ahead(S.b64 + n.r0, n.rows * 8u);
+                c16_ahead(S.diag64 + n.r0, n.rows * 8u);
+            },
+            [&](const C16View& t) {
+            c16_stage(reinterpret_cast<double*>(sm), t.cl, t.ncol, [&](const uint32_t (&j)[4], double (&o)[4]) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) o[u] = __ldcg(S.x64 + j[u]);
+            });
+            product<double>(t, [&](uint32_t col) { return __ldcg(S.x64 + col); });
+            for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+                const uint32_t g = t.r0 + k;
+                const double bi = __ldg(S.b64 + g);
+                const double x = reinterpret_cast<const double*>(sm)[k];
+                const double ri = bi - (__ldg(S.diag64 + g) * x + rowsum<double>(k));
+                acc[0] += ri * ri;
+                acc[1] += bi * bi;
+                body(t, k, ri);
+            }
+        });
+    }
+};
+
+// the smallest reduction one FP32 inner solve is asked for, squared
+__device__ __forceinline__ double inner_target(const C16Args& S, double relres) {
+    double eta = 0.3 * S.tol / relres;
+    if (eta < S.eta_min) eta = S.eta_min;
+    if (eta > 0.5) eta = 0.5;
+    return eta * eta;
+}
+
+// ok: every grid sum completed (else the timeout is the error)
+__device__ __forceinline__ void c16_finish_solve(const C16Args& S, const C16Sync& sy, int total, int outers,
+                                                 double relres, bool converged, bool ok) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    *S.epoch = sy.epoch + 2;  // past every epoch any block has used
+    if (!ok) return;
+    S.sc->cg_iters = total;
+    S.sc->cg_outer = outers;
+    S.sc->cg_relres = relres;
+    if (!converged) atomicOr(&S.sc->err, ERR_CG_NOT_CONVERGED);
+}
+
+// Diagonally scaled CG in the single-reduction form of Chronopoulos and Gear
+// (1989): with u = D^-1 r and w = A u, one sum of (r.u, w.u, r.r) gives the
+// next alpha and beta, and s = w + beta s, p = u + beta p follow by
+// recurrence.  A row publishes (r, w, s, 1 / diagonal); whoever needs its
+// next u forms it from those while staging (16 bytes per staged column, not
+// per entry), so an iteration has one grid-wide wait.  The same iterates as
+// CG's in exact arithmetic; the FP64 true residual ends the solve.
+__global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16(C16Args S) {
+    extern __shared__ __align__(16) unsigned char c16_sm[];
+    C16Sync sy{S.slots, *S.epoch, S.sc};
+    const C16Block B(S, c16_sm, false);
+    float* vec = reinterpret_cast<float*>(c16_sm);
+    float4* pc = S.pub0;  // published rows: read by this iteration
+    float4* pn = S.pub1;  // and written
+    int total = 0, outers = 0;
+    double relres = 0.0;
+    bool converged = false, ok = true;
+    for (int outer = 0; outer < S.max_outer; outer++) {
+        double acc[2] = {0.0, 0.0};
+        B.residual(acc, [&](const C16View& t, uint32_t k, double ri) {
+            const float r = (float)ri;
+            if (B.single) {
+                B.rf(C16Block::C16_R)[k] = r;
+                B.rf(C16Block::C16_W)[k] = 0.f;
+                B.rf(C16Block::C16_S)[k] = 0.f;
+                B.rf(C16Block::C16_P)[k] = 0.f;
+                pc[t.r0 + k] = make_float4(r, 0.f, 0.f, B.rf(C16Block::C16_INV)[k]);
+            } else {
+                S.p[t.r0 + k] = 0.f;
+                pc[t.r0 + k] = make_float4(r, 0.f, 0.f, __ldg(S.inv_diag + t.r0 + k));
+            }
+        });
+        double tot[2];
+        ok = c16_sum<2>(acc, sy, B.got(), tot);
+        if (!ok) break;
         outers++;
-        const double rr64 = tot[0], bb = tot[1];
-        relres = bb > 0.0 ? sqrt(rr64 / bb) : 0.0;
+        relres = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : 0.0;
         if (relres <= S.tol) {
             converged = true;
             break;
         }
         if (total >= S.max_iter) break;
-        if (LRN) {
-            // z = S' r of the new residual, r.z
-            double rz0[1] = {0.0};
-            for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < R; k += gridDim.x * blockDim.x) {
-                const float* rr_ = rc;
-                const float zs = sp_row(S, k, [rr_](uint32_t j) { return rr_[j]; });
-                zc[k] = make_float2(zs, 0.f);
-                rz0[0] += (double)rc[k] * (double)zs;
-            }
-            double trz[1];
-            if (!grid_reduce<1>(rz0, S.part, S.result, S.bar, S.sc, trz)) return;
-            tot[2] = trz[0];
-        }
-        double eta = 0.3 * S.tol / relres;
-        if (eta < S.eta_min) eta = S.eta_min;
-        if (eta > 0.5) eta = 0.5;
-        const double stop = eta * eta * rr64;
-        double rz = tot[2];
-        float beta = 0.f;
-        for (int it = 0; it < S.inner_cap && total < S.max_iter; it++) {
-            // ---- q = A p_new with p_new = z + beta p (fused), p.q
-            double pq[1] = {0.0};
-            u = 0;
-            for (uint32_t sl = gw; sl < nsl; sl += nw) {
-                const uint32_t g0 = __ldg(S.off + sl), T = __ldg(S.off + sl + 1) - g0;
-                const uint32_t ts = u0 > u ? min(T, u0 - u) : 0u;
-                const int base = (int)(sl * C16_ROWS) - C16_BIAS;
-                float s0 = 0.f, s1 = 0.f;
-#pragma unroll 2
-                for (uint32_t t = 0; t < ts; t++) {
-                    const uint64_t pol = c16_policy(g0 + t, S.keep);
-                    const uint2 cw = ld_codes(gcodes + (size_t)(g0 + t) * 32 + lane, pol);
-                    const float4 w = ld_mat(gw4 + (size_t)(g0 + t) * 32 + lane, pol);
-                    uint32_t col[4];
-                    c16_cols(cw, base, S.side, (size_t)(g0 + t) * C16_CHUNK + 4u * lane, col);
-                    const float2 a0 = zc[col[0]], a1 = zc[col[1]], a2 = zc[col[2]], a3 = zc[col[3]];
-                    s0 = fmaf(w.x, fmaf(beta, a0.y, a0.x), s0);
-                    s1 = fmaf(w.y, fmaf(beta, a1.y, a1.x), s1);
-                    s0 = fmaf(w.z, fmaf(beta, a2.y, a2.x), s0);
-                    s1 = fmaf(w.w, fmaf(beta, a3.y, a3.x), s1);
+        const double stop = inner_target(S, relres) * tot[0];
+        double alpha = 0.0, beta = 0.0, gamma = 0.0;
+        // it = -1: w = A u of the start, nothing moves (alpha = beta = 0)
+        for (int it = -1;; it++) {
+            const float af = (float)alpha, bf = (float)beta;
+            double g[3] = {0.0, 0.0, 0.0};
+            B.tiles(
+                [&](const C16View& n) {
+                    c16_ahead(S.x64 + n.r0, n.rows * 8u);
+                    c16_ahead(S.p + n.r0, n.rows * 4u);
+                    c16_ahead(S.diag32 + n.r0, n.rows * 4u);
+                },
+                [&](const C16View& t) {
+                auto next_u = [&](const float4& v) {
+                    return v.w * fmaf(-af, fmaf(bf, v.z, v.y), v.x);
+                };
+                c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
+                    float4 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) v[u] = __ldcg(pc + j[u]);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) o[u] = next_u(v[u]);
+                });
+                B.product<float>(t, [&](uint32_t col) { return next_u(__ldcg(pc + col)); });
+                for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+                    const uint32_t gk = t.r0 + k;
+                    float4 o;
+                    float p, dg;
+                    double x;
+                    if (B.single) {
+                        o = make_float4(B.rf(C16Block::C16_R)[k], B.rf(C16Block::C16_W)[k], B.rf(C16Block::C16_S)[k],
+                                        B.rf(C16Block::C16_INV)[k]);
+                        p = B.rf(C16Block::C16_P)[k];
+                        dg = B.rf(C16Block::C16_DG)[k];
+                        x = B.rx()[k];
+                    } else {
+                        o = pc[gk];
+                        p = S.p[gk];
+                        dg = __ldg(S.diag32 + gk);
+                        x = S.x64[gk];
+                    }
+                    const float sn = fmaf(bf, o.z, o.y);
+                    p = fmaf(bf, p, o.w * o.x);
+                    x += alpha * (double)p;
+                    const float r = fmaf(-af, sn, o.x);
+                    const float u = vec[k];
+                    const float w = fmaf(dg, u, B.rowsum<float>(k));
+                    pn[gk] = make_float4(r, w, sn, o.w);
+                    S.x64[gk] = x;
+                    if (B.single) {
+                        B.rf(C16Block::C16_R)[k] = r;
+                        B.rf(C16Block::C16_W)[k] = w;
+                        B.rf(C16Block::C16_S)[k] = sn;
+                        B.rf(C16Block::C16_P)[k] = p;
+                        B.rx()[k] = x;
+                    } else {
+                        S.p[gk] = p;
+                    }
+                    g[0] += (double)r * (double)u;
+                    g[1] += (double)w * (double)u;
+                    g[2] += (double)r * (double)r;
                 }
-#pragma unroll 2
-                for (uint32_t t = ts; t < T; t++) {
-                    const uint2 cw = smc[(u + t - u0) * 32 + lane];
-                    const float4 w = smw[(u + t - u0) * 32 + lane];
-                    uint32_t col[4];
-                    c16_cols(cw, base, S.side, (size_t)(g0 + t) * C16_CHUNK + 4u * lane, col);
-                    const float2 a0 = zc[col[0]], a1 = zc[col[1]], a2 = zc[col[2]], a3 = zc[col[3]];
-                    s0 = fmaf(w.x, fmaf(beta, a0.y, a0.x), s0);
-                    s1 = fmaf(w.y, fmaf(beta, a1.y, a1.x), s1);
-                    s0 = fmaf(w.z, fmaf(beta, a2.y, a2.x), s0);
-                    s1 = fmaf(w.w, fmaf(beta, a3.y, a3.x), s1);
-                }
-                u += T;
-                float s = s0 + s1;
-                s += __shfl_xor_sync(0xffffffffu, s, 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
-                s += __shfl_xor_sync(0xffffffffu, s, 4);
-                const uint32_t k = sl * C16_ROWS + rr;
-                if (l == 0 && k < R) {
-                    const float2 o = zc[k];
-                    const float pn = fmaf(beta, o.y, o.x);
-                    const float qi = fmaf(S.diag32[k], pn, s);
-                    zn[k].y = pn;
-                    S.q[k] = qi;
-                    pq[0] += (double)pn * (double)qi;
-                }
-            }
-            double totp[1];
-            if (!grid_reduce<1>(pq, S.part, S.result, S.bar, S.sc, totp)) return;
-            const double alpha = rz / totp[0];
-            const float alpha_f = (float)alpha;
-            // ---- x64 += alpha p, r -= alpha q, z = M^-1 r, r.z, r.r
-            double acc2[2] = {0.0, 0.0};
-            if (LRN) {
-                // z_k = sum_j S'_kj (r_j - alpha q_j), the new residual into
-                // the other buffer (the neighbours read the old one)
-                for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < R; k += gridDim.x * blockDim.x) {
-                    const float* rr_ = rc;
-                    const float* qq_ = S.q;
-                    const float zs =
-                        sp_row(S, k, [rr_, qq_, alpha_f](uint32_t j) { return fmaf(-alpha_f, qq_[j], rr_[j]); });
-                    const float pn = zn[k].y;
-                    S.x64[k] += alpha * (double)pn;
-                    const float ri = fmaf(-alpha_f, S.q[k], rc[k]);
-                    ra[k] = ri;
-                    zn[k] = make_float2(zs, pn);
-                    acc2[0] += (double)ri * (double)zs;
-                    acc2[1] += (double)ri * (double)ri;
-                }
+            });
+            double gt[3];
+            ok = c16_sum<3>(g, sy, B.got(), gt);
+            if (!ok) break;
+            float4* x = pc;
+            pc = pn;
+            pn = x;
+            if (it >= 0) {
+                total++;
+                if (gt[2] <= stop) break;
+                beta = gt[0] / gamma;
+                alpha = gt[0] / (gt[1] - beta * gt[0] / alpha);
             } else {
-                for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < R; k += gridDim.x * blockDim.x) {
-                    const float pn = zn[k].y;
-                    S.x64[k] += alpha * (double)pn;
-                    const float ri = fmaf(-alpha_f, S.q[k], rc[k]);
-                    const float zi = ri * S.inv_diag[k];
-                    rc[k] = ri;
-                    zn[k] = make_float2(zi, pn);
-                    acc2[0] += (double)ri * (double)zi;
-                    acc2[1] += (double)ri * (double)ri;
-                }
+                alpha = gt[0] / gt[1];
             }
-            double tot2[2];
-            if (!grid_reduce<2>(acc2, S.part, S.result, S.bar, S.sc, tot2)) return;
-            if (LRN) {
-                float* t_ = rc;
-                rc = ra;
-                ra = t_;
-            }
-            total++;
-            beta = (float)(tot2[0] / rz);
-            rz = tot2[0];
-            float2* tt = zc;
-            zc = zn;
-            zn = tt;
-            if (tot2[1] <= stop) break;
+            gamma = gt[0];
+            if (it + 1 >= S.inner_cap || total >= S.max_iter) break;
+        }
+        if (!ok) break;
+    }
+    c16_finish_solve(S, sy, total, outers, relres, converged, ok);
+}
+
+// Row k of S' x over the staged x (own rows first in the tile's list); an
+// escaped column's x comes from remote.  S' is in shared memory or read
+// again every iteration.
+template <class REMOTE>
+__device__ __forceinline__ float c16_sp_row(const C16Args& S, const C16Block& B, const C16View& t, const float* vec,
+                                            uint32_t k, REMOTE remote) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    auto add = [&](uint32_t e, size_t at, float& a) {
+        const uint32_t c = e >> 16;
+        float x;
+        if (t.esc && c == C16_ESC) x = remote(__ldg(S.sp_side + at));
+        else x = vec[c >> 2];
+        a = fmaf(__uint_as_float(e << 16), x, a);
+    };
+    auto four = [&](const uint4& e, uint32_t f, float& a0, float& a1, float& a2, float& a3) {  // four f of the array
+        add(e.x, 4 * (size_t)f, a0);
+        add(e.y, 4 * (size_t)f + 1, a1);
+        add(e.z, 4 * (size_t)f + 2, a2);
+        add(e.w, 4 * (size_t)f + 3, a3);
+    };
+    float dg;
+    if (B.sp_res) {
+        const float* diag = reinterpret_cast<const float*>(B.sm + B.sp_at);
+        const uint32_t nsp = (t.rows + SP_SLICE - 1) / SP_SLICE;
+        const uint32_t* first = reinterpret_cast<const uint32_t*>(diag + nsp * SP_SLICE) + k / SP_SLICE;
+        const uint32_t a = first[0] + k % SP_SLICE, b = first[1];
+        const uint4* w = reinterpret_cast<const uint4*>(B.sm + B.sp_words);
+        dg = diag[k];
+        uint32_t f = a;
+        for (; f + SP_SLICE < b; f += 2 * SP_SLICE) {
+            four(w[f], __ldg(t.spf) + f, acc[0], acc[1], acc[2], acc[3]);
+            four(w[f + SP_SLICE], __ldg(t.spf) + f + SP_SLICE, acc[4], acc[5], acc[6], acc[7]);
+        }
+        if (f < b) four(w[f], __ldg(t.spf) + f, acc[0], acc[1], acc[2], acc[3]);
+    } else {
+        constexpr int UN = 8;  // fours in flight: a whole row mostly
+        const uint32_t a = __ldg(t.spf + k / SP_SLICE) + k % SP_SLICE, b = __ldg(t.spf + k / SP_SLICE + 1);
+        dg = __ldg(S.sp_diag + t.r0 + k);
+        const uint4* w = reinterpret_cast<const uint4*>(S.sp_ent);
+        for (uint32_t f = a; f < b; f += UN * SP_SLICE) {
+            uint4 e[UN];
+#pragma unroll
+            for (int u = 0; u < UN; u++) e[u] = __ldg(w + (f + u * SP_SLICE < b ? f + u * SP_SLICE : f));
+#pragma unroll
+            for (int u = 0; u < UN; u++)
+                if (f + u * SP_SLICE < b) four(e[u], f + u * SP_SLICE, acc[4 * (u & 1)], acc[4 * (u & 1) + 1], acc[4 * (u & 1) + 2],
+                                               acc[4 * (u & 1) + 3]);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        S.sc->cg_iters = total;
-        S.sc->cg_outer = outers;
-        S.sc->cg_relres = relres;
-        if (!converged) atomicOr(&S.sc->err, ERR_CG_NOT_CONVERGED);
+    const float offd = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+    return fmaf(dg, vec[k], offd);
+}
+
+// The learned preconditioner z = S' r.  An iteration is two passes, each
+// ending in a grid-wide sum: the update (residuals r - alpha q staged, x, z =
+// S' r, r.z and r.r) and the product (directions z + beta p staged, q = A p,
+// p.q).  A row publishes (z, p) in the first and (r, q) in the second, each
+// read by the other blocks only in the other pass.
+__global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16_learned(C16Args S) {
+    extern __shared__ __align__(16) unsigned char c16_sm[];
+    C16Sync sy{S.slots, *S.epoch, S.sc};
+    const C16Block B(S, c16_sm, true);
+    float* vec = reinterpret_cast<float*>(c16_sm);
+    float2* zp = reinterpret_cast<float2*>(S.pub0);
+    float2* rq = reinterpret_cast<float2*>(S.pub1);
+    int total = 0, outers = 0;
+    double relres = 0.0;
+    bool converged = false, ok = true;
+    for (int outer = 0; outer < S.max_outer; outer++) {
+        double acc[2] = {0.0, 0.0};
+        B.residual(acc, [&](const C16View& t, uint32_t k, double ri) {
+            rq[t.r0 + k] = make_float2((float)ri, 0.f);
+            if (B.single) B.rf(C16Block::C16_P)[k] = 0.f;
+            else S.p[t.r0 + k] = 0.f;
+        });
+        double tot[2];
+        ok = c16_sum<2>(acc, sy, B.got(), tot);
+        if (!ok) break;
+        outers++;
+        relres = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : 0.0;
+        if (relres <= S.tol) {
+            converged = true;
+            break;
+        }
+        if (total >= S.max_iter) break;
+        const double stop = inner_target(S, relres) * tot[0];
+        double alpha = 0.0, rz = 0.0;
+        // it = -1: z of the start, nothing moves (alpha = 0)
+        for (int it = -1;; it++) {
+            const float af = (float)alpha;
+            double g[2] = {0.0, 0.0};
+            B.tiles(
+                [&](const C16View& n) {
+                    const uint32_t nsp = (n.rows + SP_SLICE - 1) / SP_SLICE;
+                    const uint32_t f = __ldg(n.spf);
+                    c16_ahead(S.sp_ent + 4 * (size_t)f, (__ldg(n.spf + nsp) - f) * 16u);
+                    c16_ahead(n.spf, (nsp + 1) * 4u);
+                    c16_ahead(S.sp_diag + n.r0, n.rows * 4u);
+                    c16_ahead(S.x64 + n.r0, n.rows * 8u);
+                    c16_ahead(S.p + n.r0, n.rows * 4u);
+                },
+                [&](const C16View& t) {
+                auto next_r = [&](const float2& v) { return fmaf(-af, v.y, v.x); };
+                c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
+                    float2 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) v[u] = __ldcg(rq + j[u]);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) o[u] = next_r(v[u]);
+                });
+                __syncthreads();
+                for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+                    const uint32_t gk = t.r0 + k;
+                    const float r = vec[k];
+                    const float p = B.single ? B.rf(C16Block::C16_P)[k] : S.p[gk];
+                    const double x = (B.single ? B.rx()[k] : S.x64[gk]) + alpha * (double)p;
+                    const float z = c16_sp_row(S, B, t, vec, k, [&](uint32_t col) { return next_r(__ldcg(rq + col)); });
+                    zp[gk] = make_float2(z, p);
+                    S.x64[gk] = x;
+                    if (B.single) {
+                        B.rx()[k] = x;
+                        B.rf(C16Block::C16_R)[k] = r;
+                    } else {
+                        S.r[gk] = r;
+                    }
+                    g[0] += (double)r * (double)z;
+                    g[1] += (double)r * (double)r;
+                }
+            });
+            double gt[2];
+            ok = c16_sum<2>(g, sy, B.got(), gt);
+            if (!ok) break;
+            float beta = 0.f;
+            if (it >= 0) {
+                total++;
+                if (gt[1] <= stop) break;
+                beta = (float)(gt[0] / rz);
+            }
+            rz = gt[0];
+            if (it + 1 >= S.inner_cap || total >= S.max_iter) break;
+            double pq[1] = {0.0};
+            B.tiles(
+                [&](const C16View& n) {
+                    c16_ahead(S.diag32 + n.r0, n.rows * 4u);
+                    c16_ahead(S.r + n.r0, n.rows * 4u);
+                },
+                [&](const C16View& t) {
+                auto next_p = [&](const float2& v) { return fmaf(beta, v.y, v.x); };
+                c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
+                    float2 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) v[u] = __ldcg(zp + j[u]);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) o[u] = next_p(v[u]);
+                });
+                B.product<float>(t, [&](uint32_t col) { return next_p(__ldcg(zp + col)); });
+                for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+                    const uint32_t gk = t.r0 + k;
+                    const float p = vec[k];
+                    const float dg = B.single ? B.rf(C16Block::C16_DG)[k] : __ldg(S.diag32 + gk);
+                    const float q = fmaf(dg, p, B.rowsum<float>(k));
+                    if (B.single) B.rf(C16Block::C16_P)[k] = p;
+                    else S.p[gk] = p;
+                    rq[gk] = make_float2(B.single ? B.rf(C16Block::C16_R)[k] : S.r[gk], q);
+                    pq[0] += (double)p * (double)q;
+                }
+            });
+            double totp[1];
+            ok = c16_sum<1>(pq, sy, B.got(), totp);
+            if (!ok) break;
+            alpha = rz / totp[0];
+        }
+        if (!ok) break;
     }
+    c16_finish_solve(S, sy, total, outers, relres, converged, ok);
 }
 
 template <class T>
@@ -588,52 +1507,142 @@ bool c16_alloc(T** p, size_t count) {
     return cudaMalloc((void**)p, (count ? count : 1) * sizeof(T)) == cudaSuccess;
 }
 
-size_t c16_smem_bytes(int threads, int chunks) {
-    return (size_t)(threads / 32) * (size_t)chunks * 32 * (sizeof(uint2) + sizeof(float4));
+// Position of cell (x, y, z) of a 2^bits cube along the Hilbert curve
+// (J. Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004:
+// the axes are turned into the curve's transposed index in place, whose bits
+// are then interleaved).
+uint64_t hilbert_index(uint32_t x, uint32_t y, uint32_t z, int bits) {
+    uint32_t v[3] = {x, y, z};
+    for (uint32_t q = 1u << (bits - 1); q > 1; q >>= 1) {
+        const uint32_t low = q - 1;
+        for (int a = 0; a < 3; a++) {
+            if (v[a] & q) {
+                v[0] ^= low;
+            } else {
+                const uint32_t t = (v[0] ^ v[a]) & low;
+                v[0] ^= t;
+                v[a] ^= t;
+            }
+        }
+    }
+    v[1] ^= v[0];
+    v[2] ^= v[1];
+    uint32_t t = 0;
+    for (uint32_t q = 1u << (bits - 1); q > 1; q >>= 1)
+        if (v[2] & q) t ^= q - 1;
+    uint64_t h = 0;
+    for (int b = bits - 1; b >= 0; b--)
+        for (int a = 0; a < 3; a++) h = (h << 1) | (((v[a] ^ t) >> b) & 1u);
+    return h;
 }
+
+// The linked cells of a grid in curve order: their up to 4 cells of the
+// sorted grid (global ids) and the 27 linked cells around each.
+void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint32_t>* nbr) {
+    const uint32_t f = (uint32_t)g.reach;  // 2 on the refined grid, else 1
+    const uint32_t nx = g.cdx, ny = (g.cdy + f - 1) / f, nz = (g.cdz + f - 1) / f;
+    const uint32_t most = std::max(nx, std::max(ny, nz));
+    int bits = 1;
+    while ((1u << bits) < most) bits++;
+    struct Key {
+        uint64_t h;
+        uint32_t x, y, z;
+    };
+    std::vector<Key> order;
+    order.reserve((size_t)nx * ny * nz);
+    for (uint32_t z = 0; z < nz; z++)
+        for (uint32_t y = 0; y < ny; y++)
+            for (uint32_t x = 0; x < nx; x++) order.push_back({hilbert_index(x, y, z, bits), x, y, z});
+    std::sort(order.begin(), order.end(), [](const Key& a, const Key& b) { return a.h < b.h; });
+    const uint32_t first = (uint32_t)(cells->size() / 4);
+    std::vector<uint32_t> rank(order.size());
+    for (size_t k = 0; k < order.size(); k++)
+        rank[((size_t)order[k].z * ny + order[k].y) * nx + order[k].x] = first + (uint32_t)k;
+    for (const Key& o : order) {
+        for (uint32_t b = 0; b < 2; b++)
+            for (uint32_t a = 0; a < 2; a++) {
+                const uint32_t y = o.y * f + a, z = o.z * f + b;
+                const bool in = a < f && b < f && y < g.cdy && z < g.cdz;
+                cells->push_back(in ? g.base + z * g.sheet + y * g.cdx + o.x : C16_NONE);
+            }
+        for (int dz = -1; dz <= 1; dz++)
+            for (int dy = -1; dy <= 1; dy++)
+                for (int dx = -1; dx <= 1; dx++) {
+                    const int64_t x = (int64_t)o.x + dx, y = (int64_t)o.y + dy, z = (int64_t)o.z + dz;
+                    const bool in = x >= 0 && y >= 0 && z >= 0 && x < nx && y < ny && z < nz;
+                    nbr->push_back(in ? rank[((size_t)z * ny + (size_t)y) * nx + (size_t)x] : C16_NONE);
+                }
+    }
+}
+
+// shared memory of the pack's page table and of a solver block (the rest of
+// an SM's 228 KB stays L1 and the kernels' static arrays)
+size_t c16_page_bytes(uint32_t cap) { return (((size_t)cap + C16_PAGE - 1) / C16_PAGE + 1) * sizeof(uint16_t); }
+constexpr size_t C16_PAGE_BYTES_MAX = 160 * 1024;
+constexpr size_t C16_SMEM = 220 * 1024;
 
 }  // namespace
 
-int ppe_c16_enable(PpeWork& w, std::string* err) {
+// the pack's page table is in shared memory: 20 M particles
+bool ppe_c16_takes(uint32_t cap, const Grid& grid) {
+    return grid.reach <= 2 && c16_page_bytes(cap) <= C16_PAGE_BYTES_MAX;
+}
+
+int ppe_c16_enable(PpeWork& w, const Grid& grid, std::string* err) {
     if (w.c16_ready) return MPS_OK;
     const size_t cap = w.cap;
-    const size_t vec = cap + 8;  // the last slice's padding rows read up to 3 past R
+    if (!ppe_c16_takes(w.cap, grid)) {
+        if (err) *err = "the compact PPE layout does not take this grid";
+        return MPS_ERR_INVALID;
+    }
+    const size_t vec = cap + 8;
     const size_t slices = (cap + C16_ROWS - 1) / C16_ROWS + 2;
-    w.c16_cap_chunks = slices * ((PPE_W + 31) / 32);
-    const size_t ent = w.c16_cap_chunks * C16_CHUNK;
+    const size_t chunks = slices * ((PPE_W + 15) / 16);
+    const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms);
+    std::vector<uint32_t> cells, nbr;
+    linked_cells(grid, &cells, &nbr);
+    w.c16_nsuper = (uint32_t)(cells.size() / 4);
     bool ok = true;
+    ok &= c16_alloc(&w.c16_cells, cells.size());
+    ok &= c16_alloc(&w.c16_nbr, nbr.size());
+    ok &= c16_alloc(&w.c16_base, (size_t)w.c16_nsuper + 2);
     ok &= c16_alloc(&w.cpos, cap);
-    ok &= c16_alloc(&w.c16_width, slices + 2);
-    ok &= c16_alloc(&w.c16_codes, ent);
-    ok &= c16_alloc(&w.c16_w, ent);
-    ok &= c16_alloc(&w.c16_side, ent);
-    ok &= c16_alloc(&w.c16_esc, 1);
+    ok &= c16_alloc(&w.clen, vec);
+    ok &= c16_alloc(&w.c16_off, slices + 2);
+    ok &= c16_alloc(&w.c16_ent, chunks * C16_CHUNK_BYTES);
+    ok &= c16_alloc(&w.c16_side, chunks * C16_CHUNK);
+    ok &= c16_alloc(&w.c16_tile, tiles * (sizeof(C16Tile) / sizeof(uint32_t)));
+    ok &= c16_alloc(&w.c16_collist, tiles * C16_COLS);
+    ok &= c16_alloc(&w.c16_stats, C16_STATS);
     ok &= c16_alloc(&w.cb64, vec);
     ok &= c16_alloc(&w.cx64, vec);
     ok &= c16_alloc(&w.cdiag64, vec);
     ok &= c16_alloc(&w.cdiag32, vec);
     ok &= c16_alloc(&w.cinv_diag, vec);
+    ok &= c16_alloc(&w.cdsq, vec);
     ok &= c16_alloc(&w.cr, vec);
-    ok &= c16_alloc(&w.cq, vec);
-    ok &= c16_alloc(&w.czp[0], vec);
-    ok &= c16_alloc(&w.czp[1], vec);
+    ok &= c16_alloc(&w.cp, vec);
+    ok &= c16_alloc(&w.cpub[0], vec);
+    ok &= c16_alloc(&w.cpub[1], vec);
+    ok &= c16_alloc(&w.c16_slots, 2 * (size_t)w.sms * w.sms * C16_SUMS);
+    ok &= c16_alloc(&w.c16_epoch, 1);
     if (!ok) {
         ppe_c16_free(w);
         if (err) *err = "cudaMalloc failed for the compact PPE layout";
         return MPS_ERR_CUDA;
     }
-    // padding rows beyond R read these: keep them finite
-    cudaMemset(w.cx64, 0, vec * sizeof(double));
-    cudaMemset(w.czp[0], 0, vec * sizeof(float2));
-    cudaMemset(w.czp[1], 0, vec * sizeof(float2));
-    const size_t most = c16_smem_bytes(PPE_THREADS, 8);
-    if (cudaFuncSetAttribute(k_ppe_solve_c16<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
+    cudaMemset(w.c16_stats, 0, C16_STATS * sizeof(uint32_t));
+    cudaMemset(w.c16_epoch, 0, sizeof(unsigned long long));
+    cudaMemset(w.c16_slots, 0, 2 * (size_t)w.sms * w.sms * C16_SUMS * sizeof(ulonglong2));
+    if (cudaMemcpy(w.c16_cells, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(w.c16_nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaFuncSetAttribute(k_c16_pack<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)C16_PAGE_BYTES_MAX) != cudaSuccess ||
+        cudaFuncSetAttribute(k_c16_pack<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)C16_PAGE_BYTES_MAX) != cudaSuccess ||
+        cudaFuncSetAttribute(k_ppe_solve_c16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C16_SMEM) !=
             cudaSuccess ||
-        cudaFuncSetAttribute(k_ppe_solve_c16<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_ppe_solve_c16<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_ppe_solve_c16<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
+        cudaFuncSetAttribute(k_ppe_solve_c16_learned, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C16_SMEM) !=
             cudaSuccess) {
         ppe_c16_free(w);
         if (err) *err = "the compact PPE solver cannot have its shared memory";
@@ -644,82 +1653,140 @@ int ppe_c16_enable(PpeWork& w, std::string* err) {
 }
 
 void ppe_c16_free(PpeWork& w) {
-    void* ps[] = {w.cpos, w.c16_width, w.c16_codes, w.c16_w, w.c16_side, w.c16_esc, w.cb64, w.cx64, w.cdiag64,
-                  w.cdiag32, w.cinv_diag, w.cr, w.cq, w.czp[0], w.czp[1], w.cr2};
+    void* ps[] = {w.c16_cells, w.c16_nbr, w.c16_base, w.cpos, w.clen, w.c16_off, w.c16_ent, w.c16_side, w.c16_tile,
+                  w.c16_collist, w.c16_stats, w.cb64, w.cx64, w.cdiag64, w.cdiag32, w.cinv_diag, w.cdsq, w.cr, w.cp,
+                  w.cpub[0], w.cpub[1], w.c16_slots, w.c16_epoch, w.c16_spfirst, w.c16_spent, w.c16_spside};
     for (void* p : ps)
         if (p) cudaFree(p);
-    w.cpos = w.c16_width = w.c16_esc = nullptr;
-    w.c16_codes = nullptr;
-    w.c16_w = nullptr;
-    w.c16_side = nullptr;
+    w.c16_cells = w.c16_nbr = w.c16_base = w.cpos = w.clen = w.c16_off = w.c16_side = w.c16_tile = nullptr;
+    w.c16_collist = w.c16_stats = nullptr;
+    w.c16_ent = nullptr;
     w.cb64 = w.cx64 = w.cdiag64 = nullptr;
-    w.cdiag32 = w.cinv_diag = w.cr = w.cq = nullptr;
-    w.czp[0] = w.czp[1] = nullptr;
-    w.cr2 = nullptr;
+    w.cdiag32 = w.cinv_diag = w.cdsq = w.cr = w.cp = nullptr;
+    w.cpub[0] = w.cpub[1] = nullptr;
+    w.c16_slots = nullptr;
+    w.c16_epoch = nullptr;
+    w.c16_spfirst = w.c16_spent = w.c16_spside = nullptr;
     w.c16_ready = false;
     w.c16 = false;
     w.c16_learned = false;
 }
 
+// the learned S' in the tiles' codes
+int ppe_c16_learned_enable(PpeWork& w, std::string* err) {
+    const int e = ppe_sp_enable(w, err);
+    if (e != MPS_OK) return e;
+    if (w.c16_spfirst) return MPS_OK;
+    const size_t tiles = c16_tiles(w.cap, (uint32_t)w.sms);
+    const size_t ent = ((size_t)w.cap / SP_SLICE + tiles + 1) * SP_SLICE * LP_GW;
+    bool ok = c16_alloc(&w.c16_spfirst, tiles * C16_SP_SLICES);
+    ok &= c16_alloc(&w.c16_spent, ent);
+    ok &= c16_alloc(&w.c16_spside, ent);
+    if (!ok) {
+        if (err) *err = "cudaMalloc failed for the learned compact preconditioner";
+        return MPS_ERR_CUDA;
+    }
+    return MPS_OK;
+}
+
+// The row numbers, before the assembly.
+int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st) {
+    C16Flag F;
+    F.pos = a.cur.pos;
+    F.n = a.cur.n;
+    F.id = a.cur.id;
+    F.sid_of_id = a.batch.n ? a.batch.sid_of_id : nullptr;
+    F.scenes = a.batch.n ? w.scenes : nullptr;
+    F.bthr = bthr;
+    k_c16_count<<<cblocks((w.c16_nsuper + 1) * 32u, 256), 256, 0, st>>>(F, w.c16_cells, w.c16_nsuper, a.cell_start,
+                                                                        w.c16_base, w.c16_stats);
+    launch_scan_exclusive(w.c16_base, w.c16_nsuper + 1, st);
+    k_c16_rows<<<cblocks(w.c16_nsuper * 32u, 256), 256, 0, st>>>(F, w.c16_cells, w.c16_nsuper, a.cell_start,
+                                                                 w.c16_base, w.cpos, w.rowlist, w.nrows, w.rlen,
+                                                                 w.diag64);
+    return 3;
+}
+
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
-    (void)a;
     const uint32_t maxslices = (cap + C16_ROWS - 1) / C16_ROWS;
-    k_c16_rows<<<cblocks(C16_ROWS * (maxslices + 1), 256), 256, 0, st>>>(
-        w.rowlist, w.nrows, w.rlen, w.b64, w.x64, w.diag64, w.diag32, w.inv_diag, w.cpos, w.cb64, w.cx64, w.cdiag64,
-        w.cdiag32, w.cinv_diag, w.c16_width, maxslices);
-    launch_scan_exclusive(w.c16_width, maxslices + 1, st);
-    cudaMemsetAsync(w.c16_esc, 0, sizeof(uint32_t), st);
-    k_c16_pack<<<cblocks(maxslices * 32u, 256), 256, 0, st>>>(w.cols, w.wrm, w.rlen, w.rowlist, w.nrows, w.c16_width,
-                                                             w.cpos, w.c16_codes, w.c16_w, w.c16_side, w.c16_esc);
+    k_c16_width<<<cblocks(C16_ROWS * (maxslices + 1), 256), 256, 0, st>>>(w.clen, w.nrows, w.c16_off, maxslices);
+    launch_scan_exclusive(w.c16_off, maxslices + 1, st);
+    C16PackArgs P;
+    P.cols_rm = w.cols;
+    P.w_rm = w.wrm;
+    P.clen = w.clen;
+    P.nrows = w.nrows;
+    P.off = w.c16_off;
+    P.base = w.c16_base;
+    P.nbr = w.c16_nbr;
+    P.nsuper = w.c16_nsuper;
+    P.blocks = (uint32_t)w.sms;
+    P.tiles = reinterpret_cast<C16Tile*>(w.c16_tile);
+    P.collist = w.c16_collist;
+    P.ent = w.c16_ent;
+    P.side = w.c16_side;
+    P.stats = w.c16_stats;
+    P.rowlist = w.rowlist;
+    P.cpos = w.cpos;
+    P.idv = a.cur.id;
+    P.index_of_id = w.index_of_id;
+    P.dsq = w.cdsq;
+    P.s_cnt = w.lp.s_cnt;
+    P.s_col = w.lp.s_col;
+    P.s_val = w.lp.s_val;
+    P.s_diag = w.lp.s_diag;
+    P.sc = a.sc;
+    P.sp_first = w.c16_spfirst;
+    P.sp_ent = w.c16_spent;
+    P.sp_side = w.c16_spside;
+    P.sp_diag = w.sp_diag;
+    const uint32_t tiles = c16_tiles(cap, (uint32_t)w.sms);
+    if (w.c16_learned) k_c16_pack<true><<<tiles, C16_PACK_THREADS, c16_page_bytes(cap), st>>>(P);
+    else k_c16_pack<false><<<tiles, C16_PACK_THREADS, c16_page_bytes(cap), st>>>(P);
     return 3;
 }
 
 int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, uint32_t cap, cudaStream_t st) {
     C16Args S;
     S.nrows = w.nrows;
-    S.off = w.c16_width;
-    S.codes = w.c16_codes;
-    S.wts = w.c16_w;
+    S.off = w.c16_off;
+    S.ent = w.c16_ent;
     S.side = w.c16_side;
+    S.tiles = reinterpret_cast<const C16Tile*>(w.c16_tile);
+    S.collist = w.c16_collist;
+    S.stats = w.c16_stats;
     S.b64 = w.cb64;
     S.diag64 = w.cdiag64;
     S.diag32 = w.cdiag32;
     S.inv_diag = w.cinv_diag;
     S.x64 = w.cx64;
+    S.p = w.cp;
     S.r = w.cr;
-    S.zp0 = w.czp[0];
-    S.zp1 = w.czp[1];
-    S.q = w.cq;
-    S.part = w.part;
-    S.result = w.result;
-    S.bar = w.bar;
+    S.pub0 = w.cpub[0];
+    S.pub1 = w.cpub[1];
+    S.slots = w.c16_slots;
+    S.epoch = w.c16_epoch;
     S.sc = a.sc;
     S.tol = opt.cg_tol;
     S.max_iter = opt.cg_max_iter;
     S.inner_cap = opt.cg_check_every > 0 ? opt.cg_check_every : 500;
     S.eta_min = pow(10.0, -(double)(opt.cg_inner_digits > 0 ? opt.cg_inner_digits : 4));
     S.max_outer = 40;
-    // the matrix head kept in L2: the same byte budget as the 8-byte layout
+    // the share of the matrix kept in L2: the same byte budget as the 8-byte layout
     S.keep = w.l2_keep_entries == 0xFFFFFFFFu ? 0xFFFFFFFFu
-                                               : (uint32_t)((size_t)w.l2_keep_entries * 8 / (C16_CHUNK * 6));
-    // chunks per warp in shared memory (an SM holds 32 warps whichever the
-    // block size, so the per-SM total is the same)
-    int chunks = w.c16_smem_chunks;
-    if (chunks < 0) chunks = 0;
-    if (chunks > 8) chunks = 8;
-    S.smem_chunks = chunks;
-    const size_t smem = c16_smem_bytes(w.threads, chunks);
-    S.sp_off = w.sp_off;
-    S.sp_ent = w.sp_ent;
+                                               : (uint32_t)((size_t)w.l2_keep_entries * 8 / C16_CHUNK_BYTES);
+    const int chunks = w.c16_smem_chunks < 0 ? 0 : (w.c16_smem_chunks > 8 ? 8 : w.c16_smem_chunks);
+    S.smem_chunks = (uint32_t)chunks * 32;  // of the 32 warps an SM's share is counted in
+    S.smem_bytes = (uint32_t)C16_SMEM;
+    S.sp_first = w.c16_spfirst;
+    S.sp_ent = w.c16_spent;
+    S.sp_side = w.c16_spside;
     S.sp_diag = w.sp_diag;
-    S.r2 = w.cr2;
     void* args[] = {&S};
-    const bool lrn = w.c16_learned;
-    const void* fn = a.exact ? (lrn ? (const void*)k_ppe_solve_c16<true, true> : (const void*)k_ppe_solve_c16<true, false>)
-                             : (lrn ? (const void*)k_ppe_solve_c16<false, true> : (const void*)k_ppe_solve_c16<false, false>);
-    w.launch_err = launch_cooperative_smem(fn, w.blocks, w.threads, smem, args, st);
+    const void* fn = w.c16_learned ? (const void*)k_ppe_solve_c16_learned : (const void*)k_ppe_solve_c16;
+    w.launch_err = launch_cooperative_smem(fn, w.sms, C16_THREADS, C16_SMEM, args, st);
     if (!w.write_pressure) return 1;
-    k_c16_finish<<<cblocks(cap, 256), 256, 0, st>>>(w.cx64, w.rlen, w.cpos, a.cur.press, a.sc);
+    k_c16_finish<<<cblocks(cap, 256), 256, 0, st>>>(w.cx64, w.cpos, a.cur.press, a.sc);
     return 2;
 }
 
@@ -745,26 +1812,13 @@ int ppe_sp_enable(PpeWork& w, std::string* err) {
     return MPS_OK;
 }
 
-int ppe_c16_learned_enable(PpeWork& w, std::string* err) {
-    const int e = ppe_sp_enable(w, err);
-    if (e != MPS_OK) return e;
-    if (w.cr2) return MPS_OK;
-    if (!c16_alloc(&w.cr2, (size_t)w.cap + 8)) {
-        if (err) *err = "cudaMalloc failed for the learned compact preconditioner";
-        return MPS_ERR_CUDA;
-    }
-    cudaMemset(w.cr2, 0, ((size_t)w.cap + 8) * sizeof(float));
-    return MPS_OK;
-}
-
-int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st, bool by_particle) {
+int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
     SpArgs A;
     A.rowlist = w.rowlist;
     A.nrows = w.nrows;
     A.idv = a.cur.id;
     A.index_of_id = w.index_of_id;
     A.rlen = w.rlen;
-    A.cpos = w.cpos;
     A.diag64 = w.diag64;
     A.s_cnt = w.lp.s_cnt;
     A.s_col = w.lp.s_col;
@@ -779,18 +1833,16 @@ int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream
     const uint32_t wb = cblocks((maxslices + 1) * SP_SLICE, 256), pb = cblocks(maxslices * SP_SLICE, 256);
     k_sp_width<<<wb, 256, 0, st>>>(A);
     launch_scan_exclusive(w.sp_off, maxslices + 1, st);
-    if (by_particle) k_sp_pack<true><<<pb, 256, 0, st>>>(A);
-    else k_sp_pack<false><<<pb, 256, 0, st>>>(A);
+    k_sp_pack<<<pb, 256, 0, st>>>(A);
     return 3;
 }
 
 int ppe_c16_export(const PpeWork& w, uint32_t np, const uint32_t* d_row_start, uint32_t* d_cols, float* d_w,
                    cudaStream_t st) {
-    const uint32_t maxslices = (np + C16_ROWS - 1) / C16_ROWS;
-    if (maxslices)
-        k_c16_export<<<cblocks(maxslices * 32u, 256), 256, 0, st>>>(w.rlen, w.rowlist, w.nrows, w.c16_width,
-                                                                   w.c16_codes, w.c16_w, w.c16_side, d_row_start,
-                                                                   d_cols, d_w);
+    const uint32_t tiles = c16_tiles(np, (uint32_t)w.sms);
+    k_c16_export<<<tiles, 256, 0, st>>>(reinterpret_cast<const C16Tile*>(w.c16_tile), w.c16_collist, (uint32_t)w.sms,
+                                        w.clen, w.rowlist, w.nrows, w.c16_off, w.c16_ent, w.c16_side, d_row_start,
+                                        d_cols, d_w);
     return MPS_OK;
 }
 

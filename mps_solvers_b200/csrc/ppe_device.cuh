@@ -152,8 +152,7 @@ __device__ __forceinline__ float4 ld_mat(const float4* p, uint64_t pol) {
 // consecutive row positions, width = the longest row of the slice, entry t
 // of row position k at off[k / 32] + 32 t + k % 32.  Each entry is one
 // 32-bit word: (column - c) in the upper 16 bits, the value in BF16 in the
-// lower 16, where c is the row's own column (its compact position in the
-// compact solver, its particle index in the particle-indexed solvers);
+// lower 16, where c is the row's own column; columns are particle indices;
 // padding is 0 (the row itself, value 0).  The diagonal is kept in FP32 by
 // row position.
 constexpr uint32_t SP_SLICE = 32;
