@@ -342,8 +342,8 @@ mps_status mps_cell_sort_dev(const float* pos4_dev, uint32_t n, const mps_grid* 
  * else MPS_ERR_CAPACITY.  All calls on a device share the array, so calls
  * whose GPU work overlaps race and must be serialised.  Every call looks the
  * array's address up for the current device and context (so it stays valid
- * after cudaDeviceReset).  The call waits for its stream before returning and
- * copies n from host memory, so it cannot be captured in a CUDA graph.  The
+ * after cudaDeviceReset).  The call waits for its stream before returning, so
+ * it cannot be captured in a CUDA graph.  The
  * array stays allocated on every device that loaded the library until the
  * process exits. */
 #define MPS_NOALLOC_MAX_PARTICLES 524288u

@@ -465,7 +465,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         CK(dalloc(h, &h->sort.keys[b], cap));
         CK(dalloc(h, &h->sort.vals[b], cap));
     }
-    CK(dalloc(h, &h->sort.hist, (size_t)SORT_RADIX * h->sort.tiles));
+    CK(dalloc(h, &h->sort.hist, (size_t)SORT_RADIX * (h->sort.tiles + 1)));
     CK(dalloc(h, &h->stage.pos3, 3 * (size_t)cap));
     CK(dalloc(h, &h->stage.vel3, 3 * (size_t)cap));
     CK(dalloc(h, &h->stage.press, cap));
@@ -736,7 +736,7 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
         CK(dalloc(h, &h->sort.keys[b], cap));
         CK(dalloc(h, &h->sort.vals[b], cap));
     }
-    CK(dalloc(h, &h->sort.hist, (size_t)SORT_RADIX * h->sort.tiles));
+    CK(dalloc(h, &h->sort.hist, (size_t)SORT_RADIX * (h->sort.tiles + 1)));
     CK(dalloc(h, &h->stage.pos3, 3 * (size_t)cap));
     CK(dalloc(h, &h->stage.vel3, 3 * (size_t)cap));
     CK(dalloc(h, &h->stage.press, cap));
@@ -1922,7 +1922,7 @@ extern "C" mps_status mps_cell_sort_dev(const float* pos4_dev, uint32_t n, const
     s.tiles = tiles;
     void* blk = nullptr;
     const size_t nk = (size_t)(n > 0 ? n : 1);
-    const size_t bytes = 4 * nk * sizeof(uint32_t) + (size_t)SORT_RADIX * tiles * sizeof(uint32_t) +
+    const size_t bytes = 4 * nk * sizeof(uint32_t) + (size_t)SORT_RADIX * (tiles + 1) * sizeof(uint32_t) +
                          ((size_t)g.ncells + 1) * sizeof(uint32_t) + sizeof(uint32_t) + 256;
     if (cudaMalloc(&blk, bytes) != cudaSuccess) return MPS_ERR_CUDA;
     uint32_t* b = (uint32_t*)blk;
@@ -1931,11 +1931,9 @@ extern "C" mps_status mps_cell_sort_dev(const float* pos4_dev, uint32_t n, const
     s.keys[1] = b + 2 * nk;
     s.vals[1] = b + 3 * nk;
     s.hist = b + 4 * nk;
-    uint32_t* cs = s.hist + (size_t)SORT_RADIX * tiles;
+    uint32_t* cs = s.hist + (size_t)SORT_RADIX * (tiles + 1);
     uint32_t* n_dev = cs + g.ncells + 1;
-    cudaMemcpyAsync(n_dev, &n, sizeof n, cudaMemcpyHostToDevice, st);
-    launch_cell_keys_plain((const float4*)pos4_dev, n, g, s.keys[0], s.vals[0], st);
-    const int r = launch_radix_sort(s, n_dev, sort_passes(g.ncells), n, st);
+    const int r = launch_keys_and_sort_plain((const float4*)pos4_dev, n, g, s, n_dev, sort_passes(g.ncells), st);
     launch_cell_start_plain(s.keys[r], n, g, cs, n_in_grid_dev, st);
     if (n) {
         cudaMemcpyAsync(perm_dev, s.vals[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);

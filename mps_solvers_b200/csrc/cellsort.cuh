@@ -27,7 +27,7 @@ inline int sort_passes(uint32_t ncells) {
 struct SortScratch {
     uint32_t* keys[2];
     uint32_t* vals[2];
-    uint32_t* hist;  // SORT_RADIX * tiles
+    uint32_t* hist;  // SORT_RADIX * (tiles + 1): digit rows of tile counts, then the digits' totals
     uint32_t tiles;
 };
 
@@ -40,14 +40,12 @@ enum ApplyMode : int {
 };
 
 // Launchers (all asynchronous on `st`).
-// Stable LSD radix sort of (keys[0], vals[0]) over *n_dev keys; returns the
-// buffer index (0/1) that holds the result.
-int launch_radix_sort(SortScratch& s, const uint32_t* n_dev, int passes, uint32_t cap, cudaStream_t st);
 // The rebuild's keys and sort: the cell key of every active particle (after
 // the pending update; with batch.n > 0 g is the whole cell space and each
 // particle, by id, uses its scene's grid) computed by the first pass's
-// upsweep, then the sort over sc->np keys.  Returns the buffer index as
-// launch_radix_sort.  The cell table is filled by the gather that follows.
+// upsweep, then a stable LSD radix sort of (keys[0], vals[0]) over sc->np
+// keys.  Returns the buffer index (0/1) that holds the result (`passes` odd: 1).
+// The cell table is filled by the gather that follows.
 int launch_keys_and_sort(const float4* pos, const float4* tmp, int apply, const Grid& g, Scalars* sc,
                          const uint32_t* id, const BatchDev& batch, SortScratch& s, int passes, cudaStream_t st);
 
@@ -82,8 +80,8 @@ void launch_merge_keys_sort(const float4* pos, const float4* tmp, int apply, con
 cudaError_t merge_sort_setup();
 
 // Same pieces with n given on the host (for the device-pointer primitive).
-void launch_cell_keys_plain(const float4* pos, uint32_t n, const Grid& g, uint32_t* keys, uint32_t* vals,
-                            cudaStream_t st);
+int launch_keys_and_sort_plain(const float4* pos, uint32_t n, const Grid& g, SortScratch& s, uint32_t* n_dev,
+                               int passes, cudaStream_t st);
 void launch_cell_start_plain(const uint32_t* keys_sorted, uint32_t n, const Grid& g, uint32_t* cell_start,
                              uint32_t* n_in_grid, cudaStream_t st);
 // exclusive scan of `total` uint32 counters in place (one block)

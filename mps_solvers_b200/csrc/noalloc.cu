@@ -28,8 +28,8 @@
 //     the device address up with cudaGetSymbolAddress for the current device
 //     and context, so the address stays right after a cudaDeviceReset or when
 //     another context becomes current (nothing is cached);
-//   * the call cannot be captured in a CUDA graph: it copies n from host
-//     memory and ends by waiting for its stream (cudaStreamSynchronize);
+//   * the call cannot be captured in a CUDA graph: it ends by waiting for
+//     its stream (cudaStreamSynchronize);
 //   * errors: the launches' configurations are valid by construction for
 //     every accepted size, and the call reports the copies' return codes and
 //     the stream's result; it neither reads nor clears errors that other
@@ -54,7 +54,7 @@ constexpr size_t kVals0 = kKeys0 + round64(kMaxP);
 constexpr size_t kKeys1 = kVals0 + round64(kMaxP);
 constexpr size_t kVals1 = kKeys1 + round64(kMaxP);
 constexpr size_t kHist = kVals1 + round64(kMaxP);
-constexpr size_t kCells = kHist + round64((size_t)SORT_RADIX * kMaxTiles);
+constexpr size_t kCells = kHist + round64((size_t)SORT_RADIX * (kMaxTiles + 1));
 constexpr size_t kCount = kCells + round64((size_t)kMaxC + 1);
 constexpr size_t kWords = kCount + 64;
 
@@ -106,9 +106,7 @@ extern "C" mps_status mps_cell_sort_dev_noalloc(const float* pos4_dev, uint32_t 
     s.hist = base + kHist;
     uint32_t* cs = base + kCells;
     uint32_t* n_dev = base + kCount;
-    if (cudaMemcpyAsync(n_dev, &n, sizeof n, cudaMemcpyHostToDevice, st) != cudaSuccess) return MPS_ERR_CUDA;
-    launch_cell_keys_plain((const float4*)pos4_dev, n, g, s.keys[0], s.vals[0], st);
-    const int r = launch_radix_sort(s, n_dev, sort_passes(g.ncells), n, st);
+    const int r = launch_keys_and_sort_plain((const float4*)pos4_dev, n, g, s, n_dev, sort_passes(g.ncells), st);
     launch_cell_start_plain(s.keys[r], n, g, cs, n_in_grid_dev, st);
     bool copies_ok = true;
     if (n) {
