@@ -324,8 +324,9 @@ const char* mps_last_error(mps_handle* h);
  * stable sort by cell, cell start/end tables.  perm_dev[new] = old index;
  * cell_of_dev[new] = cell id (ncells for a particle outside the grid, sorted
  * last); start_dev/end_dev get ncells entries; *n_in_grid_dev (device) the
- * count of particles inside the grid.  Scratch memory is allocated and freed
- * by the call; stream may be NULL (legacy default stream). */
+ * count of particles inside the grid.  Scratch memory comes from the device's
+ * memory pool (cudaMallocAsync) and goes back to it; stream may be NULL
+ * (legacy default stream). */
 mps_status mps_cell_sort_dev(const float* pos4_dev, uint32_t n, const mps_grid* g,
                              uint32_t* perm_dev, uint32_t* cell_of_dev, uint32_t* start_dev,
                              uint32_t* end_dev, uint32_t* n_in_grid_dev, void* stream);
@@ -343,8 +344,7 @@ mps_status mps_cell_sort_dev(const float* pos4_dev, uint32_t n, const mps_grid* 
  * whose GPU work overlaps race and must be serialised.  Every call looks the
  * array's address up for the current device and context (so it stays valid
  * after cudaDeviceReset).  The call waits for its stream before returning, so
- * it cannot be captured in a CUDA graph.  The
- * array stays allocated on every device that loaded the library until the
+ * it cannot be captured in a CUDA graph.  The array stays allocated on every device that loaded the library until the
  * process exits. */
 #define MPS_NOALLOC_MAX_PARTICLES 524288u
 #define MPS_NOALLOC_MAX_CELLS 524288u

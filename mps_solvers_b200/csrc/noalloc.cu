@@ -2,11 +2,10 @@
 // (cell keys, stable sort by cell, cell start/end tables) without any device
 // memory allocation.
 //
-// Why it exists: mps_cell_sort_dev allocates its scratch with cudaMalloc and
-// frees it with cudaFree on every call.  Some callers cannot do that: a host
-// application that hands all device memory to its own pool allocator and
-// forbids any other allocation, or a latency-critical loop in which
-// cudaMalloc/cudaFree (which synchronise the device) would stall other work.
+// Why it exists: mps_cell_sort_dev takes its scratch from the device's memory
+// pool on every call.  Some callers cannot do that: a host application that
+// hands all device memory to its own pool allocator and forbids any other
+// allocation.
 // This variant keeps its scratch in one fixed device array instead, so it
 // allocates nothing; the caller still provides the input positions and all
 // output arrays.
@@ -31,8 +30,7 @@
 //   * the call cannot be captured in a CUDA graph: it ends by waiting for
 //     its stream (cudaStreamSynchronize);
 //   * errors: the launches' configurations are valid by construction for
-//     every accepted size, and the call reports the copies' return codes and
-//     the stream's result; it neither reads nor clears errors that other
+//     every accepted size, and the call reports the stream's result; it neither reads nor clears errors that other
 //     work left on the thread (no cudaGetLastError).
 #include <cstdint>
 
@@ -106,17 +104,13 @@ extern "C" mps_status mps_cell_sort_dev_noalloc(const float* pos4_dev, uint32_t 
     s.hist = base + kHist;
     uint32_t* cs = base + kCells;
     uint32_t* n_dev = base + kCount;
-    const int r = launch_keys_and_sort_plain((const float4*)pos4_dev, n, g, s, n_dev, sort_passes(g.ncells), st);
-    launch_cell_start_plain(s.keys[r], n, g, cs, n_in_grid_dev, st);
-    bool copies_ok = true;
-    if (n) {
-        copies_ok &= cudaMemcpyAsync(perm_dev, s.vals[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st) ==
-                     cudaSuccess;
-        copies_ok &= cudaMemcpyAsync(cell_of_dev, s.keys[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st) ==
-                     cudaSuccess;
+    const int passes = sort_passes(g.ncells);
+    if (n) {  // the last pass writes the caller's arrays
+        s.keys[passes & 1] = cell_of_dev;
+        s.vals[passes & 1] = perm_dev;
     }
+    const int r = launch_keys_and_sort_plain((const float4*)pos4_dev, n, g, s, n_dev, passes, st);
+    launch_cell_start_plain(s.keys[r], n, g, cs, n_in_grid_dev, st);
     launch_cell_end_from_start(cs, g.ncells, start_dev, end_dev, st);
-    const cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess || !copies_ok) return MPS_ERR_CUDA;
-    return MPS_OK;
+    return cudaStreamSynchronize(st) == cudaSuccess ? MPS_OK : MPS_ERR_CUDA;
 }
