@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(256) k_surface_vertex(StageArgs a, SurfaceGrid
         return t < 0.f ? -1 : (t >= (float)dim ? (int)dim - 1 : (int)t);
     };
     const float hx = g.cell_size, hyz = g.cell_yz;
+    const float far2 = r0 * r0 * 1.0001f;
     const int x0 = cell_lo(x, g.left, hx, g.cdx), x1 = cell_hi(x, g.left, hx, g.cdx);
     const int y0 = cell_lo(y, g.back, hyz, g.cdy), y1 = cell_hi(y, g.back, hyz, g.cdy);
     const int z0 = g.dim == 3 ? cell_lo(z, g.bottom, hyz, g.cdz) : 0;
@@ -179,7 +180,8 @@ __global__ void __launch_bounds__(256) k_surface_vertex(StageArgs a, SurfaceGrid
                     const float4 pj = __ldg(a.cur.pos + j);
                     if (ptype(pj) != T_FLUID) continue;
                     const float dx = pj.x - x, dy = pj.y - y, dz = pj.z - z;
-                    acc += cubic_w(r0, sqrtf(dx * dx + dy * dy + dz * dz));
+                    const float rr = dx * dx + dy * dy + dz * dz;
+                    if (rr <= far2) acc += cubic_w(r0, sqrtf(rr));  // beyond, w is 0
                 }
             }
     }
@@ -200,20 +202,46 @@ __device__ __forceinline__ uint32_t cube_case(const float* __restrict__ vn, cons
     return idx;
 }
 
+// Triangles per cube, scanned within blocks of SURFACE_SCAN cubes: cnt[c] =
+// those of the earlier cubes of c's block, sum[b] the block's, and one slot
+// past the last for the total.  The scan over the blocks follows (2,000 sums
+// for a 256 x 64 x 128 grid); one block scanning all 2 M cubes took 0.5 ms.
+constexpr uint32_t SURFACE_SCAN = 1024;
 __global__ void __launch_bounds__(256) k_surface_count(const float* __restrict__ vn, SurfaceGrid sg,
                                                        const uint32_t* __restrict__ iso_bits,
-                                                       const uint8_t* __restrict__ tab_n, uint32_t* __restrict__ cnt) {
-    const uint32_t mx = sg.nx - 1, my = sg.ny - 1, mz = sg.nz - 1;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > mx * my * mz) return;
-    if (c == mx * my * mz) {
-        cnt[c] = 0;  // the scan's total slot
-        return;
-    }
+                                                       const uint8_t* __restrict__ tab_n, uint32_t* __restrict__ cnt,
+                                                       uint32_t* __restrict__ sum, uint32_t nblocks) {
+    __shared__ uint32_t ws[8];
+    const uint32_t mx = sg.nx - 1, my = sg.ny - 1, mz = sg.nz - 1, ncube = mx * my * mz;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float iso = __uint_as_float(iso_bits[1]);
-    float val[8];
-    const uint32_t idx = cube_case(vn, sg, c % mx, (c / mx) % my, c / (mx * my), iso, val);
-    cnt[c] = tab_n[idx];
+    uint32_t carry = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < SURFACE_SCAN / 256; r++) {
+        const uint32_t c = blockIdx.x * SURFACE_SCAN + r * 256 + threadIdx.x;
+        uint32_t n = 0;
+        if (c < ncube) {
+            float val[8];
+            n = tab_n[cube_case(vn, sg, c % mx, (c / mx) % my, c / (mx * my), iso, val)];
+        }
+        uint32_t x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)lane >= o) x += t;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        uint32_t before = carry;
+        for (uint32_t w = 0; w < warp; w++) before += ws[w];
+        for (uint32_t w = 0; w < 8; w++) carry += ws[w];
+        if (c < ncube) cnt[c] = before + x - n;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        sum[blockIdx.x] = carry;
+        if (blockIdx.x == 0) sum[nblocks] = 0;  // the scan's total slot
+    }
 }
 
 // -grad n at a vertex (central differences; one-sided at the grid's faces)
@@ -233,13 +261,14 @@ __device__ float3 vertex_normal(const float* __restrict__ vn, const SurfaceGrid&
 __global__ void __launch_bounds__(256) k_surface_emit(const float* __restrict__ vn, SurfaceGrid sg,
                                                       const uint32_t* __restrict__ iso_bits,
                                                       const uint8_t* __restrict__ tab_n, const int8_t* __restrict__ tab_t,
-                                                      const uint32_t* __restrict__ off, uint32_t max_tri,
+                                                      const uint32_t* __restrict__ off,
+                                                      const uint32_t* __restrict__ sum, uint32_t max_tri,
                                                       float* __restrict__ pos9, float* __restrict__ nrm9,
                                                       uint32_t* __restrict__ ntri) {
     const uint32_t mx = sg.nx - 1, my = sg.ny - 1, mz = sg.nz - 1;
     const uint32_t ncube = mx * my * mz;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c == 0) ntri[0] = off[ncube];
+    if (c == 0) ntri[0] = sum[(ncube + SURFACE_SCAN - 1) / SURFACE_SCAN];
     if (c >= ncube) return;
     const float iso = __uint_as_float(iso_bits[1]);
     const uint32_t ix = c % mx, iy = (c / mx) % my, iz = c / (mx * my);
@@ -247,7 +276,7 @@ __global__ void __launch_bounds__(256) k_surface_emit(const float* __restrict__ 
     const uint32_t idx = cube_case(vn, sg, ix, iy, iz, iso, val);
     const uint32_t nt = tab_n[idx];
     if (nt == 0) return;
-    const uint32_t base = off[c];
+    const uint32_t base = off[c] + sum[c / SURFACE_SCAN];
     for (uint32_t t = 0; t < nt; t++) {
         if (base + t >= max_tri) return;
         for (int k = 0; k < 3; k++) {
@@ -306,7 +335,8 @@ int surface_setup(SurfaceWork& w, const SurfaceGrid& g, uint32_t max_tri, cudaSt
         cudaMemsetAsync(*p, 0, bytes + 64, st);
     };
     al((void**)&w.vn, nv * sizeof(float));
-    al((void**)&w.cube_cnt, (ncube + 1) * sizeof(uint32_t));
+    al((void**)&w.cube_cnt, ncube * sizeof(uint32_t));
+    al((void**)&w.block_cnt, ((ncube + SURFACE_SCAN - 1) / SURFACE_SCAN + 1) * sizeof(uint32_t));
     al((void**)&w.tri_pos, (size_t)max_tri * 9 * sizeof(float));
     al((void**)&w.tri_nrm, (size_t)max_tri * 9 * sizeof(float));
     al((void**)&w.ntri, 2 * sizeof(uint32_t));
@@ -341,14 +371,15 @@ void surface_enqueue_extract(SurfaceWork& w, const StageArgs& a, cudaStream_t st
     const uint32_t nv = g.nx * g.ny * g.nz;
     const uint32_t ncube = (g.nx - 1) * (g.ny - 1) * (g.nz - 1);
     k_surface_vertex<<<blocks_for(nv, 256), 256, 0, st>>>(a, g, w.vn);
-    k_surface_count<<<blocks_for(ncube + 1, 256), 256, 0, st>>>(w.vn, g, w.ntri, w.tab_n, w.cube_cnt);
-    launch_scan_exclusive(w.cube_cnt, ncube + 1, st);
-    k_surface_emit<<<blocks_for(ncube, 256), 256, 0, st>>>(w.vn, g, w.ntri, w.tab_n, w.tab_t, w.cube_cnt, w.max_tri,
+    const uint32_t nb = blocks_for(ncube, SURFACE_SCAN);
+    k_surface_count<<<nb, 256, 0, st>>>(w.vn, g, w.ntri, w.tab_n, w.cube_cnt, w.block_cnt, nb);
+    launch_scan_exclusive(w.block_cnt, nb + 1, st);
+    k_surface_emit<<<blocks_for(ncube, 256), 256, 0, st>>>(w.vn, g, w.ntri, w.tab_n, w.tab_t, w.cube_cnt, w.block_cnt, w.max_tri,
                                                            w.tri_pos, w.tri_nrm, w.ntri);
 }
 
 void surface_free(SurfaceWork& w) {
-    void* ps[] = {w.vn, w.cube_cnt, w.tri_pos, w.tri_nrm, w.ntri, w.tab_n, w.tab_t, w.best};
+    void* ps[] = {w.vn, w.cube_cnt, w.block_cnt, w.tri_pos, w.tri_nrm, w.ntri, w.tab_n, w.tab_t, w.best};
     for (void* p : ps)
         if (p) cudaFree(p);
     w = SurfaceWork();

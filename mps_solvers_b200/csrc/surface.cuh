@@ -46,6 +46,7 @@ struct SurfaceWork {
     uint32_t max_tri = 0;
     float* vn = nullptr;          // vertex values
     uint32_t* cube_cnt = nullptr; // triangles per cube, then exclusive offsets
+    uint32_t* block_cnt = nullptr;  // triangles before each block of cubes
     float* tri_pos = nullptr;     // 9 floats per triangle
     float* tri_nrm = nullptr;     // 9 floats per triangle
     uint32_t* ntri = nullptr;     // [0] triangles found (may exceed max_tri), [1] iso bits
