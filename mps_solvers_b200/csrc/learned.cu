@@ -70,6 +70,38 @@ __device__ __forceinline__ Feat edge_feat(const LpSystem& S, const float4& pi, f
     return e;
 }
 
+// A warp's walk over stencil entries [begin, end) of a row: each lane takes the
+// features of one entry (feat(t, neighbour), with a value of its own), 32 at
+// a time through shared memory, and body(t, neighbour, features, value) then
+// sees the entries in order with the whole warp.  Every lane working out the
+// same entry's square root and divisions was a third of these kernels.
+template <class FE, class B>
+__device__ __forceinline__ void for_edges(const uint32_t* __restrict__ cols, uint32_t begin, uint32_t end, FE feat,
+                                          B body) {
+    __shared__ float4 buf_all[8][32][3];  // blocks of 256 threads
+    float4(*buf)[3] = buf_all[(threadIdx.x >> 5) & 7u];
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t t0 = begin; t0 < end; t0 += 32) {
+        const uint32_t n = min(32u, end - t0);
+        __syncwarp();
+        if (lane < n) {
+            const uint32_t j = cols[t0 + lane];
+            float x = 0.f;
+            const Feat e = feat(t0 + lane, j, x);
+            buf[lane][0] = make_float4(e.f[0], e.f[1], e.f[2], e.f[3]);
+            buf[lane][1] = make_float4(e.f[4], e.f[5], e.f[6], x);
+            buf[lane][2].x = __uint_as_float(j);
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (uint32_t u = 0; u < n; u++) {
+            const float4 p = buf[u][0], q = buf[u][1];
+            const Feat e{{p.x, p.y, p.z, p.w, q.x, q.y, q.z}};
+            body(t0 + u, __float_as_uint(buf[u][2].x), e, q.w);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- stencil
 // One warp per non-Dirichlet row: its non-Dirichlet neighbours within r0 in
 // ascending index (so the j < i entries come first), and D^-1/2.
@@ -167,9 +199,8 @@ __global__ void __launch_bounds__(256) k_lp_edge_fwd(FwdArgs A) {
     const float ni = __ldg(S.n + i);
     const uint32_t cnt = A.scnt[i];
     float acc0 = 0.f, acc1 = 0.f;
-    for (uint32_t t = 0; t < cnt; t++) {
-        const uint32_t j = A.scols[(size_t)i * LP_GW + t];
-        const Feat e = edge_feat(S, pi, ni, j, kc);
+    auto feat = [&](uint32_t, uint32_t j, float&) { return edge_feat(S, pi, ni, j, kc); };
+    for_edges(A.scols + (size_t)i * LP_GW, 0u, cnt, feat, [&](uint32_t, uint32_t j, const Feat& e, float) {
         float s0 = b0, s1 = b1;
 #pragma unroll
         for (int f = 0; f < LP_F; f++) {
@@ -182,40 +213,108 @@ __global__ void __launch_bounds__(256) k_lp_edge_fwd(FwdArgs A) {
         }
         acc0 += gelu_t(s0, nullptr);
         acc1 += gelu_t(s1, nullptr);
-    }
+    });
     const float inv = cnt ? 1.f / (float)cnt : 0.f;
     float* a = PASS == 1 ? A.a1 : A.a2;
     a[(size_t)i * LP_H + lane] = acc0 * inv;
     a[(size_t)i * LP_H + lane + 32] = acc1 * inv;
 }
 
+// The dense 64 -> 64 layers work on tiles of 64 rows in shared memory, a
+// thread on 4 rows by 4 columns: four 16-byte and four 8-byte shared-memory
+// loads feed 64 multiply-adds.  (One output a thread over 4 rows loaded two words a
+// multiply-add: 60 and 155 us a layer forward and backward for 57,000 rows.)
+constexpr int DT = 64;            // rows of a tile
+constexpr int DT_LD = LP_H + 4;   // floats a row of a staged tile
+
+// rows [k0, k0 + DT) of the row list into a tile (zeros past R)
+__device__ __forceinline__ void dense_stage(float (*t)[DT_LD], const float* __restrict__ x,
+                                            const uint32_t* __restrict__ idx) {
+    for (int e = threadIdx.x; e < DT * LP_H / 4; e += 256) {
+        const int r = e / (LP_H / 4), c = e % (LP_H / 4);
+        const uint32_t i = idx[r];
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i != 0xffffffffu) v = *reinterpret_cast<const float4*>(x + (size_t)i * LP_H + 4 * c);
+        *reinterpret_cast<float4*>(&t[r][4 * c]) = v;
+    }
+}
+
+// acc[a][b] += sum over c of t[r0 + a][c] m[c][4 q + b], c ascending
+__device__ __forceinline__ void dense_mul(const float (*t)[DT_LD], const __nv_bfloat16 (*m)[LP_H], int r0, int q,
+                                          float (&acc)[4][4]) {
+#pragma unroll 4
+    for (int c = 0; c < LP_H; c += 4) {
+        float4 x[4], w[4];
+#pragma unroll
+        for (int a = 0; a < 4; a++) x[a] = *reinterpret_cast<const float4*>(&t[r0 + a][c]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint2 v = *reinterpret_cast<const uint2*>(&m[c + u][4 * q]);
+            w[u] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u),
+                               __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const float xv = u == 0 ? x[a].x : (u == 1 ? x[a].y : (u == 2 ? x[a].z : x[a].w));
+                acc[a][0] = fmaf(w[u].x, xv, acc[a][0]);
+                acc[a][1] = fmaf(w[u].y, xv, acc[a][1]);
+                acc[a][2] = fmaf(w[u].z, xv, acc[a][2]);
+                acc[a][3] = fmaf(w[u].w, xv, acc[a][3]);
+            }
+    }
+}
+
+__device__ __forceinline__ void dense_rows(uint32_t* idx, uint32_t k0, uint32_t R, const uint32_t* __restrict__ rowlist) {
+    if (threadIdx.x < DT) idx[threadIdx.x] = k0 + threadIdx.x < R ? __ldg(rowlist + k0 + threadIdx.x) : 0xffffffffu;
+}
+
 // dense 64 -> 64 layer on every row: pre = W x + b (b optional), out =
-// act(pre) + resid (act: 0 none, 1 GELU); 4 rows per 256-thread block.
+// act(pre) + resid (act: 0 none, 1 GELU)
 __global__ void __launch_bounds__(256) k_lp_dense_fwd(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                       int woff, int boff, const float* __restrict__ resid,
                                                       float* __restrict__ pre_out, float* __restrict__ out, int act,
                                                       const uint32_t* __restrict__ rowlist,
                                                       const uint32_t* __restrict__ nrows) {
-    __shared__ float W[LP_H][LP_H + 1];
-    __shared__ float xs[4][LP_H];
+    __shared__ __align__(16) __nv_bfloat16 Wt[LP_H][LP_H];  // W transposed: [input][output]
+    __shared__ __align__(16) float xs[DT][DT_LD];
+    __shared__ uint32_t idx[DT];
     const uint32_t R = *nrows;
-    for (int t = threadIdx.x; t < LP_H * LP_H; t += blockDim.x) W[t / LP_H][t % LP_H] = wbf(w, woff + t);
-    const int r = threadIdx.x >> 6, o = threadIdx.x & 63;
-    const float bias = boff >= 0 ? wbf(w, boff + o) : 0.f;
-    for (uint32_t k0 = blockIdx.x * 4; k0 < R; k0 += gridDim.x * 4) {
+    for (int t = threadIdx.x; t < LP_H * LP_H; t += blockDim.x) Wt[t % LP_H][t / LP_H] = w[woff + t];
+    const int q = threadIdx.x & 15, r0 = 4 * (threadIdx.x >> 4);
+    float bias[4];
+#pragma unroll
+    for (int b = 0; b < 4; b++) bias[b] = boff >= 0 ? wbf(w, boff + 4 * q + b) : 0.f;
+    for (uint32_t k0 = blockIdx.x * DT; k0 < R; k0 += gridDim.x * DT) {
         __syncthreads();
-        const uint32_t k = k0 + r;
-        const uint32_t i = k < R ? __ldg(rowlist + k) : 0u;
-        if (k < R) xs[r][o] = x[(size_t)i * LP_H + o];
+        dense_rows(idx, k0, R, rowlist);
         __syncthreads();
-        if (k < R) {
-            float s = bias;
-#pragma unroll 16
-            for (int c = 0; c < LP_H; c++) s = fmaf(W[o][c], xs[r][c], s);
-            if (pre_out) pre_out[(size_t)i * LP_H + o] = s;
-            float v = act ? gelu_t(s, nullptr) : s;
-            if (resid) v += resid[(size_t)i * LP_H + o];
-            out[(size_t)i * LP_H + o] = v;
+        dense_stage(xs, x, idx);
+        __syncthreads();
+        float acc[4][4];
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int b = 0; b < 4; b++) acc[a][b] = bias[b];
+        dense_mul(xs, Wt, r0, q, acc);
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+            const uint32_t i = idx[r0 + a];
+            if (i == 0xffffffffu) continue;
+            const size_t o = (size_t)i * LP_H + 4 * q;
+            if (pre_out) *reinterpret_cast<float4*>(pre_out + o) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+            float v[4];
+#pragma unroll
+            for (int b = 0; b < 4; b++) v[b] = act ? gelu_t(acc[a][b], nullptr) : acc[a][b];
+            if (resid) {
+                const float4 z = *reinterpret_cast<const float4*>(resid + o);
+                v[0] += z.x;
+                v[1] += z.y;
+                v[2] += z.z;
+                v[3] += z.w;
+            }
+            *reinterpret_cast<float4*>(out + o) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
 }
@@ -241,9 +340,8 @@ __global__ void __launch_bounds__(256) k_lp_readout_fwd(FwdArgs A) {
     const float2 kc = lp_consts(S, i);
     const float ni = __ldg(S.n + i);
     const uint32_t nl = A.nlow[i];
-    for (uint32_t t = 0; t < nl; t++) {
-        const uint32_t j = A.scols[(size_t)i * LP_GW + t];
-        const Feat e = edge_feat(S, pi, ni, j, kc);
+    auto feat = [&](uint32_t, uint32_t j, float&) { return edge_feat(S, pi, ni, j, kc); };
+    for_edges(A.scols + (size_t)i * LP_GW, 0u, nl, feat, [&](uint32_t t, uint32_t j, const Feat& e, float) {
         float s0 = ra0 + A.rb[(size_t)j * LP_H + lane], s1 = ra1 + A.rb[(size_t)j * LP_H + lane + 32];
 #pragma unroll
         for (int f = 0; f < LP_F; f++) {
@@ -252,7 +350,7 @@ __global__ void __launch_bounds__(256) k_lp_readout_fwd(FwdArgs A) {
         }
         const float g = warp_sum(om0 * gelu_t(s0, nullptr) + om1 * gelu_t(s1, nullptr));
         if (lane == 0) A.gval[(size_t)i * LP_GW + t] = g;
-    }
+    });
     const float d = warp_sum(wbf(A.w, LP_DL + lane) * A.h2[(size_t)i * LP_H + lane] +
                              wbf(A.w, LP_DL + lane + 32) * A.h2[(size_t)i * LP_H + lane + 32]);
     if (lane == 0) {
@@ -435,9 +533,11 @@ __global__ void __launch_bounds__(256) k_lp_readout_bwd_a(BwdArgs A) {
         const float2 kc = lp_consts(S, i);
         const float ni = __ldg(S.n + i);
         float dra0 = 0.f, dra1 = 0.f;
-        for (uint32_t t = 0; t < A.nlow[i]; t++) {
-            const uint32_t j = A.scols[(size_t)i * LP_GW + t];
-            const Feat e = edge_feat(S, pi, ni, j, kc);
+        auto feat = [&](uint32_t t, uint32_t j, float& x) {
+            x = A.dgval[(size_t)i * LP_GW + t];
+            return edge_feat(S, pi, ni, j, kc);
+        };
+        for_edges(A.scols + (size_t)i * LP_GW, 0u, A.nlow[i], feat, [&](uint32_t, uint32_t j, const Feat& e, float dg) {
             float s0 = ra0 + A.rb[(size_t)j * LP_H + lane], s1 = ra1 + A.rb[(size_t)j * LP_H + lane + 32];
 #pragma unroll
             for (int f = 0; f < LP_F; f++) {
@@ -446,7 +546,6 @@ __global__ void __launch_bounds__(256) k_lp_readout_bwd_a(BwdArgs A) {
             }
             float d0, d1;
             const float g0 = gelu_t(s0, &d0), g1 = gelu_t(s1, &d1);
-            const float dg = A.dgval[(size_t)i * LP_GW + t];
             gom0 += dg * g0;
             gom1 += dg * g1;
             const float dt0 = dg * om0 * d0, dt1 = dg * om1 * d1;
@@ -459,7 +558,7 @@ __global__ void __launch_bounds__(256) k_lp_readout_bwd_a(BwdArgs A) {
             gbr1 += dt1;
             dra0 += dt0;
             dra1 += dt1;
-        }
+        });
         A.dra[(size_t)i * LP_H + lane] = dra0;
         A.dra[(size_t)i * LP_H + lane + 32] = dra1;
         // diagonal: G_ii = softplus(pre) + GMIN
@@ -513,11 +612,11 @@ __global__ void __launch_bounds__(256) k_lp_readout_bwd_b(BwdArgs A) {
     const float rbj0 = A.rb[(size_t)j * LP_H + lane], rbj1 = A.rb[(size_t)j * LP_H + lane + 32];
     float drb0 = 0.f, drb1 = 0.f;
     const uint32_t cnt = A.scnt[j];
-    for (uint32_t t = A.nlow[j]; t < cnt; t++) {
-        const uint32_t i = A.scols[(size_t)j * LP_GW + t];
-        const float4 pi = __ldg(S.pos + i);
-        const float2 kc = lp_consts(S, i);
-        const Feat e = edge_feat(S, pi, __ldg(S.n + i), j, kc);
+    auto feat = [&](uint32_t t, uint32_t i, float& x) {
+        x = A.dgval[(size_t)j * LP_GW + t];  // transposed: dG of (i, j)
+        return edge_feat(S, __ldg(S.pos + i), __ldg(S.n + i), j, lp_consts(S, i));
+    };
+    for_edges(A.scols + (size_t)j * LP_GW, A.nlow[j], cnt, feat, [&](uint32_t, uint32_t i, const Feat& e, float dg) {
         float s0 = A.ra[(size_t)i * LP_H + lane] + br0 + rbj0;
         float s1 = A.ra[(size_t)i * LP_H + lane + 32] + br1 + rbj1;
 #pragma unroll
@@ -528,63 +627,80 @@ __global__ void __launch_bounds__(256) k_lp_readout_bwd_b(BwdArgs A) {
         float d0, d1;
         gelu_t(s0, &d0);
         gelu_t(s1, &d1);
-        const float dg = A.dgval[(size_t)j * LP_GW + t];  // transposed: dG of (i, j)
         drb0 += dg * om0 * d0;
         drb1 += dg * om1 * d1;
-    }
+    });
     A.drb[(size_t)j * LP_H + lane] = drb0;
     A.drb[(size_t)j * LP_H + lane + 32] = drb1;
 }
 
-// dense backward on every row: dx (+)= W^T dy, dW += dy x^T, db += dy
+// dense backward on every row: dx (+)= W^T dy, dW += dy x^T, db += dy.  dW
+// is summed over a tile's rows, the tiles' sums over the block, and the
+// blocks' sums with atomics.
 __global__ void __launch_bounds__(256) k_lp_dense_bwd(const float* __restrict__ dy, const float* __restrict__ x,
                                                       const __nv_bfloat16* __restrict__ w, int woff, float* __restrict__ dx,
                                                       int accumulate, float* __restrict__ grad, int boff,
                                                       const uint32_t* __restrict__ rowlist,
                                                       const uint32_t* __restrict__ nrows) {
-    __shared__ float W[LP_H][LP_H + 1];
-    __shared__ float dW[LP_H][LP_H + 1];
-    __shared__ float dys[4][LP_H], xs[4][LP_H];
+    __shared__ __align__(16) __nv_bfloat16 W[LP_H][LP_H];  // [output][input]
+    __shared__ __align__(16) float dys[DT][DT_LD], xs[DT][DT_LD];
+    __shared__ uint32_t idx[DT];
     const uint32_t R = *nrows;
-    for (int t = threadIdx.x; t < LP_H * LP_H; t += blockDim.x) {
-        W[t / LP_H][t % LP_H] = wbf(w, woff + t);
-        dW[t / LP_H][t % LP_H] = 0.f;
-    }
-    const int r = threadIdx.x >> 6, c = threadIdx.x & 63;
+    for (int t = threadIdx.x; t < LP_H * LP_H; t += blockDim.x) W[t / LP_H][t % LP_H] = w[woff + t];
+    const int q = threadIdx.x & 15, r0 = 4 * (threadIdx.x >> 4);
+    float dw[4][4] = {};  // outputs r0 + a, inputs 4 q + b
     float db = 0.f;
-    for (uint32_t k0 = blockIdx.x * 4; k0 < R; k0 += gridDim.x * 4) {
+    for (uint32_t k0 = blockIdx.x * DT; k0 < R; k0 += gridDim.x * DT) {
         __syncthreads();
-        const uint32_t k = k0 + r;
-        const uint32_t i = k < R ? __ldg(rowlist + k) : 0u;
-        dys[r][c] = k < R ? dy[(size_t)i * LP_H + c] : 0.f;
-        xs[r][c] = k < R ? x[(size_t)i * LP_H + c] : 0.f;
+        dense_rows(idx, k0, R, rowlist);
         __syncthreads();
-        if (k < R && dx) {
-            float s = 0.f;
-#pragma unroll 16
-            for (int o = 0; o < LP_H; o++) s = fmaf(W[o][c], dys[r][o], s);
-            if (accumulate) dx[(size_t)i * LP_H + c] += s;
-            else dx[(size_t)i * LP_H + c] = s;
+        dense_stage(dys, dy, idx);
+        dense_stage(xs, x, idx);
+        __syncthreads();
+        if (dx) {
+            float acc[4][4] = {};
+            dense_mul(dys, W, r0, q, acc);
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const uint32_t i = idx[r0 + a];
+                if (i == 0xffffffffu) continue;
+                float4* o = reinterpret_cast<float4*>(dx + (size_t)i * LP_H + 4 * q);
+                float4 v = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+                if (accumulate) {
+                    const float4 z = *o;
+                    v = make_float4(z.x + v.x, z.y + v.y, z.z + v.z, z.w + v.w);
+                }
+                *o = v;
+            }
         }
-        // dW[o][c'] for o = threadIdx.x / 4 .. : 256 threads x 16 entries
-        const int o = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
+        float t[4][4] = {};
+#pragma unroll 8
+        for (int r = 0; r < DT; r++) {
+            const float4 d = *reinterpret_cast<const float4*>(&dys[r][r0]);
+            const float4 v = *reinterpret_cast<const float4*>(&xs[r][4 * q]);
+            const float dv[4] = {d.x, d.y, d.z, d.w}, xv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int cc = 0; cc < 16; cc++) {
-            float s = 0.f;
+            for (int a = 0; a < 4; a++)
 #pragma unroll
-            for (int rr = 0; rr < 4; rr++) s = fmaf(dys[rr][o], xs[rr][c0 + cc], s);
-            dW[o][c0 + cc] += s;
+                for (int b = 0; b < 4; b++) t[a][b] = fmaf(dv[a], xv[b], t[a][b]);
         }
-        if (r == 0) {
 #pragma unroll
-            for (int rr = 0; rr < 4; rr++) db += dys[rr][c];
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int b = 0; b < 4; b++) dw[a][b] += t[a][b];
+        if (boff >= 0 && threadIdx.x < LP_H) {
+            float sum = 0.f;
+#pragma unroll 8
+            for (int r = 0; r < DT; r++) sum += dys[r][threadIdx.x];
+            db += sum;
         }
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < LP_H * LP_H; t += blockDim.x) atomicAdd(grad + woff + t, dW[t / LP_H][t % LP_H]);
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) atomicAdd(grad + woff + (r0 + a) * LP_H + 4 * q + b, dw[a][b]);
     if (boff >= 0 && threadIdx.x < LP_H) atomicAdd(grad + boff + threadIdx.x, db);
 }
-
 // elementwise: out = dh * GELU'(pre)
 __global__ void __launch_bounds__(256) k_lp_gelu_bwd(const float* __restrict__ dh, const float* __restrict__ pre,
                                                      float* __restrict__ out, const uint32_t* __restrict__ rowlist,
@@ -642,9 +758,8 @@ __global__ void __launch_bounds__(256) k_lp_edge_bwd_a(BwdArgs A) {
         const uint32_t cnt = A.scnt[i];
         const float inv = cnt ? 1.f / (float)cnt : 0.f;
         const float da0 = A.da[(size_t)i * LP_H + lane] * inv, da1 = A.da[(size_t)i * LP_H + lane + 32] * inv;
-        for (uint32_t t = 0; t < cnt; t++) {
-            const uint32_t j = A.scols[(size_t)i * LP_GW + t];
-            const Feat e = edge_feat(S, pi, ni, j, kc);
+        auto feat = [&](uint32_t, uint32_t j, float&) { return edge_feat(S, pi, ni, j, kc); };
+        for_edges(A.scols + (size_t)i * LP_GW, 0u, cnt, feat, [&](uint32_t, uint32_t j, const Feat& e, float) {
             float s0 = b0, s1 = b1;
 #pragma unroll
             for (int f = 0; f < LP_F; f++) {
@@ -666,7 +781,7 @@ __global__ void __launch_bounds__(256) k_lp_edge_bwd_a(BwdArgs A) {
             }
             gb0 += ds0;
             gb1 += ds1;
-        }
+        });
     }
 #pragma unroll
     for (int f = 0; f < LP_F; f++) {
@@ -698,13 +813,12 @@ __global__ void __launch_bounds__(256) k_lp_edge2_bwd_b(BwdArgs A, float* __rest
     const float b1 = wbf(A.w, LP_B2 + lane + 32) + A.uh1[(size_t)j * LP_H + lane + 32];
     float acc0 = 0.f, acc1 = 0.f;
     const uint32_t cnt = A.scnt[j];
-    for (uint32_t t = 0; t < cnt; t++) {
-        const uint32_t i = A.scols[(size_t)j * LP_GW + t];
+    auto feat = [&](uint32_t, uint32_t i, float& x) {
         const uint32_t ci = A.scnt[i];
-        const float inv = ci ? 1.f / (float)ci : 0.f;
-        const float4 pi = __ldg(S.pos + i);
-        const float2 kc = lp_consts(S, i);
-        const Feat e = edge_feat(S, pi, __ldg(S.n + i), j, kc);
+        x = ci ? 1.f / (float)ci : 0.f;
+        return edge_feat(S, __ldg(S.pos + i), __ldg(S.n + i), j, lp_consts(S, i));
+    };
+    for_edges(A.scols + (size_t)j * LP_GW, 0u, cnt, feat, [&](uint32_t, uint32_t i, const Feat& e, float inv) {
         float s0 = b0, s1 = b1;
 #pragma unroll
         for (int f = 0; f < LP_F; f++) {
@@ -716,7 +830,7 @@ __global__ void __launch_bounds__(256) k_lp_edge2_bwd_b(BwdArgs A, float* __rest
         gelu_t(s1, &d1);
         acc0 += A.da[(size_t)i * LP_H + lane] * inv * d0;
         acc1 += A.da[(size_t)i * LP_H + lane + 32] * inv * d1;
-    }
+    });
     duh1[(size_t)j * LP_H + lane] = acc0;
     duh1[(size_t)j * LP_H + lane + 32] = acc1;
 }
@@ -1283,8 +1397,8 @@ void lp_forward(LearnedWork& L, const LpSystem& S, bool exact, uint32_t cap, cud
                 bool keep_pre) {
     (void)exact;
     const uint32_t wb = blocks_for(cap * 32u, 256);   // warp per row
-    const uint32_t db = blocks_for(cap, 4);           // 4 rows per dense block
-    const uint32_t dgrid = db < 148u * 8u ? db : 148u * 8u;
+    const uint32_t db = blocks_for(cap, DT);          // tiles of the dense layers
+    const uint32_t dgrid = db < 148u * 4u ? db : 148u * 4u;
     const uint32_t tgrid = tensor_cores ? tc_grids(cap).dense : 0u;
     uint32_t* err = const_cast<uint32_t*>(&S.sc->err);
     auto dense = [&](const float* x, int woff, int boff, const float* resid, float* pre, float* out, int act) {
@@ -1372,8 +1486,8 @@ int lp_loss_grad(LearnedWork& L, const LpSystem& S, bool exact, uint64_t seed, u
     const bool tc = L.train_tensor_cores;
     lp_forward(L, S, exact, cap, st, tc, true);
     const uint32_t tb = blocks_for(cap, 256), wb = blocks_for(cap * 32u, 256);
-    const uint32_t db = blocks_for(cap, 4);
-    const uint32_t dgrid = db < 148u * 8u ? db : 148u * 8u;
+    const uint32_t db = blocks_for(cap, DT);
+    const uint32_t dgrid = db < 148u * 3u ? db : 148u * 3u;
     const TcGrids tg = tc ? tc_grids(cap) : TcGrids{0u, 0u};
     uint32_t* err = const_cast<uint32_t*>(&S.sc->err);
     // dx (+)= W^T dy, grad(W) += dy x^T, grad(b) += dy (boff >= 0)
