@@ -106,16 +106,16 @@ typedef struct {
                             particles can move (fluid and moving walls), else
                             a full radix sort; -1 = always the full sort.  Both
                             give the same stable order.                       */
-    int ppe_layout;      /* PPE matrix in the solver: 0 = compact (rows
-                            numbered densely, 16-bit column codes, 6 bytes
-                            per entry) for single scenes with diagonal
-                            scaling, else the 8-byte layout; -1 = always the
-                            8-byte layout.  Same matrix either way;
-                            mps_autotune may change it.                       */
-    int ppe_smem_chunks; /* 128-entry chunks of the matrix each warp keeps
-                            in shared memory across CG iterations (0: 8;
-                            -1: none; at most 8 in the compact layout, 6 in
-                            the 8-byte layout with stored weights)           */
+    int ppe_layout;      /* PPE matrix in the solver: 0 = compact (tiles of
+                            neighbouring rows, 16-bit codes into each tile's
+                            list of columns, 6 bytes per entry); -1 = always
+                            the 8-byte layout.  Same matrix either way;
+                            mps_autotune may change a single scene's.         */
+    int ppe_smem_chunks; /* 128-entry chunks of the matrix kept in shared
+                            memory across CG iterations, per each of an SM's
+                            32 warps (0: 8; -1: none; at most 8 in the
+                            compact layout, 6 in the 8-byte layout with
+                            stored weights)                                  */
     int precond_every;   /* learned preconditioner (every layout, batches
                             too): steps between two evaluations of the
                             network; between them the symmetric form of the
@@ -216,8 +216,9 @@ mps_status mps_get_grid(mps_handle* h, mps_grid* g);
  * cg relative residual, step, status, number of cells, kernels launched by
  * one step, FP64 residual passes of the last PPE solve, 1 when steps replay
  * a captured CUDA graph (0: direct launches), and the matrix entries of the
- * last PPE assembly whose column did not fit the compact layout's 16-bit
- * code (-1 when the solver uses the 8-byte layout). */
+ * last PPE assembly whose column lies beyond a 16-bit offset from their own
+ * rows in the compact layout's numbering (reached through the tile's column
+ * list; -1 when the solver uses the 8-byte layout). */
 mps_status mps_get_scalars(mps_handle* h, double out16[16]);
 /* i_normal as GEO.dat indices: for each particle (by GEO index) the GEO index
  * of its wall particle (itself when it has none), np0 entries. */
@@ -459,9 +460,10 @@ typedef struct mps_tune_report {
     /* PPE solve ms per step: [3 f + t] for form f (0 stored, 1 recomputed,
      * 2 pipelined) at 1024, 512, 256 threads per block (-1: not run) */
     float ppe_ms[9];
-    int ppe_compact;           /* chosen: 1 the compact 16-bit layout        */
-    float ppe_compact_ms[3];   /* its PPE solve ms per step at 1024, 512, 256
-                                  threads per block (-1: not run)            */
+    int ppe_compact;           /* chosen: 1 the compact 16-bit layout (a batch
+                                  keeps the layout of its options: 0)        */
+    float ppe_compact_ms[3];   /* its PPE solve ms per step: it has one shape,
+                                  reported first (-1: not run)               */
 } mps_tune_report;
 mps_status mps_autotune(mps_handle* h, int steps, mps_tune_report* report);
 /* Apply the choices of a report (the chosen fields: stage_threads,

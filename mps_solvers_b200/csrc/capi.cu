@@ -381,6 +381,18 @@ static int walk_reach(float cell_size, float cell_yz) {
     return cell_yz < cell_size ? (int)std::ceil((double)cell_size / (double)cell_yz - 1e-9) : 1;
 }
 
+// options.ppe_l2_keep_mb in 8-byte matrix entries
+static uint32_t l2_keep_entries(const mps_options& opt) {
+    if (opt.ppe_l2_keep_mb < 0) return 0xFFFFFFFFu;
+    size_t keep_bytes = (size_t)opt.ppe_l2_keep_mb << 20;
+    if (opt.ppe_l2_keep_mb == 0) {  // half the L2: the best of a sweep at 310,912 particles
+        int l2 = 0;
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, opt.device);
+        keep_bytes = (size_t)l2 / 2;
+    }
+    return (uint32_t)(keep_bytes / 8);
+}
+
 // the fluid list's capacity: every fluid particle, and one gap for each warp
 // of a gather over cap particles (blocks of 256) that can hold fluid
 static uint32_t fluid_list_cap(uint32_t nfluid, uint32_t cap) {
@@ -566,13 +578,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         int e = ppe_setup(h->ppe, h->cap, h->g, h->P, h->prm, h->stream, &h->err);
         if (e != MPS_OK) return (mps_status)e;
         h->ppe.pipelined = h->opt.ppe_pipelined != 0;
-        size_t keep_bytes = (size_t)h->opt.ppe_l2_keep_mb << 20;
-        if (h->opt.ppe_l2_keep_mb == 0) {  // half the L2: the best of a sweep at 310,912 particles
-            int l2 = 0;
-            cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->opt.device);
-            keep_bytes = (size_t)l2 / 2;
-        }
-        h->ppe.l2_keep_entries = h->opt.ppe_l2_keep_mb < 0 ? 0xFFFFFFFFu : (uint32_t)(keep_bytes / 8);
+        h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
         if (h->opt.precond == MPS_PRECOND_LEARNED) {
             e = ppe_enable_learned(h->ppe, &h->err);
             if (e == MPS_OK) e = ppe_sp_enable(h->ppe, &h->err);
@@ -585,8 +591,8 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         h->ppe.c16_smem_chunks = h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
         h->ppe.precond_every = h->opt.precond_every > 0 ? h->opt.precond_every : 40;
         h->ppe.index_of_id = h->index_of_id;
-        if (h->opt.ppe_layout == 0 && !h->nscenes && ppe_c16_takes(h->cap, h->g)) {
-            e = ppe_c16_enable(h->ppe, h->g, &h->err);
+        if (h->opt.ppe_layout == 0 && ppe_c16_takes(h->cap, &h->g, 1)) {
+            e = ppe_c16_enable(h->ppe, &h->g, 1, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
             set_compact(h, true);
@@ -892,6 +898,15 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
             e = ppe_enable_learned(h->ppe, &h->err);
             if (e == MPS_OK) e = ppe_sp_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
+        }
+        if (h->opt.ppe_layout == 0 && ppe_c16_takes(cap, h->scene_grid.data(), S)) {
+            h->ppe.c16_smem_chunks =
+                h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
+            e = ppe_c16_enable(h->ppe, h->scene_grid.data(), S, &h->err);
+            if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
+            if (e != MPS_OK) return (mps_status)e;
+            h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
+            set_compact(h, true);
         }
     }
     Scalars sc;
@@ -1668,11 +1683,12 @@ extern "C" mps_status mps_autotune(mps_handle* h, int steps, mps_tune_report* re
         ppe_set_threads(h->ppe, best_p);
         h->ppe.stored_weights = best_sw;
         h->ppe.pipelined = best_pipe;
+        if (h->nscenes) best_c16 = h->ppe.c16_ready;  // a batch keeps the layout of its options
         set_compact(h, best_c16);
         r.ppe_threads = best_p;
         r.ppe_stored_weights = best_sw ? 1 : 0;
         r.ppe_pipelined = best_pipe ? 1 : 0;
-        r.ppe_compact = best_c16 ? 1 : 0;
+        r.ppe_compact = best_c16 && !h->nscenes ? 1 : 0;
     }
     drop_graphs(h);
     if (rep) *rep = r;
@@ -1692,7 +1708,7 @@ extern "C" mps_status mps_apply_tuning(mps_handle* h, const mps_tune_report* r) 
                 h->err = "the compact PPE layout is for single scenes";
                 return MPS_ERR_INVALID;
             }
-            int e = ppe_c16_enable(h->ppe, h->g, &h->err);
+            int e = ppe_c16_enable(h->ppe, &h->g, 1, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
         }
@@ -1706,7 +1722,7 @@ extern "C" mps_status mps_apply_tuning(mps_handle* h, const mps_tune_report* r) 
         }
         h->ppe.stored_weights = r->ppe_stored_weights != 0;
         h->ppe.pipelined = r->ppe_pipelined != 0;
-        set_compact(h, r->ppe_compact != 0);
+        set_compact(h, h->nscenes ? h->ppe.c16_ready : r->ppe_compact != 0);
     }
     drop_graphs(h);
     return MPS_OK;

@@ -64,6 +64,18 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
     if (blockIdx.x == 0 && threadIdx.x == 0) A.bar[0] = 0u;  // the solver's barrier starts empty
     if (k >= (C16 ? *A.nrows : n)) return;
     const uint32_t i = C16 ? __ldg(A.rowlist + k) : k;
+    if (C16 && BT && i == PPE_DIRICHLET) {  // a gap between two scenes' rows: an identity row with b = 0
+        if (lane == 0) {
+            A.clen[k] = 0;
+            A.cdiag64[k] = -1.0;
+            A.cdiag32[k] = -1.f;
+            A.cinv_diag[k] = -1.f;
+            A.cdsq[k] = 1.f;
+            A.cb64[k] = 0.0;
+            A.cx64[k] = 0.0;
+        }
+        return;
+    }
     const float4* __restrict__ pos = a.cur.pos;
     const float* __restrict__ nn = a.cur.n;
     const float4 pi = pos[i];
@@ -1642,8 +1654,8 @@ int ppe_enqueue_setup(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     A.rho_lambda_alpha_n0 = rho * w.lambda64 * alpha * w.n0_64;
     A.dim2 = 2.0 * dim;
     A.scenes = w.scenes;
-    A.rowlist = w.rowlist;
-    A.nrows = w.nrows;
+    A.rowlist = ppe_c16_rowlist(w);
+    A.nrows = ppe_c16_nrows(w);
     A.cpos = w.cpos;
     A.clen = w.clen;
     A.cb64 = w.cb64;
@@ -1652,13 +1664,18 @@ int ppe_enqueue_setup(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     A.cdiag32 = w.cdiag32;
     A.cinv_diag = w.cinv_diag;
     A.cdsq = w.cdsq;
-    const bool c16 = w.c16 && !a.batch.n;
-    const uint32_t warps_blocks = blocks_for((c16 ? a.cap_solid : cap) * 32u, 256);
+    const bool c16 = w.c16;
+    const uint32_t warps_blocks = blocks_for((c16 ? a.cap_solid + 8u * w.nscenes : cap) * 32u, 256);
     int launched = 1;
     if (c16) {
         launched += ppe_c16_enqueue_rows(w, a, A.beta * A.n0, st);
-        if (a.exact) k_ppe_assemble<true, false, true><<<warps_blocks, 256, 0, st>>>(A);
-        else k_ppe_assemble<false, false, true><<<warps_blocks, 256, 0, st>>>(A);
+        if (a.batch.n) {
+            if (a.exact) k_ppe_assemble<true, true, true><<<warps_blocks, 256, 0, st>>>(A);
+            else k_ppe_assemble<false, true, true><<<warps_blocks, 256, 0, st>>>(A);
+        } else {
+            if (a.exact) k_ppe_assemble<true, false, true><<<warps_blocks, 256, 0, st>>>(A);
+            else k_ppe_assemble<false, false, true><<<warps_blocks, 256, 0, st>>>(A);
+        }
     } else if (a.batch.n) {
         if (a.exact) k_ppe_assemble<true, true, false><<<warps_blocks, 256, 0, st>>>(A);
         else k_ppe_assemble<false, true, false><<<warps_blocks, 256, 0, st>>>(A);
@@ -1699,7 +1716,7 @@ LpSystem ppe_lp_system(const PpeWork& w, const StageArgs& a) {
     L.rowlist = w.rowlist;
     L.nrows = w.nrows;
     L.acols = w.cols;
-    L.acols_by_row = w.c16 && !a.batch.n;
+    L.acols_by_row = w.c16;
     L.cell = a.cur.cell;
     L.cell_start = a.cell_start;
     L.g = a.g;
@@ -1760,6 +1777,8 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     // PPE_SMEM_CHUNKS, 192 KB for the 32 warps of an SM
     S.smem_chunks = w.stored_weights ? (w.c16_smem_chunks < PPE_SMEM_CHUNKS ? w.c16_smem_chunks : PPE_SMEM_CHUNKS) : 0;
     if (S.smem_chunks < 0) S.smem_chunks = 0;
+    const bool learned = opt.precond == MPS_PRECOND_LEARNED && w.lp.ready && w.sp_ent;
+    if (w.c16 && (!learned || w.c16_learned)) return ppe_c16_enqueue_solve(w, a, opt, cap, st);
     if (a.batch.n) {
         BatchSolveArgs B;
         B.rowlist = w.rowlist;
@@ -1799,9 +1818,8 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
         B.rq0 = w.rq[0];
         B.rq1 = w.rq[1];
         void* bargs[] = {&B};
-        const bool blearned = opt.precond == MPS_PRECOND_LEARNED && w.lp.ready && w.sp_ent;
         const void* bfn;
-        if (blearned)
+        if (learned)
             bfn = w.stored_weights ? (a.exact ? (const void*)k_ppe_solve_batch<true, true, 1>
                                               : (const void*)k_ppe_solve_batch<false, true, 1>)
                                    : (a.exact ? (const void*)k_ppe_solve_batch<true, false, 1>
@@ -1816,8 +1834,6 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
         k_ppe_finish<<<blocks_for(cap, 256), 256, 0, st>>>(w.x64, w.rlen, a.cur.press, a.sc);
         return 2;
     }
-    const bool learned = opt.precond == MPS_PRECOND_LEARNED && w.lp.ready && w.sp_ent;
-    if (w.c16 && (!learned || w.c16_learned)) return ppe_c16_enqueue_solve(w, a, opt, cap, st);
     if (w.pipelined && !learned) {
         PipeArgs Pa;
         Pa.rowlist = w.rowlist;

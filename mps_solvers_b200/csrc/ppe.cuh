@@ -88,7 +88,7 @@ struct PpeWork {
     double* scene_relres = nullptr;
     // compact layout (ppe_compact.cu): rows numbered along a Hilbert curve
     // over the linked cells, tiles of consecutive rows with a column list
-    // each, 16-bit codes into it beside FP32 weights; single scenes
+    // each, 16-bit codes into it beside FP32 weights
     bool c16 = false;                  // the solve uses this layout
     bool c16_ready = false;            // its buffers exist
     int c16_smem_chunks = 8;           // chunks per warp held in shared memory across iterations
@@ -108,6 +108,15 @@ struct PpeWork {
     float *cdiag32 = nullptr, *cinv_diag = nullptr, *cr = nullptr, *cp = nullptr;
     float* cdsq = nullptr;             // 1 / sqrt(-diagonal)
     float4* cpub[2] = {nullptr, nullptr};  // what the other blocks read of a row, two buffers
+    // a batch: the scenes' linked cells and rows, its own row list with the
+    // scenes' starts at multiples of 8, the scenes' first tiles, tile sums
+    uint32_t* c16_dense = nullptr;
+    uint32_t* c16_sfirst = nullptr;
+    uint32_t* c16_srow = nullptr;
+    uint32_t* c16_tb = nullptr;
+    uint32_t* c16_rowlist = nullptr;
+    uint32_t* c16_nrows = nullptr;
+    double* c16_tsum = nullptr;
     ulonglong2* c16_slots = nullptr;   // the solver's grid sums
     unsigned long long* c16_epoch = nullptr;  // and the epochs its launches have used
     // the learned S' in the tiles' codes (code << 16 | BF16 value): the
@@ -166,8 +175,10 @@ int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint3
 // The compact 16-bit layout and its persistent solver (ppe_compact.cu):
 // whether it takes a grid and capacity, buffers, the pack after the assembly, the solve with p = max(x, 0), the
 // escaped-entry count of the last pack, and the stencil export.
-bool ppe_c16_takes(uint32_t cap, const Grid& grid);
-int ppe_c16_enable(PpeWork& w, const Grid& grid, std::string* err);
+bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids);
+int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* err);
+const uint32_t* ppe_c16_rowlist(const PpeWork& w);
+const uint32_t* ppe_c16_nrows(const PpeWork& w);
 // the row numbers, before the assembly (bthr = beta n0; a batch uses its
 // scenes' own)
 int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st);

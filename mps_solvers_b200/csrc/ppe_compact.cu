@@ -67,15 +67,18 @@ constexpr uint32_t C16_STATS = 4;
 constexpr uint32_t C16_SP_SLICES = C16_COLS / 32 + 1;  // S' slices (32 rows) a tile can have, and one
 
 // One tile: slices [s0, s1), its columns (its own rows first, then the others
-// in ascending order), whether entries are escaped, and its longest slice.
+// in ascending order), whether entries are escaped, its longest slice and,
+// in a batch, its scene.
 struct C16Tile {
-    uint32_t s0, s1, ncol, esc, wmax, pad[3];
+    uint32_t s0, s1, ncol, esc, wmax, scene, pad[2];
 };
 
-// Tiles of R rows for G solver blocks: the same number for every block.
-__host__ __device__ __forceinline__ uint32_t c16_tiles(uint32_t R, uint32_t G) {
-    const uint32_t per = G * C16_TILE_ROWS;
-    const uint32_t k = (R + per - 1) / per;
+// Tiles of R rows for G solver blocks: the same number for every block.  The
+// scenes of a batch (ns, 0 for a single scene) have tiles of their own; one
+// tile of each is spoken for before the rows are shared out.
+__host__ __device__ __forceinline__ uint32_t c16_tiles(uint32_t R, uint32_t G, uint32_t ns) {
+    const uint32_t t = (R + C16_TILE_ROWS - 1) / C16_TILE_ROWS + ns;
+    const uint32_t k = (t + G - 1) / G;
     return G * (k > 0 ? k : 1u);
 }
 
@@ -123,36 +126,94 @@ __global__ void __launch_bounds__(256) k_c16_count(C16Flag F, const uint32_t* __
     if (lane == 0) base[h] = n;  // base[nsuper] = 0: the scan leaves R there
 }
 
-// After the scan: row numbers and the row list.  A particle without a row
-// gets the identity row of the particle-indexed arrays.
-__global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, const uint32_t* __restrict__ cells, uint32_t nsuper,
-                                                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ base,
-                                                  uint32_t* __restrict__ cpos, uint32_t* __restrict__ rowlist,
-                                                  uint32_t* __restrict__ nrows, uint32_t* __restrict__ rlen,
-                                                  double* __restrict__ diag64) {
+// A batch: the scenes' rows start at multiples of 8, so that no slice (and no
+// tile) spans two scenes.  dense: the scanned counts; base: the linked
+// cells' first rows with the scenes' starts moved up; srow: the scenes'
+// first rows and the end.  The up to 7 places left at a scene's end have no
+// row (C16_NONE in the row list).
+__global__ void __launch_bounds__(256) k_c16_shift(const uint32_t* __restrict__ dense, uint32_t nsuper,
+                                                   const uint32_t* __restrict__ sfirst, uint32_t ns,
+                                                   uint32_t* __restrict__ base, uint32_t* __restrict__ srow,
+                                                   uint32_t* __restrict__ rowlist, uint32_t* __restrict__ nrows) {
+    __shared__ uint32_t first[PPE_MAX_SCENES + 1], at[PPE_MAX_SCENES + 1];
+    for (uint32_t x = threadIdx.x; x <= ns; x += blockDim.x) first[x] = sfirst[x];
+    if (threadIdx.x < 32) {
+        uint32_t carry = 0;
+        for (uint32_t s0 = 0; s0 < ns; s0 += 32) {
+            const uint32_t s = s0 + threadIdx.x;
+            const uint32_t v = s < ns ? (dense[sfirst[s + 1]] - dense[sfirst[s]] + 7u) & ~7u : 0u;
+            uint32_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+                if ((int)threadIdx.x >= o) x += t;
+            }
+            if (s < ns) at[s] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (threadIdx.x == 0) at[ns] = carry;
+    }
+    __syncthreads();
+    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h <= nsuper) {
+        uint32_t lo = 0, hi = ns;  // the scene of cell h (past the last: the end)
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (first[mid] <= h) lo = mid;
+            else hi = mid;
+        }
+        base[h] = h == nsuper ? at[ns] : dense[h] - dense[first[lo]] + at[lo];
+    }
+    if (blockIdx.x == 0) {
+        for (uint32_t s = threadIdx.x; s <= ns; s += blockDim.x) {
+            srow[s] = at[s];
+            if (s < ns)
+                for (uint32_t k = at[s] + dense[first[s + 1]] - dense[first[s]]; k < at[s + 1]; k++) rowlist[k] = C16_NONE;
+        }
+        if (threadIdx.x == 0) *nrows = at[ns];
+    }
+}
+
+// After the scan: row numbers and the row list (in a batch also the list
+// without the scenes' gaps, of dense_n rows).  A particle without a row gets
+// the identity row of the particle-indexed arrays.
+struct C16RowArgs {
+    const uint32_t *cells, *cs, *base;
+    uint32_t nsuper;
+    const uint32_t* dense;  // batch: first row of every linked cell without the gaps
+    uint32_t *cpos, *rowlist, *nrows, *dense_list, *dense_n, *rlen;
+    double* diag64;
+};
+
+__global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, C16RowArgs A) {
     const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
-    if (h >= nsuper) return;
-    uint32_t at = base[h];
-    const uint4 c4 = *reinterpret_cast<const uint4*>(cells + 4 * (size_t)h);
+    if (h >= A.nsuper) return;
+    uint32_t at = A.base[h];
+    const uint32_t dd = A.dense ? at - A.dense[h] : 0u;  // gaps before this cell
+    const uint4 c4 = *reinterpret_cast<const uint4*>(A.cells + 4 * (size_t)h);
     const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
-    if (h == nsuper - 1 && lane == 0) *nrows = base[nsuper];
+    if (h == A.nsuper - 1 && lane == 0) {
+        if (A.dense) *A.dense_n = A.dense[A.nsuper];
+        else *A.nrows = A.base[A.nsuper];
+    }
 #pragma unroll
     for (int u = 0; u < 4; u++) {
         if (c[u] == C16_NONE) continue;
-        const uint32_t lo = cs[c[u]], hi = cs[c[u] + 1];
+        const uint32_t lo = A.cs[c[u]], hi = A.cs[c[u] + 1];
         for (uint32_t i0 = lo; i0 < hi; i0 += 32) {
             const uint32_t i = i0 + lane;
             const bool f = i < hi && c16_is_row(F, i);
             const uint32_t m = __ballot_sync(0xffffffffu, f);
             if (f) {
                 const uint32_t k = at + __popc(m & lt);
-                cpos[i] = k;
-                rowlist[k] = i;
+                A.cpos[i] = k;
+                A.rowlist[k] = i;
+                if (A.dense) A.dense_list[k - dd] = i;
             } else if (i < hi) {
-                cpos[i] = C16_NONE;
-                rlen[i] = PPE_DIRICHLET;
-                diag64[i] = 1.0;
+                A.cpos[i] = C16_NONE;
+                A.rlen[i] = PPE_DIRICHLET;
+                A.diag64[i] = 1.0;
             }
             at += __popc(m);
         }
@@ -169,6 +230,63 @@ __global__ void __launch_bounds__(256) k_c16_width(const uint32_t* __restrict__ 
     for (int o = 1; o < (int)C16_ROWS; o <<= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
     const uint32_t s = k / C16_ROWS;
     if (k % C16_ROWS == 0 && s <= maxslices) width[s] = (len + 15u) / 16u;
+}
+
+// Weight of the slices before s when tiles are cut.
+__device__ __forceinline__ uint64_t c16_weight(const uint32_t* __restrict__ off, uint32_t s) {
+    return (uint64_t)__ldg(off + s) + (uint64_t)C16_SLICE_COST * s;
+}
+
+// A batch's tiles: tb[s] = first tile of scene s, tb[ns] = all of them.  One
+// tile a scene, the rest by weight, what rounding leaves to the scenes with
+// the heaviest tiles.
+__global__ void __launch_bounds__(32) k_c16_cut(const uint32_t* __restrict__ off, const uint32_t* __restrict__ srow,
+                                                const uint32_t* __restrict__ nrows, uint32_t ns, uint32_t G,
+                                                uint32_t* __restrict__ tb) {
+    constexpr uint32_t PER = PPE_MAX_SCENES / 32;
+    const uint32_t lane = threadIdx.x, R = *nrows, T = c16_tiles(R, G, ns);
+    const double W = (double)c16_weight(off, R / C16_ROWS);
+    double w[PER];
+    uint32_t n[PER], given = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < PER; u++) {
+        const uint32_t s = u * 32 + lane;
+        w[u] = s < ns ? (double)(c16_weight(off, srow[s + 1] / C16_ROWS) - c16_weight(off, srow[s] / C16_ROWS)) : -1.0;
+        n[u] = s < ns ? 1u + (W > 0.0 ? (uint32_t)((double)(T - ns) * (w[u] / W)) : 0u) : 0u;
+        given += n[u];
+    }
+    given = __reduce_add_sync(0xffffffffu, given);
+    for (; given < T; given++) {
+        double most = -2.0;
+        uint32_t at = 0;
+#pragma unroll
+        for (uint32_t u = 0; u < PER; u++) {
+            const double load = n[u] ? w[u] / n[u] : -2.0;
+            if (load > most) { most = load; at = u * 32 + lane; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double m2 = __shfl_xor_sync(0xffffffffu, most, o);
+            const uint32_t a2 = __shfl_xor_sync(0xffffffffu, at, o);
+            if (m2 > most || (m2 == most && a2 < at)) { most = m2; at = a2; }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < PER; u++)
+            if (at == u * 32 + lane) n[u]++;
+    }
+    uint32_t carry = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < PER; u++) {
+        uint32_t x = n[u];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)lane >= o) x += t;
+        }
+        if (u * 32 + lane <= ns) tb[u * 32 + lane] = carry + x - n[u];
+        carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) tb[ns] = carry;
 }
 
 // ---------------------------------------------------------------- pack
@@ -198,6 +316,9 @@ struct C16PackArgs {
     const uint32_t* base;     // first row of every linked cell
     const uint32_t* nbr;      // 27 linked cells around each (C16_NONE: outside)
     uint32_t nsuper, blocks;
+    uint32_t ns;              // scenes of a batch (0: a single scene)
+    const uint32_t* srow;     // their first rows
+    const uint32_t* tb;       // and first tiles
     C16Tile* tiles;
     uint32_t* collist;        // C16_COLS per tile
     unsigned char* ent;
@@ -265,24 +386,32 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
     __shared__ uint32_t ws[32], found[4];
     const uint32_t R = *A.nrows;
     const uint32_t nsl = (R + C16_ROWS - 1) / C16_ROWS;
-    const uint32_t T = c16_tiles(R, A.blocks);
+    const uint32_t T = c16_tiles(R, A.blocks, A.ns);
     const uint32_t t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
     const uint32_t lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     if (t >= T) return;
-    // equal shares of the chunks, a slice counting C16_SLICE_COST more
-    const uint64_t W = (uint64_t)A.off[nsl] + (uint64_t)C16_SLICE_COST * nsl;
+    // equal shares of the chunks of the tile's scene, a slice counting
+    // C16_SLICE_COST more
+    uint32_t scene = 0, t0 = 0, t1 = T, lo = 0, hi = nsl;
+    if (A.ns) {
+        scene = warp_lower(A.ns, (uint64_t)t + 1, [&](uint32_t x) { return (uint64_t)__ldg(A.tb + x); }) - 1;
+        t0 = __ldg(A.tb + scene);
+        t1 = __ldg(A.tb + scene + 1);
+        lo = __ldg(A.srow + scene) / C16_ROWS;
+        hi = __ldg(A.srow + scene + 1) / C16_ROWS;
+    }
     if (warp < 2) {
-        const uint32_t s = warp_lower(nsl, W * (t + warp) / T, [&](uint32_t x) {
-            return (uint64_t)__ldg(A.off + x) + (uint64_t)C16_SLICE_COST * x;
-        });
-        if (lane == 0) found[warp] = t + warp == T ? nsl : s;
+        const uint64_t w0 = c16_weight(A.off, lo), w1 = c16_weight(A.off, hi);
+        const uint32_t s = warp_lower(nsl, w0 + (w1 - w0) * (t - t0 + warp) / (t1 - t0),
+                                      [&](uint32_t x) { return c16_weight(A.off, x); });
+        if (lane == 0) found[warp] = t + warp == t1 ? hi : s;
     }
     const uint32_t npages = (R + C16_PAGE - 1) / C16_PAGE;
     for (uint32_t p = tid; p < npages; p += nthr) page_slot[p] = 0;
     __syncthreads();
     const uint32_t s0 = found[0], s1 = found[1];
     if (s0 >= s1) {
-        if (tid == 0) A.tiles[t] = C16Tile{s0, s0, 0u, 0u, 0u, {0u, 0u, 0u}};
+        if (tid == 0) A.tiles[t] = C16Tile{s0, s0, 0u, 0u, 0u, scene, {0u, 0u}};
         return;
     }
     const uint32_t r0 = s0 * C16_ROWS, r1 = min(s1 * C16_ROWS, R), rows = r1 - r0;
@@ -349,7 +478,9 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
     };
     if (LRN) {
         for (uint32_t x = tid; x < rows * 8u; x += nthr) {  // eight threads a row
-            const uint32_t id = __ldg(A.idv + __ldg(A.rowlist + r0 + x / 8u));
+            const uint32_t i = __ldg(A.rowlist + r0 + x / 8u);
+            if (i == C16_NONE) continue;
+            const uint32_t id = __ldg(A.idv + i);
             const uint32_t n = __ldg(A.s_cnt + id);
             for (uint32_t u = x & 7u; u < n; u += 8) {
                 const uint32_t col = sp_row_of(id, u);
@@ -441,8 +572,8 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
         const uint32_t nsp = (rows + SP_SLICE - 1) / SP_SLICE;
         for (uint32_t j = warp; j < nsp; j += nwarps) {
             const uint32_t k = j * SP_SLICE + lane;
-            const uint32_t n =
-                k < rows ? (__ldg(A.s_cnt + __ldg(A.idv + __ldg(A.rowlist + r0 + k))) + 3u) / 4u : 0u;
+            const uint32_t i = k < rows ? __ldg(A.rowlist + r0 + k) : C16_NONE;
+            const uint32_t n = i != C16_NONE ? (__ldg(A.s_cnt + __ldg(A.idv + i)) + 3u) / 4u : 0u;
             const uint32_t w = __reduce_max_sync(0xffffffffu, n);
             if (lane == 0) first[j + 1] = w * SP_SLICE;
         }
@@ -458,10 +589,11 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
         // a pair without a row now is left out (of both its rows), which
         // keeps S' symmetric and diagonally dominant
         for (uint32_t k = tid; k < rows; k += nthr) {
-            const uint32_t id = __ldg(A.idv + __ldg(A.rowlist + r0 + k));
-            const uint32_t n = __ldg(A.s_cnt + id);
+            const uint32_t i = __ldg(A.rowlist + r0 + k);
+            const uint32_t id = i != C16_NONE ? __ldg(A.idv + i) : 0u;
+            const uint32_t n = i != C16_NONE ? __ldg(A.s_cnt + id) : 0u;
             const float di = __ldg(A.dsq + r0 + k);
-            A.sp_diag[r0 + k] = __ldg(A.s_diag + id) * (di * di);
+            A.sp_diag[r0 + k] = i != C16_NONE ? __ldg(A.s_diag + id) * (di * di) : 1.f;
             const uint32_t f0 = first[k / SP_SLICE], words = (first[k / SP_SLICE + 1] - f0) / SP_SLICE * 4u;
             auto place = [&](uint32_t w) { return ((size_t)f0 + w / 4u * SP_SLICE + k % SP_SLICE) * 4u + (w & 3u); };
             uint32_t m = 0;
@@ -496,7 +628,7 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
     const int any = __syncthreads_or((int)nesc);
     if (tid == 0) {
         for (uint32_t w = 0; w < nwarps; w++) wmax = max(wmax, ws[w]);
-        A.tiles[t] = C16Tile{s0, s1, ncol, any ? 1u : 0u, wmax, {0u, 0u, 0u}};
+        A.tiles[t] = C16Tile{s0, s1, ncol, any ? 1u : 0u, wmax, scene, {0u, 0u}};
         atomicMax(A.stats + 1, ncol);
         atomicMax(A.stats + 2, rows);
     }
@@ -521,7 +653,7 @@ __global__ void __launch_bounds__(256) k_c16_finish(const double* __restrict__ c
 // Export: the stored entries of every row as particle indices, at
 // row_start[i] (the particle's list) in stored order.  One block per tile.
 __global__ void __launch_bounds__(256) k_c16_export(const C16Tile* __restrict__ tiles,
-                                                    const uint32_t* __restrict__ collist, uint32_t blocks,
+                                                    const uint32_t* __restrict__ collist, uint32_t blocks, uint32_t ns,
                                                     const uint32_t* __restrict__ clen,
                                                     const uint32_t* __restrict__ rowlist,
                                                     const uint32_t* __restrict__ nrows, const uint32_t* __restrict__ off,
@@ -530,14 +662,16 @@ __global__ void __launch_bounds__(256) k_c16_export(const C16Tile* __restrict__ 
                                                     const uint32_t* __restrict__ row_start, uint32_t* __restrict__ cols,
                                                     float* __restrict__ out_w) {
     const uint32_t R = *nrows;
-    if (blockIdx.x >= c16_tiles(R, blocks)) return;
+    if (blockIdx.x >= c16_tiles(R, blocks, ns)) return;
     const C16Tile ti = tiles[blockIdx.x];
     const uint32_t lane = threadIdx.x & 31, r = lane & 7u, q = lane >> 3;
     for (uint32_t s = ti.s0 + (threadIdx.x >> 5); s < ti.s1; s += blockDim.x >> 5) {
         const uint32_t k = s * C16_ROWS + r;
         if (k >= R) continue;
         const uint32_t g0 = off[s], W = off[s + 1] - g0;
-        const uint32_t o = row_start[rowlist[k]], len = clen[k];
+        const uint32_t len = clen[k];
+        if (len == 0) continue;
+        const uint32_t o = row_start[rowlist[k]];
         for (uint32_t x = 0; x < W; x++)
             for (uint32_t u = 0; u < 4; u++) {
                 const uint32_t e = 16u * x + 4u * q + u;  // the pack's order (k_c16_pack)
@@ -673,6 +807,11 @@ struct C16Args {
     const C16Tile* tiles;
     const uint32_t* collist;
     const uint32_t* stats;      // [1] most columns and [2] most rows of a tile
+    uint32_t ns;                // scenes of a batch (0: a single scene)
+    const uint32_t* tb;         // their first tiles
+    double* tsum;               // a batch's sums of every tile, two buffers
+    int *iters, *outers;        // a batch's results by scene
+    double* srel;
     const double* b64;
     const double* diag64;
     const float* diag32;
@@ -798,13 +937,15 @@ struct C16View {
     uint32_t esc;
     const uint32_t* cl;
     const uint32_t* spf;  // its S' slices (k_c16_pack)
+    uint32_t tile, scene;
 };
 
 constexpr uint32_t C16_SEGS = 4;  // most pieces a slice's chunks are cut into
 
 __device__ __forceinline__ uint32_t c16_align(uint32_t v) { return (v + 15u) & ~15u; }
 
-__device__ __forceinline__ C16View c16_view(const C16Args& S, uint32_t t, uint32_t R, uint32_t C, uint32_t nwarps) {
+__device__ __forceinline__ C16View c16_view(const C16Args& S, uint32_t t, uint32_t R, uint32_t C, uint32_t nwarps,
+                                             uint32_t keep) {
     const C16Tile ti = S.tiles[t];
     C16View v;
     v.s0 = ti.s0;
@@ -821,9 +962,11 @@ __device__ __forceinline__ C16View c16_view(const C16Args& S, uint32_t t, uint32
     v.cpw = max(v.cpw, 1u);
     v.nseg = ti.wmax ? (ti.wmax + v.cpw - 2) / v.cpw + 1 : 1u;
     v.resw = 0;
-    v.keepw = S.keep == 0xffffffffu ? S.keep : (uint32_t)((uint64_t)v.cpw * min(S.keep, C) / C);
+    v.keepw = keep == 0xffffffffu ? keep : (uint32_t)((uint64_t)v.cpw * min(keep, C) / C);
     v.cl = S.collist + (size_t)t * C16_COLS;
     v.spf = S.sp_first + (size_t)t * C16_SP_SLICES;
+    v.tile = t;
+    v.scene = ti.scene;
     return v;
 }
 
@@ -990,13 +1133,22 @@ __device__ __forceinline__ void c16_stage(T* vec, const uint32_t* cl, uint32_t n
 // and, in a block of one tile
 // (single), its column list and its rows' state, which then never leave the
 // SM.  The rest holds chunks of the matrix.
+// The solve of the scene a tile belongs to (a batch; every tile has a copy).
+struct C16Scene {
+    double alpha, beta, gamma, stop, relres;
+    int total, outers, it, phase;
+    uint32_t flip;  // which of the published buffers is read
+    uint32_t pad;
+};
+
 struct C16Plan {
-    uint32_t q, soff, sseg, got, views, cl, row, res;  // byte offsets
+    uint32_t q, soff, sseg, got, views, scn, cl, row, res;  // byte offsets
     uint32_t rs;                           // row stride of the sums and the state
 };
 constexpr uint32_t C16_ROW_BYTES = 32;     // x in double; r, w, s, 1 / diagonal, p, diagonal
 
-__device__ __forceinline__ C16Plan c16_plan(uint32_t ncol, uint32_t rows, uint32_t nseg, uint32_t ntiles, bool single) {
+__device__ __forceinline__ C16Plan c16_plan(uint32_t ncol, uint32_t rows, uint32_t nseg, uint32_t ntiles, bool single,
+                                            bool batch) {
     C16Plan p;
     const uint32_t ns = (rows + C16_ROWS - 1) / C16_ROWS;
     p.rs = ns * C16_ROWS;
@@ -1005,7 +1157,8 @@ __device__ __forceinline__ C16Plan c16_plan(uint32_t ncol, uint32_t rows, uint32
     p.sseg = p.soff + c16_align((ns + 1) * 4u);
     p.got = p.sseg + c16_align(ns);
     p.views = p.got + c16_align(gridDim.x * C16_SUMS * 8u);
-    p.cl = p.views + c16_align(single ? 0u : ntiles * (uint32_t)sizeof(C16View));
+    p.scn = p.views + c16_align(single ? 0u : ntiles * (uint32_t)sizeof(C16View));
+    p.cl = p.scn + c16_align(batch ? ntiles * (uint32_t)sizeof(C16Scene) : 0u);
     p.row = p.cl + (single ? c16_align(ncol * 4u) : 0u);
     p.res = c16_align(p.row + (single ? p.rs * C16_ROW_BYTES : 0u));
     return p;
@@ -1034,21 +1187,21 @@ struct C16Block {
     __device__ __forceinline__ C16Block(const C16Args& S_, unsigned char* sm_, bool learned) : S(S_), sm(sm_) {
         R = *S.nrows;
         G = gridDim.x;
-        ntiles = c16_tiles(R, G) / G;
+        ntiles = c16_tiles(R, G, S.ns) / G;
         C = max(__ldg(S.off + (R + C16_ROWS - 1) / C16_ROWS), 1u);
-        v = c16_view(S, blockIdx.x + G * (ntiles - 1), R, C, blockDim.x >> 5);
+        v = c16_view(S, blockIdx.x + G * (ntiles - 1), R, C, blockDim.x >> 5, S.keep);
         single = false;
         whole = false;
         if (ntiles == 1) {
-            pl = c16_plan(v.ncol, v.rows, v.nseg, 1u, true);
+            pl = c16_plan(v.ncol, v.rows, v.nseg, 1u, true, S.ns != 0u);
             single = pl.res <= S.smem_bytes;
         }
         if (!single) {
             // a tile with so many rows and columns that the pieces do not fit
             // is done by one warp, slices whole: slow, but right
-            pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), C16_SEGS, ntiles, false);
+            pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), C16_SEGS, ntiles, false, S.ns != 0u);
             whole = pl.res > S.smem_bytes;
-            if (whole) pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), 1u, ntiles, false);
+            if (whole) pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), 1u, ntiles, false, S.ns != 0u);
         }
         if (whole) v.cpw = max(v.nch, 1u);
         sp_res = false;
@@ -1064,9 +1217,18 @@ struct C16Block {
             for (uint32_t x = lane; x < n * (C16_CHUNK_BYTES / 16); x += 32) dst[x] = __ldg(src + x);
         }
         if (!single) {
+            // half the L2 budget less the rows' vectors (48 bytes a row) and
+            // S', which are read again every iteration too: with all of it
+            // 293,971 rows take 4.19 (learned 4.49) ms a solve, so 4.08 (4.23)
+            uint32_t keep = S.keep;
+            if (keep != 0xffffffffu) {
+                const uint64_t other = (uint64_t)R * 48u + (learned ? (uint64_t)__ldg(S.stats + 3) * 16u : 0u);
+                const uint32_t n = (uint32_t)min(other / C16_CHUNK_BYTES, (uint64_t)0x7fffffffu);
+                keep = keep / 2u > n ? keep / 2u - n : 0u;
+            }
             C16View* views = reinterpret_cast<C16View*>(sm + pl.views);
             for (uint32_t m = threadIdx.x; m < ntiles; m += blockDim.x) {
-                C16View t = c16_view(S, blockIdx.x + G * m, R, C, nw);
+                C16View t = c16_view(S, blockIdx.x + G * m, R, C, nw, keep);
                 if (whole) t.cpw = max(t.nch, 1u);
                 if (m == ntiles - 1) t.resw = v.resw;
                 views[m] = t;
@@ -1117,25 +1279,32 @@ struct C16Block {
     // body(view) for each of the block's tiles; the slice offsets are loaded
     // (the body's first barrier publishes them).  While a tile is worked on,
     // ahead(view) brings what the next one reads once into L2.
-    template <class F, class P>
-    __device__ __forceinline__ void tiles(P ahead, F body) const {
-        if (single) {
-            body(v);
-            return;
-        }
+    template <class P, class F, class W>
+    __device__ __forceinline__ void tiles(P ahead, F body, W want) const {
         const C16View* views = reinterpret_cast<const C16View*>(sm + pl.views);
         for (uint32_t m = 0; m < ntiles; m++) {
-            const C16View t = views[m];
-            __syncthreads();
-            c16_slices(S, t, soff(), sseg());
-            if (m + 1 < ntiles) {
+            if (m + 1 < ntiles && want(m + 1)) {
                 const C16View& n = views[m + 1];
                 c16_ahead(n.cl, n.ncol * 4u);
                 c16_ahead(S.off + n.s0, (n.ns + 1) * 4u);
                 ahead(n);
             }
-            body(t);
+            if (!want(m)) continue;
+            C16View t = v;
+            if (!single) {
+                t = views[m];
+                __syncthreads();
+                c16_slices(S, t, soff(), sseg());
+            }
+            body(t);  // the only call: the compiler inlines it
         }
+    }
+    template <class P, class F>
+    __device__ __forceinline__ void tiles(P ahead, F body) const {
+        tiles(ahead, body, [](uint32_t) { return true; });
+    }
+    __device__ __forceinline__ const C16View& view(uint32_t m) const {
+        return single ? v : reinterpret_cast<const C16View*>(sm + pl.views)[m];
     }
     // the tile's products over the staged vector, barriers included; row k's
     // sum is then rowsum<T>(k)
@@ -1151,34 +1320,33 @@ struct C16Block {
     __device__ __forceinline__ T rowsum(uint32_t k) const {
         return c16_rowsum(reinterpret_cast<const T*>(sm + pl.q), pl.rs, sseg(), k);
     }
-    // r64 = b - A x64 of every row in FP64; body(view, k, r64, x)
+    // r64 = b - A x64 of the tile's rows in FP64, |r64|^2 and |b|^2;
+    // body(k, r64)
     template <class F>
-    __device__ __forceinline__ void residual(double (&acc)[2], F body) const {
-        tiles(
-            [&](const C16View& n) {
-                c16_ahead(S.b64 + n.r0, n.rows * 8u);
-                c16_ahead(S.diag64 + n.r0, n.rows * 8u);
-            },
-            [&](const C16View& t) {
-            c16_stage(reinterpret_cast<double*>(sm), t.cl, t.ncol, [&](const uint32_t (&j)[4], double (&o)[4]) {
+    __device__ __forceinline__ void residual(const C16View& t, double (&acc)[C16_SUMS], F body) const {
+        c16_stage(reinterpret_cast<double*>(sm), t.cl, t.ncol, [&](const uint32_t (&j)[4], double (&o)[4]) {
 #pragma unroll
-                for (int u = 0; u < 4; u++) o[u] = __ldcg(S.x64 + j[u]);
-            });
-            product<double>(t, [&](uint32_t col) { return __ldcg(S.x64 + col); });
-            for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
-                const uint32_t g = t.r0 + k;
-                const double bi = __ldg(S.b64 + g);
-                const double x = reinterpret_cast<const double*>(sm)[k];
-                const double ri = bi - (__ldg(S.diag64 + g) * x + rowsum<double>(k));
-                acc[0] += ri * ri;
-                acc[1] += bi * bi;
-                body(t, k, ri);
-            }
+            for (int u = 0; u < 4; u++) o[u] = __ldcg(S.x64 + j[u]);
         });
+        product<double>(t, [&](uint32_t col) { return __ldcg(S.x64 + col); });
+        for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+            const uint32_t g = t.r0 + k;
+            const double bi = __ldg(S.b64 + g);
+            const double x = reinterpret_cast<const double*>(sm)[k];
+            const double ri = bi - (__ldg(S.diag64 + g) * x + rowsum<double>(k));
+            acc[0] += ri * ri;
+            acc[1] += bi * bi;
+            body(k, ri);
+        }
+    }
+    // what that reads of a tile once
+    __device__ __forceinline__ void ahead_residual(const C16View& n) const {
+        c16_ahead(S.b64 + n.r0, n.rows * 8u);
+        c16_ahead(S.diag64 + n.r0, n.rows * 8u);
     }
 };
 
-// the smallest reduction one FP32 inner solve is asked for, squared
+// the reduction one FP32 inner solve is asked for, squared
 __device__ __forceinline__ double inner_target(const C16Args& S, double relres) {
     double eta = 0.3 * S.tol / relres;
     if (eta < S.eta_min) eta = S.eta_min;
@@ -1186,145 +1354,89 @@ __device__ __forceinline__ double inner_target(const C16Args& S, double relres) 
     return eta * eta;
 }
 
-// ok: every grid sum completed (else the timeout is the error)
-__device__ __forceinline__ void c16_finish_solve(const C16Args& S, const C16Sync& sy, int total, int outers,
-                                                 double relres, bool converged, bool ok) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    *S.epoch = sy.epoch + 2;  // past every epoch any block has used
-    if (!ok) return;
-    S.sc->cg_iters = total;
-    S.sc->cg_outer = outers;
-    S.sc->cg_relres = relres;
-    if (!converged) atomicOr(&S.sc->err, ERR_CG_NOT_CONVERGED);
-}
-
-// Diagonally scaled CG in the single-reduction form of Chronopoulos and Gear
-// (1989): with u = D^-1 r and w = A u, one sum of (r.u, w.u, r.r) gives the
-// next alpha and beta, and s = w + beta s, p = u + beta p follow by
-// recurrence.  A row publishes (r, w, s, 1 / diagonal); whoever needs its
-// next u forms it from those while staging (16 bytes per staged column, not
-// per entry), so an iteration has one grid-wide wait.  The same iterates as
-// CG's in exact arithmetic; the FP64 true residual ends the solve.
-__global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16(C16Args S) {
-    extern __shared__ __align__(16) unsigned char c16_sm[];
-    C16Sync sy{S.slots, *S.epoch, S.sc};
-    const C16Block B(S, c16_sm, false);
-    float* vec = reinterpret_cast<float*>(c16_sm);
-    float4* pc = S.pub0;  // published rows: read by this iteration
-    float4* pn = S.pub1;  // and written
-    int total = 0, outers = 0;
-    double relres = 0.0;
-    bool converged = false, ok = true;
-    for (int outer = 0; outer < S.max_outer; outer++) {
-        double acc[2] = {0.0, 0.0};
-        B.residual(acc, [&](const C16View& t, uint32_t k, double ri) {
-            const float r = (float)ri;
-            if (B.single) {
-                B.rf(C16Block::C16_R)[k] = r;
-                B.rf(C16Block::C16_W)[k] = 0.f;
-                B.rf(C16Block::C16_S)[k] = 0.f;
-                B.rf(C16Block::C16_P)[k] = 0.f;
-                pc[t.r0 + k] = make_float4(r, 0.f, 0.f, B.rf(C16Block::C16_INV)[k]);
-            } else {
-                S.p[t.r0 + k] = 0.f;
-                pc[t.r0 + k] = make_float4(r, 0.f, 0.f, __ldg(S.inv_diag + t.r0 + k));
-            }
-        });
-        double tot[2];
-        ok = c16_sum<2>(acc, sy, B.got(), tot);
-        if (!ok) break;
-        outers++;
-        relres = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : 0.0;
-        if (relres <= S.tol) {
-            converged = true;
-            break;
-        }
-        if (total >= S.max_iter) break;
-        const double stop = inner_target(S, relres) * tot[0];
-        double alpha = 0.0, beta = 0.0, gamma = 0.0;
-        // it = -1: w = A u of the start, nothing moves (alpha = beta = 0)
-        for (int it = -1;; it++) {
-            const float af = (float)alpha, bf = (float)beta;
-            double g[3] = {0.0, 0.0, 0.0};
-            B.tiles(
-                [&](const C16View& n) {
-                    c16_ahead(S.x64 + n.r0, n.rows * 8u);
-                    c16_ahead(S.p + n.r0, n.rows * 4u);
-                    c16_ahead(S.diag32 + n.r0, n.rows * 4u);
-                },
-                [&](const C16View& t) {
-                auto next_u = [&](const float4& v) {
-                    return v.w * fmaf(-af, fmaf(bf, v.z, v.y), v.x);
-                };
-                c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
-                    float4 v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) v[u] = __ldcg(pc + j[u]);
-#pragma unroll
-                    for (int u = 0; u < 4; u++) o[u] = next_u(v[u]);
-                });
-                B.product<float>(t, [&](uint32_t col) { return next_u(__ldcg(pc + col)); });
-                for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
-                    const uint32_t gk = t.r0 + k;
-                    float4 o;
-                    float p, dg;
-                    double x;
-                    if (B.single) {
-                        o = make_float4(B.rf(C16Block::C16_R)[k], B.rf(C16Block::C16_W)[k], B.rf(C16Block::C16_S)[k],
-                                        B.rf(C16Block::C16_INV)[k]);
-                        p = B.rf(C16Block::C16_P)[k];
-                        dg = B.rf(C16Block::C16_DG)[k];
-                        x = B.rx()[k];
-                    } else {
-                        o = pc[gk];
-                        p = S.p[gk];
-                        dg = __ldg(S.diag32 + gk);
-                        x = S.x64[gk];
-                    }
-                    const float sn = fmaf(bf, o.z, o.y);
-                    p = fmaf(bf, p, o.w * o.x);
-                    x += alpha * (double)p;
-                    const float r = fmaf(-af, sn, o.x);
-                    const float u = vec[k];
-                    const float w = fmaf(dg, u, B.rowsum<float>(k));
-                    pn[gk] = make_float4(r, w, sn, o.w);
-                    S.x64[gk] = x;
-                    if (B.single) {
-                        B.rf(C16Block::C16_R)[k] = r;
-                        B.rf(C16Block::C16_W)[k] = w;
-                        B.rf(C16Block::C16_S)[k] = sn;
-                        B.rf(C16Block::C16_P)[k] = p;
-                        B.rx()[k] = x;
-                    } else {
-                        S.p[gk] = p;
-                    }
-                    g[0] += (double)r * (double)u;
-                    g[1] += (double)w * (double)u;
-                    g[2] += (double)r * (double)r;
-                }
-            });
-            double gt[3];
-            ok = c16_sum<3>(g, sy, B.got(), gt);
-            if (!ok) break;
-            float4* x = pc;
-            pc = pn;
-            pn = x;
-            if (it >= 0) {
-                total++;
-                if (gt[2] <= stop) break;
-                beta = gt[0] / gamma;
-                alpha = gt[0] / (gt[1] - beta * gt[0] / alpha);
-            } else {
-                alpha = gt[0] / gt[1];
-            }
-            gamma = gt[0];
-            if (it + 1 >= S.inner_cap || total >= S.max_iter) break;
-        }
-        if (!ok) break;
+// ---- a tile's part of an iteration with diagonal scaling
+// CG in the single-reduction form of Chronopoulos and Gear (1989): with u =
+// D^-1 r and w = A u, one sum of (r.u, w.u, r.r) gives the next alpha and
+// beta, and s = w + beta s, p = u + beta p follow by recurrence.  A row
+// publishes (r, w, s, 1 / diagonal); whoever needs its next u forms it from
+// those while staging (16 bytes per staged column, not per entry), so an
+// iteration has one grid-wide wait.  The same iterates as CG's in exact
+// arithmetic; the FP64 true residual ends the solve.  pc is read, pn written.
+__device__ __forceinline__ void c16_start_row(const C16Args& S, const C16Block& B, const C16View& t, uint32_t k,
+                                              double ri, float4* pc) {
+    const float r = (float)ri;
+    if (B.single) {
+        B.rf(C16Block::C16_R)[k] = r;
+        B.rf(C16Block::C16_W)[k] = 0.f;
+        B.rf(C16Block::C16_S)[k] = 0.f;
+        B.rf(C16Block::C16_P)[k] = 0.f;
+        pc[t.r0 + k] = make_float4(r, 0.f, 0.f, B.rf(C16Block::C16_INV)[k]);
+    } else {
+        S.p[t.r0 + k] = 0.f;
+        pc[t.r0 + k] = make_float4(r, 0.f, 0.f, __ldg(S.inv_diag + t.r0 + k));
     }
-    c16_finish_solve(S, sy, total, outers, relres, converged, ok);
 }
 
+__device__ __forceinline__ void c16_iterate(const C16Args& S, const C16Block& B, const C16View& t, double alpha,
+                                            double beta, const float4* pc, float4* pn, double (&g)[C16_SUMS]) {
+    float* vec = reinterpret_cast<float*>(B.sm);
+    const float af = (float)alpha, bf = (float)beta;
+    auto next_u = [&](const float4& v) { return v.w * fmaf(-af, fmaf(bf, v.z, v.y), v.x); };
+    c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldcg(pc + j[u]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) o[u] = next_u(v[u]);
+    });
+    B.product<float>(t, [&](uint32_t col) { return next_u(__ldcg(pc + col)); });
+    for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+        const uint32_t gk = t.r0 + k;
+        float4 o;
+        float p, dg;
+        double x;
+        if (B.single) {
+            o = make_float4(B.rf(C16Block::C16_R)[k], B.rf(C16Block::C16_W)[k], B.rf(C16Block::C16_S)[k],
+                            B.rf(C16Block::C16_INV)[k]);
+            p = B.rf(C16Block::C16_P)[k];
+            dg = B.rf(C16Block::C16_DG)[k];
+            x = B.rx()[k];
+        } else {
+            o = pc[gk];
+            p = S.p[gk];
+            dg = __ldg(S.diag32 + gk);
+            x = S.x64[gk];
+        }
+        const float sn = fmaf(bf, o.z, o.y);
+        p = fmaf(bf, p, o.w * o.x);
+        x += alpha * (double)p;
+        const float r = fmaf(-af, sn, o.x);
+        const float u = vec[k];
+        const float w = fmaf(dg, u, B.rowsum<float>(k));
+        pn[gk] = make_float4(r, w, sn, o.w);
+        S.x64[gk] = x;
+        if (B.single) {
+            B.rf(C16Block::C16_R)[k] = r;
+            B.rf(C16Block::C16_W)[k] = w;
+            B.rf(C16Block::C16_S)[k] = sn;
+            B.rf(C16Block::C16_P)[k] = p;
+            B.rx()[k] = x;
+        } else {
+            S.p[gk] = p;
+        }
+        g[0] += (double)r * (double)u;
+        g[1] += (double)w * (double)u;
+        g[2] += (double)r * (double)r;
+    }
+}
+
+__device__ __forceinline__ void c16_ahead_iterate(const C16Args& S, const C16View& n) {
+    c16_ahead(S.x64 + n.r0, n.rows * 8u);
+    c16_ahead(S.p + n.r0, n.rows * 4u);
+    c16_ahead(S.diag32 + n.r0, n.rows * 4u);
+}
+
+// ---- and with the learned preconditioner z = S' r
 // Row k of S' x over the staged x (own rows first in the tile's list); an
 // escaped column's x comes from remote.  S' is in shared memory or read
 // again every iteration.
@@ -1378,30 +1490,127 @@ __device__ __forceinline__ float c16_sp_row(const C16Args& S, const C16Block& B,
     return fmaf(dg, vec[k], offd);
 }
 
-// The learned preconditioner z = S' r.  An iteration is two passes, each
-// ending in a grid-wide sum: the update (residuals r - alpha q staged, x, z =
-// S' r, r.z and r.r) and the product (directions z + beta p staged, q = A p,
-// p.q).  A row publishes (z, p) in the first and (r, q) in the second, each
-// read by the other blocks only in the other pass.
-__global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16_learned(C16Args S) {
+// An iteration is two passes, each ending in a grid-wide sum: the update
+// (residuals r - alpha q staged, x, z = S' r, r.z and r.r) and the product
+// (directions z + beta p staged, q = A p, p.q).  A row publishes (z, p) in
+// the first and (r, q) in the second, each read by the other blocks only in
+// the other pass.
+__device__ __forceinline__ void c16_update(const C16Args& S, const C16Block& B, const C16View& t, double alpha,
+                                           float2* zp, const float2* rq, double (&g)[C16_SUMS]) {
+    float* vec = reinterpret_cast<float*>(B.sm);
+    const float af = (float)alpha;
+    auto next_r = [&](const float2& v) { return fmaf(-af, v.y, v.x); };
+    c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
+        float2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldcg(rq + j[u]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) o[u] = next_r(v[u]);
+    });
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+        const uint32_t gk = t.r0 + k;
+        const float r = vec[k];
+        const float p = B.single ? B.rf(C16Block::C16_P)[k] : S.p[gk];
+        const double x = (B.single ? B.rx()[k] : S.x64[gk]) + alpha * (double)p;
+        const float z = c16_sp_row(S, B, t, vec, k, [&](uint32_t col) { return next_r(__ldcg(rq + col)); });
+        zp[gk] = make_float2(z, p);
+        S.x64[gk] = x;
+        if (B.single) {
+            B.rx()[k] = x;
+            B.rf(C16Block::C16_R)[k] = r;
+        } else {
+            S.r[gk] = r;
+        }
+        g[0] += (double)r * (double)z;
+        g[1] += (double)r * (double)r;
+    }
+}
+
+__device__ __forceinline__ void c16_ahead_update(const C16Args& S, const C16View& n) {
+    const uint32_t nsp = (n.rows + SP_SLICE - 1) / SP_SLICE;
+    const uint32_t f = __ldg(n.spf);
+    c16_ahead(S.sp_ent + 4 * (size_t)f, (__ldg(n.spf + nsp) - f) * 16u);
+    c16_ahead(n.spf, (nsp + 1) * 4u);
+    c16_ahead(S.sp_diag + n.r0, n.rows * 4u);
+    c16_ahead(S.x64 + n.r0, n.rows * 8u);
+    c16_ahead(S.p + n.r0, n.rows * 4u);
+}
+
+__device__ __forceinline__ void c16_direction(const C16Args& S, const C16Block& B, const C16View& t, float beta,
+                                              const float2* zp, float2* rq, double& pq) {
+    float* vec = reinterpret_cast<float*>(B.sm);
+    auto next_p = [&](const float2& v) { return fmaf(beta, v.y, v.x); };
+    c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
+        float2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldcg(zp + j[u]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) o[u] = next_p(v[u]);
+    });
+    B.product<float>(t, [&](uint32_t col) { return next_p(__ldcg(zp + col)); });
+    for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
+        const uint32_t gk = t.r0 + k;
+        const float p = vec[k];
+        const float dg = B.single ? B.rf(C16Block::C16_DG)[k] : __ldg(S.diag32 + gk);
+        const float q = fmaf(dg, p, B.rowsum<float>(k));
+        if (B.single) B.rf(C16Block::C16_P)[k] = p;
+        else S.p[gk] = p;
+        rq[gk] = make_float2(B.single ? B.rf(C16Block::C16_R)[k] : S.r[gk], q);
+        pq += (double)p * (double)q;
+    }
+}
+
+__device__ __forceinline__ void c16_ahead_direction(const C16Args& S, const C16View& n) {
+    c16_ahead(S.diag32 + n.r0, n.rows * 4u);
+    c16_ahead(S.r + n.r0, n.rows * 4u);
+}
+
+// the start of an inner solve from r64: r published, p = 0
+__device__ __forceinline__ void c16_start_row_learned(const C16Args& S, const C16Block& B, const C16View& t,
+                                                      uint32_t k, double ri, float2* rq) {
+    rq[t.r0 + k] = make_float2((float)ri, 0.f);
+    if (B.single) B.rf(C16Block::C16_P)[k] = 0.f;
+    else S.p[t.r0 + k] = 0.f;
+}
+
+// ---- one scene
+// ok: every grid sum completed (else the timeout is the error)
+__device__ __forceinline__ void c16_finish_solve(const C16Args& S, const C16Sync& sy, int total, int outers,
+                                                 double relres, bool converged, bool ok) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    *S.epoch = sy.epoch + 2;  // past every epoch any block has used
+    if (!ok) return;
+    S.sc->cg_iters = total;
+    S.sc->cg_outer = outers;
+    S.sc->cg_relres = relres;
+    if (!converged) atomicOr(&S.sc->err, ERR_CG_NOT_CONVERGED);
+}
+
+template <bool LRN>
+__global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16(C16Args S) {
     extern __shared__ __align__(16) unsigned char c16_sm[];
     C16Sync sy{S.slots, *S.epoch, S.sc};
-    const C16Block B(S, c16_sm, true);
-    float* vec = reinterpret_cast<float*>(c16_sm);
+    const C16Block B(S, c16_sm, LRN);
+    float4* pc = S.pub0;  // published rows: read by this iteration
+    float4* pn = S.pub1;  // and written
     float2* zp = reinterpret_cast<float2*>(S.pub0);
     float2* rq = reinterpret_cast<float2*>(S.pub1);
     int total = 0, outers = 0;
     double relres = 0.0;
     bool converged = false, ok = true;
     for (int outer = 0; outer < S.max_outer; outer++) {
-        double acc[2] = {0.0, 0.0};
-        B.residual(acc, [&](const C16View& t, uint32_t k, double ri) {
-            rq[t.r0 + k] = make_float2((float)ri, 0.f);
-            if (B.single) B.rf(C16Block::C16_P)[k] = 0.f;
-            else S.p[t.r0 + k] = 0.f;
-        });
+        double acc[C16_SUMS] = {0.0, 0.0, 0.0};
+        B.tiles([&](const C16View& n) { B.ahead_residual(n); },
+                [&](const C16View& t) {
+                    B.residual(t, acc, [&](uint32_t k, double ri) {
+                        if (LRN) c16_start_row_learned(S, B, t, k, ri, rq);
+                        else c16_start_row(S, B, t, k, ri, pc);
+                    });
+                });
+        const double two[2] = {acc[0], acc[1]};
         double tot[2];
-        ok = c16_sum<2>(acc, sy, B.got(), tot);
+        ok = c16_sum<2>(two, sy, B.got(), tot);
         if (!ok) break;
         outers++;
         relres = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : 0.0;
@@ -1411,95 +1620,250 @@ __global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16_learned(C16Arg
         }
         if (total >= S.max_iter) break;
         const double stop = inner_target(S, relres) * tot[0];
-        double alpha = 0.0, rz = 0.0;
-        // it = -1: z of the start, nothing moves (alpha = 0)
+        double alpha = 0.0, beta = 0.0, gamma = 0.0;
+        // it = -1: w = A u, or z = S' r, of the start; nothing moves (alpha = beta = 0)
         for (int it = -1;; it++) {
-            const float af = (float)alpha;
-            double g[2] = {0.0, 0.0};
-            B.tiles(
-                [&](const C16View& n) {
-                    const uint32_t nsp = (n.rows + SP_SLICE - 1) / SP_SLICE;
-                    const uint32_t f = __ldg(n.spf);
-                    c16_ahead(S.sp_ent + 4 * (size_t)f, (__ldg(n.spf + nsp) - f) * 16u);
-                    c16_ahead(n.spf, (nsp + 1) * 4u);
-                    c16_ahead(S.sp_diag + n.r0, n.rows * 4u);
-                    c16_ahead(S.x64 + n.r0, n.rows * 8u);
-                    c16_ahead(S.p + n.r0, n.rows * 4u);
-                },
-                [&](const C16View& t) {
-                auto next_r = [&](const float2& v) { return fmaf(-af, v.y, v.x); };
-                c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
-                    float2 v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) v[u] = __ldcg(rq + j[u]);
-#pragma unroll
-                    for (int u = 0; u < 4; u++) o[u] = next_r(v[u]);
-                });
-                __syncthreads();
-                for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
-                    const uint32_t gk = t.r0 + k;
-                    const float r = vec[k];
-                    const float p = B.single ? B.rf(C16Block::C16_P)[k] : S.p[gk];
-                    const double x = (B.single ? B.rx()[k] : S.x64[gk]) + alpha * (double)p;
-                    const float z = c16_sp_row(S, B, t, vec, k, [&](uint32_t col) { return next_r(__ldcg(rq + col)); });
-                    zp[gk] = make_float2(z, p);
-                    S.x64[gk] = x;
-                    if (B.single) {
-                        B.rx()[k] = x;
-                        B.rf(C16Block::C16_R)[k] = r;
-                    } else {
-                        S.r[gk] = r;
-                    }
-                    g[0] += (double)r * (double)z;
-                    g[1] += (double)r * (double)r;
+            double g[C16_SUMS] = {0.0, 0.0, 0.0};
+            if (LRN) {
+                B.tiles([&](const C16View& n) { c16_ahead_update(S, n); },
+                        [&](const C16View& t) { c16_update(S, B, t, alpha, zp, rq, g); });
+                const double v2[2] = {g[0], g[1]};
+                double gt[2];
+                ok = c16_sum<2>(v2, sy, B.got(), gt);
+                if (!ok) break;
+                beta = 0.0;
+                if (it >= 0) {
+                    total++;
+                    if (gt[1] <= stop) break;
+                    beta = gt[0] / gamma;
                 }
-            });
-            double gt[2];
-            ok = c16_sum<2>(g, sy, B.got(), gt);
-            if (!ok) break;
-            float beta = 0.f;
-            if (it >= 0) {
-                total++;
-                if (gt[1] <= stop) break;
-                beta = (float)(gt[0] / rz);
+                gamma = gt[0];
+                if (it + 1 >= S.inner_cap || total >= S.max_iter) break;
+                double pq[1] = {0.0}, tp[1];
+                B.tiles([&](const C16View& n) { c16_ahead_direction(S, n); },
+                        [&](const C16View& t) { c16_direction(S, B, t, (float)beta, zp, rq, pq[0]); });
+                ok = c16_sum<1>(pq, sy, B.got(), tp);
+                if (!ok) break;
+                alpha = gamma / tp[0];
+            } else {
+                B.tiles([&](const C16View& n) { c16_ahead_iterate(S, n); },
+                        [&](const C16View& t) { c16_iterate(S, B, t, alpha, beta, pc, pn, g); });
+                double gt[C16_SUMS];
+                ok = c16_sum<C16_SUMS>(g, sy, B.got(), gt);
+                if (!ok) break;
+                float4* x = pc;
+                pc = pn;
+                pn = x;
+                if (it >= 0) {
+                    total++;
+                    if (gt[2] <= stop) break;
+                    beta = gt[0] / gamma;
+                    alpha = gt[0] / (gt[1] - beta * gt[0] / alpha);
+                } else {
+                    alpha = gt[0] / gt[1];
+                }
+                gamma = gt[0];
+                if (it + 1 >= S.inner_cap || total >= S.max_iter) break;
             }
-            rz = gt[0];
-            if (it + 1 >= S.inner_cap || total >= S.max_iter) break;
-            double pq[1] = {0.0};
-            B.tiles(
-                [&](const C16View& n) {
-                    c16_ahead(S.diag32 + n.r0, n.rows * 4u);
-                    c16_ahead(S.r + n.r0, n.rows * 4u);
-                },
-                [&](const C16View& t) {
-                auto next_p = [&](const float2& v) { return fmaf(beta, v.y, v.x); };
-                c16_stage(vec, t.cl, t.ncol, [&](const uint32_t (&j)[4], float (&o)[4]) {
-                    float2 v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) v[u] = __ldcg(zp + j[u]);
-#pragma unroll
-                    for (int u = 0; u < 4; u++) o[u] = next_p(v[u]);
-                });
-                B.product<float>(t, [&](uint32_t col) { return next_p(__ldcg(zp + col)); });
-                for (uint32_t k = threadIdx.x; k < t.rows; k += blockDim.x) {
-                    const uint32_t gk = t.r0 + k;
-                    const float p = vec[k];
-                    const float dg = B.single ? B.rf(C16Block::C16_DG)[k] : __ldg(S.diag32 + gk);
-                    const float q = fmaf(dg, p, B.rowsum<float>(k));
-                    if (B.single) B.rf(C16Block::C16_P)[k] = p;
-                    else S.p[gk] = p;
-                    rq[gk] = make_float2(B.single ? B.rf(C16Block::C16_R)[k] : S.r[gk], q);
-                    pq[0] += (double)p * (double)q;
-                }
-            });
-            double totp[1];
-            ok = c16_sum<1>(pq, sy, B.got(), totp);
-            if (!ok) break;
-            alpha = rz / totp[0];
         }
         if (!ok) break;
     }
     c16_finish_solve(S, sy, total, outers, relres, converged, ok);
+}
+
+// ---- the scenes of a batch
+// Every scene runs its own solve, with its own FP64 passes and stop, and its
+// tiles are spread over the blocks.  In a round every tile does what its
+// scene is at (the FP64 residual, the start, an iteration; with the learned
+// form an update or a product) and leaves its sums; after one grid-wide
+// barrier every block adds up the sums of its tiles' scenes, in tile order,
+// and moves them on.  A scene that is done is skipped; the barrier's own sum
+// counts the scenes that are not.
+enum : int { SCN_RESID = 0, SCN_START, SCN_ITER, SCN_PROD, SCN_DONE };
+
+// the block's sum of g to out[0 .. C16_SUMS)
+__device__ __forceinline__ void c16_tile_sum(const double (&g)[C16_SUMS], double* out) {
+    __shared__ double part[C16_SUMS][32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < (int)C16_SUMS; k++) {
+        const double t = warp_sum_d(g[k]);
+        if (lane == 0) part[k][warp] = t;
+    }
+    __syncthreads();
+    if (warp < C16_SUMS) {
+        const double t = warp_sum_d(lane < nw ? part[warp][lane] : 0.0);
+        if (lane == 0) out[warp] = t;
+    }
+}
+
+// a scene's next step from the sums of its last one (g); true when it ends
+template <bool LRN>
+__device__ __forceinline__ void c16_advance(const C16Args& S, C16Scene& c, const double (&g)[C16_SUMS], bool* failed) {
+    switch (c.phase) {
+        case SCN_RESID:
+            c.outers++;
+            c.relres = g[1] > 0.0 ? sqrt(g[0] / g[1]) : 0.0;
+            if (c.relres <= S.tol) {
+                c.phase = SCN_DONE;
+            } else if (c.total >= S.max_iter || c.outers >= S.max_outer) {
+                c.phase = SCN_DONE;
+                *failed = true;
+            } else {
+                c.stop = inner_target(S, c.relres) * g[0];
+                c.alpha = c.beta = c.gamma = 0.0;
+                c.it = -1;
+                c.phase = SCN_START;
+            }
+            return;
+        case SCN_PROD:
+            c.alpha = c.gamma / g[0];
+            c.it++;
+            c.phase = SCN_ITER;
+            return;
+        default: break;
+    }
+    const bool started = c.phase == SCN_ITER;
+    if (started) c.total++;
+    if (LRN) {
+        if (started && g[1] <= c.stop) {
+            c.phase = SCN_RESID;
+            return;
+        }
+        c.beta = started ? g[0] / c.gamma : 0.0;
+        c.gamma = g[0];
+        c.phase = c.it + 1 >= S.inner_cap || c.total >= S.max_iter ? SCN_RESID : SCN_PROD;
+    } else {
+        c.flip ^= 1u;
+        if (started && g[2] <= c.stop) {
+            c.phase = SCN_RESID;
+            return;
+        }
+        if (started) {
+            c.beta = g[0] / c.gamma;
+            c.alpha = g[0] / (g[1] - c.beta * g[0] / c.alpha);
+        } else {
+            c.alpha = g[0] / g[1];
+        }
+        c.gamma = g[0];
+        c.phase = c.it + 1 >= S.inner_cap || c.total >= S.max_iter ? SCN_RESID : SCN_ITER;
+        c.it++;
+    }
+}
+
+template <bool LRN>
+__global__ void __launch_bounds__(C16_THREADS, 1) k_ppe_solve_c16_batch(C16Args S) {
+    extern __shared__ __align__(16) unsigned char c16_sm[];
+    C16Sync sy{S.slots, *S.epoch, S.sc};
+    const C16Block B(S, c16_sm, LRN);
+    C16Scene* scn = reinterpret_cast<C16Scene*>(c16_sm + B.pl.scn);
+    __shared__ int open_s;  // scenes not done whose first tile is this block's
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint32_t T = B.ntiles * B.G;
+    for (uint32_t m = threadIdx.x; m < B.ntiles; m += blockDim.x) {
+        C16Scene c;
+        c.alpha = c.beta = c.gamma = c.stop = c.relres = 0.0;
+        c.total = c.outers = 0;
+        c.it = -1;
+        c.phase = SCN_RESID;
+        c.flip = 0;
+        scn[m] = c;
+    }
+    auto own = [&](uint32_t m) { return __ldg(S.tb + B.view(m).scene) == B.view(m).tile; };
+    auto count_open = [&] {  // thread 0
+        int n = 0;
+        for (uint32_t m = 0; m < B.ntiles; m++) n += scn[m].phase != SCN_DONE && own(m) ? 1 : 0;
+        open_s = n;
+    };
+    __syncthreads();
+    if (threadIdx.x == 0) count_open();
+    __syncthreads();
+    float2* zp = reinterpret_cast<float2*>(S.pub0);
+    float2* rq = reinterpret_cast<float2*>(S.pub1);
+    bool ok;
+    for (uint32_t round = 0;; round++) {
+        double* ts = S.tsum + (size_t)(round & 1u) * T * C16_SUMS;
+        auto index = [&](const C16View& t) { return (t.tile - blockIdx.x) / B.G; };
+        B.tiles(
+            [&](const C16View& n) {
+                const int ph = scn[index(n)].phase;
+                if (ph == SCN_RESID) B.ahead_residual(n);
+                else if (!LRN) c16_ahead_iterate(S, n);
+                else if (ph == SCN_PROD) c16_ahead_direction(S, n);
+                else c16_ahead_update(S, n);
+            },
+            [&](const C16View& t) {
+                const C16Scene& c = scn[index(t)];
+                double g[C16_SUMS] = {0.0, 0.0, 0.0};
+                if (c.phase == SCN_RESID) {
+                    float4* pc = c.flip ? S.pub1 : S.pub0;
+                    B.residual(t, g, [&](uint32_t k, double ri) {
+                        if (LRN) c16_start_row_learned(S, B, t, k, ri, rq);
+                        else c16_start_row(S, B, t, k, ri, pc);
+                    });
+                } else if (!LRN) {
+                    c16_iterate(S, B, t, c.alpha, c.beta, c.flip ? S.pub1 : S.pub0, c.flip ? S.pub0 : S.pub1, g);
+                } else if (c.phase == SCN_PROD) {
+                    c16_direction(S, B, t, (float)c.beta, zp, rq, g[0]);
+                } else {
+                    c16_update(S, B, t, c.alpha, zp, rq, g);
+                }
+                c16_tile_sum(g, ts + (size_t)t.tile * C16_SUMS);
+            },
+            [&](uint32_t m) { return scn[m].phase != SCN_DONE; });
+        const double open[1] = {threadIdx.x == 0 ? (double)open_s : 0.0};
+        double left[1];
+        ok = c16_sum<1>(open, sy, B.got(), left);
+        if (!ok || left[0] == 0.0) break;
+        // a scene's sums once for its consecutive tiles here; the others copy
+        auto leads = [&](uint32_t m) { return m == 0 || B.view(m - 1).scene != B.view(m).scene; };
+        for (uint32_t m = warp; m < B.ntiles; m += nw) {
+            if (scn[m].phase == SCN_DONE || !leads(m)) continue;
+            const uint32_t s = B.view(m).scene, t0 = __ldg(S.tb + s), t1 = __ldg(S.tb + s + 1);
+            double g[C16_SUMS] = {0.0, 0.0, 0.0};
+            for (uint32_t t = t0 + lane; t < t1; t += 32)
+#pragma unroll
+                for (int k = 0; k < (int)C16_SUMS; k++) g[k] += __ldcg(ts + (size_t)t * C16_SUMS + k);
+#pragma unroll
+            for (int k = 0; k < (int)C16_SUMS; k++) g[k] = warp_sum_d(g[k]);
+            if (lane == 0) {
+                bool failed = false;
+                c16_advance<LRN>(S, scn[m], g, &failed);
+                if (failed) atomicOr(&S.sc->err, ERR_CG_NOT_CONVERGED);
+            }
+        }
+        __syncthreads();
+        for (uint32_t m = threadIdx.x; m < B.ntiles; m += blockDim.x) {
+            uint32_t l = m;
+            while (!leads(l)) l--;
+            if (l != m) scn[m] = scn[l];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) count_open();
+        for (uint32_t m = threadIdx.x; m < B.ntiles; m += blockDim.x)
+            if (own(m)) {
+                const uint32_t s = B.view(m).scene;
+                S.iters[s] = scn[m].total;
+                S.outers[s] = scn[m].outers;
+                S.srel[s] = scn[m].relres;
+            }
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *S.epoch = sy.epoch + 2;
+        if (ok) {
+            int mi = 0, mo = 0;
+            double mr = 0.0;
+            for (uint32_t s = 0; s < S.ns; s++) {
+                mi = max(mi, __ldcg(S.iters + s));
+                mo = max(mo, __ldcg(S.outers + s));
+                mr = fmax(mr, __ldcg(S.srel + s));
+            }
+            S.sc->cg_iters = mi;
+            S.sc->cg_outer = mo;
+            S.sc->cg_relres = mr;
+        }
+    }
 }
 
 template <class T>
@@ -1550,6 +1914,8 @@ void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint3
     };
     std::vector<Key> order;
     order.reserve((size_t)nx * ny * nz);
+    cells->reserve(cells->size() + 4 * (size_t)nx * ny * nz);
+    nbr->reserve(nbr->size() + 27 * (size_t)nx * ny * nz);
     for (uint32_t z = 0; z < nz; z++)
         for (uint32_t y = 0; y < ny; y++)
             for (uint32_t x = 0; x < nx; x++) order.push_back({hilbert_index(x, y, z, bits), x, y, z});
@@ -1579,33 +1945,59 @@ void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint3
 // an SM's 228 KB stays L1 and the kernels' static arrays)
 size_t c16_page_bytes(uint32_t cap) { return (((size_t)cap + C16_PAGE - 1) / C16_PAGE + 1) * sizeof(uint16_t); }
 constexpr size_t C16_PAGE_BYTES_MAX = 160 * 1024;
+// row numbers a handle can need: a scene of a batch starts at a multiple of 8
+uint32_t c16_rows_cap(uint32_t cap, uint32_t ns) { return cap + 8u * ns; }
 constexpr size_t C16_SMEM = 220 * 1024;
 
 }  // namespace
 
-// the pack's page table is in shared memory: 20 M particles
-bool ppe_c16_takes(uint32_t cap, const Grid& grid) {
-    return grid.reach <= 2 && c16_page_bytes(cap) <= C16_PAGE_BYTES_MAX;
+static bool c16_solver_smem() {
+    for (const void* f : {(const void*)k_ppe_solve_c16<false>, (const void*)k_ppe_solve_c16<true>,
+                          (const void*)k_ppe_solve_c16_batch<false>, (const void*)k_ppe_solve_c16_batch<true>})
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C16_SMEM) != cudaSuccess)
+            return false;
+    return true;
 }
 
-int ppe_c16_enable(PpeWork& w, const Grid& grid, std::string* err) {
+// the pack's page table is in shared memory: 20 M particles
+bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
+    for (uint32_t s = 0; s < ngrids; s++)
+        if (grids[s].reach > 2) return false;
+    return c16_page_bytes(c16_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
+}
+
+int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* err) {
     if (w.c16_ready) return MPS_OK;
-    const size_t cap = w.cap;
-    if (!ppe_c16_takes(w.cap, grid)) {
+    const uint32_t ns = w.nscenes;
+    if (!ppe_c16_takes(w.cap, grids, ngrids)) {
         if (err) *err = "the compact PPE layout does not take this grid";
         return MPS_ERR_INVALID;
     }
+    const size_t cap = c16_rows_cap(w.cap, ns);
     const size_t vec = cap + 8;
     const size_t slices = (cap + C16_ROWS - 1) / C16_ROWS + 2;
     const size_t chunks = slices * ((PPE_W + 15) / 16);
-    const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms);
-    std::vector<uint32_t> cells, nbr;
-    linked_cells(grid, &cells, &nbr);
+    const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms, ns);
+    std::vector<uint32_t> cells, nbr, sfirst;
+    for (uint32_t s = 0; s < ngrids; s++) {
+        sfirst.push_back((uint32_t)(cells.size() / 4));
+        linked_cells(grids[s], &cells, &nbr);
+    }
+    sfirst.push_back((uint32_t)(cells.size() / 4));
     w.c16_nsuper = (uint32_t)(cells.size() / 4);
     bool ok = true;
     ok &= c16_alloc(&w.c16_cells, cells.size());
     ok &= c16_alloc(&w.c16_nbr, nbr.size());
     ok &= c16_alloc(&w.c16_base, (size_t)w.c16_nsuper + 2);
+    if (ns) {
+        ok &= c16_alloc(&w.c16_dense, (size_t)w.c16_nsuper + 2);
+        ok &= c16_alloc(&w.c16_sfirst, ns + 1);
+        ok &= c16_alloc(&w.c16_srow, ns + 1);
+        ok &= c16_alloc(&w.c16_tb, PPE_MAX_SCENES + 1);
+        ok &= c16_alloc(&w.c16_rowlist, vec);
+        ok &= c16_alloc(&w.c16_nrows, 1);
+        ok &= c16_alloc(&w.c16_tsum, 2 * tiles * C16_SUMS);
+    }
     ok &= c16_alloc(&w.cpos, cap);
     ok &= c16_alloc(&w.clen, vec);
     ok &= c16_alloc(&w.c16_off, slices + 2);
@@ -1634,16 +2026,14 @@ int ppe_c16_enable(PpeWork& w, const Grid& grid, std::string* err) {
     cudaMemset(w.c16_stats, 0, C16_STATS * sizeof(uint32_t));
     cudaMemset(w.c16_epoch, 0, sizeof(unsigned long long));
     cudaMemset(w.c16_slots, 0, 2 * (size_t)w.sms * w.sms * C16_SUMS * sizeof(ulonglong2));
-    if (cudaMemcpy(w.c16_cells, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+    if ((ns && cudaMemcpy(w.c16_sfirst, sfirst.data(), sfirst.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) ||
+        cudaMemcpy(w.c16_cells, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(w.c16_nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaFuncSetAttribute(k_c16_pack<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)C16_PAGE_BYTES_MAX) != cudaSuccess ||
         cudaFuncSetAttribute(k_c16_pack<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)C16_PAGE_BYTES_MAX) != cudaSuccess ||
-        cudaFuncSetAttribute(k_ppe_solve_c16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C16_SMEM) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_ppe_solve_c16_learned, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C16_SMEM) !=
-            cudaSuccess) {
+        !c16_solver_smem()) {
         ppe_c16_free(w);
         if (err) *err = "the compact PPE solver cannot have its shared memory";
         return MPS_ERR_CUDA;
@@ -1655,7 +2045,8 @@ int ppe_c16_enable(PpeWork& w, const Grid& grid, std::string* err) {
 void ppe_c16_free(PpeWork& w) {
     void* ps[] = {w.c16_cells, w.c16_nbr, w.c16_base, w.cpos, w.clen, w.c16_off, w.c16_ent, w.c16_side, w.c16_tile,
                   w.c16_collist, w.c16_stats, w.cb64, w.cx64, w.cdiag64, w.cdiag32, w.cinv_diag, w.cdsq, w.cr, w.cp,
-                  w.cpub[0], w.cpub[1], w.c16_slots, w.c16_epoch, w.c16_spfirst, w.c16_spent, w.c16_spside};
+                  w.cpub[0], w.cpub[1], w.c16_slots, w.c16_epoch, w.c16_dense, w.c16_sfirst, w.c16_srow, w.c16_tb,
+                  w.c16_rowlist, w.c16_nrows, w.c16_tsum, w.c16_spfirst, w.c16_spent, w.c16_spside};
     for (void* p : ps)
         if (p) cudaFree(p);
     w.c16_cells = w.c16_nbr = w.c16_base = w.cpos = w.clen = w.c16_off = w.c16_side = w.c16_tile = nullptr;
@@ -1665,6 +2056,8 @@ void ppe_c16_free(PpeWork& w) {
     w.cdiag32 = w.cinv_diag = w.cdsq = w.cr = w.cp = nullptr;
     w.cpub[0] = w.cpub[1] = nullptr;
     w.c16_slots = nullptr;
+    w.c16_dense = w.c16_sfirst = w.c16_srow = w.c16_tb = w.c16_rowlist = w.c16_nrows = nullptr;
+    w.c16_tsum = nullptr;
     w.c16_epoch = nullptr;
     w.c16_spfirst = w.c16_spent = w.c16_spside = nullptr;
     w.c16_ready = false;
@@ -1677,8 +2070,9 @@ int ppe_c16_learned_enable(PpeWork& w, std::string* err) {
     const int e = ppe_sp_enable(w, err);
     if (e != MPS_OK) return e;
     if (w.c16_spfirst) return MPS_OK;
-    const size_t tiles = c16_tiles(w.cap, (uint32_t)w.sms);
-    const size_t ent = ((size_t)w.cap / SP_SLICE + tiles + 1) * SP_SLICE * LP_GW;
+    const size_t cap = c16_rows_cap(w.cap, w.nscenes);
+    const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms, w.nscenes);
+    const size_t ent = (cap / SP_SLICE + tiles + 1) * SP_SLICE * LP_GW;
     bool ok = c16_alloc(&w.c16_spfirst, tiles * C16_SP_SLICES);
     ok &= c16_alloc(&w.c16_spent, ent);
     ok &= c16_alloc(&w.c16_spside, ent);
@@ -1689,6 +2083,12 @@ int ppe_c16_learned_enable(PpeWork& w, std::string* err) {
     return MPS_OK;
 }
 
+// the tiles' row list and count (a batch's have gaps, the others' do not)
+const uint32_t* ppe_c16_rowlist(const PpeWork& w) { return w.c16_rowlist ? w.c16_rowlist : w.rowlist; }
+const uint32_t* ppe_c16_nrows(const PpeWork& w) { return w.c16_nrows ? w.c16_nrows : w.nrows; }
+static uint32_t* c16_rowlist(PpeWork& w) { return const_cast<uint32_t*>(ppe_c16_rowlist(w)); }
+static uint32_t* c16_nrows(PpeWork& w) { return const_cast<uint32_t*>(ppe_c16_nrows(w)); }
+
 // The row numbers, before the assembly.
 int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st) {
     C16Flag F;
@@ -1698,24 +2098,45 @@ int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream
     F.sid_of_id = a.batch.n ? a.batch.sid_of_id : nullptr;
     F.scenes = a.batch.n ? w.scenes : nullptr;
     F.bthr = bthr;
+    uint32_t* counts = a.batch.n ? w.c16_dense : w.c16_base;
     k_c16_count<<<cblocks((w.c16_nsuper + 1) * 32u, 256), 256, 0, st>>>(F, w.c16_cells, w.c16_nsuper, a.cell_start,
-                                                                        w.c16_base, w.c16_stats);
-    launch_scan_exclusive(w.c16_base, w.c16_nsuper + 1, st);
-    k_c16_rows<<<cblocks(w.c16_nsuper * 32u, 256), 256, 0, st>>>(F, w.c16_cells, w.c16_nsuper, a.cell_start,
-                                                                 w.c16_base, w.cpos, w.rowlist, w.nrows, w.rlen,
-                                                                 w.diag64);
-    return 3;
+                                                                        counts, w.c16_stats);
+    launch_scan_exclusive(counts, w.c16_nsuper + 1, st);
+    C16RowArgs A;
+    A.cells = w.c16_cells;
+    A.cs = a.cell_start;
+    A.base = w.c16_base;
+    A.nsuper = w.c16_nsuper;
+    A.dense = a.batch.n ? w.c16_dense : nullptr;
+    A.cpos = w.cpos;
+    A.rowlist = c16_rowlist(w);
+    A.nrows = c16_nrows(w);
+    A.dense_list = w.rowlist;
+    A.dense_n = w.nrows;
+    A.rlen = w.rlen;
+    A.diag64 = w.diag64;
+    if (a.batch.n)
+        k_c16_shift<<<cblocks(w.c16_nsuper + 1, 256), 256, 0, st>>>(w.c16_dense, w.c16_nsuper, w.c16_sfirst, w.nscenes,
+                                                                    w.c16_base, w.c16_srow, A.rowlist, A.nrows);
+    k_c16_rows<<<cblocks(w.c16_nsuper * 32u, 256), 256, 0, st>>>(F, A);
+    return a.batch.n ? 4 : 3;
 }
 
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
-    const uint32_t maxslices = (cap + C16_ROWS - 1) / C16_ROWS;
-    k_c16_width<<<cblocks(C16_ROWS * (maxslices + 1), 256), 256, 0, st>>>(w.clen, w.nrows, w.c16_off, maxslices);
+    const uint32_t ns = w.nscenes, rows = c16_rows_cap(cap, ns);
+    const uint32_t maxslices = (rows + C16_ROWS - 1) / C16_ROWS;
+    k_c16_width<<<cblocks(C16_ROWS * (maxslices + 1), 256), 256, 0, st>>>(w.clen, c16_nrows(w), w.c16_off,
+                                                                          maxslices);
     launch_scan_exclusive(w.c16_off, maxslices + 1, st);
+    if (ns) k_c16_cut<<<1, 32, 0, st>>>(w.c16_off, w.c16_srow, c16_nrows(w), ns, (uint32_t)w.sms, w.c16_tb);
     C16PackArgs P;
     P.cols_rm = w.cols;
     P.w_rm = w.wrm;
     P.clen = w.clen;
-    P.nrows = w.nrows;
+    P.nrows = c16_nrows(w);
+    P.ns = ns;
+    P.srow = w.c16_srow;
+    P.tb = w.c16_tb;
     P.off = w.c16_off;
     P.base = w.c16_base;
     P.nbr = w.c16_nbr;
@@ -1726,7 +2147,7 @@ int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStrea
     P.ent = w.c16_ent;
     P.side = w.c16_side;
     P.stats = w.c16_stats;
-    P.rowlist = w.rowlist;
+    P.rowlist = c16_rowlist(w);
     P.cpos = w.cpos;
     P.idv = a.cur.id;
     P.index_of_id = w.index_of_id;
@@ -1740,15 +2161,21 @@ int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStrea
     P.sp_ent = w.c16_spent;
     P.sp_side = w.c16_spside;
     P.sp_diag = w.sp_diag;
-    const uint32_t tiles = c16_tiles(cap, (uint32_t)w.sms);
-    if (w.c16_learned) k_c16_pack<true><<<tiles, C16_PACK_THREADS, c16_page_bytes(cap), st>>>(P);
-    else k_c16_pack<false><<<tiles, C16_PACK_THREADS, c16_page_bytes(cap), st>>>(P);
-    return 3;
+    const uint32_t tiles = c16_tiles(rows, (uint32_t)w.sms, ns);
+    if (w.c16_learned) k_c16_pack<true><<<tiles, C16_PACK_THREADS, c16_page_bytes(rows), st>>>(P);
+    else k_c16_pack<false><<<tiles, C16_PACK_THREADS, c16_page_bytes(rows), st>>>(P);
+    return ns ? 4 : 3;
 }
 
 int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, uint32_t cap, cudaStream_t st) {
     C16Args S;
-    S.nrows = w.nrows;
+    S.nrows = c16_nrows(w);
+    S.ns = w.nscenes;
+    S.tb = w.c16_tb;
+    S.tsum = w.c16_tsum;
+    S.iters = w.scene_iters;
+    S.outers = w.scene_outer;
+    S.srel = w.scene_relres;
     S.off = w.c16_off;
     S.ent = w.c16_ent;
     S.side = w.c16_side;
@@ -1783,7 +2210,9 @@ int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt
     S.sp_side = w.c16_spside;
     S.sp_diag = w.sp_diag;
     void* args[] = {&S};
-    const void* fn = w.c16_learned ? (const void*)k_ppe_solve_c16_learned : (const void*)k_ppe_solve_c16;
+    const void* fn = w.nscenes ? (w.c16_learned ? (const void*)k_ppe_solve_c16_batch<true>
+                                                : (const void*)k_ppe_solve_c16_batch<false>)
+                               : (w.c16_learned ? (const void*)k_ppe_solve_c16<true> : (const void*)k_ppe_solve_c16<false>);
     w.launch_err = launch_cooperative_smem(fn, w.sms, C16_THREADS, C16_SMEM, args, st);
     if (!w.write_pressure) return 1;
     k_c16_finish<<<cblocks(cap, 256), 256, 0, st>>>(w.cx64, w.cpos, a.cur.press, a.sc);
@@ -1839,9 +2268,9 @@ int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream
 
 int ppe_c16_export(const PpeWork& w, uint32_t np, const uint32_t* d_row_start, uint32_t* d_cols, float* d_w,
                    cudaStream_t st) {
-    const uint32_t tiles = c16_tiles(np, (uint32_t)w.sms);
+    const uint32_t tiles = c16_tiles(c16_rows_cap(np, w.nscenes), (uint32_t)w.sms, w.nscenes);
     k_c16_export<<<tiles, 256, 0, st>>>(reinterpret_cast<const C16Tile*>(w.c16_tile), w.c16_collist, (uint32_t)w.sms,
-                                        w.clen, w.rowlist, w.nrows, w.c16_off, w.c16_ent, w.c16_side, d_row_start,
+                                        w.nscenes, w.clen, ppe_c16_rowlist(w), ppe_c16_nrows(w), w.c16_off, w.c16_ent, w.c16_side, d_row_start,
                                         d_cols, d_w);
     return MPS_OK;
 }
