@@ -417,6 +417,8 @@ static Grid device_grid(const HostGrid& hg, uint32_t base) {
     g.base = base;
     g.cell_yz = hg.cell_yz;
     g.reach = walk_reach(hg.cell_size, hg.cell_yz);
+    g.by_sheet = UDiv(g.sheet);
+    g.by_cdx = UDiv(g.cdx);
     return g;
 }
 

@@ -5,6 +5,20 @@
 
 namespace mpsb {
 
+// Division of a number below 2^31 by a divisor fixed on the host, 1 <= d < 2^31:
+// with 2^(s-1) < d <= 2^s and m = ceil(2^(31+s) / d) < 2^32, floor(n m / 2^(31+s)) is
+// floor(n / d) for every n < 2^31 (Granlund and Montgomery 1994, theorem 4.2):
+// a multiplication and a shift where a 32-bit division takes some 20 instructions.
+struct UDiv {
+    uint32_t m = 0, s = 0;
+    UDiv() = default;
+    explicit UDiv(uint32_t d) {
+        while ((1ull << s) < d) s++;
+        m = (uint32_t)(((1ull << (31 + s)) + d - 1) / d);
+    }
+    __device__ __forceinline__ uint32_t of(uint32_t n) const { return __umulhi(n << 1, m) >> s; }
+};
+
 // Cell grid of the reference's cell list (MPS_CAL_expl_v1.0/MPS.cpp:567-642).
 // The fast-arithmetic 3-D path halves the cells along y and z (cell_yz =
 // cell_size / 2, twice the cells along y and z, reach 2): a walk then visits
@@ -18,7 +32,8 @@ struct Grid {
     int dim;
     uint32_t base;  // first global cell id of this grid (scenes of a batch; 0 otherwise)
     float cell_yz;  // cell edge along y and z (cell_size along x)
-    int reach;      // cell rows walked on each side along y and z to cover cell_size
+    int reach;      // cell rows walked on each side along y and z to cover cell_size (1 or 2)
+    UDiv by_sheet, by_cdx;  // a cell's place in the grid (cell_near)
 };
 
 // Per-scene constants, fixed after initialisation.
@@ -160,8 +175,14 @@ struct RowRange { uint32_t lo, hi; };
 
 __device__ __forceinline__ void row_offsets(const Grid& g, int row, int* dz, int* dy) {
     const int w = 2 * g.reach + 1;
-    if (g.dim == 3) { *dz = row / w - g.reach; *dy = row % w - g.reach; }
-    else { *dz = 0; *dy = row - g.reach; }
+    if (g.dim == 3) {
+        const int q = (row * (w == 3 ? 22 : 13)) >> 6;  // row / w for rows 0 to 24 and w = 3 or 5
+        *dz = q - g.reach;
+        *dy = row - q * w - g.reach;
+    } else {
+        *dz = 0;
+        *dy = row - g.reach;
+    }
 }
 
 __device__ __forceinline__ RowRange link_row(const Grid& g, const uint32_t* __restrict__ cell_start, uint32_t c,
@@ -199,8 +220,8 @@ struct CellNear {
 };
 
 __device__ __forceinline__ CellNear cell_near(const Grid& g, uint32_t c, float x, float y, float z, float re) {
-    const uint32_t cz = c / g.sheet, rem = c - cz * g.sheet;
-    const uint32_t cy = rem / g.cdx, cx = rem - cy * g.cdx;
+    const uint32_t cz = g.by_sheet.of(c), rem = c - cz * g.sheet;
+    const uint32_t cy = g.by_cdx.of(rem), cx = rem - cy * g.cdx;
     const float x0 = g.left + g.cell_size * (float)cx;
     const float y0 = g.back + g.cell_yz * (float)cy;
     const float z0 = g.bottom + g.cell_yz * (float)cz;
@@ -276,15 +297,14 @@ __device__ __forceinline__ RowRange link_row_near_ref(const Grid& g, const uint3
 // A warp's walk over all its rows as one list of candidates.  Lane r looks
 // up row r (link_row_near; at most 25 rows, so one lookup per lane, all in
 // parallel), an inclusive scan of the row lengths numbers the candidates of
-// all rows in walk order (rows in order, indices ascending within a row),
-// and candidate f of that numbering is fetched with a 5-step search over the
-// lanes' row ends.  Every 32 consecutive candidates fill one batch of the
-// warp, whichever rows they come from, in the same order as the row-by-row
-// walk: ordered sums over the batches add the same terms in the same order.
+// all rows in walk order (rows in order, indices ascending within a row).
+// Every 32 consecutive candidates fill one batch of the warp, whichever rows
+// they come from, in the same order as the row-by-row walk: ordered sums
+// over the batches add the same terms in the same order.
 struct FlatWalk {
     uint32_t total;  // candidates over all rows
-    uint32_t end;    // this lane's row: one past its last candidate in walk order (total past the rows)
-    int base;        // this lane's row: particle index minus walk position
+    uint32_t start;  // first candidate of this lane's non-empty row in walk order (~0 past the rows)
+    int base;        // particle index minus walk position in that row
 };
 
 __device__ __forceinline__ FlatWalk flat_walk_of(RowRange rg, uint32_t lane) {
@@ -295,10 +315,18 @@ __device__ __forceinline__ FlatWalk flat_walk_of(RowRange rg, uint32_t lane) {
         const uint32_t t = __shfl_up_sync(0xffffffffu, e, o);
         if ((int)lane >= o) e += t;
     }
+    // the rows that hold candidates move to the first lanes, in their order
+    __shared__ uint2 moved[8][32];  // a warp's own 32; blocks that walk have at most 8 warps
+    uint2* mine = moved[threadIdx.x >> 5];
+    const uint32_t some = __ballot_sync(0xffffffffu, len > 0);
+    __syncwarp();
+    if (len > 0) mine[__popc(some & ((1u << lane) - 1u))] = make_uint2(e - len, rg.lo - (e - len));
+    __syncwarp();
+    const uint2 m = mine[lane];
     FlatWalk w;
     w.total = __shfl_sync(0xffffffffu, e, 31);
-    w.end = e;
-    w.base = (int)rg.lo - (int)(e - len);
+    w.start = (int)lane < __popc(some) ? m.x : 0xffffffffu;
+    w.base = (int)m.y;
     return w;
 }
 
@@ -309,15 +337,24 @@ __device__ __forceinline__ FlatWalk flat_walk(const Grid& g, const uint32_t* __r
     return flat_walk_of(rg, lane);
 }
 
-// the particle index of candidate f (f < total; every lane calls it)
-__device__ __forceinline__ uint32_t flat_at(const FlatWalk& w, uint32_t f) {
-    int r = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-        const uint32_t e = __shfl_sync(0xffffffffu, w.end, r + step - 1);
-        if (e <= f) r += step;
+// body(j, in) for each batch of 32 candidates of a walk.  A batch finds its
+// rows from one OR over the warp of the places at which a row starts in it:
+// the rows up to a candidate are those of the batches before and the bits up
+// to its lane.  One reduction and one shuffle a batch, where a search over
+// the rows' ends took six dependent shuffles.
+template <class F>
+__device__ __forceinline__ void flat_batches(const FlatWalk& w, uint32_t lane, F&& body) {
+    const uint32_t upto = 0xffffffffu >> (31u - lane);
+    int r0 = -1;  // the row of the candidate before the batch
+    for (uint32_t f0 = 0; f0 < w.total; f0 += 32) {
+        const uint32_t at = w.start - f0;
+        const uint32_t starts = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+        const int r = r0 + __popc(starts & upto);
+        r0 += __popc(starts);
+        const int base = __shfl_sync(0xffffffffu, w.base, r);
+        const bool in = f0 + lane < w.total;
+        body((uint32_t)((int)min(f0 + lane, w.total - 1u) + base), in);  // past the end: the last one again
     }
-    return (uint32_t)((int)f + __shfl_sync(0xffffffffu, w.base, r));
 }
 
 // body(j, in) for each batch of 32 candidates of a warp's walk, in walk
@@ -333,11 +370,7 @@ template <bool FLAT, class F>
 __device__ __forceinline__ void walk_cells(const Grid& g, const uint32_t* __restrict__ cs, uint32_t c,
                                            const CellNear& nr, uint32_t lane, F&& body) {
     if (FLAT) {
-        const FlatWalk fw = flat_walk(g, cs, c, nr, lane);
-        for (uint32_t f0 = 0; f0 < fw.total; f0 += 32) {
-            const bool in = f0 + lane < fw.total;
-            body(flat_at(fw, in ? f0 + lane : fw.total - 1), in);
-        }
+        flat_batches(flat_walk(g, cs, c, nr, lane), lane, body);
     } else {
         const int rows = g.dim == 3 ? 9 : 3;
         for (int row = 0; row < rows; row++) {

@@ -402,6 +402,38 @@ __device__ __forceinline__ float warp_tree_add(float v) {
     return v;
 }
 
+// one level of warp_tree_add for two values: lanes without the bit go on with
+// a, lanes with it with b
+__device__ __forceinline__ float fold2(uint32_t lane, uint32_t bit, float a, float b) {
+    const bool up = lane & bit;
+    return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, bit);
+}
+
+// warp_tree_add of x, y and z for lane 0, the same additions with 8 shuffles for 15
+__device__ __forceinline__ void warp_tree_add3(uint32_t lane, float& x, float& y, float& z) {
+    float v = fold2(lane, 8, fold2(lane, 16, x, y), z + __shfl_xor_sync(0xffffffffu, z, 16));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    x = v;  // x in lane 0, y in lane 16, z in lane 8
+    y = __shfl_sync(0xffffffffu, v, 16);
+    z = __shfl_sync(0xffffffffu, v, 8);
+}
+
+// warp_tree_add of two particles' x, y and z, the first's for lane 0 and the
+// second's for lane 16: 10 shuffles for 30
+__device__ __forceinline__ void warp_tree_add3x2(uint32_t lane, float& x1, float& y1, float& z1, float x2, float y2,
+                                                 float z2) {
+    const float xy = fold2(lane, 8, fold2(lane, 16, x1, x2), fold2(lane, 16, y1, y2));
+    float z = fold2(lane, 16, z1, z2);
+    z += __shfl_xor_sync(0xffffffffu, z, 8);
+    float v = fold2(lane, 4, xy, z);
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    x1 = v;  // x in lanes 0 and 16, y 8 lanes on, z 4 lanes on
+    y1 = __shfl_sync(0xffffffffu, v, (lane & 16u) + 8u);
+    z1 = __shfl_sync(0xffffffffu, v, (lane & 16u) + 4u);
+}
+
 template <bool EX, bool ORD, bool BT>
 __global__ void __launch_bounds__(256) k_visc_w(StageArgs a, const uint32_t* __restrict__ list,
                                                 const uint32_t* __restrict__ list_n) {
@@ -442,7 +474,7 @@ __global__ void __launch_bounds__(256) k_visc_w(StageArgs a, const uint32_t* __r
             else { ax += tx; ay += ty; az += tz; }
         }
     });
-    if (!ORD) { ax = warp_tree_add(ax); ay = warp_tree_add(ay); az = warp_tree_add(az); }
+    if (!ORD) warp_tree_add3(lane, ax, ay, az);
     if (lane != 0) return;
     const float dt = dt_of<BT>(a, L.s);
     float gx, gy, gz;
@@ -526,11 +558,7 @@ __global__ void __launch_bounds__(256, BT ? 3 : 5) k_visc_w2(StageArgs a, const 
                 row_offsets(L1.g, (int)lane, &dz, &dy);
                 ru = union_row(dz, dy);
             }
-            const FlatWalk fw = flat_walk_of(ru, lane);
-            for (uint32_t f0 = 0; f0 < fw.total; f0 += 32) {
-                const bool in = f0 + lane < fw.total;
-                both(flat_at(fw, in ? f0 + lane : fw.total - 1), in);
-            }
+            flat_batches(flat_walk_of(ru, lane), lane, both);
         } else {
             const int R = L1.g.reach, nz = L1.g.dim == 3 ? R : 0;
             for (int dz = -nz; dz <= nz; dz++)
@@ -553,14 +581,12 @@ __global__ void __launch_bounds__(256, BT ? 3 : 5) k_visc_w2(StageArgs a, const 
             else walk_cells<false>(L.g, L.cs, L.c, nr, lane, one);
         }
     }
-    a1x = warp_tree_add(a1x); a1y = warp_tree_add(a1y); a1z = warp_tree_add(a1z);
-    a2x = warp_tree_add(a2x); a2y = warp_tree_add(a2y); a2z = warp_tree_add(a2z);
-    if (lane > 1 || (lane == 1 && !two)) return;
+    warp_tree_add3x2(lane, a1x, a1y, a1z, a2x, a2y, a2z);
+    if ((lane & 15u) || (lane && !two)) return;
     const uint32_t i = lane ? i2 : i1;
     const float4 ui = lane ? u2 : u1;
     const Local& L = lane ? L2 : L1;
     const Phys Pi = phys_of<BT>(a, L.s);
-    const float ax = lane ? a2x : a1x, ay = lane ? a2y : a1y, az = lane ? a2z : a1z;
     const float dt = dt_of<BT>(a, L.s);
     float gx, gy, gz;
     if (BT) {
@@ -569,7 +595,7 @@ __global__ void __launch_bounds__(256, BT ? 3 : 5) k_visc_w2(StageArgs a, const 
     } else {
         gx = a.sc->g_eff[0]; gy = a.sc->g_eff[1]; gz = a.sc->g_eff[2];
     }
-    const float lx = Pi.c_lap * ax, ly = Pi.c_lap * ay, lz = Pi.c_lap * az;
+    const float lx = Pi.c_lap * a1x, ly = Pi.c_lap * a1y, lz = Pi.c_lap * a1z;
     float4 t;
     t.x = ui.x + dt * (Pi.niu * lx + gx);
     t.y = ui.y + dt * (Pi.niu * ly + gy);
@@ -624,7 +650,7 @@ __global__ void __launch_bounds__(256) k_collision_w(StageArgs a, const uint32_t
             else { cx += tx; cy += ty; cz += tz; }
         }
     });
-    if (!ORD) { cx = warp_tree_add(cx); cy = warp_tree_add(cy); cz = warp_tree_add(cz); }
+    if (!ORD) warp_tree_add3(lane, cx, cy, cz);
     if (lane == 0) a.tmp[i] = make_float4(cx, cy, cz, 0.f);
 }
 
@@ -754,7 +780,7 @@ __global__ void __launch_bounds__(256) k_dash_w(StageArgs a, const uint32_t* __r
     } else {
         walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, grad);
     }
-    if (!ORD) { gx = warp_tree_add(gx); gy = warp_tree_add(gy); gz = warp_tree_add(gz); }
+    if (!ORD) warp_tree_add3(lane, gx, gy, gz);
     if (lane != 0) return;
     const float cg = fmul<EX>(P.dim_f, P.one_over_nzero);
     const float kk = fmul<EX>(-dt_of<BT>(a, L.s), P.one_over_rho);
