@@ -671,13 +671,11 @@ __global__ void __launch_bounds__(256) k_pnd_w(StageArgs a, int eos, int all_typ
     const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
     walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
         {
-            float w = 0.f;
-            if (in && j != i) {
-                const float4 pj = __ldg(pos + j);
-                const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
-                const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
-                if (rr < thr) w = weight_rr<EX>(re, rr);
-            }
+            // the flat walk's lists have no place that cannot be read: no branches (113 -> 109 us at 310,912)
+            const float4 pj = __ldg(pos + (!EX || in ? j : i));
+            const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
+            const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
+            const float w = in && j != i && rr < thr ? weight_rr<EX>(re, rr) : 0.f;
             if (ORD) ordered_add1<true>(reinterpret_cast<float*>(obuf), lane, w != 0.f, w, acc);
             else acc += w;
         }

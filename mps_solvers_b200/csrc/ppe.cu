@@ -41,41 +41,19 @@ struct AsmArgs {
     unsigned* bar;
     double n0, lambda, beta, b_tmp, rho_lambda_alpha_n0, dim2;
     const PpeScene* scenes;  // per scene of a batch (these constants otherwise)
-    // the compact layout (C16): rows in its order, columns as row numbers,
-    // the rows' vectors by row; the particle-indexed arrays above then hold
-    // only what other code reads of them (rlen, diag64)
-    const uint32_t* rowlist;
-    const uint32_t* nrows;
-    const uint32_t* cpos;
-    uint32_t* clen;
-    double *cb64, *cx64, *cdiag64;
-    float *cdiag32, *cinv_diag, *cdsq;
 };
 
 // One warp per particle: scan the reference's 27 linked cells for rlap
 // neighbours of type != 2, accumulate the diagonal, append the non-Dirichlet
 // ones in ascending index order (MPS_CAL_v4.0/MPS_CPU.cpp:651-698).
-template <bool EX, bool BT, bool C16>
+template <bool EX, bool BT>
 __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
     const StageArgs& a = A.a;
     const uint32_t n = a.sc->np;
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // row (C16) or particle
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (blockIdx.x == 0 && threadIdx.x == 0) A.bar[0] = 0u;  // the solver's barrier starts empty
-    if (k >= (C16 ? *A.nrows : n)) return;
-    const uint32_t i = C16 ? __ldg(A.rowlist + k) : k;
-    if (C16 && BT && i == PPE_DIRICHLET) {  // a gap between two scenes' rows: an identity row with b = 0
-        if (lane == 0) {
-            A.clen[k] = 0;
-            A.cdiag64[k] = -1.0;
-            A.cdiag32[k] = -1.f;
-            A.cinv_diag[k] = -1.f;
-            A.cdsq[k] = 1.f;
-            A.cb64[k] = 0.0;
-            A.cx64[k] = 0.0;
-        }
-        return;
-    }
+    if (i >= n) return;
     const float4* __restrict__ pos = a.cur.pos;
     const float* __restrict__ nn = a.cur.n;
     const float4 pi = pos[i];
@@ -90,7 +68,7 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
         rlan0 = ps.rho_lambda_alpha_n0;
     }
     const bool dir_i = ptype(pi) == T_DUMMY || ni < beta * n0;
-    if (!C16 && dir_i) {
+    if (dir_i) {
         if (lane == 0) {
             A.rlen[i] = PPE_DIRICHLET;
             A.diag64[i] = 1.0;
@@ -109,8 +87,8 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
     // n_j < bthr (double) exactly when n_j < bthr_f, the least float >= bthr
     float bthr_f = (float)bthr;
     if ((double)bthr_f < bthr) bthr_f = nextafterf(bthr_f, INFINITY);
-    uint32_t* cols = A.cols + (size_t)k * PPE_W;
-    float* wrow = A.wrm + (size_t)k * PPE_W;
+    uint32_t* cols = A.cols + (size_t)i * PPE_W;
+    float* wrow = A.wrm + (size_t)i * PPE_W;
     uint32_t count = 0;
     float diag_lane = 0.f;  // this lane's few nonzero weights, then a FP64 warp sum
     const uint32_t lt = (1u << lane) - 1u;
@@ -119,7 +97,6 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
         {
             bool app = false;
             float w = 0.f;
-            uint32_t col = j;
             if (in && j != i) {
                 const float4 pj = __ldg(pos + j);
                 if (ptype(pj) != T_DUMMY) {
@@ -127,14 +104,7 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
                     const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
                     if (rr < thr) {
                         w = weight_rr<EX>(re, rr);
-                        if (w > 0.f) {
-                            if (C16) {
-                                col = __ldg(A.cpos + j);
-                                app = col != PPE_DIRICHLET;
-                            } else {
-                                app = !(__ldg(nn + j) < bthr_f);
-                            }
-                        }
+                        if (w > 0.f) app = !(__ldg(nn + j) < bthr_f);
                     }
                 }
             }
@@ -143,7 +113,7 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
             if (app) {
                 const uint32_t at = count + __popc(m & lt);
                 if (at < PPE_W) {
-                    cols[at] = col;
+                    cols[at] = j;
                     wrow[at] = w;
                 }
             }
@@ -159,20 +129,10 @@ __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
         const double dg = -diag - Aii;
         A.rlen[i] = count;
         A.diag64[i] = dg;
-        if (C16) {
-            A.clen[k] = count;
-            A.cdiag64[k] = dg;
-            A.cdiag32[k] = (float)dg;
-            A.cinv_diag[k] = (float)(1.0 / dg);
-            A.cdsq[k] = (float)(1.0 / sqrt(-dg));
-            A.cb64[k] = b_tmp * (n0 - ni);
-            A.cx64[k] = (double)a.cur.press[i];
-        } else {
-            A.diag32[i] = (float)dg;
-            A.inv_diag[i] = (float)(1.0 / dg);
-            A.b64[i] = b_tmp * (n0 - ni);
-            A.x64[i] = (double)a.cur.press[i];
-        }
+        A.diag32[i] = (float)dg;
+        A.inv_diag[i] = (float)(1.0 / dg);
+        A.b64[i] = b_tmp * (n0 - ni);
+        A.x64[i] = (double)a.cur.press[i];
     }
 }
 
@@ -1654,36 +1614,27 @@ int ppe_enqueue_setup(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     A.rho_lambda_alpha_n0 = rho * w.lambda64 * alpha * w.n0_64;
     A.dim2 = 2.0 * dim;
     A.scenes = w.scenes;
-    A.rowlist = ppe_c16_rowlist(w);
-    A.nrows = ppe_c16_nrows(w);
-    A.cpos = w.cpos;
-    A.clen = w.clen;
-    A.cb64 = w.cb64;
-    A.cx64 = w.cx64;
-    A.cdiag64 = w.cdiag64;
-    A.cdiag32 = w.cdiag32;
-    A.cinv_diag = w.cinv_diag;
-    A.cdsq = w.cdsq;
     const bool c16 = w.c16;
-    const uint32_t warps_blocks = blocks_for((c16 ? a.cap_solid + 8u * w.nscenes : cap) * 32u, 256);
-    int launched = 1;
+    int launched = 0;
     if (c16) {
-        launched += ppe_c16_enqueue_rows(w, a, A.beta * A.n0, st);
-        if (a.batch.n) {
-            if (a.exact) k_ppe_assemble<true, true, true><<<warps_blocks, 256, 0, st>>>(A);
-            else k_ppe_assemble<false, true, true><<<warps_blocks, 256, 0, st>>>(A);
-        } else {
-            if (a.exact) k_ppe_assemble<true, false, true><<<warps_blocks, 256, 0, st>>>(A);
-            else k_ppe_assemble<false, false, true><<<warps_blocks, 256, 0, st>>>(A);
-        }
-    } else if (a.batch.n) {
-        if (a.exact) k_ppe_assemble<true, true, false><<<warps_blocks, 256, 0, st>>>(A);
-        else k_ppe_assemble<false, true, false><<<warps_blocks, 256, 0, st>>>(A);
+        C16Assemble K;
+        K.n0 = A.n0;
+        K.beta = A.beta;
+        K.b_tmp = A.b_tmp;
+        K.rho_lambda_alpha_n0 = A.rho_lambda_alpha_n0;
+        K.dim2 = A.dim2;
+        launched += ppe_c16_enqueue_assemble(w, a, K, cap, st);
     } else {
-        if (a.exact) k_ppe_assemble<true, false, false><<<warps_blocks, 256, 0, st>>>(A);
-        else k_ppe_assemble<false, false, false><<<warps_blocks, 256, 0, st>>>(A);
+        const uint32_t blocks = blocks_for(cap * 32u, 256);
+        if (a.batch.n) {
+            if (a.exact) k_ppe_assemble<true, true><<<blocks, 256, 0, st>>>(A);
+            else k_ppe_assemble<false, true><<<blocks, 256, 0, st>>>(A);
+        } else {
+            if (a.exact) k_ppe_assemble<true, false><<<blocks, 256, 0, st>>>(A);
+            else k_ppe_assemble<false, false><<<blocks, 256, 0, st>>>(A);
+        }
+        launched += 1 + enqueue_rows_pack(w, a, cap, st);
     }
-    if (!c16) launched += enqueue_rows_pack(w, a, cap, st);
     // the state this system was assembled from
     cudaMemcpyAsync(w.pos_snap, a.cur.pos, (size_t)cap * sizeof(float4), cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(w.n_snap, a.cur.n, (size_t)cap * sizeof(float), cudaMemcpyDeviceToDevice, st);

@@ -177,11 +177,12 @@ int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint3
 // escaped-entry count of the last pack, and the stencil export.
 bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids);
 int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* err);
-const uint32_t* ppe_c16_rowlist(const PpeWork& w);
-const uint32_t* ppe_c16_nrows(const PpeWork& w);
-// the row numbers, before the assembly (bthr = beta n0; a batch uses its
-// scenes' own)
-int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st);
+// the PPE's constants (a batch uses its scenes' own; dim2 is the same for all)
+struct C16Assemble {
+    double n0, beta, b_tmp, rho_lambda_alpha_n0, dim2;
+};
+// the row numbers, the rows' entries, diagonals and vectors
+int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& K, uint32_t cap, cudaStream_t st);
 int ppe_c16_learned_enable(PpeWork& w, std::string* err);
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st);
 int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, uint32_t cap, cudaStream_t st);

@@ -220,16 +220,141 @@ __global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, C16RowArgs A) {
     }
 }
 
-// Chunks of every slice (the longest of its 8 rows), then scanned.
-__global__ void __launch_bounds__(256) k_c16_width(const uint32_t* __restrict__ clen, const uint32_t* __restrict__ nrows,
-                                                   uint32_t* __restrict__ width, uint32_t maxslices) {
-    const uint32_t R = *nrows;
+// ---------------------------------------------------------------- assembly
+struct C16AsmArgs {
+    StageArgs a;
+    C16Assemble K;
+    const PpeScene* scenes;
+    const uint32_t* rowlist;
+    const uint32_t* nrows;
+    const uint32_t* cpos;
+    uint32_t* cols;   // row-major, PPE_W a row
+    float* wrm;
+    uint32_t* clen;
+    uint32_t* rlen;   // by particle: entries of its row
+    unsigned* bar;
+    double *diag64, *cb64, *cx64, *cdiag64;
+    float *cdiag32, *cinv_diag, *cdsq;
+    uint32_t* width;
+    uint32_t maxslices;
+};
+
+// A warp a row: the neighbours within rlap of type != 2 in ascending particle
+// index, those with rows appended as row numbers, every weight added to the
+// diagonal (MPS_CAL_v4.0/MPS_CPU.cpp:651-698).  Bound by issued instructions:
+// of some 640 candidates a third is within rlap.  The walk only tests a
+// candidate; the hits collect in shared memory, and every 32 of them are
+// weighed, looked up and appended together.  136,582 rows: 300 -> 240 us
+// against all of it for every batch of candidates, with the row's divisions
+// (now k_c16_rowend's, a thread a row).  Two and four rows a warp over the
+// union of their candidates take fewer instructions and more registers:
+// 20 us slower and 60 us slower.
+template <bool EX, bool BT>
+__global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
+    __shared__ __align__(512) char hits[8 * 512];  // a warp's hits (particle, r^2): a ring of two halves of 32
+    const StageArgs& a = A.a;
+    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.bar[0] = 0u;  // the 8-byte solvers' barrier starts empty
+    if (k >= *A.nrows) return;
+    const uint32_t i = __ldg(A.rowlist + k);
+    if (BT && i == C16_NONE) return;  // a gap between two scenes' rows
+    const uint32_t mine = (threadIdx.x >> 5) * 512u;
+    auto hit_at = [&](uint32_t n) -> float2& { return *reinterpret_cast<float2*>(hits + ((n * 8u & 511u) | mine)); };
+    const float4* __restrict__ pos = a.cur.pos;
+    const float4 pi = pos[i];
+    const Local L = local_of<BT>(a, i);
+    const Phys P = phys_of<BT>(a, L.s);
+    const float re = P.rlap, thr = P.rlap_thr;
+    uint32_t* cols = A.cols + (size_t)k * PPE_W;
+    float* wrow = A.wrm + (size_t)k * PPE_W;
+    uint32_t found = 0, count = 0;
+    float diag_lane = 0.f;  // a lane's few weights, then a FP64 sum over the warp
+    auto weigh = [&](uint32_t at, uint32_t m) {
+        __syncwarp();
+        const float2 h = hit_at(at + lane);
+        float w = 0.f;
+        uint32_t col = PPE_DIRICHLET;
+        if (lane < m) {
+            w = weight_rr<EX>(re, h.y);
+            if (w > 0.f) col = __ldg(A.cpos + __float_as_uint(h.x));
+        }
+        diag_lane += w;
+        const uint32_t ma = __ballot_sync(0xffffffffu, col != PPE_DIRICHLET);
+        const uint32_t to = count + __popc(ma & lt);
+        if (col != PPE_DIRICHLET && to < PPE_W) {
+            cols[to] = col;
+            wrow[to] = w;
+        }
+        count += __popc(ma);
+    };
+    const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
+    flat_batches(flat_walk(L.g, L.cs, L.c, nr, lane), lane, [&](uint32_t j, bool in) {
+        const float4 pj = __ldg(pos + j);
+        const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
+        const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
+        const bool hit = in && ptype(pj) != T_DUMMY && rr < thr && j != i;
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        if (hit) hit_at(found + __popc(m & lt)) = make_float2(__uint_as_float(j), rr);
+        const uint32_t was = found;
+        found += __popc(m);
+        if ((found ^ was) & 32u) weigh(was & 32u, 32u);
+    });
+    weigh(found & 32u, found & 31u);
+    const double d = warp_sum_d((double)diag_lane);
+    if (lane) return;
+    if (count > PPE_W) {
+        atomicOr(&a.sc->err, ERR_CAPACITY);  // more than PPE_W neighbours
+        count = PPE_W;
+    }
+    A.clen[k] = count;
+    A.rlen[i] = count;
+    A.cdiag64[k] = d;
+}
+
+// A thread a row: its diagonal from the weights' sum and its vectors; and the
+// chunks of every slice (the longest of its 8 rows), scanned next.  A gap
+// between two scenes' rows is an identity row with b = 0.
+template <bool BT>
+__global__ void __launch_bounds__(256) k_c16_rowend(C16AsmArgs A) {
+    const StageArgs& a = A.a;
+    const uint32_t R = *A.nrows;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t len = k < R ? clen[k] : 0u;
+    const uint32_t i = k < R ? A.rowlist[k] : C16_NONE;
+    uint32_t len = 0;
+    if (i != C16_NONE) {
+        len = A.clen[k];
+        double n0 = A.K.n0, b_tmp = A.K.b_tmp, rlan0 = A.K.rho_lambda_alpha_n0;
+        uint32_t s = 0;
+        if (BT) {
+            s = a.batch.sid_of_id[a.cur.id[i]];
+            const PpeScene& ps = A.scenes[s];
+            n0 = ps.n0;
+            b_tmp = ps.b_tmp;
+            rlan0 = ps.rho_lambda_alpha_n0;
+        }
+        const double dt = (double)dt_of<BT>(a, s);
+        const double dg = -A.cdiag64[k] - rlan0 / (A.K.dim2 * dt * dt);
+        A.diag64[i] = dg;
+        A.cdiag64[k] = dg;
+        A.cdiag32[k] = (float)dg;
+        A.cinv_diag[k] = (float)(1.0 / dg);
+        A.cdsq[k] = (float)(1.0 / sqrt(-dg));
+        A.cb64[k] = b_tmp * (n0 - (double)a.cur.n[i]);
+        A.cx64[k] = (double)a.cur.press[i];
+    } else if (BT && k < R) {
+        A.clen[k] = 0;
+        A.cdiag64[k] = -1.0;
+        A.cdiag32[k] = -1.f;
+        A.cinv_diag[k] = -1.f;
+        A.cdsq[k] = 1.f;
+        A.cb64[k] = 0.0;
+        A.cx64[k] = 0.0;
+    }
 #pragma unroll
     for (int o = 1; o < (int)C16_ROWS; o <<= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
     const uint32_t s = k / C16_ROWS;
-    if (k % C16_ROWS == 0 && s <= maxslices) width[s] = (len + 15u) / 16u;
+    if (k % C16_ROWS == 0 && s <= A.maxslices) A.width[s] = (len + 15u) / 16u;
 }
 
 // Weight of the slices before s when tiles are cut.
@@ -2084,13 +2209,13 @@ int ppe_c16_learned_enable(PpeWork& w, std::string* err) {
 }
 
 // the tiles' row list and count (a batch's have gaps, the others' do not)
-const uint32_t* ppe_c16_rowlist(const PpeWork& w) { return w.c16_rowlist ? w.c16_rowlist : w.rowlist; }
-const uint32_t* ppe_c16_nrows(const PpeWork& w) { return w.c16_nrows ? w.c16_nrows : w.nrows; }
+static const uint32_t* ppe_c16_rowlist(const PpeWork& w) { return w.c16_rowlist ? w.c16_rowlist : w.rowlist; }
+static const uint32_t* ppe_c16_nrows(const PpeWork& w) { return w.c16_nrows ? w.c16_nrows : w.nrows; }
 static uint32_t* c16_rowlist(PpeWork& w) { return const_cast<uint32_t*>(ppe_c16_rowlist(w)); }
 static uint32_t* c16_nrows(PpeWork& w) { return const_cast<uint32_t*>(ppe_c16_nrows(w)); }
 
-// The row numbers, before the assembly.
-int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st) {
+// The row numbers.
+static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st) {
     C16Flag F;
     F.pos = a.cur.pos;
     F.n = a.cur.n;
@@ -2122,11 +2247,50 @@ int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream
     return a.batch.n ? 4 : 3;
 }
 
+static uint32_t c16_maxslices(const PpeWork& w, uint32_t cap) {
+    return (c16_rows_cap(cap, w.nscenes) + C16_ROWS - 1) / C16_ROWS;
+}
+
+int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& K, uint32_t cap, cudaStream_t st) {
+    const int launched = ppe_c16_enqueue_rows(w, a, K.beta * K.n0, st);
+    C16AsmArgs A;
+    A.a = a;
+    A.K = K;
+    A.scenes = w.scenes;
+    A.rowlist = c16_rowlist(w);
+    A.nrows = c16_nrows(w);
+    A.cpos = w.cpos;
+    A.cols = w.cols;
+    A.wrm = w.wrm;
+    A.clen = w.clen;
+    A.rlen = w.rlen;
+    A.bar = w.bar;
+    A.diag64 = w.diag64;
+    A.cb64 = w.cb64;
+    A.cx64 = w.cx64;
+    A.cdiag64 = w.cdiag64;
+    A.cdiag32 = w.cdiag32;
+    A.cinv_diag = w.cinv_diag;
+    A.cdsq = w.cdsq;
+    A.width = w.c16_off;
+    A.maxslices = c16_maxslices(w, cap);
+    // a.cap_solid: particles that can have rows (not dummies)
+    const uint32_t blocks = cblocks(c16_rows_cap(a.cap_solid, w.nscenes) * 32u, 256);
+    const uint32_t eblocks = cblocks(C16_ROWS * (A.maxslices + 1), 256);
+    if (a.batch.n) {
+        if (a.exact) k_c16_assemble<true, true><<<blocks, 256, 0, st>>>(A);
+        else k_c16_assemble<false, true><<<blocks, 256, 0, st>>>(A);
+        k_c16_rowend<true><<<eblocks, 256, 0, st>>>(A);
+    } else {
+        if (a.exact) k_c16_assemble<true, false><<<blocks, 256, 0, st>>>(A);
+        else k_c16_assemble<false, false><<<blocks, 256, 0, st>>>(A);
+        k_c16_rowend<false><<<eblocks, 256, 0, st>>>(A);
+    }
+    return launched + 2;
+}
+
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
-    const uint32_t ns = w.nscenes, rows = c16_rows_cap(cap, ns);
-    const uint32_t maxslices = (rows + C16_ROWS - 1) / C16_ROWS;
-    k_c16_width<<<cblocks(C16_ROWS * (maxslices + 1), 256), 256, 0, st>>>(w.clen, c16_nrows(w), w.c16_off,
-                                                                          maxslices);
+    const uint32_t ns = w.nscenes, rows = c16_rows_cap(cap, ns), maxslices = c16_maxslices(w, cap);
     launch_scan_exclusive(w.c16_off, maxslices + 1, st);
     if (ns) k_c16_cut<<<1, 32, 0, st>>>(w.c16_off, w.c16_srow, c16_nrows(w), ns, (uint32_t)w.sms, w.c16_tb);
     C16PackArgs P;
@@ -2164,7 +2328,7 @@ int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStrea
     const uint32_t tiles = c16_tiles(rows, (uint32_t)w.sms, ns);
     if (w.c16_learned) k_c16_pack<true><<<tiles, C16_PACK_THREADS, c16_page_bytes(rows), st>>>(P);
     else k_c16_pack<false><<<tiles, C16_PACK_THREADS, c16_page_bytes(rows), st>>>(P);
-    return ns ? 4 : 3;
+    return ns ? 3 : 2;
 }
 
 int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, uint32_t cap, cudaStream_t st) {

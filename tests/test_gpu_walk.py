@@ -1,8 +1,7 @@
 """The warps' walk over the linked cells (mps_device.cuh: flat_batches) and the
-tile layout's assembly, two rows a warp (ppe_compact.cu), against sums over
-all pairs in double precision: grids whose edges no power of two divides,
-cells with one particle and with a dozen, warps whose two rows are in one cell
-and in two, a last warp with one row.
+tile layout's assembly on it (ppe_compact.cu), against sums over all pairs in
+double precision: grids whose edges no power of two divides, cells with none,
+one and a dozen particles, few rows and many.
 
 A weight re/r - 1 comes from 2-ulp reciprocal square roots of r^2 (relative
 error 1.5e-7 from the rounded differences): at most 5e-7 re/r.  A sum of up
