@@ -357,15 +357,42 @@ __device__ __forceinline__ void flat_batches(const FlatWalk& w, uint32_t lane, F
     }
 }
 
+// The hits of a walk (particle, r^2), 32 at a time: a warp's ring of two
+// halves of 32 in shared memory, 512 bytes aligned to as much.  Every lane
+// calls add for every batch of candidates; work(at, n) is called with each
+// full half (n = 32) and reads its hits with get(at + lane); the caller ends
+// with work(found & 32, found & 31).
+struct HitRing {
+    char* ring;
+    uint32_t found = 0;
+    __device__ __forceinline__ explicit HitRing(char* warps_ring) : ring(warps_ring) {}
+    __device__ __forceinline__ float2& get(uint32_t n) const { return *reinterpret_cast<float2*>(ring + (n * 8u & 511u)); }
+    template <class F>
+    __device__ __forceinline__ void add(uint32_t lane, bool hit, uint32_t j, float rr, F&& work) {
+        const uint32_t m = __ballot_sync(0xffffffffu, hit), was = found;
+        if (hit) get(found + __popc(m & ((1u << lane) - 1u))) = make_float2(__uint_as_float(j), rr);
+        found += __popc(m);
+        if ((found ^ was) & 32u) {
+            __syncwarp();
+            work(was & 32u, 32u);
+        }
+    }
+    template <class F>
+    __device__ __forceinline__ void rest(F&& work) {
+        __syncwarp();
+        work(found & 32u, found & 31u);
+    }
+};
+
 // body(j, in) for each batch of 32 candidates of a warp's walk, in walk
 // order (lane L gets the batch's L-th candidate; `in` is false past the
 // end).  FLAT walks the rows as one list (flat_walk: the rows' lookups in
 // parallel, full batches) on any grid; the other form walks the reference's
 // grid (reach 1) row by row.  Both visit the same candidates in the same
-// order.  The flat form pays on the refined grid (up to 25 short rows); on
-// the reference's grid (9 rows of about 200 candidates) the row form is as
-// fast and is what the exact kernels use: exact arithmetic keeps the
-// reference's grid (the refined one is built for fast arithmetic only).
+// order.  Sums over the lanes depend on the batches, so exact arithmetic
+// without ordered sums (the semi-implicit method: rows of about 200
+// candidates, where the row form is as fast) keeps the row form; ordered sums
+// do not, and on the explicit method's rows of about 28 the list is faster.
 template <bool FLAT, class F>
 __device__ __forceinline__ void walk_cells(const Grid& g, const uint32_t* __restrict__ cs, uint32_t c,
                                            const CellNear& nr, uint32_t lane, F&& body) {

@@ -357,20 +357,6 @@ __device__ __forceinline__ WarpTask warp_task(const StageArgs& a, const uint32_t
 // additions as a loop over the hits, without a shuffle chain every lane runs.
 // Only lane 0's sums are the result.  buf holds 32 entries per warp.
 template <bool EX>
-__device__ __forceinline__ void ordered_add1(float* buf, uint32_t lane, bool hit, float t, float& acc) {
-    const uint32_t m = __ballot_sync(0xffffffffu, hit);
-    if (m == 0u) return;
-    if (hit) buf[__popc(m & ((1u << lane) - 1u))] = t;
-    __syncwarp();
-    if (lane == 0) {
-        const int nh = __popc(m);
-#pragma unroll 4
-        for (int k = 0; k < nh; k++) acc = fadd<EX>(acc, buf[k]);
-    }
-    __syncwarp();
-}
-
-template <bool EX>
 __device__ __forceinline__ void ordered_add3(float4* buf, uint32_t lane, bool hit, float tx, float ty, float tz,
                                              float& ax, float& ay, float& az) {
     const uint32_t m = __ballot_sync(0xffffffffu, hit);
@@ -388,6 +374,53 @@ __device__ __forceinline__ void ordered_add3(float4* buf, uint32_t lane, bool hi
         }
     }
     __syncwarp();
+}
+
+// Ordered sums of the first n lanes' terms in lane order; the others give 0
+// (which changes no sum).  Every lane adds them all, four a load; of three
+// components lane c adds component c.  With the hits of several batches of
+// candidates together (HitRing), and the exact square roots and divisions done
+// for them alone, PND at 70,912 particles took 44 us for 56, viscosity 42 for 59
+// (a third of it the linked cells' rows as one list).
+__device__ __forceinline__ void ordered_sum1(float4* buf, uint32_t lane, uint32_t n, float t, float& acc) {
+    reinterpret_cast<float*>(buf)[lane] = t;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++) {
+        if (4u * k >= n) break;
+        const float4 v = buf[k];
+        acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ void ordered_sum3(float4* buf, uint32_t lane, uint32_t n, float tx, float ty, float tz, float& acc) {
+    float* f = reinterpret_cast<float*>(buf);
+    f[lane] = tx;
+    f[32 + lane] = ty;
+    f[64 + lane] = tz;
+    __syncwarp();
+    const float4* mine = buf + (lane < 3u ? lane * 8u : 0u);
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++) {
+        if (4u * k >= n) break;
+        const float4 v = mine[k];
+        acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+    }
+    __syncwarp();
+}
+
+// the components of an ordered_sum3 for lane 0
+__device__ __forceinline__ void ordered_gather3(float acc, float& x, float& y, float& z) {
+    x = acc;
+    y = __shfl_sync(0xffffffffu, acc, 1);
+    z = __shfl_sync(0xffffffffu, acc, 2);
+}
+
+// the warp's ring of hits (blocks of up to 256 threads)
+__device__ __forceinline__ char* hit_ring() {
+    __shared__ __align__(512) char rings[8][512];
+    return rings[(threadIdx.x >> 5) & 7u];
 }
 
 // the warp's 32-entry buffer for ordered sums (blocks of up to 256 threads)
@@ -451,30 +484,52 @@ __global__ void __launch_bounds__(256) k_visc_w(StageArgs a, const uint32_t* __r
     float ax = 0.f, ay = 0.f, az = 0.f;
     float4* obuf = ordered_buf();
     const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
-    walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
-        {
+    if constexpr (ORD) {
+        HitRing hits(hit_ring());
+        float acc = 0.f;
+        auto laplace = [&](uint32_t at, uint32_t m) {
             float tx = 0.f, ty = 0.f, tz = 0.f;
-            bool hit = false;
-            if (in && j != i) {
-                const float4 pj = __ldg(pos + j);
-                const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
-                const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
-                if (rr < thr) {
-                    const float w = weight_rr<EX>(re, rr);
-                    if (w != 0.f) {
-                        const float4 uj = __ldg(vel + j);
-                        tx = fmul<EX>(w, fsub<EX>(uj.x, ui.x));
-                        ty = fmul<EX>(w, fsub<EX>(uj.y, ui.y));
-                        tz = fmul<EX>(w, fsub<EX>(uj.z, ui.z));
-                        hit = true;
+            const float2 h = hits.get(at + lane);
+            const float w = lane < m ? weight_rr<true>(re, h.y) : 0.f;
+            if (w != 0.f) {
+                const float4 uj = __ldg(vel + __float_as_uint(h.x));
+                tx = __fmul_rn(w, __fsub_rn(uj.x, ui.x));
+                ty = __fmul_rn(w, __fsub_rn(uj.y, ui.y));
+                tz = __fmul_rn(w, __fsub_rn(uj.z, ui.z));
+            }
+            ordered_sum3(obuf, lane, m, tx, ty, tz, acc);
+        };
+        walk_cells<true>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
+            const float4 pj = __ldg(pos + j);
+            const float dx = __fsub_rn(pj.x, pi.x), dy = __fsub_rn(pj.y, pi.y), dz = __fsub_rn(pj.z, pi.z);
+            const float rr = dot3<true>(dx, dy, dz, dx, dy, dz);
+            hits.add(lane, in && j != i && rr < thr, j, rr, laplace);
+        });
+        hits.rest(laplace);
+        ordered_gather3(acc, ax, ay, az);
+    } else {
+        walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
+            {
+                float tx = 0.f, ty = 0.f, tz = 0.f;
+                if (in && j != i) {
+                    const float4 pj = __ldg(pos + j);
+                    const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
+                    const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
+                    if (rr < thr) {
+                        const float w = weight_rr<EX>(re, rr);
+                        if (w != 0.f) {
+                            const float4 uj = __ldg(vel + j);
+                            tx = fmul<EX>(w, fsub<EX>(uj.x, ui.x));
+                            ty = fmul<EX>(w, fsub<EX>(uj.y, ui.y));
+                            tz = fmul<EX>(w, fsub<EX>(uj.z, ui.z));
+                        }
                     }
                 }
+                ax += tx; ay += ty; az += tz;
             }
-            if (ORD) ordered_add3<true>(obuf, lane, hit, tx, ty, tz, ax, ay, az);
-            else { ax += tx; ay += ty; az += tz; }
-        }
-    });
-    if (!ORD) warp_tree_add3(lane, ax, ay, az);
+        });
+        warp_tree_add3(lane, ax, ay, az);
+    }
     if (lane != 0) return;
     const float dt = dt_of<BT>(a, L.s);
     float gx, gy, gz;
@@ -620,7 +675,7 @@ __global__ void __launch_bounds__(256) k_collision_w(StageArgs a, const uint32_t
     const Local L = local_of<BT>(a, i);
     const Phys P = phys_of<BT>(a, L.s);
     const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, P.col_dis);
-    walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
+    walk_cells<!EX || ORD>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
         {
             float tx = 0.f, ty = 0.f, tz = 0.f;
             bool hit = false;
@@ -669,18 +724,29 @@ __global__ void __launch_bounds__(256) k_pnd_w(StageArgs a, int eos, int all_typ
     float acc = 0.f;
     float4* obuf = ordered_buf();
     const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
-    walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
-        {
+    if constexpr (ORD) {
+        HitRing hits(hit_ring());
+        auto weigh = [&](uint32_t at, uint32_t m) {
+            const float2 h = hits.get(at + lane);
+            ordered_sum1(obuf, lane, m, lane < m ? weight_rr<true>(re, h.y) : 0.f, acc);
+        };
+        walk_cells<true>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
+            const float4 pj = __ldg(pos + j);
+            const float dx = __fsub_rn(pj.x, pi.x), dy = __fsub_rn(pj.y, pi.y), dz = __fsub_rn(pj.z, pi.z);
+            const float rr = dot3<true>(dx, dy, dz, dx, dy, dz);
+            hits.add(lane, in && j != i && rr < thr, j, rr, weigh);
+        });
+        hits.rest(weigh);
+    } else {
+        walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
             // the flat walk's lists have no place that cannot be read: no branches (113 -> 109 us at 310,912)
             const float4 pj = __ldg(pos + (!EX || in ? j : i));
             const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
             const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
-            const float w = in && j != i && rr < thr ? weight_rr<EX>(re, rr) : 0.f;
-            if (ORD) ordered_add1<true>(reinterpret_cast<float*>(obuf), lane, w != 0.f, w, acc);
-            else acc += w;
-        }
-    });
-    if (!ORD) acc = warp_tree_add(acc);
+            acc += in && j != i && rr < thr ? weight_rr<EX>(re, rr) : 0.f;
+        });
+        acc = warp_tree_add(acc);
+    }
     if (lane != 0) return;
     a.cur.n[i] = acc;
     if (eos) {
@@ -714,7 +780,7 @@ __global__ void __launch_bounds__(256) k_dash_w(StageArgs a, const uint32_t* __r
     const uint32_t lt = (1u << lane) - 1u;
     uint32_t nhit = 0;
     float hat = press[i];
-    walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
+    walk_cells<!EX || ORD>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
         {
             bool near = false;
             if (in) {
@@ -740,15 +806,14 @@ __global__ void __launch_bounds__(256) k_dash_w(StageArgs a, const uint32_t* __r
     for (int o = 16; o > 0; o >>= 1) hat = fminf(hat, __shfl_xor_sync(0xffffffffu, hat, o));
     const float re = P.rzero, thr = P.rzero_thr;
     const bool skip_dummy = a.semi != 0;
-    float gx = 0.f, gy = 0.f, gz = 0.f;
+    float gx = 0.f, gy = 0.f, gz = 0.f, gacc = 0.f;
     float4* obuf = ordered_buf();
     // the gradient's terms: candidates of the kept slots, in the same
     // ascending order as the cell walk, or the cell walk itself
     const bool slotted = nhit <= DASH_SLOTS;
-    auto grad = [&](uint32_t j, bool in) {
+    auto grad = [&](uint32_t j, bool in, uint32_t n) {  // n candidates in this batch's first lanes
         {
             float tx = 0.f, ty = 0.f, tz = 0.f;
-            bool hit = false;
             if (in && j != i) {
                 const float4 pj = __ldg(pos + j);
                 if (!(skip_dummy && ptype(pj) == T_DUMMY)) {
@@ -761,24 +826,24 @@ __global__ void __launch_bounds__(256) k_dash_w(StageArgs a, const uint32_t* __r
                             tx = fmul<EX>(k, dx);
                             ty = fmul<EX>(k, dy);
                             tz = fmul<EX>(k, dz);
-                            hit = true;
                         }
                     }
                 }
             }
-            if (ORD) ordered_add3<true>(obuf, lane, hit, tx, ty, tz, gx, gy, gz);
+            if (ORD) ordered_sum3(obuf, lane, n, tx, ty, tz, gacc);
             else { gx += tx; gy += ty; gz += tz; }
         }
     };
     if (slotted) {
         for (uint32_t f0 = 0; f0 < nhit; f0 += 32) {
             const bool in = f0 + lane < nhit;
-            grad(in ? my[f0 + lane] : 0xFFFFFFFFu, in);
+            grad(in ? my[f0 + lane] : 0xFFFFFFFFu, in, min(nhit - f0, 32u));
         }
     } else {
-        walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, grad);
+        walk_cells<!EX || ORD>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) { grad(j, in, 32u); });
     }
-    if (!ORD) warp_tree_add3(lane, gx, gy, gz);
+    if (ORD) ordered_gather3(gacc, gx, gy, gz);
+    else warp_tree_add3(lane, gx, gy, gz);
     if (lane != 0) return;
     const float cg = fmul<EX>(P.dim_f, P.one_over_nzero);
     const float kk = fmul<EX>(-dt_of<BT>(a, L.s), P.one_over_rho);

@@ -251,7 +251,7 @@ struct C16AsmArgs {
 // 20 us slower and 60 us slower.
 template <bool EX, bool BT>
 __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
-    __shared__ __align__(512) char hits[8 * 512];  // a warp's hits (particle, r^2): a ring of two halves of 32
+    __shared__ __align__(512) char rings[8][512];
     const StageArgs& a = A.a;
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
     const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -259,8 +259,7 @@ __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
     if (k >= *A.nrows) return;
     const uint32_t i = __ldg(A.rowlist + k);
     if (BT && i == C16_NONE) return;  // a gap between two scenes' rows
-    const uint32_t mine = (threadIdx.x >> 5) * 512u;
-    auto hit_at = [&](uint32_t n) -> float2& { return *reinterpret_cast<float2*>(hits + ((n * 8u & 511u) | mine)); };
+    HitRing hits(rings[threadIdx.x >> 5]);
     const float4* __restrict__ pos = a.cur.pos;
     const float4 pi = pos[i];
     const Local L = local_of<BT>(a, i);
@@ -268,11 +267,10 @@ __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
     const float re = P.rlap, thr = P.rlap_thr;
     uint32_t* cols = A.cols + (size_t)k * PPE_W;
     float* wrow = A.wrm + (size_t)k * PPE_W;
-    uint32_t found = 0, count = 0;
+    uint32_t count = 0;
     float diag_lane = 0.f;  // a lane's few weights, then a FP64 sum over the warp
     auto weigh = [&](uint32_t at, uint32_t m) {
-        __syncwarp();
-        const float2 h = hit_at(at + lane);
+        const float2 h = hits.get(at + lane);
         float w = 0.f;
         uint32_t col = PPE_DIRICHLET;
         if (lane < m) {
@@ -294,13 +292,9 @@ __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
         const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
         const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
         const bool hit = in && ptype(pj) != T_DUMMY && rr < thr && j != i;
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (hit) hit_at(found + __popc(m & lt)) = make_float2(__uint_as_float(j), rr);
-        const uint32_t was = found;
-        found += __popc(m);
-        if ((found ^ was) & 32u) weigh(was & 32u, 32u);
+        hits.add(lane, hit, j, rr, weigh);
     });
-    weigh(found & 32u, found & 31u);
+    hits.rest(weigh);
     const double d = warp_sum_d((double)diag_lane);
     if (lane) return;
     if (count > PPE_W) {
