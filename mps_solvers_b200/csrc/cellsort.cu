@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_keys_upsweep(const float4* __r
                                                                uint32_t* __restrict__ vals,
                                                                const uint32_t* __restrict__ id, BatchDev batch,
                                                                uint32_t* __restrict__ hist, uint32_t tiles) {
+    after_previous();
     __shared__ uint32_t h[SORT_RADIX];
     const uint32_t n = sc->np;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_keys_upsweep_plain(const float
 __global__ void __launch_bounds__(SORT_THREADS) k_radix_upsweep(const uint32_t* __restrict__ keys,
                                                                 const uint32_t* __restrict__ n_dev, int shift,
                                                                 uint32_t* __restrict__ hist, uint32_t tiles) {
+    after_previous();
     __shared__ uint32_t h[SORT_RADIX];
     const uint32_t n = *n_dev;
     for (int d = threadIdx.x; d < SORT_RADIX; d += SORT_THREADS) h[d] = 0;
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_radix_upsweep(const uint32_t* 
 // turn took 12 us for 152 tiles (310,912 keys), 38 us for 787; this takes
 // 3.0 and 4.5 us.
 __global__ void __launch_bounds__(256) k_radix_scan(uint32_t* __restrict__ hist, uint32_t tiles) {
+    after_previous();
     const uint32_t d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (d >= (uint32_t)SORT_RADIX) return;
     uint32_t* row = hist + (size_t)d * tiles;
@@ -158,6 +161,7 @@ __global__ void __launch_bounds__(256) k_radix_scan(uint32_t* __restrict__ hist,
 // array starts 16-byte aligned), a block scan of the thread sums, and a
 // running carry between chunks.
 __global__ void __launch_bounds__(1024) k_scan_exclusive(uint32_t* __restrict__ a, uint32_t total) {
+    after_previous();
     __shared__ uint32_t warp_sums[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t carry = 0;
@@ -232,6 +236,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_radix_downsweep(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, const uint32_t* __restrict__ hist, const uint32_t* __restrict__ n_dev, int shift,
     uint32_t tiles, int scanned) {
+    after_previous();
     constexpr int WARPS = SORT_THREADS / 32;
     static_assert(SORT_THREADS == SORT_RADIX, "one digit per thread");
     __shared__ uint32_t warp_hist[WARPS][SORT_RADIX];
@@ -326,6 +331,7 @@ __global__ void __launch_bounds__(256) k_merge_keys(const float4* __restrict__ p
                                                     int apply, Grid g, Scalars* __restrict__ sc,
                                                     const uint32_t* __restrict__ id, BatchDev batch,
                                                     const uint32_t* __restrict__ cell_old, MergeScratch m) {
+    after_previous();
     const uint32_t n = sc->np;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->n_fluid = 0;  // the merge gather refills the particle lists
@@ -372,6 +378,7 @@ __device__ __forceinline__ void block_bitonic(T* x, uint32_t P) {
 // shared memory; more (a state set from the host that moved many particles
 // across cells) in the scratch arrays themselves, sized for every particle.
 __global__ void __launch_bounds__(MERGE_SORT_THREADS) k_merge_sort(MergeScratch m) {
+    after_previous();
     extern __shared__ uint64_t msh[];
     const uint32_t cnt = *(volatile uint32_t*)&m.count[0];
     __syncthreads();
@@ -439,8 +446,8 @@ cudaError_t merge_sort_setup() {
 void launch_merge_keys_sort(const float4* pos, const float4* tmp, int apply, const Grid& g, Scalars* sc,
                             const uint32_t* id, const BatchDev& batch, const uint32_t* cell_old,
                             const MergeScratch& m, uint32_t cap, cudaStream_t st) {
-    k_merge_keys<<<(cap + 255) / 256, 256, 0, st>>>(pos, tmp, apply, g, sc, id, batch, cell_old, m);
-    k_merge_sort<<<1, MERGE_SORT_THREADS, MERGE_SMEM_CAP * (sizeof(uint64_t) + sizeof(uint32_t)), st>>>(m);
+    launch(k_merge_keys, (cap + 255) / 256, 256, 0, st, pos, tmp, apply, g, sc, id, batch, cell_old, m);
+    launch(k_merge_sort, 1, MERGE_SORT_THREADS, MERGE_SMEM_CAP * (sizeof(uint64_t) + sizeof(uint32_t)), st, m);
 }
 
 // ---------------------------------------------------------------- cell tables
@@ -475,13 +482,13 @@ static int radix_passes(SortScratch& s, const uint32_t* n_dev, int passes, cudaS
     for (int p = 0; p < passes; p++) {
         const int shift = 8 * p;
         if (p > 0)
-            k_radix_upsweep<<<s.tiles, SORT_THREADS, 0, st>>>(s.keys[cur], n_dev, shift, s.hist, s.tiles);
+            launch(k_radix_upsweep, s.tiles, SORT_THREADS, 0, st, s.keys[cur], n_dev, shift, s.hist, s.tiles);
         // few tiles: each downsweep block scans the histograms itself (one
         // launch less per pass); many: one scan kernel
         const int scanned = s.tiles > SORT_FUSED_SCAN_TILES;
-        if (scanned) k_radix_scan<<<SORT_RADIX / 8, 256, 0, st>>>(s.hist, s.tiles);
-        k_radix_downsweep<<<s.tiles, SORT_THREADS, 0, st>>>(s.keys[cur], s.vals[cur], s.keys[cur ^ 1],
-                                                             s.vals[cur ^ 1], s.hist, n_dev, shift, s.tiles, scanned);
+        if (scanned) launch(k_radix_scan, SORT_RADIX / 8, 256, 0, st, s.hist, s.tiles);
+        launch(k_radix_downsweep, s.tiles, SORT_THREADS, 0, st, s.keys[cur], s.vals[cur], s.keys[cur ^ 1],
+               s.vals[cur ^ 1], s.hist, n_dev, shift, s.tiles, scanned);
         cur ^= 1;
     }
     return cur;
@@ -489,13 +496,13 @@ static int radix_passes(SortScratch& s, const uint32_t* n_dev, int passes, cudaS
 
 int launch_keys_and_sort(const float4* pos, const float4* tmp, int apply, const Grid& g, Scalars* sc,
                          const uint32_t* id, const BatchDev& batch, SortScratch& s, int passes, cudaStream_t st) {
-    k_keys_upsweep<<<s.tiles, SORT_THREADS, 0, st>>>(pos, tmp, apply, g, sc, s.keys[0], s.vals[0], id, batch, s.hist,
-                                                     s.tiles);
+    launch(k_keys_upsweep, s.tiles, SORT_THREADS, 0, st, pos, tmp, apply, g, sc, s.keys[0], s.vals[0], id, batch,
+           s.hist, s.tiles);
     return radix_passes(s, &sc->np, passes, st);
 }
 
 void launch_scan_exclusive(uint32_t* a, uint32_t total, cudaStream_t st) {
-    k_scan_exclusive<<<1, 1024, 0, st>>>(a, total);
+    launch(k_scan_exclusive, 1, 1024, 0, st, a, total);
 }
 
 

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(256) k_gather(State src, State dst, const uint
                                                 uint32_t* __restrict__ index_of_id, Scalars* __restrict__ sc,
                                                 uint32_t* __restrict__ list_fluid, uint32_t* __restrict__ list_solid,
                                                 BatchDev batch, uint32_t* __restrict__ cell_start, uint32_t ncells) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     // the cell table (one thread per sorted position and one past the end)
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(256) k_merge_gather(State src, State dst, cons
                                                       uint32_t* __restrict__ index_of_id, Scalars* __restrict__ sc,
                                                       uint32_t* __restrict__ list_fluid,
                                                       uint32_t* __restrict__ list_solid, BatchDev batch) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t m = count[1];
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -206,17 +208,16 @@ void launch_merge_gather(const State& src, const State& dst, const MergeScratch&
                          Scalars* sc, uint32_t cap, cudaStream_t st, uint32_t* list_fluid, uint32_t* list_solid,
                          const BatchDev& batch) {
     const uint32_t threads = cap > ncells + 1 ? cap : ncells + 1;
-    k_merge_gather<<<blocks_for(threads, 256), 256, 0, st>>>(src, dst, m.newkey, m.a, m.b, m.count, cs_old, cs_new,
-                                                              ncells, tmp, apply, index_of_id, sc, list_fluid,
-                                                              list_solid, batch);
+    launch(k_merge_gather, blocks_for(threads, 256), 256, 0, st, src, dst, m.newkey, m.a, m.b, m.count, cs_old, cs_new,
+           ncells, tmp, apply, index_of_id, sc, list_fluid, list_solid, batch);
 }
 
 void launch_gather(const State& src, const State& dst, const uint32_t* perm, const uint32_t* keys_sorted,
                    const float4* tmp, int apply, uint32_t* index_of_id, Scalars* sc, uint32_t cap, cudaStream_t st,
                    uint32_t* list_fluid, uint32_t* list_solid, const BatchDev& batch, uint32_t* cell_start,
                    uint32_t ncells) {
-    k_gather<<<blocks_for(cap + 1, 256), 256, 0, st>>>(src, dst, perm, keys_sorted, tmp, apply, index_of_id, sc,
-                                                        list_fluid, list_solid, batch, cell_start, ncells);
+    launch(k_gather, blocks_for(cap + 1, 256), 256, 0, st, src, dst, perm, keys_sorted, tmp, apply, index_of_id, sc,
+           list_fluid, list_solid, batch, cell_start, ncells);
 }
 
 // ---------------------------------------------------------------- update_dt
@@ -225,6 +226,7 @@ void launch_gather(const State& src, const State& dst, const uint32_t* perm, con
 // rounded to float), capped at dt_max.  The minimum over particles is the
 // value at the largest |u|^2, so a max-reduction of |u|^2 gives the same dt.
 __global__ void __launch_bounds__(256) k_update_dt(const float4* __restrict__ vel, Phys P, Scalars* __restrict__ sc) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t m = 0;
@@ -260,6 +262,7 @@ __global__ void __launch_bounds__(256) k_update_dt(const float4* __restrict__ ve
 // and constants, and its body force at its own time.
 __global__ void __launch_bounds__(256) k_update_dt_batch(const float4* __restrict__ vel, const uint32_t* __restrict__ id,
                                                          BatchDev b, Scalars* __restrict__ sc) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
@@ -310,18 +313,21 @@ __global__ void __launch_bounds__(256) k_update_dt_batch(const float4* __restric
 }
 
 void launch_update_dt(const StageArgs& a, uint32_t cap, cudaStream_t st) {
-    if (a.batch.n) k_update_dt_batch<<<blocks_for(cap, 256), 256, 0, st>>>(a.cur.vel, a.cur.id, a.batch, a.sc);
-    else k_update_dt<<<blocks_for(cap, 256), 256, 0, st>>>(a.cur.vel, a.P, a.sc);
+    if (a.batch.n) launch(k_update_dt_batch, blocks_for(cap, 256), 256, 0, st, a.cur.vel, a.cur.id, a.batch, a.sc);
+    else launch(k_update_dt, blocks_for(cap, 256), 256, 0, st, a.cur.vel, a.P, a.sc);
 }
 
 __global__ void k_step_end(Scalars* sc, BatchDev b) {
+    after_previous();
     sc->time = __fadd_rn(sc->time, sc->dt);
     sc->step += 1;
     for (uint32_t s = 0; s < b.n; s++) b.time[s] = __fadd_rn(b.time[s], b.dt[s]);
     if (b.n) sc->time = b.time[0];
 }
 
-void launch_step_end(Scalars* sc, const BatchDev& batch, cudaStream_t st) { k_step_end<<<1, 1, 0, st>>>(sc, batch); }
+void launch_step_end(Scalars* sc, const BatchDev& batch, cudaStream_t st) {
+    launch(k_step_end, 1, 1, 0, st, sc, batch);
+}
 
 // ---------------------------------------------------------------- warp per particle
 // One warp per particle; lane l takes candidate j = base + l of each row
@@ -470,6 +476,7 @@ __device__ __forceinline__ void warp_tree_add3x2(uint32_t lane, float& x1, float
 template <bool EX, bool ORD, bool BT>
 __global__ void __launch_bounds__(256) k_visc_w(StageArgs a, const uint32_t* __restrict__ list,
                                                 const uint32_t* __restrict__ list_n) {
+    after_previous();
     const WarpTask tk = warp_task(a, list, list_n);
     if (!tk.ok) return;
     const uint32_t i = tk.i, lane = threadIdx.x & 31;
@@ -557,6 +564,7 @@ __global__ void __launch_bounds__(256) k_visc_w(StageArgs a, const uint32_t* __r
 template <bool BT>  // single scenes: 5 blocks an SM (48 registers) measured 5 % faster than 4
 __global__ void __launch_bounds__(256, BT ? 3 : 5) k_visc_w2(StageArgs a, const uint32_t* __restrict__ list,
                                                  const uint32_t* __restrict__ list_n) {
+    after_previous();
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nl = *list_n;
@@ -662,6 +670,7 @@ __global__ void __launch_bounds__(256, BT ? 3 : 5) k_visc_w2(StageArgs a, const 
 template <bool EX, bool ORD, bool BT>
 __global__ void __launch_bounds__(256) k_collision_w(StageArgs a, const uint32_t* __restrict__ list,
                                                      const uint32_t* __restrict__ list_n) {
+    after_previous();
     const WarpTask tk = warp_task(a, list, list_n);
     if (!tk.ok) return;
     const uint32_t i = tk.i, lane = threadIdx.x & 31;
@@ -712,6 +721,7 @@ __global__ void __launch_bounds__(256) k_collision_w(StageArgs a, const uint32_t
 template <bool EX, bool ORD, bool BT>
 __global__ void __launch_bounds__(256) k_pnd_w(StageArgs a, int eos, int all_types, const uint32_t* __restrict__ list,
                                                const uint32_t* __restrict__ list_n) {
+    after_previous();
     const WarpTask tk = warp_task(a, list, list_n);
     if (!tk.ok) return;
     const uint32_t i = tk.i, lane = threadIdx.x & 31;
@@ -760,6 +770,7 @@ constexpr uint32_t DASH_SLOTS = 64;  // neighbours within r0 kept per particle (
 template <bool EX, bool ORD, bool BT>
 __global__ void __launch_bounds__(256) k_dash_w(StageArgs a, const uint32_t* __restrict__ list,
                                                 const uint32_t* __restrict__ list_n) {
+    after_previous();
     const WarpTask tk = warp_task(a, list, list_n);
     if (!tk.ok) return;
     const uint32_t i = tk.i, lane = threadIdx.x & 31;
@@ -860,15 +871,15 @@ void launch_visc(const StageArgs& a, uint32_t cap, cudaStream_t st) {
     const uint32_t nb2 = blocks_for((a.cap_fluid + 1) / 2 * 32u, (uint32_t)a.threads);  // two particles a warp
     const bool ord = a.exact && !a.semi;
     if (a.batch.n) {
-        if (a.exact && ord) k_visc_w<true, true, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.exact) k_visc_w<true, false, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.list_fluid) k_visc_w2<true><<<nb2, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else k_visc_w<false, false, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
+        if (a.exact && ord) launch(k_visc_w<true, true, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.exact) launch(k_visc_w<true, false, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.list_fluid) launch(k_visc_w2<true>, nb2, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else launch(k_visc_w<false, false, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
     } else {
-        if (a.exact && ord) k_visc_w<true, true, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.exact) k_visc_w<true, false, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.list_fluid) k_visc_w2<false><<<nb2, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else k_visc_w<false, false, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
+        if (a.exact && ord) launch(k_visc_w<true, true, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.exact) launch(k_visc_w<true, false, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.list_fluid) launch(k_visc_w2<false>, nb2, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else launch(k_visc_w<false, false, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
     }
 }
 
@@ -880,13 +891,14 @@ void launch_collision(const StageArgs& a, uint32_t cap, cudaStream_t st) {
     const uint32_t nb = blocks_for((a.list_fluid ? a.cap_fluid : cap) * 32u, (uint32_t)a.threads);
     const bool ord = a.exact && !a.semi;
     if (a.batch.n) {
-        if (a.exact && ord) k_collision_w<true, true, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.exact) k_collision_w<true, false, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else k_collision_w<false, false, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
+        if (a.exact && ord) launch(k_collision_w<true, true, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.exact) launch(k_collision_w<true, false, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else launch(k_collision_w<false, false, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
     } else {
-        if (a.exact && ord) k_collision_w<true, true, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.exact) k_collision_w<true, false, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else k_collision_w<false, false, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
+        if (a.exact && ord) launch(k_collision_w<true, true, false>, nb, a.threads, 0, st, a, a.list_fluid,
+                                   a.n_fluid);
+        else if (a.exact) launch(k_collision_w<true, false, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else launch(k_collision_w<false, false, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
     }
 }
 
@@ -901,13 +913,17 @@ void launch_pnd(const StageArgs& a, int eos, int all_types, uint32_t cap, cudaSt
     const uint32_t nb = blocks_for((use_list ? a.cap_solid : cap) * 32u, (uint32_t)a.threads);
     const bool ord = a.exact && !a.semi;
     if (a.batch.n) {
-        if (a.exact && ord) k_pnd_w<true, true, true><<<nb, a.threads, 0, st>>>(a, eos, all_types, list, a.n_solid);
-        else if (a.exact) k_pnd_w<true, false, true><<<nb, a.threads, 0, st>>>(a, eos, all_types, list, a.n_solid);
-        else k_pnd_w<false, false, true><<<nb, a.threads, 0, st>>>(a, eos, all_types, list, a.n_solid);
+        if (a.exact && ord) launch(k_pnd_w<true, true, true>, nb, a.threads, 0, st, a, eos, all_types, list,
+                                   a.n_solid);
+        else if (a.exact) launch(k_pnd_w<true, false, true>, nb, a.threads, 0, st, a, eos, all_types, list,
+                                 a.n_solid);
+        else launch(k_pnd_w<false, false, true>, nb, a.threads, 0, st, a, eos, all_types, list, a.n_solid);
     } else {
-        if (a.exact && ord) k_pnd_w<true, true, false><<<nb, a.threads, 0, st>>>(a, eos, all_types, list, a.n_solid);
-        else if (a.exact) k_pnd_w<true, false, false><<<nb, a.threads, 0, st>>>(a, eos, all_types, list, a.n_solid);
-        else k_pnd_w<false, false, false><<<nb, a.threads, 0, st>>>(a, eos, all_types, list, a.n_solid);
+        if (a.exact && ord) launch(k_pnd_w<true, true, false>, nb, a.threads, 0, st, a, eos, all_types, list,
+                                   a.n_solid);
+        else if (a.exact) launch(k_pnd_w<true, false, false>, nb, a.threads, 0, st, a, eos, all_types, list,
+                                 a.n_solid);
+        else launch(k_pnd_w<false, false, false>, nb, a.threads, 0, st, a, eos, all_types, list, a.n_solid);
     }
 }
 
@@ -916,6 +932,7 @@ void launch_pnd(const StageArgs& a, int eos, int all_types, uint32_t cap, cudaSt
 __global__ void __launch_bounds__(256) k_dummy_press(State s, const uint32_t* __restrict__ normal_id_of,
                                                      const uint32_t* __restrict__ index_of_id,
                                                      const Scalars* __restrict__ sc) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -926,7 +943,7 @@ __global__ void __launch_bounds__(256) k_dummy_press(State s, const uint32_t* __
 
 void launch_dummy_press(const StageArgs& a, const uint32_t* normal_id_of, const uint32_t* index_of_id, uint32_t cap,
                         cudaStream_t st) {
-    k_dummy_press<<<blocks_for(cap, 256), 256, 0, st>>>(a.cur, normal_id_of, index_of_id, a.sc);
+    launch(k_dummy_press, blocks_for(cap, 256), 256, 0, st, a.cur, normal_id_of, index_of_id, a.sc);
 }
 
 // ---------------------------------------------------------------- gradient
@@ -939,13 +956,13 @@ void launch_dash(const StageArgs& a, uint32_t cap, cudaStream_t st) {
     const uint32_t nb = blocks_for((a.list_fluid ? a.cap_fluid : cap) * 32u, (uint32_t)a.threads);
     const bool ord = a.exact && !a.semi;
     if (a.batch.n) {
-        if (a.exact && ord) k_dash_w<true, true, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.exact) k_dash_w<true, false, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else k_dash_w<false, false, true><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
+        if (a.exact && ord) launch(k_dash_w<true, true, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.exact) launch(k_dash_w<true, false, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else launch(k_dash_w<false, false, true>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
     } else {
-        if (a.exact && ord) k_dash_w<true, true, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else if (a.exact) k_dash_w<true, false, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
-        else k_dash_w<false, false, false><<<nb, a.threads, 0, st>>>(a, a.list_fluid, a.n_fluid);
+        if (a.exact && ord) launch(k_dash_w<true, true, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else if (a.exact) launch(k_dash_w<true, false, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
+        else launch(k_dash_w<false, false, false>, nb, a.threads, 0, st, a, a.list_fluid, a.n_fluid);
     }
 }
 

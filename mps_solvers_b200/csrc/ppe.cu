@@ -48,6 +48,7 @@ struct AsmArgs {
 // ones in ascending index order (MPS_CAL_v4.0/MPS_CPU.cpp:651-698).
 template <bool EX, bool BT>
 __global__ void __launch_bounds__(256) k_ppe_assemble(AsmArgs A) {
+    after_previous();
     const StageArgs& a = A.a;
     const uint32_t n = a.sc->np;
     const uint32_t lane = threadIdx.x & 31;
@@ -1158,6 +1159,7 @@ __global__ void __launch_bounds__(PPE_THREADS) k_ppe_solve_batch(BatchSolveArgs 
 __global__ void __launch_bounds__(256) k_row_scene(const uint32_t* __restrict__ rowlist, const uint32_t* __restrict__ nrows,
                                                    const uint32_t* __restrict__ id, const uint32_t* __restrict__ sid_of_id,
                                                    uint32_t* __restrict__ row_scene, uint32_t cap) {
+    after_previous();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= *nrows || k >= cap) return;
     row_scene[k] = sid_of_id[id[rowlist[k]]];
@@ -1171,6 +1173,7 @@ constexpr uint32_t ROW_TILE = 2048;
 
 __global__ void __launch_bounds__(256) k_rows_count(const uint32_t* __restrict__ rlen, const Scalars* __restrict__ sc,
                                                     uint32_t* __restrict__ tilecnt) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t base = blockIdx.x * ROW_TILE;
     uint32_t c = 0;
@@ -1192,6 +1195,7 @@ __global__ void __launch_bounds__(256) k_rows_count(const uint32_t* __restrict__
 __global__ void __launch_bounds__(256) k_rows_scatter(const uint32_t* __restrict__ rlen, const Scalars* __restrict__ sc,
                                                       const uint32_t* __restrict__ tileoff, uint32_t ntiles,
                                                       uint32_t* __restrict__ rowlist, uint32_t* __restrict__ nrows) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t base = blockIdx.x * ROW_TILE;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1233,6 +1237,7 @@ __global__ void __launch_bounds__(256) k_sell_width(const uint32_t* __restrict__
                                                     const uint32_t* __restrict__ rowlist,
                                                     const uint32_t* __restrict__ nrows, uint32_t* __restrict__ width,
                                                     uint32_t maxslices) {
+    after_previous();
     const uint32_t R = *nrows;
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;  // slice
     if (s > maxslices) return;
@@ -1254,6 +1259,7 @@ __global__ void __launch_bounds__(256) k_sell_pack(const uint32_t* __restrict__ 
                                                    const uint32_t* __restrict__ rlen, const uint32_t* __restrict__ rowlist,
                                                    const uint32_t* __restrict__ nrows, const uint32_t* __restrict__ off,
                                                    uint32_t* __restrict__ scols, float* __restrict__ sw) {
+    after_previous();
     const uint32_t R = *nrows;
     const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31, r = lane & 7, q = lane >> 3;
@@ -1288,6 +1294,7 @@ __global__ void __launch_bounds__(256) k_sell_pack(const uint32_t* __restrict__ 
 // p = max(x, 0) (pressCorr, MPS_CAL_v4.0/MPS_CPU.cpp:734-743); Dirichlet rows 0.
 __global__ void __launch_bounds__(256) k_ppe_finish(const double* __restrict__ x64, const uint32_t* __restrict__ rlen,
                                                     float* __restrict__ press, const Scalars* __restrict__ sc) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1499,21 +1506,22 @@ static cudaError_t launch_cooperative(const void* fn, int blocks, int threads, v
 // stored weights), from the assembled row-major system.
 static int enqueue_rows_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
     const uint32_t ntiles = (cap + ROW_TILE - 1) / ROW_TILE;
-    k_rows_count<<<ntiles, 256, 0, st>>>(w.rlen, a.sc, w.tilecnt);
+    launch(k_rows_count, ntiles, 256, 0, st, w.rlen, a.sc, w.tilecnt);
     launch_scan_exclusive(w.tilecnt, ntiles, st);
-    k_rows_scatter<<<ntiles, 256, 0, st>>>(w.rlen, a.sc, w.tilecnt, ntiles, w.rowlist, w.nrows);
+    launch(k_rows_scatter, ntiles, 256, 0, st, w.rlen, a.sc, w.tilecnt, ntiles, w.rowlist, w.nrows);
     int launched = 6;
     if (a.batch.n) {
-        k_row_scene<<<blocks_for(cap, 256), 256, 0, st>>>(w.rowlist, w.nrows, a.cur.id, a.batch.sid_of_id, w.row_scene,
-                                                          cap);
+        launch(k_row_scene, blocks_for(cap, 256), 256, 0, st, w.rowlist, w.nrows, a.cur.id, a.batch.sid_of_id,
+               w.row_scene, cap);
         launched++;
     }
     // SELL-8 layout of the non-Dirichlet rows
     const uint32_t maxslices = (cap + SELL_C - 1) / SELL_C;
-    k_sell_width<<<blocks_for(maxslices + 1, 256), 256, 0, st>>>(w.rlen, w.rowlist, w.nrows, w.sell_off, maxslices);
+    launch(k_sell_width, blocks_for(maxslices + 1, 256), 256, 0, st, w.rlen, w.rowlist, w.nrows, w.sell_off,
+           maxslices);
     launch_scan_exclusive(w.sell_off, maxslices + 1, st);
-    k_sell_pack<<<blocks_for(maxslices * 32u, 256), 256, 0, st>>>(w.cols, w.wrm, w.rlen, w.rowlist, w.nrows,
-                                                                  w.sell_off, w.sell_cols, w.sell_w);
+    launch(k_sell_pack, blocks_for(maxslices * 32u, 256), 256, 0, st, w.cols, w.wrm, w.rlen, w.rowlist, w.nrows,
+           w.sell_off, w.sell_cols, w.sell_w);
     return launched;
 }
 
@@ -1627,11 +1635,11 @@ int ppe_enqueue_setup(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     } else {
         const uint32_t blocks = blocks_for(cap * 32u, 256);
         if (a.batch.n) {
-            if (a.exact) k_ppe_assemble<true, true><<<blocks, 256, 0, st>>>(A);
-            else k_ppe_assemble<false, true><<<blocks, 256, 0, st>>>(A);
+            if (a.exact) launch(k_ppe_assemble<true, true>, blocks, 256, 0, st, A);
+            else launch(k_ppe_assemble<false, true>, blocks, 256, 0, st, A);
         } else {
-            if (a.exact) k_ppe_assemble<true, false><<<blocks, 256, 0, st>>>(A);
-            else k_ppe_assemble<false, false><<<blocks, 256, 0, st>>>(A);
+            if (a.exact) launch(k_ppe_assemble<true, false>, blocks, 256, 0, st, A);
+            else launch(k_ppe_assemble<false, false>, blocks, 256, 0, st, A);
         }
         launched += 1 + enqueue_rows_pack(w, a, cap, st);
     }
@@ -1782,7 +1790,7 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
                                               : (const void*)k_ppe_solve_batch<false, false, 0>);
         w.launch_err = launch_cooperative(bfn, w.blocks, w.threads, bargs, st);
         if (!w.write_pressure) return 1;
-        k_ppe_finish<<<blocks_for(cap, 256), 256, 0, st>>>(w.x64, w.rlen, a.cur.press, a.sc);
+        launch(k_ppe_finish, blocks_for(cap, 256), 256, 0, st, w.x64, w.rlen, a.cur.press, a.sc);
         return 2;
     }
     if (w.pipelined && !learned) {
@@ -1825,7 +1833,7 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
                               : (a.exact ? (const void*)k_ppe_solve_pipe<true, false> : (const void*)k_ppe_solve_pipe<false, false>);
         w.launch_err = launch_cooperative(pfn, w.blocks, w.threads, pargs, st);
         if (!w.write_pressure) return 1;
-        k_ppe_finish<<<blocks_for(cap, 256), 256, 0, st>>>(w.x64, w.rlen, a.cur.press, a.sc);
+        launch(k_ppe_finish, blocks_for(cap, 256), 256, 0, st, w.x64, w.rlen, a.cur.press, a.sc);
         return 2;
     }
     void* args[] = {&S};
@@ -1839,7 +1847,7 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     const size_t smem = (size_t)(w.threads / 32) * (size_t)S.smem_chunks * 32 * (sizeof(uint4) + sizeof(float4));
     w.launch_err = launch_cooperative_smem(fn, w.blocks, w.threads, smem, args, st);
     if (!w.write_pressure) return 1;
-    k_ppe_finish<<<blocks_for(cap, 256), 256, 0, st>>>(w.x64, w.rlen, a.cur.press, a.sc);
+    launch(k_ppe_finish, blocks_for(cap, 256), 256, 0, st, w.x64, w.rlen, a.cur.press, a.sc);
     return 2;
 }
 
@@ -1873,6 +1881,7 @@ __device__ __forceinline__ float comp(const float4& v, int c) { return c == 0 ? 
 
 template <bool EX>
 __global__ void __launch_bounds__(256) k_cn_assemble(CnArgs A) {
+    after_previous();
     const StageArgs& a = A.a;
     const uint32_t n = a.sc->np;
     const uint32_t lane = threadIdx.x & 31;
@@ -1952,6 +1961,7 @@ __global__ void __launch_bounds__(256) k_cn_assemble(CnArgs A) {
 // fluid u_c = x, x_c += dt u_c.
 __global__ void k_cn_finish(const double* __restrict__ x64, const uint32_t* __restrict__ rlen, State s, int c,
                             const Scalars* sc) {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sc->np || rlen[i] == PPE_DIRICHLET) return;
     const float x = (float)x64[i];
@@ -1980,11 +1990,11 @@ int ppe_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c
     A.bar = w.bar;
     A.lambda_n0_over_dim_niu = lambda * n0 / ((double)a.P.dim_f * (double)a.P.niu);
     const uint32_t warps_blocks = blocks_for(cap * 32u, 256);
-    if (a.exact) k_cn_assemble<true><<<warps_blocks, 256, 0, st>>>(A);
-    else k_cn_assemble<false><<<warps_blocks, 256, 0, st>>>(A);
+    if (a.exact) launch(k_cn_assemble<true>, warps_blocks, 256, 0, st, A);
+    else launch(k_cn_assemble<false>, warps_blocks, 256, 0, st, A);
     int launched = 1 + enqueue_rows_pack(w, a, cap, st);
     launched += ppe_enqueue_solve(w, a, opt, cap, st);
-    k_cn_finish<<<blocks_for(cap, 256), 256, 0, st>>>(w.x64, w.rlen, a.cur, c, a.sc);
+    launch(k_cn_finish, blocks_for(cap, 256), 256, 0, st, w.x64, w.rlen, a.cur, c, a.sc);
     return launched + 1;
 }
 

@@ -107,6 +107,7 @@ __device__ __forceinline__ bool c16_is_row(const C16Flag& F, uint32_t i) {
 __global__ void __launch_bounds__(256) k_c16_count(C16Flag F, const uint32_t* __restrict__ cells, uint32_t nsuper,
                                                    const uint32_t* __restrict__ cs, uint32_t* __restrict__ base,
                                                    uint32_t* __restrict__ stats) {
+    after_previous();
     const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x < C16_STATS) stats[threadIdx.x] = 0u;
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(256) k_c16_shift(const uint32_t* __restrict__ 
                                                    const uint32_t* __restrict__ sfirst, uint32_t ns,
                                                    uint32_t* __restrict__ base, uint32_t* __restrict__ srow,
                                                    uint32_t* __restrict__ rowlist, uint32_t* __restrict__ nrows) {
+    after_previous();
     __shared__ uint32_t first[PPE_MAX_SCENES + 1], at[PPE_MAX_SCENES + 1];
     for (uint32_t x = threadIdx.x; x <= ns; x += blockDim.x) first[x] = sfirst[x];
     if (threadIdx.x < 32) {
@@ -186,6 +188,7 @@ struct C16RowArgs {
 };
 
 __global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, C16RowArgs A) {
+    after_previous();
     const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
     if (h >= A.nsuper) return;
@@ -251,6 +254,7 @@ struct C16AsmArgs {
 // 20 us slower and 60 us slower.
 template <bool EX, bool BT>
 __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
+    after_previous();
     __shared__ __align__(512) char rings[8][512];
     const StageArgs& a = A.a;
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
@@ -311,6 +315,7 @@ __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
 // between two scenes' rows is an identity row with b = 0.
 template <bool BT>
 __global__ void __launch_bounds__(256) k_c16_rowend(C16AsmArgs A) {
+    after_previous();
     const StageArgs& a = A.a;
     const uint32_t R = *A.nrows;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -362,6 +367,7 @@ __device__ __forceinline__ uint64_t c16_weight(const uint32_t* __restrict__ off,
 __global__ void __launch_bounds__(32) k_c16_cut(const uint32_t* __restrict__ off, const uint32_t* __restrict__ srow,
                                                 const uint32_t* __restrict__ nrows, uint32_t ns, uint32_t G,
                                                 uint32_t* __restrict__ tb) {
+    after_previous();
     constexpr uint32_t PER = PPE_MAX_SCENES / 32;
     const uint32_t lane = threadIdx.x, R = *nrows, T = c16_tiles(R, G, ns);
     const double W = (double)c16_weight(off, R / C16_ROWS);
@@ -499,6 +505,7 @@ __device__ __forceinline__ uint32_t sp_bf16_bits(float v) {
 // S' is coded the same way, one thread per row.
 template <bool LRN>
 __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
+    after_previous();
     extern __shared__ uint16_t page_slot[];  // slot of every page of rows (0xffff: none)
     __shared__ uint2 bits[C16_PAGES * 8];    // columns in use, and those before the word
     __shared__ uint32_t slot_page[C16_PAGES];
@@ -757,6 +764,7 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
 // MPS_CAL_v4.0/MPS_CPU.cpp:734-743).
 __global__ void __launch_bounds__(256) k_c16_finish(const double* __restrict__ cx64, const uint32_t* __restrict__ cpos,
                                                     float* __restrict__ press, const Scalars* __restrict__ sc) {
+    after_previous();
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -867,6 +875,7 @@ __device__ __forceinline__ void sp_batch(const SpArgs& A, uint32_t id, uint32_t 
 // row with zeros), so this pass reads one count a row instead of following
 // every entry to its row.
 __global__ void __launch_bounds__(256) k_sp_width(SpArgs A) {
+    after_previous();
     const uint32_t R = *A.nrows;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t s = k / SP_SLICE;
@@ -880,6 +889,7 @@ __global__ void __launch_bounds__(256) k_sp_width(SpArgs A) {
 // Pass 2 (after the scan of off): the kept entries of row k in stored order,
 // then zeros up to the slice's width.
 __global__ void __launch_bounds__(256) k_sp_pack(SpArgs A) {
+    after_previous();
     const uint32_t R = *A.nrows, np = A.sc->np;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t s = k / SP_SLICE, lane = k % SP_SLICE;
@@ -2218,8 +2228,8 @@ static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cud
     F.scenes = a.batch.n ? w.scenes : nullptr;
     F.bthr = bthr;
     uint32_t* counts = a.batch.n ? w.c16_dense : w.c16_base;
-    k_c16_count<<<cblocks((w.c16_nsuper + 1) * 32u, 256), 256, 0, st>>>(F, w.c16_cells, w.c16_nsuper, a.cell_start,
-                                                                        counts, w.c16_stats);
+    launch(k_c16_count, cblocks((w.c16_nsuper + 1) * 32u, 256), 256, 0, st, F, w.c16_cells, w.c16_nsuper, a.cell_start,
+           counts, w.c16_stats);
     launch_scan_exclusive(counts, w.c16_nsuper + 1, st);
     C16RowArgs A;
     A.cells = w.c16_cells;
@@ -2235,9 +2245,9 @@ static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cud
     A.rlen = w.rlen;
     A.diag64 = w.diag64;
     if (a.batch.n)
-        k_c16_shift<<<cblocks(w.c16_nsuper + 1, 256), 256, 0, st>>>(w.c16_dense, w.c16_nsuper, w.c16_sfirst, w.nscenes,
-                                                                    w.c16_base, w.c16_srow, A.rowlist, A.nrows);
-    k_c16_rows<<<cblocks(w.c16_nsuper * 32u, 256), 256, 0, st>>>(F, A);
+        launch(k_c16_shift, cblocks(w.c16_nsuper + 1, 256), 256, 0, st, w.c16_dense, w.c16_nsuper, w.c16_sfirst,
+               w.nscenes, w.c16_base, w.c16_srow, A.rowlist, A.nrows);
+    launch(k_c16_rows, cblocks(w.c16_nsuper * 32u, 256), 256, 0, st, F, A);
     return a.batch.n ? 4 : 3;
 }
 
@@ -2272,13 +2282,13 @@ int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& 
     const uint32_t blocks = cblocks(c16_rows_cap(a.cap_solid, w.nscenes) * 32u, 256);
     const uint32_t eblocks = cblocks(C16_ROWS * (A.maxslices + 1), 256);
     if (a.batch.n) {
-        if (a.exact) k_c16_assemble<true, true><<<blocks, 256, 0, st>>>(A);
-        else k_c16_assemble<false, true><<<blocks, 256, 0, st>>>(A);
-        k_c16_rowend<true><<<eblocks, 256, 0, st>>>(A);
+        if (a.exact) launch(k_c16_assemble<true, true>, blocks, 256, 0, st, A);
+        else launch(k_c16_assemble<false, true>, blocks, 256, 0, st, A);
+        launch(k_c16_rowend<true>, eblocks, 256, 0, st, A);
     } else {
-        if (a.exact) k_c16_assemble<true, false><<<blocks, 256, 0, st>>>(A);
-        else k_c16_assemble<false, false><<<blocks, 256, 0, st>>>(A);
-        k_c16_rowend<false><<<eblocks, 256, 0, st>>>(A);
+        if (a.exact) launch(k_c16_assemble<true, false>, blocks, 256, 0, st, A);
+        else launch(k_c16_assemble<false, false>, blocks, 256, 0, st, A);
+        launch(k_c16_rowend<false>, eblocks, 256, 0, st, A);
     }
     return launched + 2;
 }
@@ -2286,7 +2296,7 @@ int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& 
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
     const uint32_t ns = w.nscenes, rows = c16_rows_cap(cap, ns), maxslices = c16_maxslices(w, cap);
     launch_scan_exclusive(w.c16_off, maxslices + 1, st);
-    if (ns) k_c16_cut<<<1, 32, 0, st>>>(w.c16_off, w.c16_srow, c16_nrows(w), ns, (uint32_t)w.sms, w.c16_tb);
+    if (ns) launch(k_c16_cut, 1, 32, 0, st, w.c16_off, w.c16_srow, c16_nrows(w), ns, (uint32_t)w.sms, w.c16_tb);
     C16PackArgs P;
     P.cols_rm = w.cols;
     P.w_rm = w.wrm;
@@ -2320,8 +2330,8 @@ int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStrea
     P.sp_side = w.c16_spside;
     P.sp_diag = w.sp_diag;
     const uint32_t tiles = c16_tiles(rows, (uint32_t)w.sms, ns);
-    if (w.c16_learned) k_c16_pack<true><<<tiles, C16_PACK_THREADS, c16_page_bytes(rows), st>>>(P);
-    else k_c16_pack<false><<<tiles, C16_PACK_THREADS, c16_page_bytes(rows), st>>>(P);
+    if (w.c16_learned) launch(k_c16_pack<true>, tiles, C16_PACK_THREADS, c16_page_bytes(rows), st, P);
+    else launch(k_c16_pack<false>, tiles, C16_PACK_THREADS, c16_page_bytes(rows), st, P);
     return ns ? 3 : 2;
 }
 
@@ -2373,7 +2383,7 @@ int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt
                                : (w.c16_learned ? (const void*)k_ppe_solve_c16<true> : (const void*)k_ppe_solve_c16<false>);
     w.launch_err = launch_cooperative_smem(fn, w.sms, C16_THREADS, C16_SMEM, args, st);
     if (!w.write_pressure) return 1;
-    k_c16_finish<<<cblocks(cap, 256), 256, 0, st>>>(w.cx64, w.cpos, a.cur.press, a.sc);
+    launch(k_c16_finish, cblocks(cap, 256), 256, 0, st, w.cx64, w.cpos, a.cur.press, a.sc);
     return 2;
 }
 
@@ -2418,9 +2428,9 @@ int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream
     const uint32_t maxslices = (cap + SP_SLICE - 1) / SP_SLICE;
     A.maxslices = maxslices;
     const uint32_t wb = cblocks((maxslices + 1) * SP_SLICE, 256), pb = cblocks(maxslices * SP_SLICE, 256);
-    k_sp_width<<<wb, 256, 0, st>>>(A);
+    launch(k_sp_width, wb, 256, 0, st, A);
     launch_scan_exclusive(w.sp_off, maxslices + 1, st);
-    k_sp_pack<<<pb, 256, 0, st>>>(A);
+    launch(k_sp_pack, pb, 256, 0, st, A);
     return 3;
 }
 

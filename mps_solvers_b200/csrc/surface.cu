@@ -115,6 +115,7 @@ __device__ __forceinline__ float cubic_w(float r0, float r) {
 // sum over the linked cells of w(r_ij; r0), j != i, every type; max over i
 // (MPS_GPU::calOnce, MPS_CAL_/MPS_GPU.cpp:222-272)
 __global__ void __launch_bounds__(256) k_surface_iso(StageArgs a, unsigned long long* best) {
+    after_previous();
     const uint32_t n = a.sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float acc = 0.f;
@@ -142,12 +143,14 @@ __global__ void __launch_bounds__(256) k_surface_iso(StageArgs a, unsigned long 
 }
 
 __global__ void k_surface_iso_set(const unsigned long long* best, uint32_t* out_bits) {
+    after_previous();
     out_bits[1] = __float_as_uint(0.8f * __uint_as_float((uint32_t)*best));
 }
 
 // vertex value: fluid particles within r0 of the vertex, from the cells
 // that overlap [v - r0, v + r0], in ascending particle index
 __global__ void __launch_bounds__(256) k_surface_vertex(StageArgs a, SurfaceGrid sg, float* __restrict__ vn) {
+    after_previous();
     const uint32_t nv = sg.nx * sg.ny * sg.nz;
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nv) return;
@@ -211,6 +214,7 @@ __global__ void __launch_bounds__(256) k_surface_count(const float* __restrict__
                                                        const uint32_t* __restrict__ iso_bits,
                                                        const uint8_t* __restrict__ tab_n, uint32_t* __restrict__ cnt,
                                                        uint32_t* __restrict__ sum, uint32_t nblocks) {
+    after_previous();
     __shared__ uint32_t ws[8];
     const uint32_t mx = sg.nx - 1, my = sg.ny - 1, mz = sg.nz - 1, ncube = mx * my * mz;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -265,6 +269,7 @@ __global__ void __launch_bounds__(256) k_surface_emit(const float* __restrict__ 
                                                       const uint32_t* __restrict__ sum, uint32_t max_tri,
                                                       float* __restrict__ pos9, float* __restrict__ nrm9,
                                                       uint32_t* __restrict__ ntri) {
+    after_previous();
     const uint32_t mx = sg.nx - 1, my = sg.ny - 1, mz = sg.nz - 1;
     const uint32_t ncube = mx * my * mz;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -362,20 +367,20 @@ int surface_setup(SurfaceWork& w, const SurfaceGrid& g, uint32_t max_tri, cudaSt
 
 void surface_enqueue_iso(SurfaceWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
     cudaMemsetAsync(w.best, 0, sizeof(unsigned long long), st);
-    k_surface_iso<<<blocks_for(cap, 256), 256, 0, st>>>(a, w.best);
-    k_surface_iso_set<<<1, 1, 0, st>>>(w.best, w.ntri);
+    launch(k_surface_iso, blocks_for(cap, 256), 256, 0, st, a, w.best);
+    launch(k_surface_iso_set, 1, 1, 0, st, w.best, w.ntri);
 }
 
 void surface_enqueue_extract(SurfaceWork& w, const StageArgs& a, cudaStream_t st) {
     const SurfaceGrid& g = w.g;
     const uint32_t nv = g.nx * g.ny * g.nz;
     const uint32_t ncube = (g.nx - 1) * (g.ny - 1) * (g.nz - 1);
-    k_surface_vertex<<<blocks_for(nv, 256), 256, 0, st>>>(a, g, w.vn);
+    launch(k_surface_vertex, blocks_for(nv, 256), 256, 0, st, a, g, w.vn);
     const uint32_t nb = blocks_for(ncube, SURFACE_SCAN);
-    k_surface_count<<<nb, 256, 0, st>>>(w.vn, g, w.ntri, w.tab_n, w.cube_cnt, w.block_cnt, nb);
+    launch(k_surface_count, nb, 256, 0, st, w.vn, g, w.ntri, w.tab_n, w.cube_cnt, w.block_cnt, nb);
     launch_scan_exclusive(w.block_cnt, nb + 1, st);
-    k_surface_emit<<<blocks_for(ncube, 256), 256, 0, st>>>(w.vn, g, w.ntri, w.tab_n, w.tab_t, w.cube_cnt, w.block_cnt, w.max_tri,
-                                                           w.tri_pos, w.tri_nrm, w.ntri);
+    launch(k_surface_emit, blocks_for(ncube, 256), 256, 0, st, w.vn, g, w.ntri, w.tab_n, w.tab_t, w.cube_cnt,
+           w.block_cnt, w.max_tri, w.tri_pos, w.tri_nrm, w.ntri);
 }
 
 void surface_free(SurfaceWork& w) {
