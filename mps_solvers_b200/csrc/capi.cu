@@ -594,7 +594,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         h->ppe.precond_every = h->opt.precond_every > 0 ? h->opt.precond_every : 40;
         h->ppe.index_of_id = h->index_of_id;
         if (h->opt.ppe_layout == 0 && ppe_c16_takes(h->cap, &h->g, 1)) {
-            e = ppe_c16_enable(h->ppe, &h->g, 1, &h->err);
+            e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
             set_compact(h, true);
@@ -604,6 +604,11 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
             if (e != MPS_OK) return (mps_status)e;
             h->cn.write_pressure = false;
             h->cn.l2_keep_entries = h->ppe.l2_keep_entries;
+            if (h->ppe.c16_ready) {  // its tiles hold the fluid's rows; the 8-byte layout where they do not fit
+                h->cn.c16_smem_chunks = h->ppe.c16_smem_chunks;
+                h->cn.c16 = ppe_c16_enable(h->cn, &h->g, 1, &h->ppe, nullptr) == MPS_OK;
+                if (!h->cn.c16) cudaGetLastError();
+            }
         }
     }
     Scalars s;
@@ -904,11 +909,16 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
         if (h->opt.ppe_layout == 0 && ppe_c16_takes(cap, h->scene_grid.data(), S)) {
             h->ppe.c16_smem_chunks =
                 h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
-            e = ppe_c16_enable(h->ppe, h->scene_grid.data(), S, &h->err);
+            e = ppe_c16_enable(h->ppe, h->scene_grid.data(), S, nullptr, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
-            if (e != MPS_OK) return (mps_status)e;
-            h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
-            set_compact(h, true);
+            if (e == MPS_OK) {
+                h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
+                set_compact(h, true);
+            } else {  // no memory for the tiles beside the 8-byte layout: that one stays
+                ppe_c16_free(h->ppe);
+                h->err.clear();
+                cudaGetLastError();
+            }
         }
     }
     Scalars sc;
@@ -1086,8 +1096,8 @@ extern "C" void mps_destroy(mps_handle* h) {
     for (int b = 2; b < 4; b++)
         if (h->graph[b]) cudaGraphExecDestroy(h->graph[b]);
     for (cudaEvent_t e : h->prof_ev) cudaEventDestroy(e);
+    ppe_free(h->cn);  // before the one whose linked cells it uses
     ppe_free(h->ppe);
-    ppe_free(h->cn);
     surface_free(h->surf);
     for (void* p : h->allocs) cudaFree(p);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1710,7 +1720,7 @@ extern "C" mps_status mps_apply_tuning(mps_handle* h, const mps_tune_report* r) 
                 h->err = "the compact PPE layout is for single scenes";
                 return MPS_ERR_INVALID;
             }
-            int e = ppe_c16_enable(h->ppe, &h->g, 1, &h->err);
+            int e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
         }

@@ -1976,6 +1976,8 @@ __global__ void k_cn_finish(const double* __restrict__ x64, const uint32_t* __re
 
 int ppe_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c, double n0, double lambda,
                    uint32_t cap, cudaStream_t st) {
+    const double lambda_n0_over_dim_niu = lambda * n0 / ((double)a.P.dim_f * (double)a.P.niu);
+    if (w.c16) return ppe_c16_enqueue_cn(w, a, opt, c, lambda_n0_over_dim_niu, cap, st);
     CnArgs A;
     A.a = a;
     A.c = c;
@@ -1988,7 +1990,7 @@ int ppe_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c
     A.b64 = w.b64;
     A.x64 = w.x64;
     A.bar = w.bar;
-    A.lambda_n0_over_dim_niu = lambda * n0 / ((double)a.P.dim_f * (double)a.P.niu);
+    A.lambda_n0_over_dim_niu = lambda_n0_over_dim_niu;
     const uint32_t warps_blocks = blocks_for(cap * 32u, 256);
     if (a.exact) launch(k_cn_assemble<true>, warps_blocks, 256, 0, st, A);
     else launch(k_cn_assemble<false>, warps_blocks, 256, 0, st, A);

@@ -91,6 +91,7 @@ struct PpeWork {
     // each, 16-bit codes into it beside FP32 weights
     bool c16 = false;                  // the solve uses this layout
     bool c16_ready = false;            // its buffers exist
+    bool c16_shared = false;           // c16_cells and c16_nbr are another work's
     int c16_smem_chunks = 8;           // chunks per warp held in shared memory across iterations
     uint32_t c16_nsuper = 0;           // linked cells, in curve order
     uint32_t* c16_cells = nullptr;     // the up to 4 cells of the sorted grid of each
@@ -176,7 +177,8 @@ int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint3
 // whether it takes a grid and capacity, buffers, the pack after the assembly, the solve with p = max(x, 0), the
 // escaped-entry count of the last pack, and the stencil export.
 bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids);
-int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* err);
+// same: a work of the same grids whose linked cells are used (it is freed with or after w), or null
+int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, std::string* err);
 // the PPE's constants (a batch uses its scenes' own; dim2 is the same for all)
 struct C16Assemble {
     double n0, beta, b_tmp, rho_lambda_alpha_n0, dim2;
@@ -186,6 +188,8 @@ int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& 
 int ppe_c16_learned_enable(PpeWork& w, std::string* err);
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st);
 int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, uint32_t cap, cudaStream_t st);
+int ppe_c16_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c, double lambda_n0_over_dim_niu,
+                       uint32_t cap, cudaStream_t st);
 int ppe_c16_export(const PpeWork& w, uint32_t np, const uint32_t* d_row_start, uint32_t* d_cols, float* d_w,
                    cudaStream_t st);
 void ppe_c16_free(PpeWork& w);

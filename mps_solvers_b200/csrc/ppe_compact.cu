@@ -92,9 +92,11 @@ struct C16Flag {
     const uint32_t* sid_of_id;  // batch: the scene of each particle id
     const PpeScene* scenes;
     double bthr;
+    bool fluid;                 // the viscosity's system: a row for every fluid particle
 };
 
 __device__ __forceinline__ bool c16_is_row(const C16Flag& F, uint32_t i) {
+    if (F.fluid) return ptype(F.pos[i]) == T_FLUID;
     double b = F.bthr;
     if (F.scenes) {
         const PpeScene& s = F.scenes[F.sid_of_id[F.id[i]]];
@@ -310,6 +312,14 @@ __global__ void __launch_bounds__(256) k_c16_assemble(C16AsmArgs A) {
     A.cdiag64[k] = d;
 }
 
+// chunks of the slice of rows k / 8 (every thread of a warp calls it)
+__device__ __forceinline__ void c16_slice_width(uint32_t k, uint32_t len, const C16AsmArgs& A) {
+#pragma unroll
+    for (int o = 1; o < (int)C16_ROWS; o <<= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
+    const uint32_t s = k / C16_ROWS;
+    if (k % C16_ROWS == 0 && s <= A.maxslices) A.width[s] = (len + 15u) / 16u;
+}
+
 // A thread a row: its diagonal from the weights' sum and its vectors; and the
 // chunks of every slice (the longest of its 8 rows), scanned next.  A gap
 // between two scenes' rows is an identity row with b = 0.
@@ -350,10 +360,119 @@ __global__ void __launch_bounds__(256) k_c16_rowend(C16AsmArgs A) {
         A.cb64[k] = 0.0;
         A.cx64[k] = 0.0;
     }
-#pragma unroll
-    for (int o = 1; o < (int)C16_ROWS; o <<= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
-    const uint32_t s = k / C16_ROWS;
-    if (k % C16_ROWS == 0 && s <= A.maxslices) A.width[s] = (len + 15u) / 16u;
+    c16_slice_width(k, len, A);
+}
+
+// ---------------------------------------------------------------- Crank-Nicolson viscosity
+// The system of ppe.cu's k_cn_assemble (every neighbour in the diagonal, the
+// ones that are no rows moved to the right-hand side) for the rows of this
+// layout: hits weighed 32 at a time as in k_c16_assemble.
+struct C16CnArgs {
+    C16AsmArgs A;
+    int c;                          // velocity component
+    double lambda_n0_over_dim_niu;  // 1/R = this / dt
+};
+
+__device__ __forceinline__ float c16_comp(const float4& v, int c) { return c == 0 ? v.x : (c == 1 ? v.y : v.z); }
+
+template <bool EX>
+__global__ void __launch_bounds__(256) k_c16_cn_assemble(C16CnArgs C) {
+    after_previous();
+    __shared__ __align__(512) char rings[8][512];
+    const C16AsmArgs& A = C.A;
+    const StageArgs& a = A.a;
+    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= *A.nrows) return;
+    const uint32_t i = __ldg(A.rowlist + k);
+    HitRing hits(rings[threadIdx.x >> 5]);
+    const float4* __restrict__ pos = a.cur.pos;
+    const float4* __restrict__ vel = a.cur.vel;
+    const float4 pi = pos[i];
+    const double ui = (double)c16_comp(vel[i], C.c);
+    const Local L = local_of<false>(a, i);
+    const float re = a.P.rlap, thr = a.P.rlap_thr;
+    uint32_t* cols = A.cols + (size_t)k * PPE_W;
+    float* wrow = A.wrm + (size_t)k * PPE_W;
+    uint32_t count = 0;
+    double diag = 0.0, bi = 0.0;
+    auto weigh = [&](uint32_t at, uint32_t m) {
+        const float2 h = hits.get(at + lane);
+        uint32_t col = C16_NONE;
+        float w = 0.f;
+        if (lane < m) w = weight_rr<EX>(re, h.y);
+        if (w > 0.f) {
+            const uint32_t j = __float_as_uint(h.x);
+            const double uj = (double)c16_comp(__ldg(vel + j), C.c);
+            col = __ldg(A.cpos + j);
+            bi -= (uj - ui) * (double)w;
+            if (col == C16_NONE) bi -= (double)w * uj;
+        }
+        diag += (double)w;
+        const uint32_t ma = __ballot_sync(0xffffffffu, col != C16_NONE);
+        const uint32_t to = count + __popc(ma & lt);
+        if (col != C16_NONE && to < PPE_W) {
+            cols[to] = col;
+            wrow[to] = w;
+        }
+        count += __popc(ma);
+    };
+    const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
+    flat_batches(flat_walk(L.g, L.cs, L.c, nr, lane), lane, [&](uint32_t j, bool in) {
+        const float4 pj = __ldg(pos + j);
+        const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
+        const float rr = dot3<EX>(dx, dy, dz, dx, dy, dz);
+        hits.add(lane, in && rr < thr && j != i, j, rr, weigh);
+    });
+    hits.rest(weigh);
+    diag = warp_sum_d(diag);
+    bi = warp_sum_d(bi);
+    if (lane) return;
+    if (count > PPE_W) {
+        atomicOr(&a.sc->err, ERR_CAPACITY);
+        count = PPE_W;
+    }
+    A.clen[k] = count;
+    A.cdiag64[k] = diag;
+    A.cb64[k] = bi;
+}
+
+__global__ void __launch_bounds__(256) k_c16_cn_rowend(C16CnArgs C) {
+    after_previous();
+    const C16AsmArgs& A = C.A;
+    const StageArgs& a = A.a;
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool row = k < *A.nrows;
+    if (row) {
+        const double ui = (double)c16_comp(a.cur.vel[A.rowlist[k]], C.c);
+        const double one_over_R = C.lambda_n0_over_dim_niu / (double)a.sc->dt;
+        const double dg = -A.cdiag64[k] - one_over_R;
+        A.cdiag64[k] = dg;
+        A.cdiag32[k] = (float)dg;
+        A.cinv_diag[k] = (float)(1.0 / dg);
+        A.cb64[k] -= one_over_R * ui + C.lambda_n0_over_dim_niu * (double)a.sc->g_eff[C.c];
+        A.cx64[k] = ui;
+    }
+    c16_slice_width(k, row ? A.clen[k] : 0u, A);
+}
+
+// MPS_CPU_IMPL::updatePosVel<dir> (MPS_CAL_v4.0/MPS_CPU_IMPL.cpp:129-190):
+// fluid u_c = x, x_c += dt u_c.
+__global__ void __launch_bounds__(256) k_c16_cn_finish(const double* __restrict__ cx64, const uint32_t* __restrict__ cpos,
+                                                       State s, int c, const Scalars* __restrict__ sc) {
+    after_previous();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= sc->np) return;
+    const uint32_t k = cpos[i];
+    if (k == C16_NONE) return;
+    const float x = (float)cx64[k];
+    float4 u = s.vel[i], p = s.pos[i];
+    const float at = __fadd_rn(c16_comp(p, c), __fmul_rn(sc->dt, x));
+    if (c == 0) { u.x = x; p.x = at; }
+    else if (c == 1) { u.y = x; p.y = at; }
+    else { u.z = x; p.z = at; }
+    s.vel[i] = u;
+    s.pos[i] = p;
 }
 
 // Weight of the slices before s when tiles are cut.
@@ -2043,8 +2162,6 @@ void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint3
     };
     std::vector<Key> order;
     order.reserve((size_t)nx * ny * nz);
-    cells->reserve(cells->size() + 4 * (size_t)nx * ny * nz);
-    nbr->reserve(nbr->size() + 27 * (size_t)nx * ny * nz);
     for (uint32_t z = 0; z < nz; z++)
         for (uint32_t y = 0; y < ny; y++)
             for (uint32_t x = 0; x < nx; x++) order.push_back({hilbert_index(x, y, z, bits), x, y, z});
@@ -2053,19 +2170,23 @@ void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint3
     std::vector<uint32_t> rank(order.size());
     for (size_t k = 0; k < order.size(); k++)
         rank[((size_t)order[k].z * ny + order[k].y) * nx + order[k].x] = first + (uint32_t)k;
+    cells->resize(cells->size() + 4 * order.size());
+    nbr->resize(nbr->size() + 27 * order.size());
+    uint32_t* c = cells->data() + 4 * (size_t)first;
+    uint32_t* n = nbr->data() + 27 * (size_t)first;
     for (const Key& o : order) {
         for (uint32_t b = 0; b < 2; b++)
             for (uint32_t a = 0; a < 2; a++) {
                 const uint32_t y = o.y * f + a, z = o.z * f + b;
                 const bool in = a < f && b < f && y < g.cdy && z < g.cdz;
-                cells->push_back(in ? g.base + z * g.sheet + y * g.cdx + o.x : C16_NONE);
+                *c++ = in ? g.base + z * g.sheet + y * g.cdx + o.x : C16_NONE;
             }
         for (int dz = -1; dz <= 1; dz++)
             for (int dy = -1; dy <= 1; dy++)
                 for (int dx = -1; dx <= 1; dx++) {
-                    const int64_t x = (int64_t)o.x + dx, y = (int64_t)o.y + dy, z = (int64_t)o.z + dz;
-                    const bool in = x >= 0 && y >= 0 && z >= 0 && x < nx && y < ny && z < nz;
-                    nbr->push_back(in ? rank[((size_t)z * ny + (size_t)y) * nx + (size_t)x] : C16_NONE);
+                    const uint32_t x = o.x + (uint32_t)dx, y = o.y + (uint32_t)dy, z = o.z + (uint32_t)dz;
+                    const bool in = x < nx && y < ny && z < nz;  // below 0 wraps
+                    *n++ = in ? rank[((size_t)z * ny + y) * nx + x] : C16_NONE;
                 }
     }
 }
@@ -2095,7 +2216,7 @@ bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
     return c16_page_bytes(c16_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
 }
 
-int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* err) {
+int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, std::string* err) {
     if (w.c16_ready) return MPS_OK;
     const uint32_t ns = w.nscenes;
     if (!ppe_c16_takes(w.cap, grids, ngrids)) {
@@ -2108,15 +2229,22 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* 
     const size_t chunks = slices * ((PPE_W + 15) / 16);
     const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms, ns);
     std::vector<uint32_t> cells, nbr, sfirst;
-    for (uint32_t s = 0; s < ngrids; s++) {
-        sfirst.push_back((uint32_t)(cells.size() / 4));
-        linked_cells(grids[s], &cells, &nbr);
-    }
-    sfirst.push_back((uint32_t)(cells.size() / 4));
-    w.c16_nsuper = (uint32_t)(cells.size() / 4);
     bool ok = true;
-    ok &= c16_alloc(&w.c16_cells, cells.size());
-    ok &= c16_alloc(&w.c16_nbr, nbr.size());
+    w.c16_shared = same && same->c16_ready;
+    if (w.c16_shared) {
+        w.c16_nsuper = same->c16_nsuper;
+        w.c16_cells = same->c16_cells;
+        w.c16_nbr = same->c16_nbr;
+    } else {
+        for (uint32_t s = 0; s < ngrids; s++) {
+            sfirst.push_back((uint32_t)(cells.size() / 4));
+            linked_cells(grids[s], &cells, &nbr);
+        }
+        sfirst.push_back((uint32_t)(cells.size() / 4));
+        w.c16_nsuper = (uint32_t)(cells.size() / 4);
+        ok &= c16_alloc(&w.c16_cells, cells.size());
+        ok &= c16_alloc(&w.c16_nbr, nbr.size());
+    }
     ok &= c16_alloc(&w.c16_base, (size_t)w.c16_nsuper + 2);
     if (ns) {
         ok &= c16_alloc(&w.c16_dense, (size_t)w.c16_nsuper + 2);
@@ -2156,8 +2284,9 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* 
     cudaMemset(w.c16_epoch, 0, sizeof(unsigned long long));
     cudaMemset(w.c16_slots, 0, 2 * (size_t)w.sms * w.sms * C16_SUMS * sizeof(ulonglong2));
     if ((ns && cudaMemcpy(w.c16_sfirst, sfirst.data(), sfirst.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) ||
-        cudaMemcpy(w.c16_cells, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(w.c16_nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        (!w.c16_shared &&
+         (cudaMemcpy(w.c16_cells, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+          cudaMemcpy(w.c16_nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess)) ||
         cudaFuncSetAttribute(k_c16_pack<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)C16_PAGE_BYTES_MAX) != cudaSuccess ||
         cudaFuncSetAttribute(k_c16_pack<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2172,6 +2301,8 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, std::string* 
 }
 
 void ppe_c16_free(PpeWork& w) {
+    if (w.c16_shared) w.c16_cells = w.c16_nbr = nullptr;
+    w.c16_shared = false;
     void* ps[] = {w.c16_cells, w.c16_nbr, w.c16_base, w.cpos, w.clen, w.c16_off, w.c16_ent, w.c16_side, w.c16_tile,
                   w.c16_collist, w.c16_stats, w.cb64, w.cx64, w.cdiag64, w.cdiag32, w.cinv_diag, w.cdsq, w.cr, w.cp,
                   w.cpub[0], w.cpub[1], w.c16_slots, w.c16_epoch, w.c16_dense, w.c16_sfirst, w.c16_srow, w.c16_tb,
@@ -2219,8 +2350,9 @@ static uint32_t* c16_rowlist(PpeWork& w) { return const_cast<uint32_t*>(ppe_c16_
 static uint32_t* c16_nrows(PpeWork& w) { return const_cast<uint32_t*>(ppe_c16_nrows(w)); }
 
 // The row numbers.
-static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, cudaStream_t st) {
+static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, bool fluid, cudaStream_t st) {
     C16Flag F;
+    F.fluid = fluid;
     F.pos = a.cur.pos;
     F.n = a.cur.n;
     F.id = a.cur.id;
@@ -2255,11 +2387,9 @@ static uint32_t c16_maxslices(const PpeWork& w, uint32_t cap) {
     return (c16_rows_cap(cap, w.nscenes) + C16_ROWS - 1) / C16_ROWS;
 }
 
-int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& K, uint32_t cap, cudaStream_t st) {
-    const int launched = ppe_c16_enqueue_rows(w, a, K.beta * K.n0, st);
-    C16AsmArgs A;
+static C16AsmArgs c16_asm_args(PpeWork& w, const StageArgs& a, uint32_t cap) {
+    C16AsmArgs A = {};
     A.a = a;
-    A.K = K;
     A.scenes = w.scenes;
     A.rowlist = c16_rowlist(w);
     A.nrows = c16_nrows(w);
@@ -2278,6 +2408,13 @@ int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& 
     A.cdsq = w.cdsq;
     A.width = w.c16_off;
     A.maxslices = c16_maxslices(w, cap);
+    return A;
+}
+
+int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& K, uint32_t cap, cudaStream_t st) {
+    const int launched = ppe_c16_enqueue_rows(w, a, K.beta * K.n0, false, st);
+    C16AsmArgs A = c16_asm_args(w, a, cap);
+    A.K = K;
     // a.cap_solid: particles that can have rows (not dummies)
     const uint32_t blocks = cblocks(c16_rows_cap(a.cap_solid, w.nscenes) * 32u, 256);
     const uint32_t eblocks = cblocks(C16_ROWS * (A.maxslices + 1), 256);
@@ -2385,6 +2522,25 @@ int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt
     if (!w.write_pressure) return 1;
     launch(k_c16_finish, cblocks(cap, 256), 256, 0, st, w.cx64, w.cpos, a.cur.press, a.sc);
     return 2;
+}
+
+// One velocity component of the Crank-Nicolson viscosity: assembly, pack,
+// solve, update.  The components' rows are the same: numbered with the first.
+int ppe_c16_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c, double lambda_n0_over_dim_niu,
+                       uint32_t cap, cudaStream_t st) {
+    int launched = c == 0 ? ppe_c16_enqueue_rows(w, a, 0.0, true, st) : 0;
+    C16CnArgs C;
+    C.A = c16_asm_args(w, a, cap);
+    C.c = c;
+    C.lambda_n0_over_dim_niu = lambda_n0_over_dim_niu;
+    const uint32_t blocks = cblocks(a.cap_fluid * 32u, 256);
+    if (a.exact) launch(k_c16_cn_assemble<true>, blocks, 256, 0, st, C);
+    else launch(k_c16_cn_assemble<false>, blocks, 256, 0, st, C);
+    launch(k_c16_cn_rowend, cblocks(C16_ROWS * (C.A.maxslices + 1), 256), 256, 0, st, C);
+    launched += 2 + ppe_c16_enqueue_pack(w, a, cap, st);
+    launched += ppe_c16_enqueue_solve(w, a, opt, cap, st);
+    launch(k_c16_cn_finish, cblocks(cap, 256), 256, 0, st, w.cx64, w.cpos, a.cur, c, a.sc);
+    return launched + 1;
 }
 
 int ppe_sp_enable(PpeWork& w, std::string* err) {
