@@ -63,6 +63,15 @@ constexpr int C16_THREADS = 512;            // a solver block
 constexpr int C16_PACK_THREADS = 1024;
 constexpr int C16_BATCH = 4;                // chunks a warp loads at a time, twice buffered
 constexpr int C16_BATCH64 = 3;              // (6 of them: 5 % slower; 768 threads with 3: 2 to 10 % slower)
+// A matrix of several L2s comes from memory: every warp has the batch after
+// the next fetched into L2, 3 KB at a time, before it loads it.  A solve of
+// 1,088,346 rows with S' 16.7 -> 15.5 ms, without S' 851,839 rows 13.0 -> 12.2
+// and 507,178 rows 7.43 -> 7.22; where L2 holds a good part of the matrix the
+// fetches are in its way (311,747 rows 4.43 -> 4.52 ms, 189,647 2.37 -> 3.19).
+// 8, 16 and 24 chunks ahead: 15.8, 15.9 and 16.1 ms; none (the loaded batch
+// itself) 15.8.
+constexpr uint32_t C16_AHEAD = 4;
+constexpr uint32_t C16_AHEAD_FROM = 700000;  // chunks: 540 MB, some 400,000 rows
 constexpr uint32_t C16_STATS = 4;
 constexpr uint32_t C16_SP_SLICES = C16_COLS / 32 + 1;  // S' slices (32 rows) a tile can have, and one
 
@@ -1182,6 +1191,7 @@ struct C16View {
     // and the first keepw are read as evict_last (mat_policy; 0xFFFFFFFF:
     // default policy), so that every warp has the same mix of near and far
     uint32_t resw, keepw;
+    uint32_t ahead;   // chunks a warp fetches into L2 before it loads them (C16_AHEAD)
     uint32_t esc;
     const uint32_t* cl;
     const uint32_t* spf;  // its S' slices (k_c16_pack)
@@ -1211,6 +1221,7 @@ __device__ __forceinline__ C16View c16_view(const C16Args& S, uint32_t t, uint32
     v.nseg = ti.wmax ? (ti.wmax + v.cpw - 2) / v.cpw + 1 : 1u;
     v.resw = 0;
     v.keepw = keep == 0xffffffffu ? keep : (uint32_t)((uint64_t)v.cpw * min(keep, C) / C);
+    v.ahead = C >= C16_AHEAD_FROM ? C16_AHEAD : 0x7fffffffu;
     v.cl = S.collist + (size_t)t * C16_COLS;
     v.spf = S.sp_first + (size_t)t * C16_SP_SLICES;
     v.tile = t;
@@ -1228,6 +1239,12 @@ __device__ __forceinline__ void c16_slices(const C16Args& S, const C16View& v, u
             sseg[s] = (unsigned char)(b > a ? (b - 1) / v.cpw - a / v.cpw + 1 : 0u);
         }
     }
+}
+
+// [p, p + bytes) into L2 ahead of its loads, by one thread of the warp
+__device__ __forceinline__ void c16_fetch(const unsigned char* p, uint32_t bytes, uint64_t pol) {
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(p), "r"(bytes), "l"(pol));
 }
 
 // The row sums of a tile's product over the staged vector (at vecb): warp w
@@ -1293,8 +1310,14 @@ __device__ __forceinline__ void c16_product(const C16Args& S, const C16View& v, 
     const uint64_t near = mat_policy(0u, xk == 0xffffffffu ? xk : 1u), far = mat_policy(1u, xk == 0xffffffffu ? xk : 0u);
     float4 wa[UN], wb[UN];
     uint2 ca[UN], cb[UN];
+    uint32_t ahead = min(v.keepw, xs - x) + x + v.ahead;
     auto load = [&](float4 (&w)[UN], uint2 (&c)[UN], uint32_t at) {
         const uint64_t pol = at < xk ? near : far;
+        if (ahead < xs) {
+            c16_fetch(S.ent + (size_t)(v.c0 + ahead) * C16_CHUNK_BYTES,
+                      min((uint32_t)UN, xs - ahead) * C16_CHUNK_BYTES, far);
+            ahead += UN;
+        }
 #pragma unroll
         for (int u = 0; u < UN; u++) {
             w[u] = ld_mat(reinterpret_cast<const float4*>(src + u * C16_CHUNK_BYTES), pol);
