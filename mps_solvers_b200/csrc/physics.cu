@@ -84,14 +84,28 @@ __device__ __forceinline__ void gather_tail(uint32_t ty, uint32_t p, uint32_t n,
         const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
         const bool f = ty == T_FLUID, s2 = ty == T_FLUID || ty == T_WALL;
         const uint32_t mf = __ballot_sync(0xffffffffu, f), ms = __ballot_sync(0xffffffffu, s2);
-        uint32_t bf = 0, bs = 0;
-        const uint32_t nf = __popc(mf);
+        const uint32_t nf = __popc(mf), warp = threadIdx.x >> 5;
+        // one atomic a list and block (256 threads): one a warp queued up
+        // 100,000 of them on two words at 1.6 million particles
+        __shared__ uint32_t at[2][8];
         if (lane == 0) {
-            if (mf) bf = atomicAdd(&sc->n_fluid, nf + (nf & 1u));
-            if (ms) bs = atomicAdd(&sc->n_solid, __popc(ms));
+            at[0][warp] = nf + (nf & 1u);
+            at[1][warp] = __popc(ms);
         }
-        bf = __shfl_sync(0xffffffffu, bf, 0);
-        bs = __shfl_sync(0xffffffffu, bs, 0);
+        __syncthreads();
+        if (lane == 0 && warp < 2) {
+            uint32_t sum = 0, c[8];
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                c[w] = sum;
+                sum += at[warp][w];
+            }
+            const uint32_t base = sum ? atomicAdd(warp ? &sc->n_solid : &sc->n_fluid, sum) : 0u;
+#pragma unroll
+            for (int w = 0; w < 8; w++) at[warp][w] = base + c[w];
+        }
+        __syncthreads();
+        const uint32_t bf = at[0][warp], bs = at[1][warp];
         if (f) list_fluid[bf + __popc(mf & lt)] = p;
         if (lane == 0 && (nf & 1u)) list_fluid[bf + nf] = LIST_GAP;
         if (s2) list_solid[bs + __popc(ms & lt)] = p;
