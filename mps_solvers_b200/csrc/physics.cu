@@ -283,16 +283,30 @@ __global__ void __launch_bounds__(256) k_update_dt_batch(const float4* __restric
     after_previous();
     const uint32_t n = sc->np;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint32_t scene, most[8];
+    uint32_t s = 0, m = 0;
     if (i < n) {
         const float4 u = vel[i];
         const float vv = dot3<true>(u.x, u.y, u.z, u.x, u.y, u.z);
-        const uint32_t s = b.sid_of_id[id[i]];
+        s = b.sid_of_id[id[i]];
+        if (vv == vv) m = __float_as_uint(vv);
+        else atomicOr(&sc->err, ERR_NAN);
+    }
+    if (threadIdx.x == 0) scene = s;
+    __syncthreads();
+    if (__syncthreads_and(i >= n || s == scene)) {  // a block of one scene: one atomic, as in k_update_dt
+        m = __reduce_max_sync(0xffffffffu, m);
+        if ((threadIdx.x & 31) == 0) most[threadIdx.x >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int w = 1; w < 8; w++) m = max(m, most[w]);
+            if (m) atomicMax(b.vmax2_bits + scene, m);
+        }
+    } else if (i < n) {
         // lanes of the same scene (consecutive particles mostly share one)
         // combine before one atomic
         const uint32_t peers = __match_any_sync(__activemask(), s);
-        uint32_t m = 0;
-        if (vv == vv) m = __float_as_uint(vv);
-        else atomicOr(&sc->err, ERR_NAN);
         uint32_t best = m;
         for (uint32_t rest = peers; rest;) {
             const int l = __ffs(rest) - 1;
