@@ -24,9 +24,10 @@ struct UDiv {
 // wait in after_previous until it has ended and its writes can be read.  Every
 // kernel launched this way calls after_previous first, in every thread, so a
 // kernel has ended only when all before it have.  Between two kernels of a
-// few microseconds this saves about one: an exact explicit step at 5,000 particles
-// (16 kernels) 79 -> 73 us, at 70,912 160 -> 155 us, a semi-implicit step at 5,000
-// 473 -> 461 us.  The learned network's kernels, 20 us and more each, gain nothing.
+// few microseconds this saves about one: an exact explicit step of 5,312
+// particles (16 kernels) 79 -> 73 us, of 70,912 160 -> 155 us, a semi-implicit
+// step of 27,699 473 -> 461 us.  The learned network's training kernels, 20 us
+// and more each, gain nothing.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
