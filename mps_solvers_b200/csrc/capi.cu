@@ -1377,7 +1377,7 @@ extern "C" mps_status mps_get_scalars(mps_handle* h, double* o) {
     o[13] = s.cg_outer;
     o[14] = (h->opt.use_graph && !h->graph_off) ? 1.0 : 0.0;
     o[15] = -1.0;
-    if (h->opt.method == MPS_METHOD_SEMI_IMPLICIT && h->ppe.c16) {
+    if (h->opt.method == MPS_METHOD_SEMI_IMPLICIT && (h->ppe.have_snapshot ? h->ppe.snap_c16 : h->ppe.c16)) {
         uint32_t esc = 0;
         CK(cudaMemcpyAsync(&esc, h->ppe.c16_stats, sizeof esc, cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));

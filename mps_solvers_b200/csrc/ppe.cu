@@ -1584,7 +1584,7 @@ int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint3
     } else {
         cudaMemcpyAsync(d_start, start.data(), (size_t)(np + 1) * 4, cudaMemcpyHostToDevice, st);
         const uint32_t maxslices = (np + SELL_C - 1) / SELL_C;
-        if (w.c16)
+        if (w.snap_c16)
             ppe_c16_export(w, np, d_start, d_cols, d_w, st);
         else if (maxslices)
             k_sell_export<<<blocks_for(maxslices * 32u, 256), 256, 0, st>>>(w.rlen, w.rowlist, w.nrows, w.sell_off,
@@ -1648,6 +1648,7 @@ int ppe_enqueue_setup(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
     cudaMemcpyAsync(w.n_snap, a.cur.n, (size_t)cap * sizeof(float), cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(w.id_snap, a.cur.id, (size_t)cap * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
     w.have_snapshot = true;
+    w.snap_c16 = c16;
     if (opt.precond == MPS_PRECOND_LEARNED && w.lp.ready && w.sp_ent) {
         // the symmetric form by GEO index, rebuilt every precond_every steps;
         // S' of the current rows every step
@@ -1675,7 +1676,7 @@ LpSystem ppe_lp_system(const PpeWork& w, const StageArgs& a) {
     L.rowlist = w.rowlist;
     L.nrows = w.nrows;
     L.acols = w.cols;
-    L.acols_by_row = w.c16;
+    L.acols_by_row = w.snap_c16;
     L.cell = a.cur.cell;
     L.cell_start = a.cell_start;
     L.g = a.g;

@@ -75,6 +75,7 @@ struct PpeWork {
     float* n_snap = nullptr;
     uint32_t* id_snap = nullptr;
     bool have_snapshot = false;
+    bool snap_c16 = false;  // its layout (cols by row in the tiles' form); c16 is the next assembly's
     double n0_64 = 0.0, lambda64 = 0.0, alpha64 = 0.0;
     cudaError_t launch_err = cudaSuccess;  // of the last cooperative launch
     // batch: per-scene constants, scene of each row, per-scene results
