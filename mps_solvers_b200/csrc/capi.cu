@@ -577,7 +577,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         return MPS_ERR_INVALID;
     }
     if (h->opt.method == MPS_METHOD_SEMI_IMPLICIT) {
-        int e = ppe_setup(h->ppe, h->cap, h->g, h->P, h->prm, h->stream, &h->err);
+        int e = ppe_setup(h->ppe, h->cap, 0, h->g, h->P, h->prm, h->stream, &h->err);
         if (e != MPS_OK) return (mps_status)e;
         h->ppe.pipelined = h->opt.ppe_pipelined != 0;
         h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
@@ -600,7 +600,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
             set_compact(h, true);
         }
         if (h->opt.visc_implicit) {
-            e = ppe_setup(h->cn, h->cap, h->g, h->P, h->prm, h->stream, &h->err);
+            e = ppe_setup(h->cn, h->cap, 0, h->g, h->P, h->prm, h->stream, &h->err);
             if (e != MPS_OK) return (mps_status)e;
             h->cn.write_pressure = false;
             h->cn.l2_keep_entries = h->ppe.l2_keep_entries;
@@ -895,7 +895,7 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
     h->P = h->scene_phys[0];
     h->hc = h->scene_hc[0];
     if (h->opt.method == MPS_METHOD_SEMI_IMPLICIT) {
-        int e = ppe_setup(h->ppe, cap, h->g, h->P, h->prm, h->stream, &h->err);
+        int e = ppe_setup(h->ppe, cap, S, h->g, h->P, h->prm, h->stream, &h->err);
         if (e != MPS_OK) return (mps_status)e;
         e = ppe_setup_batch(h->ppe, ppe_scenes.data(), S, h->stream, &h->err);
         if (e != MPS_OK) return (mps_status)e;

@@ -1407,9 +1407,10 @@ static std::vector<const void*> solve_kernels() {
             (const void*)k_ppe_solve_pipe<true, false>, (const void*)k_ppe_solve_pipe<false, false>};
 }
 
-int ppe_setup(PpeWork& w, uint32_t cap, const Grid&, const Phys&, const mps_params& prm, cudaStream_t st,
-              std::string* err) {
+int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid&, const Phys&, const mps_params& prm,
+              cudaStream_t st, std::string* err) {
     w.cap = cap;
+    const size_t rows = ppe_rows_cap(cap, nscenes);
     w.alpha64 = 1.0 / ((double)prm.rho * (double)prm.cs * (double)prm.cs);
     auto al = [&](void** p, size_t bytes) -> bool {
         if (cudaMalloc(p, bytes + 64) != cudaSuccess) return false;
@@ -1417,8 +1418,8 @@ int ppe_setup(PpeWork& w, uint32_t cap, const Grid&, const Phys&, const mps_para
         return true;
     };
     bool ok = true;
-    ok &= al((void**)&w.cols, (size_t)cap * PPE_W * sizeof(uint32_t));
-    ok &= al((void**)&w.wrm, (size_t)cap * PPE_W * sizeof(float));
+    ok &= al((void**)&w.cols, rows * PPE_W * sizeof(uint32_t));
+    ok &= al((void**)&w.wrm, rows * PPE_W * sizeof(float));
     ok &= al((void**)&w.rlen, (size_t)cap * sizeof(uint32_t));
     ok &= al((void**)&w.diag64, (size_t)cap * sizeof(double));
     ok &= al((void**)&w.diag32, (size_t)cap * sizeof(float));

@@ -152,8 +152,13 @@ inline bool ppe_begin_step(PpeWork& w) {
     return w.build_net;
 }
 
-int ppe_setup(PpeWork& w, uint32_t cap, const Grid& g, const Phys& P, const mps_params& prm, cudaStream_t st,
-              std::string* err);
+// Row numbers a handle can need: a scene of a batch (nscenes; 0 for a single
+// scene) starts at a multiple of 8 in the compact layout.  What is indexed by
+// row has as many places.
+inline uint32_t ppe_rows_cap(uint32_t cap, uint32_t nscenes) { return cap + 8u * nscenes; }
+
+int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid& g, const Phys& P, const mps_params& prm,
+              cudaStream_t st, std::string* err);
 // the per-scene tables of a batch (after ppe_setup)
 int ppe_setup_batch(PpeWork& w, const PpeScene* scenes, uint32_t nscenes, cudaStream_t st, std::string* err);
 // assembly, row list and sliced-ELL layout (and, with the learned

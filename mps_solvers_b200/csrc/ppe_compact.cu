@@ -2218,8 +2218,6 @@ void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint3
 // an SM's 228 KB stays L1 and the kernels' static arrays)
 size_t c16_page_bytes(uint32_t cap) { return (((size_t)cap + C16_PAGE - 1) / C16_PAGE + 1) * sizeof(uint16_t); }
 constexpr size_t C16_PAGE_BYTES_MAX = 160 * 1024;
-// row numbers a handle can need: a scene of a batch starts at a multiple of 8
-uint32_t c16_rows_cap(uint32_t cap, uint32_t ns) { return cap + 8u * ns; }
 constexpr size_t C16_SMEM = 220 * 1024;
 
 }  // namespace
@@ -2236,7 +2234,7 @@ static bool c16_solver_smem() {
 bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
     for (uint32_t s = 0; s < ngrids; s++)
         if (grids[s].reach > 2) return false;
-    return c16_page_bytes(c16_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
+    return c16_page_bytes(ppe_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
 }
 
 int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, std::string* err) {
@@ -2246,7 +2244,7 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork
         if (err) *err = "the compact PPE layout does not take this grid";
         return MPS_ERR_INVALID;
     }
-    const size_t cap = c16_rows_cap(w.cap, ns);
+    const size_t cap = ppe_rows_cap(w.cap, ns);
     const size_t vec = cap + 8;
     const size_t slices = (cap + C16_ROWS - 1) / C16_ROWS + 2;
     const size_t chunks = slices * ((PPE_W + 15) / 16);
@@ -2353,7 +2351,7 @@ int ppe_c16_learned_enable(PpeWork& w, std::string* err) {
     const int e = ppe_sp_enable(w, err);
     if (e != MPS_OK) return e;
     if (w.c16_spfirst) return MPS_OK;
-    const size_t cap = c16_rows_cap(w.cap, w.nscenes);
+    const size_t cap = ppe_rows_cap(w.cap, w.nscenes);
     const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms, w.nscenes);
     const size_t ent = (cap / SP_SLICE + tiles + 1) * SP_SLICE * LP_GW;
     bool ok = c16_alloc(&w.c16_spfirst, tiles * C16_SP_SLICES);
@@ -2407,7 +2405,7 @@ static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, boo
 }
 
 static uint32_t c16_maxslices(const PpeWork& w, uint32_t cap) {
-    return (c16_rows_cap(cap, w.nscenes) + C16_ROWS - 1) / C16_ROWS;
+    return (ppe_rows_cap(cap, w.nscenes) + C16_ROWS - 1) / C16_ROWS;
 }
 
 static C16AsmArgs c16_asm_args(PpeWork& w, const StageArgs& a, uint32_t cap) {
@@ -2439,7 +2437,7 @@ int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& 
     C16AsmArgs A = c16_asm_args(w, a, cap);
     A.K = K;
     // a.cap_solid: particles that can have rows (not dummies)
-    const uint32_t blocks = cblocks(c16_rows_cap(a.cap_solid, w.nscenes) * 32u, 256);
+    const uint32_t blocks = cblocks(ppe_rows_cap(a.cap_solid, w.nscenes) * 32u, 256);
     const uint32_t eblocks = cblocks(C16_ROWS * (A.maxslices + 1), 256);
     if (a.batch.n) {
         if (a.exact) launch(k_c16_assemble<true, true>, blocks, 256, 0, st, A);
@@ -2454,7 +2452,7 @@ int ppe_c16_enqueue_assemble(PpeWork& w, const StageArgs& a, const C16Assemble& 
 }
 
 int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream_t st) {
-    const uint32_t ns = w.nscenes, rows = c16_rows_cap(cap, ns), maxslices = c16_maxslices(w, cap);
+    const uint32_t ns = w.nscenes, rows = ppe_rows_cap(cap, ns), maxslices = c16_maxslices(w, cap);
     launch_scan_exclusive(w.c16_off, maxslices + 1, st);
     if (ns) launch(k_c16_cut, 1, 32, 0, st, w.c16_off, w.c16_srow, c16_nrows(w), ns, (uint32_t)w.sms, w.c16_tb);
     C16PackArgs P;
@@ -2576,7 +2574,7 @@ int ppe_sp_enable(PpeWork& w, std::string* err) {
     w.sp_cap_chunks = slices * (LP_GW + 1);  // entries per lane position: 32-row slices of up to LP_GW + 1
     bool ok = c16_alloc(&w.sp_off, slices + 2);
     ok &= c16_alloc(&w.sp_ent, w.sp_cap_chunks * SP_SLICE);
-    ok &= c16_alloc(&w.sp_diag, (size_t)w.cap + 8);
+    ok &= c16_alloc(&w.sp_diag, (size_t)ppe_rows_cap(w.cap, w.nscenes) + 8);
     ok &= c16_alloc(&w.rq[0], (size_t)w.cap + 8);
     ok &= c16_alloc(&w.rq[1], (size_t)w.cap + 8);
     if (!ok) {
@@ -2615,7 +2613,7 @@ int ppe_sp_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStream
 
 int ppe_c16_export(const PpeWork& w, uint32_t np, const uint32_t* d_row_start, uint32_t* d_cols, float* d_w,
                    cudaStream_t st) {
-    const uint32_t tiles = c16_tiles(c16_rows_cap(np, w.nscenes), (uint32_t)w.sms, w.nscenes);
+    const uint32_t tiles = c16_tiles(ppe_rows_cap(np, w.nscenes), (uint32_t)w.sms, w.nscenes);
     k_c16_export<<<tiles, 256, 0, st>>>(reinterpret_cast<const C16Tile*>(w.c16_tile), w.c16_collist, (uint32_t)w.sms,
                                         w.nscenes, w.clen, ppe_c16_rowlist(w), ppe_c16_nrows(w), w.c16_off, w.c16_ent, w.c16_side, d_row_start,
                                         d_cols, d_w);
