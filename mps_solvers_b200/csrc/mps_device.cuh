@@ -405,6 +405,7 @@ struct HitRing {
         if ((found ^ was) & 32u) {
             __syncwarp();
             work(was & 32u, 32u);
+            __syncwarp();  // its reads before the next hits in its places
         }
     }
     template <class F>
