@@ -1969,12 +1969,17 @@ extern "C" mps_status mps_cell_sort_dev(const float* pos4_dev, uint32_t n, const
     s.hist = b + 4 * nk;
     uint32_t* cs = s.hist + (size_t)SORT_RADIX * (tiles + 1);
     uint32_t* n_dev = cs + g.ncells + 1;
-    if (n) {  // the last pass writes the caller's arrays
+    const bool direct = outputs_apart(pos4_dev, perm_dev, cell_of_dev, n);
+    if (n && direct) {  // the last pass writes the caller's arrays
         s.keys[passes & 1] = cell_of_dev;
         s.vals[passes & 1] = perm_dev;
     }
     const int r = launch_keys_and_sort_plain((const float4*)pos4_dev, n, g, s, n_dev, passes, st);
     launch_cell_start_plain(s.keys[r], n, g, cs, n_in_grid_dev, st);
+    if (n && !direct) {
+        cudaMemcpyAsync(perm_dev, s.vals[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(cell_of_dev, s.keys[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
+    }
     launch_cell_end_from_start(cs, g.ncells, start_dev, end_dev, st);
     const cudaError_t e = cudaStreamSynchronize(st);
     cudaFreeAsync(blk, st);

@@ -79,6 +79,14 @@ void launch_merge_keys_sort(const float4* pos, const float4* tmp, int apply, con
                             const MergeScratch& m, uint32_t cap, cudaStream_t st);
 cudaError_t merge_sort_setup();
 
+// Whether the sort's last pass can write the caller's cells and permutation
+// itself: not where they lie over the positions, which the keys are still
+// read from when the first buffers are written.
+inline bool outputs_apart(const float* pos4, const uint32_t* perm, const uint32_t* cell_of, uint32_t n) {
+    const char *p = (const char*)pos4, *p1 = p + 16 * (size_t)n;
+    auto over = [&](const uint32_t* q) { return (const char*)q < p1 && p < (const char*)(q + n); };
+    return !over(perm) && !over(cell_of);
+}
 // Same pieces with n given on the host (for the device-pointer primitive).
 int launch_keys_and_sort_plain(const float4* pos, uint32_t n, const Grid& g, SortScratch& s, uint32_t* n_dev,
                                int passes, cudaStream_t st);

@@ -105,12 +105,19 @@ extern "C" mps_status mps_cell_sort_dev_noalloc(const float* pos4_dev, uint32_t 
     uint32_t* cs = base + kCells;
     uint32_t* n_dev = base + kCount;
     const int passes = sort_passes(g.ncells);
-    if (n) {  // the last pass writes the caller's arrays
+    const bool direct = outputs_apart(pos4_dev, perm_dev, cell_of_dev, n);
+    if (n && direct) {  // the last pass writes the caller's arrays
         s.keys[passes & 1] = cell_of_dev;
         s.vals[passes & 1] = perm_dev;
     }
     const int r = launch_keys_and_sort_plain((const float4*)pos4_dev, n, g, s, n_dev, passes, st);
     launch_cell_start_plain(s.keys[r], n, g, cs, n_in_grid_dev, st);
+    bool copied = true;
+    if (n && !direct) {
+        copied = cudaMemcpyAsync(perm_dev, s.vals[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st) == cudaSuccess;
+        copied &= cudaMemcpyAsync(cell_of_dev, s.keys[r], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st) ==
+                  cudaSuccess;
+    }
     launch_cell_end_from_start(cs, g.ncells, start_dev, end_dev, st);
-    return cudaStreamSynchronize(st) == cudaSuccess ? MPS_OK : MPS_ERR_CUDA;
+    return cudaStreamSynchronize(st) == cudaSuccess && copied ? MPS_OK : MPS_ERR_CUDA;
 }
