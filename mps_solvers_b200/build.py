@@ -77,6 +77,27 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_variant(name: str, defines) -> str:
+    """The library with ppe_compact.cu's limits set otherwise (the tests'
+    builds that reach its escaped columns), beside the objects.  The objects
+    of the library itself are taken as they are: it may be loaded."""
+    os.makedirs(BUILD, exist_ok=True)
+    lib = os.path.join(BUILD, f"libmps_b200_{name}.so")
+    objs = []
+    for f in CU + CPP:
+        src, obj = os.path.join(CSRC, f), os.path.join(BUILD, f + ".o")
+        if f == "ppe_compact.cu":
+            obj = os.path.join(BUILD, f"ppe_compact.{name}.o")
+            if _stale(obj, src):
+                _run([NVCC] + NVFLAGS + [f"-D{d}" for d in defines] + ["-c", src, "-o", obj])
+        elif not os.path.exists(obj):
+            _run(([NVCC] + NVFLAGS if f in CU else [HOSTCXX] + CXXFLAGS) + ["-c", src, "-o", obj])
+        objs.append(obj)
+    if not os.path.exists(lib) or any(os.path.getmtime(o) > os.path.getmtime(lib) for o in objs):
+        _run([NVCC] + ARCH + ["-shared", "-o", lib] + objs + ["-lcudart"])
+    return lib
+
+
 if __name__ == "__main__":
     build(force="--force" in sys.argv, verbose="-v" in sys.argv)
     print(LIB)

@@ -55,9 +55,21 @@ constexpr uint32_t C16_ESC = 0xffffu;       // escaped code
 // row sums fit a block's shared memory.
 constexpr uint32_t C16_TILE_ROWS = 1600;
 constexpr uint32_t C16_SLICE_COST = 5;
-constexpr uint32_t C16_COLS = 12288;        // columns a tile lists (4 x 12,287 is below the escape code)
-constexpr uint32_t C16_PAGE = 256;          // rows per page of the tile's column set
-constexpr uint32_t C16_PAGES = 512;         // pages a tile's column set holds
+// The limits past which an entry is escaped and a tile is done by one warp;
+// builds of the tests lower them, so that small scenes get there.
+#ifndef MPS_C16_COLS
+#define MPS_C16_COLS 12288
+#endif
+#ifndef MPS_C16_PAGES
+#define MPS_C16_PAGES 512
+#endif
+#ifndef MPS_C16_WHOLE
+#define MPS_C16_WHOLE 0
+#endif
+constexpr uint32_t C16_COLS = MPS_C16_COLS;  // columns a tile lists (4 x 12,287 is below the escape code)
+constexpr uint32_t C16_PAGE = 256;           // rows per page of the tile's column set
+constexpr uint32_t C16_PAGES = MPS_C16_PAGES;  // pages a tile's column set holds
+constexpr bool C16_WHOLE = MPS_C16_WHOLE != 0;  // every tile by one warp
 constexpr uint32_t C16_NONE = 0xffffffffu;
 constexpr int C16_THREADS = 512;            // a solver block
 constexpr int C16_PACK_THREADS = 1024;
@@ -1465,13 +1477,13 @@ struct C16Block {
         whole = false;
         if (ntiles == 1) {
             pl = c16_plan(v.ncol, v.rows, v.nseg, 1u, true, S.ns != 0u);
-            single = pl.res <= S.smem_bytes;
+            single = pl.res <= S.smem_bytes && !C16_WHOLE;
         }
         if (!single) {
             // a tile with so many rows and columns that the pieces do not fit
             // is done by one warp, slices whole: slow, but right
             pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), C16_SEGS, ntiles, false, S.ns != 0u);
-            whole = pl.res > S.smem_bytes;
+            whole = pl.res > S.smem_bytes || C16_WHOLE;
             if (whole) pl = c16_plan(__ldg(S.stats + 1), __ldg(S.stats + 2), 1u, ntiles, false, S.ns != 0u);
         }
         if (whole) v.cpw = max(v.nch, 1u);
