@@ -102,7 +102,6 @@ struct PpeWork {
     uint32_t* clen = nullptr;          // off-diagonal entries of each compact row
     uint32_t* c16_off = nullptr;       // chunks per slice, then (scanned) the slices' first chunk
     unsigned char* c16_ent = nullptr;  // chunks: 128 weights and 128 codes, 768 bytes each
-    uint32_t* c16_side = nullptr;      // compact column of an escaped entry (by entry)
     uint32_t* c16_tile = nullptr;      // tile descriptors
     uint32_t* c16_collist = nullptr;   // the tiles' columns
     uint32_t* c16_stats = nullptr;     // [0] entries past a 16-bit offset from their slice, [1] most columns of a tile

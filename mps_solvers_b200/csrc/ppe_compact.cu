@@ -20,9 +20,9 @@
 //    one with 4 lanes per row; lane L = 8 q + r holds, in every chunk of 16
 //    entries of row r, entries 4 q to 4 q + 3.  A chunk is 768 contiguous
 //    bytes: 512 of weights, then 256 of codes;
-//  * a column past the tile's list (C16_COLS columns) is coded 65535 and its
-//    number kept in a side array; only rows with far more neighbours than a
-//    lattice has get there.
+//  * a column past the tile's list (C16_COLS columns) is coded 65535 and read
+//    from the assembly's row-major columns; only rows with far more neighbours
+//    than a lattice has get there.
 //
 // In every product a block first brings the tile's columns of the vector
 // into shared memory, in coalesced runs, and then reads each entry's operand
@@ -46,8 +46,7 @@ namespace {
 inline uint32_t cblocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
 constexpr uint32_t C16_ROWS = 8;            // rows per slice
-constexpr uint32_t C16_CHUNK = 128;         // entries per chunk (8 rows x 16)
-constexpr uint32_t C16_CHUNK_BYTES = 768;   // 128 weights, then 128 codes
+constexpr uint32_t C16_CHUNK_BYTES = 768;   // a chunk, 128 entries (8 rows x 16): weights, then codes
 constexpr uint32_t C16_ESC = 0xffffu;       // escaped code
 // Rows of a tile on average, and a slice's cost beside its chunks (1 to 32 of
 // them) when tiles are cut: a tile then has at most 37 / 5 of the average,
@@ -587,7 +586,6 @@ struct C16PackArgs {
     C16Tile* tiles;
     uint32_t* collist;        // C16_COLS per tile
     unsigned char* ent;
-    uint32_t* side;
     uint32_t* stats;          // [0] entries beyond a 16-bit offset from their slice, [1] most columns, [2] most rows,
                               // [3] fours of S' given out
     // learned S' (LRN)
@@ -805,7 +803,6 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
                 w = __ldg(rw + 4u * x + q);
             }
             const uint32_t cc[4] = {cv.x, cv.y, cv.z, cv.w};
-            const size_t ch = (size_t)(g0 + x);
             uint32_t code[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -816,7 +813,6 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
                 if (d < 0 || d >= (int)C16_ESC) far++;
                 if (p == C16_NONE) {
                     code[u] = C16_ESC;
-                    A.side[ch * C16_CHUNK + 4u * lane + u] = cc[u];
                     nesc++;
                 } else {
                     code[u] = 4u * p;
@@ -825,7 +821,7 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
             if (e + 1 >= len) w.y = 0.f;
             if (e + 2 >= len) w.z = 0.f;
             if (e + 3 >= len) w.w = 0.f;
-            unsigned char* dst = A.ent + ch * C16_CHUNK_BYTES;
+            unsigned char* dst = A.ent + (size_t)(g0 + x) * C16_CHUNK_BYTES;
             *reinterpret_cast<float4*>(dst + 16u * lane) = w;
             *reinterpret_cast<uint2*>(dst + 512u + 8u * lane) =
                 make_uint2(code[0] | (code[1] << 16), code[2] | (code[3] << 16));
@@ -925,7 +921,7 @@ __global__ void __launch_bounds__(256) k_c16_export(const C16Tile* __restrict__ 
                                                     const uint32_t* __restrict__ rowlist,
                                                     const uint32_t* __restrict__ nrows, const uint32_t* __restrict__ off,
                                                     const unsigned char* __restrict__ ent,
-                                                    const uint32_t* __restrict__ side,
+                                                    const uint32_t* __restrict__ cols_rm,
                                                     const uint32_t* __restrict__ row_start, uint32_t* __restrict__ cols,
                                                     float* __restrict__ out_w) {
     const uint32_t R = *nrows;
@@ -945,7 +941,7 @@ __global__ void __launch_bounds__(256) k_c16_export(const C16Tile* __restrict__ 
                 if (e >= len) continue;
                 const unsigned char* src = ent + (size_t)(g0 + x) * C16_CHUNK_BYTES;
                 const uint32_t c = reinterpret_cast<const uint16_t*>(src + 512)[4u * lane + u];
-                const uint32_t col = c == C16_ESC ? side[(size_t)(g0 + x) * C16_CHUNK + 4u * lane + u]
+                const uint32_t col = c == C16_ESC ? cols_rm[(size_t)k * PPE_W + e]
                                                   : collist[(size_t)blockIdx.x * C16_COLS + c / 4u];
                 cols[o + e] = rowlist[col];
                 out_w[o + e] = reinterpret_cast<const float*>(src)[4u * lane + u];
@@ -1072,7 +1068,7 @@ struct C16Args {
     const uint32_t* nrows;
     const uint32_t* off;        // first chunk of every slice
     const unsigned char* ent;
-    const uint32_t* side;
+    const uint32_t* cols_rm;    // the assembly's columns, PPE_W a row (of escaped entries)
     const C16Tile* tiles;
     const uint32_t* collist;
     const uint32_t* stats;      // [1] most columns and [2] most rows of a tile
@@ -1289,7 +1285,8 @@ __device__ __forceinline__ void c16_product(const C16Args& S, const C16View& v, 
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             if (ESC && c[u] == C16_ESC)
-                o[u] = remote(__ldg(S.side + (size_t)(v.c0 + at) * C16_CHUNK + 4u * lane + u));
+                o[u] = remote(__ldg(S.cols_rm + (size_t)((v.s0 + s) * C16_ROWS + (lane & 7u)) * PPE_W +
+                                    16u * (at - soff[s]) + 4u * (lane >> 3) + u));
             else
                 o[u] = *reinterpret_cast<const T*>(vecb + c[u] * (sizeof(T) / 4));
         }
@@ -2292,7 +2289,6 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork
     ok &= c16_alloc(&w.clen, vec);
     ok &= c16_alloc(&w.c16_off, slices + 2);
     ok &= c16_alloc(&w.c16_ent, chunks * C16_CHUNK_BYTES);
-    ok &= c16_alloc(&w.c16_side, chunks * C16_CHUNK);
     ok &= c16_alloc(&w.c16_tile, tiles * (sizeof(C16Tile) / sizeof(uint32_t)));
     ok &= c16_alloc(&w.c16_collist, tiles * C16_COLS);
     ok &= c16_alloc(&w.c16_stats, C16_STATS);
@@ -2336,13 +2332,13 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork
 void ppe_c16_free(PpeWork& w) {
     if (w.c16_shared) w.c16_cells = w.c16_nbr = nullptr;
     w.c16_shared = false;
-    void* ps[] = {w.c16_cells, w.c16_nbr, w.c16_base, w.cpos, w.clen, w.c16_off, w.c16_ent, w.c16_side, w.c16_tile,
+    void* ps[] = {w.c16_cells, w.c16_nbr, w.c16_base, w.cpos, w.clen, w.c16_off, w.c16_ent, w.c16_tile,
                   w.c16_collist, w.c16_stats, w.cb64, w.cx64, w.cdiag64, w.cdiag32, w.cinv_diag, w.cdsq, w.cr, w.cp,
                   w.cpub[0], w.cpub[1], w.c16_slots, w.c16_epoch, w.c16_dense, w.c16_sfirst, w.c16_srow, w.c16_tb,
                   w.c16_rowlist, w.c16_nrows, w.c16_tsum, w.c16_spfirst, w.c16_spent, w.c16_spside};
     for (void* p : ps)
         if (p) cudaFree(p);
-    w.c16_cells = w.c16_nbr = w.c16_base = w.cpos = w.clen = w.c16_off = w.c16_side = w.c16_tile = nullptr;
+    w.c16_cells = w.c16_nbr = w.c16_base = w.cpos = w.clen = w.c16_off = w.c16_tile = nullptr;
     w.c16_collist = w.c16_stats = nullptr;
     w.c16_ent = nullptr;
     w.cb64 = w.cx64 = w.cdiag64 = nullptr;
@@ -2483,7 +2479,6 @@ int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStrea
     P.tiles = reinterpret_cast<C16Tile*>(w.c16_tile);
     P.collist = w.c16_collist;
     P.ent = w.c16_ent;
-    P.side = w.c16_side;
     P.stats = w.c16_stats;
     P.rowlist = c16_rowlist(w);
     P.cpos = w.cpos;
@@ -2516,7 +2511,7 @@ int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt
     S.srel = w.scene_relres;
     S.off = w.c16_off;
     S.ent = w.c16_ent;
-    S.side = w.c16_side;
+    S.cols_rm = w.cols;
     S.tiles = reinterpret_cast<const C16Tile*>(w.c16_tile);
     S.collist = w.c16_collist;
     S.stats = w.c16_stats;
@@ -2627,8 +2622,8 @@ int ppe_c16_export(const PpeWork& w, uint32_t np, const uint32_t* d_row_start, u
                    cudaStream_t st) {
     const uint32_t tiles = c16_tiles(ppe_rows_cap(np, w.nscenes), (uint32_t)w.sms, w.nscenes);
     k_c16_export<<<tiles, 256, 0, st>>>(reinterpret_cast<const C16Tile*>(w.c16_tile), w.c16_collist, (uint32_t)w.sms,
-                                        w.nscenes, w.clen, ppe_c16_rowlist(w), ppe_c16_nrows(w), w.c16_off, w.c16_ent, w.c16_side, d_row_start,
-                                        d_cols, d_w);
+                                        w.nscenes, w.clen, ppe_c16_rowlist(w), ppe_c16_nrows(w), w.c16_off, w.c16_ent, w.cols,
+                                        d_row_start, d_cols, d_w);
     return MPS_OK;
 }
 
