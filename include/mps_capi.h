@@ -458,7 +458,8 @@ typedef struct mps_tune_report {
     int ppe_pipelined;         /* chosen: 1 pipelined PCG */
     float stage_ms[3];         /* visc + collision + pnd + dash per step at 64, 128, 256 */
     /* PPE solve ms per step: [3 f + t] for form f (0 stored, 1 recomputed,
-     * 2 pipelined) at 1024, 512, 256 threads per block (-1: not run) */
+     * 2 pipelined) at 1024, 512, 256 threads per block (-1: not run; a batch
+     * in the compact layout has only that) */
     float ppe_ms[9];
     int ppe_compact;           /* chosen: 1 the compact 16-bit layout (a batch
                                   keeps the layout of its options: 0)        */

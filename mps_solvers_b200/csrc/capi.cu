@@ -578,6 +578,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
     }
     if (h->opt.method == MPS_METHOD_SEMI_IMPLICIT) {
         int e = ppe_setup(h->ppe, h->cap, 0, h->g, h->P, h->prm, h->stream, &h->err);
+        if (e == MPS_OK) e = ppe_sell_enable(h->ppe, h->stream, &h->err);
         if (e != MPS_OK) return (mps_status)e;
         h->ppe.pipelined = h->opt.ppe_pipelined != 0;
         h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
@@ -609,6 +610,8 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
                 h->cn.c16 = ppe_c16_enable(h->cn, &h->g, 1, &h->ppe, nullptr) == MPS_OK;
                 if (!h->cn.c16) cudaGetLastError();
             }
+            if (!h->cn.c16) e = ppe_sell_enable(h->cn, h->stream, &h->err);
+            if (e != MPS_OK) return (mps_status)e;
         }
     }
     Scalars s;
@@ -914,12 +917,14 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
             if (e == MPS_OK) {
                 h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
                 set_compact(h, true);
-            } else {  // no memory for the tiles beside the 8-byte layout: that one stays
+            } else {  // no memory for the tiles
                 ppe_c16_free(h->ppe);
                 h->err.clear();
                 cudaGetLastError();
             }
         }
+        if (!h->ppe.c16) e = ppe_sell_enable(h->ppe, h->stream, &h->err);
+        if (e != MPS_OK) return (mps_status)e;
     }
     Scalars sc;
     return read_status(h, &sc);
@@ -1652,15 +1657,16 @@ extern "C" mps_status mps_autotune(mps_handle* h, int steps, mps_tune_report* re
         const int ppe_cand[3] = {1024, 512, 256};
         const bool learned = h->opt.precond == MPS_PRECOND_LEARNED && h->ppe.lp.ready;
         const int nforms = (learned || h->nscenes) ? 2 : 3;
-        // form 3: the compact layout (single scenes, diagonal scaling)
-        const bool compact_ok = h->ppe.c16_ready && !h->nscenes && (!learned || h->ppe.sp_ent != nullptr);
+        // form 3: the compact layout; a batch that has it has no other
+        const bool compact_ok = h->ppe.c16_ready && (!learned || h->ppe.sp_ent != nullptr);
+        const bool only_compact = h->nscenes && h->ppe.c16_ready;
         best = 1e300;
         int best_p = h->ppe.threads;
         bool best_sw = h->ppe.stored_weights, best_pipe = h->ppe.pipelined, best_c16 = h->ppe.c16;
         for (int k = 0; k < 3; k++) r.ppe_compact_ms[k] = -1.f;
         for (int c = 0; c < 12; c++) {
             const int form = c / 3;
-            if (form >= nforms && form != 3) {
+            if (form != 3 && (form >= nforms || only_compact)) {
                 r.ppe_ms[c] = -1.f;
                 continue;
             }

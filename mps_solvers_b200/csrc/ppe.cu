@@ -1437,10 +1437,6 @@ int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid&, const Phy
     ok &= al((void**)&w.pos_snap, (size_t)cap * sizeof(float4));
     ok &= al((void**)&w.n_snap, (size_t)cap * sizeof(float));
     ok &= al((void**)&w.id_snap, (size_t)cap * sizeof(uint32_t));
-    ok &= al((void**)&w.sell_off, ((size_t)cap / SELL_C + 4) * sizeof(uint32_t));
-    ok &= al((void**)&w.sell_cols, ((size_t)cap + 8) * (PPE_W + 4) * sizeof(uint32_t));
-    ok &= al((void**)&w.sell_w, ((size_t)cap + 8) * (PPE_W + 4) * sizeof(float));
-    ok &= al((void**)&w.tilecnt, ((size_t)cap / 2048 + 2) * sizeof(uint32_t));
     ok &= al((void**)&w.nrows, sizeof(uint32_t));
     if (!ok) {
         *err = "cudaMalloc failed for the PPE matrix";
@@ -1484,6 +1480,24 @@ int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid&, const Phy
         return MPS_ERR_CUDA;
     }
     w.ready = true;
+    return MPS_OK;
+}
+
+int ppe_sell_enable(PpeWork& w, cudaStream_t st, std::string* err) {
+    const size_t cap = w.cap;
+    bool ok = true;
+    auto al = [&](uint32_t** p, size_t words) {
+        ok = ok && cudaMalloc((void**)p, words * sizeof(uint32_t) + 64) == cudaSuccess;
+        if (ok) cudaMemsetAsync(*p, 0, words * sizeof(uint32_t) + 64, st);
+    };
+    al(&w.sell_off, cap / SELL_C + 4);
+    al(&w.sell_cols, (cap + 8) * (PPE_W + 4));
+    al((uint32_t**)&w.sell_w, (cap + 8) * (PPE_W + 4));
+    al(&w.tilecnt, cap / ROW_TILE + 2);
+    if (!ok) {
+        *err = "cudaMalloc failed for the PPE matrix";
+        return MPS_ERR_CUDA;
+    }
     return MPS_OK;
 }
 

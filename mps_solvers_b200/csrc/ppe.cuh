@@ -158,6 +158,10 @@ inline uint32_t ppe_rows_cap(uint32_t cap, uint32_t nscenes) { return cap + 8u *
 
 int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid& g, const Phys& P, const mps_params& prm,
               cudaStream_t st, std::string* err);
+// the 8-byte layout's matrix (after ppe_setup): 4.1 KB a particle.  A single
+// scene has it beside the tiles, since the autotuner and mps_apply_tuning
+// change its layout; a batch and the viscosity have one of the two.
+int ppe_sell_enable(PpeWork& w, cudaStream_t st, std::string* err);
 // the per-scene tables of a batch (after ppe_setup)
 int ppe_setup_batch(PpeWork& w, const PpeScene* scenes, uint32_t nscenes, cudaStream_t st, std::string* err);
 // assembly, row list and sliced-ELL layout (and, with the learned
