@@ -595,7 +595,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         h->ppe.precond_every = h->opt.precond_every > 0 ? h->opt.precond_every : 40;
         h->ppe.index_of_id = h->index_of_id;
         if (h->opt.ppe_layout == 0 && ppe_c16_takes(h->cap, &h->g, 1)) {
-            e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, &h->err);
+            e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, h->stream, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
             set_compact(h, true);
@@ -607,7 +607,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
             h->cn.l2_keep_entries = h->ppe.l2_keep_entries;
             if (h->ppe.c16_ready) {  // its tiles hold the fluid's rows; the 8-byte layout where they do not fit
                 h->cn.c16_smem_chunks = h->ppe.c16_smem_chunks;
-                h->cn.c16 = ppe_c16_enable(h->cn, &h->g, 1, &h->ppe, nullptr) == MPS_OK;
+                h->cn.c16 = ppe_c16_enable(h->cn, &h->g, 1, &h->ppe, h->stream, nullptr) == MPS_OK;
                 if (!h->cn.c16) cudaGetLastError();
             }
             if (!h->cn.c16) e = ppe_sell_enable(h->cn, h->stream, &h->err);
@@ -912,7 +912,7 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
         if (h->opt.ppe_layout == 0 && ppe_c16_takes(cap, h->scene_grid.data(), S)) {
             h->ppe.c16_smem_chunks =
                 h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
-            e = ppe_c16_enable(h->ppe, h->scene_grid.data(), S, nullptr, &h->err);
+            e = ppe_c16_enable(h->ppe, h->scene_grid.data(), S, nullptr, h->stream, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e == MPS_OK) {
                 h->ppe.l2_keep_entries = l2_keep_entries(h->opt);
@@ -1726,7 +1726,7 @@ extern "C" mps_status mps_apply_tuning(mps_handle* h, const mps_tune_report* r) 
                 h->err = "the compact PPE layout is for single scenes";
                 return MPS_ERR_INVALID;
             }
-            int e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, &h->err);
+            int e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, h->stream, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
         }

@@ -94,6 +94,7 @@ struct PpeWork {
     bool c16_ready = false;            // its buffers exist
     bool c16_shared = false;           // c16_cells and c16_nbr are another work's
     int c16_smem_chunks = 8;           // chunks per warp held in shared memory across iterations
+    unsigned char* c16_block = nullptr;  // the allocation of the arrays from here to c16_epoch
     uint32_t c16_nsuper = 0;           // linked cells, in curve order
     uint32_t* c16_cells = nullptr;     // the up to 4 cells of the sorted grid of each
     uint32_t* c16_nbr = nullptr;       // the 27 linked cells around each
@@ -187,7 +188,8 @@ int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint3
 // escaped-entry count of the last pack, and the stencil export.
 bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids);
 // same: a work of the same grids whose linked cells are used (it is freed with or after w), or null
-int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, std::string* err);
+int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, cudaStream_t st,
+                   std::string* err);
 // the PPE's constants (a batch uses its scenes' own; dim2 is the same for all)
 struct C16Assemble {
     double n0, beta, b_tmp, rho_lambda_alpha_n0, dim2;

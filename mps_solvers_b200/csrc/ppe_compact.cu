@@ -2151,75 +2151,96 @@ bool c16_alloc(T** p, size_t count) {
     return cudaMalloc((void**)p, (count ? count : 1) * sizeof(T)) == cudaSuccess;
 }
 
-// Position of cell (x, y, z) of a 2^bits cube along the Hilbert curve
-// (J. Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004:
-// the axes are turned into the curve's transposed index in place, whose bits
-// are then interleaved).
-uint64_t hilbert_index(uint32_t x, uint32_t y, uint32_t z, int bits) {
-    uint32_t v[3] = {x, y, z};
-    for (uint32_t q = 1u << (bits - 1); q > 1; q >>= 1) {
-        const uint32_t low = q - 1;
-        for (int a = 0; a < 3; a++) {
-            if (v[a] & q) {
-                v[0] ^= low;
-            } else {
-                const uint32_t t = (v[0] ^ v[a]) & low;
-                v[0] ^= t;
-                v[a] ^= t;
+// Several arrays in one allocation (each starts at 256 bytes): a cudaMalloc
+// costs 0.1 ms and more, and a handle has some thirty of these arrays.
+struct C16Arrays {
+    size_t bytes = 0;
+    std::vector<std::pair<void**, size_t>> at;
+    template <class T>
+    void add(T** p, size_t count) {
+        at.push_back({(void**)p, bytes});
+        bytes += (count * sizeof(T) + 255) / 256 * 256;
+    }
+    bool get(unsigned char** block) {
+        if (!c16_alloc(block, bytes)) return false;
+        for (const auto& a : at) *a.first = *block + a.second;
+        return true;
+    }
+};
+
+// The linked cells of a grid (the fast arithmetic's halved cells grouped)
+struct C16Cells {
+    uint32_t f, nx, ny, nz;  // cells of the sorted grid in one along y and z; linked cells
+    C16Cells(const Grid& g)
+        : f((uint32_t)g.reach), nx(g.cdx), ny((g.cdy + f - 1) / f), nz((g.cdz + f - 1) / f) {}
+    uint64_t count() const { return (uint64_t)nx * ny * nz; }
+};
+
+// The cells of a box along the Hilbert curve of the cube around it.  The
+// curve is the one of J. Skilling, "Programming the Hilbert curve" (AIP Conf.
+// Proc. 707, 2004), unrolled from its top level down: in the curve's frame
+// (axis a is the box's axis p[a], mirrored where f[a]) the octants come in
+// Gray code order, backwards in cubes of odd parity; a set bit of axis a
+// mirrors axis 0 of the octant's own frame, a clear one swaps axes 0 and a.
+// Octants outside the box are passed over.  79,950 cells take 1.4 ms of host
+// time; computing and sorting the cells' positions took 11.8.
+struct C16Curve {
+    uint32_t n[3];
+    uint32_t* out;  // (z ny + y) nx + x of each cell
+    void cube(const uint32_t (&at)[3], uint32_t edge, const uint32_t (&p0)[3], const uint32_t (&f0)[3], bool odd) {
+        if (edge == 1) {
+            *out++ = (at[2] * n[1] + at[1]) * n[0] + at[0];
+            return;
+        }
+        for (uint32_t d = 0; d < 8; d++) {
+            const uint32_t v = odd ? 7u - d : d;
+            const uint32_t b[3] = {v >> 2, ((v >> 1) ^ (v >> 2)) & 1u, (v ^ (v >> 1)) & 1u};
+            uint32_t o[3] = {at[0], at[1], at[2]}, p[3] = {p0[0], p0[1], p0[2]}, f[3] = {f0[0], f0[1], f0[2]};
+            for (int a = 0; a < 3; a++) o[p[a]] += b[a] != f[a] ? edge / 2 : 0u;
+            if (o[0] >= n[0] || o[1] >= n[1] || o[2] >= n[2]) continue;
+            for (int a = 0; a < 3; a++) {
+                if (b[a]) {
+                    f[0] ^= 1u;
+                } else {
+                    std::swap(p[0], p[a]);
+                    std::swap(f[0], f[a]);
+                }
             }
+            cube(o, edge / 2, p, f, odd != ((v & 1u) != 0u));
         }
     }
-    v[1] ^= v[0];
-    v[2] ^= v[1];
-    uint32_t t = 0;
-    for (uint32_t q = 1u << (bits - 1); q > 1; q >>= 1)
-        if (v[2] & q) t ^= q - 1;
-    uint64_t h = 0;
-    for (int b = bits - 1; b >= 0; b--)
-        for (int a = 0; a < 3; a++) h = (h << 1) | (((v[a] ^ t) >> b) & 1u);
-    return h;
+};
+
+void curve_order(const C16Cells& c, uint32_t* out) {
+    C16Curve w{{c.nx, c.ny, c.nz}, out};
+    uint32_t edge = 2;
+    while (edge < std::max(c.nx, std::max(c.ny, c.nz))) edge *= 2;
+    w.cube({0, 0, 0}, edge, {0, 1, 2}, {0, 0, 0}, false);
 }
 
-// The linked cells of a grid in curve order: their up to 4 cells of the
-// sorted grid (global ids) and the 27 linked cells around each.
-void linked_cells(const Grid& g, std::vector<uint32_t>* cells, std::vector<uint32_t>* nbr) {
-    const uint32_t f = (uint32_t)g.reach;  // 2 on the refined grid, else 1
-    const uint32_t nx = g.cdx, ny = (g.cdy + f - 1) / f, nz = (g.cdz + f - 1) / f;
-    const uint32_t most = std::max(nx, std::max(ny, nz));
-    int bits = 1;
-    while ((1u << bits) < most) bits++;
-    struct Key {
-        uint64_t h;
-        uint32_t x, y, z;
-    };
-    std::vector<Key> order;
-    order.reserve((size_t)nx * ny * nz);
-    for (uint32_t z = 0; z < nz; z++)
-        for (uint32_t y = 0; y < ny; y++)
-            for (uint32_t x = 0; x < nx; x++) order.push_back({hilbert_index(x, y, z, bits), x, y, z});
-    std::sort(order.begin(), order.end(), [](const Key& a, const Key& b) { return a.h < b.h; });
-    const uint32_t first = (uint32_t)(cells->size() / 4);
-    std::vector<uint32_t> rank(order.size());
-    for (size_t k = 0; k < order.size(); k++)
-        rank[((size_t)order[k].z * ny + order[k].y) * nx + order[k].x] = first + (uint32_t)k;
-    cells->resize(cells->size() + 4 * order.size());
-    nbr->resize(nbr->size() + 27 * order.size());
-    uint32_t* c = cells->data() + 4 * (size_t)first;
-    uint32_t* n = nbr->data() + 27 * (size_t)first;
-    for (const Key& o : order) {
-        for (uint32_t b = 0; b < 2; b++)
-            for (uint32_t a = 0; a < 2; a++) {
-                const uint32_t y = o.y * f + a, z = o.z * f + b;
-                const bool in = a < f && b < f && y < g.cdy && z < g.cdz;
-                *c++ = in ? g.base + z * g.sheet + y * g.cdx + o.x : C16_NONE;
-            }
-        for (int dz = -1; dz <= 1; dz++)
-            for (int dy = -1; dy <= 1; dy++)
-                for (int dx = -1; dx <= 1; dx++) {
-                    const uint32_t x = o.x + (uint32_t)dx, y = o.y + (uint32_t)dy, z = o.z + (uint32_t)dz;
-                    const bool in = x < nx && y < ny && z < nz;  // below 0 wraps
-                    *n++ = in ? rank[((size_t)z * ny + y) * nx + x] : C16_NONE;
-                }
+// The place of every linked cell on the curve (first: the grid's first one).
+__global__ void __launch_bounds__(256) k_c16_rank(const uint32_t* __restrict__ order, uint32_t n, uint32_t first,
+                                                  uint32_t* __restrict__ rank) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) rank[order[k]] = first + k;
+}
+
+// A warp a linked cell: the 27 linked cells around it (C16_NONE: outside) and
+// its up to 4 cells of the sorted grid (global ids).
+__global__ void __launch_bounds__(256) k_c16_links(Grid g, C16Cells c, const uint32_t* __restrict__ order, uint32_t n,
+                                                   const uint32_t* __restrict__ rank, uint32_t* __restrict__ cells,
+                                                   uint32_t* __restrict__ nbr) {
+    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k >= n) return;
+    const uint32_t lin = order[k], cx = lin % c.nx, cy = lin / c.nx % c.ny, cz = lin / c.nx / c.ny;
+    if (lane < 27) {
+        const uint32_t x = cx + lane % 3 - 1, y = cy + lane / 3 % 3 - 1, z = cz + lane / 9 - 1;  // below 0 wraps
+        const bool in = x < c.nx && y < c.ny && z < c.nz;
+        nbr[27 * (size_t)k + lane] = in ? rank[(z * c.ny + y) * c.nx + x] : C16_NONE;
+    } else if (lane < 31) {
+        const uint32_t a = (lane - 27) & 1u, b = (lane - 27) >> 1, y = cy * c.f + a, z = cz * c.f + b;
+        const bool in = a < c.f && b < c.f && y < g.cdy && z < g.cdz;
+        cells[4 * (size_t)k + lane - 27] = in ? g.base + z * g.sheet + y * g.cdx + cx : C16_NONE;
     }
 }
 
@@ -2246,7 +2267,8 @@ bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
     return c16_page_bytes(ppe_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
 }
 
-int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, std::string* err) {
+int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, cudaStream_t st,
+                   std::string* err) {
     if (w.c16_ready) return MPS_OK;
     const uint32_t ns = w.nscenes;
     if (!ppe_c16_takes(w.cap, grids, ngrids)) {
@@ -2258,64 +2280,72 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork
     const size_t slices = (cap + C16_ROWS - 1) / C16_ROWS + 2;
     const size_t chunks = slices * ((PPE_W + 15) / 16);
     const size_t tiles = c16_tiles((uint32_t)cap, (uint32_t)w.sms, ns);
-    std::vector<uint32_t> cells, nbr, sfirst;
-    bool ok = true;
+    C16Arrays A;
     w.c16_shared = same && same->c16_ready;
+    std::vector<uint32_t> sfirst(1, 0u);
+    for (uint32_t s = 0; s < ngrids; s++) sfirst.push_back(sfirst.back() + (uint32_t)C16Cells(grids[s]).count());
+    w.c16_nsuper = sfirst.back();
     if (w.c16_shared) {
-        w.c16_nsuper = same->c16_nsuper;
         w.c16_cells = same->c16_cells;
         w.c16_nbr = same->c16_nbr;
     } else {
-        for (uint32_t s = 0; s < ngrids; s++) {
-            sfirst.push_back((uint32_t)(cells.size() / 4));
-            linked_cells(grids[s], &cells, &nbr);
-        }
-        sfirst.push_back((uint32_t)(cells.size() / 4));
-        w.c16_nsuper = (uint32_t)(cells.size() / 4);
-        ok &= c16_alloc(&w.c16_cells, cells.size());
-        ok &= c16_alloc(&w.c16_nbr, nbr.size());
+        A.add(&w.c16_cells, 5 * (size_t)w.c16_nsuper);  // and the curve order, behind
+        A.add(&w.c16_nbr, 27 * (size_t)w.c16_nsuper);
     }
-    ok &= c16_alloc(&w.c16_base, (size_t)w.c16_nsuper + 2);
+    A.add(&w.c16_base, (size_t)w.c16_nsuper + 2);
     if (ns) {
-        ok &= c16_alloc(&w.c16_dense, (size_t)w.c16_nsuper + 2);
-        ok &= c16_alloc(&w.c16_sfirst, ns + 1);
-        ok &= c16_alloc(&w.c16_srow, ns + 1);
-        ok &= c16_alloc(&w.c16_tb, PPE_MAX_SCENES + 1);
-        ok &= c16_alloc(&w.c16_rowlist, vec);
-        ok &= c16_alloc(&w.c16_nrows, 1);
-        ok &= c16_alloc(&w.c16_tsum, 2 * tiles * C16_SUMS);
+        A.add(&w.c16_dense, (size_t)w.c16_nsuper + 2);
+        A.add(&w.c16_sfirst, ns + 1);
+        A.add(&w.c16_srow, ns + 1);
+        A.add(&w.c16_tb, PPE_MAX_SCENES + 1);
+        A.add(&w.c16_rowlist, vec);
+        A.add(&w.c16_nrows, 1);
+        A.add(&w.c16_tsum, 2 * tiles * C16_SUMS);
     }
-    ok &= c16_alloc(&w.cpos, cap);
-    ok &= c16_alloc(&w.clen, vec);
-    ok &= c16_alloc(&w.c16_off, slices + 2);
-    ok &= c16_alloc(&w.c16_ent, chunks * C16_CHUNK_BYTES);
-    ok &= c16_alloc(&w.c16_tile, tiles * (sizeof(C16Tile) / sizeof(uint32_t)));
-    ok &= c16_alloc(&w.c16_collist, tiles * C16_COLS);
-    ok &= c16_alloc(&w.c16_stats, C16_STATS);
-    ok &= c16_alloc(&w.cb64, vec);
-    ok &= c16_alloc(&w.cx64, vec);
-    ok &= c16_alloc(&w.cdiag64, vec);
-    ok &= c16_alloc(&w.cdiag32, vec);
-    ok &= c16_alloc(&w.cinv_diag, vec);
-    ok &= c16_alloc(&w.cdsq, vec);
-    ok &= c16_alloc(&w.cr, vec);
-    ok &= c16_alloc(&w.cp, vec);
-    ok &= c16_alloc(&w.cpub[0], vec);
-    ok &= c16_alloc(&w.cpub[1], vec);
-    ok &= c16_alloc(&w.c16_slots, 2 * (size_t)w.sms * w.sms * C16_SUMS);
-    ok &= c16_alloc(&w.c16_epoch, 1);
-    if (!ok) {
+    A.add(&w.cpos, cap);
+    A.add(&w.clen, vec);
+    A.add(&w.c16_off, slices + 2);
+    A.add(&w.c16_ent, chunks * C16_CHUNK_BYTES);
+    A.add(&w.c16_tile, tiles * (sizeof(C16Tile) / sizeof(uint32_t)));
+    A.add(&w.c16_collist, tiles * C16_COLS);
+    A.add(&w.c16_stats, C16_STATS);
+    A.add(&w.cb64, vec);
+    A.add(&w.cx64, vec);
+    A.add(&w.cdiag64, vec);
+    A.add(&w.cdiag32, vec);
+    A.add(&w.cinv_diag, vec);
+    A.add(&w.cdsq, vec);
+    A.add(&w.cr, vec);
+    A.add(&w.cp, vec);
+    A.add(&w.cpub[0], vec);
+    A.add(&w.cpub[1], vec);
+    A.add(&w.c16_slots, 2 * (size_t)w.sms * w.sms * C16_SUMS);
+    A.add(&w.c16_epoch, 1);
+    const bool have = A.get(&w.c16_block);
+    if (!have) {
         ppe_c16_free(w);
         if (err) *err = "cudaMalloc failed for the compact PPE layout";
         return MPS_ERR_CUDA;
     }
-    cudaMemset(w.c16_stats, 0, C16_STATS * sizeof(uint32_t));
-    cudaMemset(w.c16_epoch, 0, sizeof(unsigned long long));
-    cudaMemset(w.c16_slots, 0, 2 * (size_t)w.sms * w.sms * C16_SUMS * sizeof(ulonglong2));
-    if ((ns && cudaMemcpy(w.c16_sfirst, sfirst.data(), sfirst.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) ||
-        (!w.c16_shared &&
-         (cudaMemcpy(w.c16_cells, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-          cudaMemcpy(w.c16_nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess)) ||
+    bool ok = true;
+    cudaMemsetAsync(w.c16_stats, 0, C16_STATS * sizeof(uint32_t), st);
+    cudaMemsetAsync(w.c16_epoch, 0, sizeof(unsigned long long), st);
+    cudaMemsetAsync(w.c16_slots, 0, 2 * (size_t)w.sms * w.sms * C16_SUMS * sizeof(ulonglong2), st);
+    if (!w.c16_shared) {
+        std::vector<uint32_t> order(w.c16_nsuper);
+        for (uint32_t s = 0; s < ngrids; s++) curve_order(C16Cells(grids[s]), order.data() + sfirst[s]);
+        uint32_t* dev = w.c16_cells + 4 * (size_t)w.c16_nsuper;
+        ok = cudaMemcpyAsync(dev, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st) == cudaSuccess;
+        for (uint32_t s = 0; s < ngrids && ok; s++) {
+            const uint32_t first = sfirst[s], n = sfirst[s + 1] - first;
+            uint32_t* rank = w.c16_base + first;  // each step writes the array anew
+            k_c16_rank<<<cblocks(n, 256), 256, 0, st>>>(dev + first, n, first, rank);
+            k_c16_links<<<cblocks(n, 8), 256, 0, st>>>(grids[s], C16Cells(grids[s]), dev + first, n, rank,
+                                                       w.c16_cells + 4 * (size_t)first, w.c16_nbr + 27 * (size_t)first);
+        }
+        ok = cudaStreamSynchronize(st) == cudaSuccess && ok;  // before the order goes
+    }
+    if (!ok || (ns && cudaMemcpyAsync(w.c16_sfirst, sfirst.data(), sfirst.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) ||
         cudaFuncSetAttribute(k_c16_pack<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)C16_PAGE_BYTES_MAX) != cudaSuccess ||
         cudaFuncSetAttribute(k_c16_pack<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2330,14 +2360,9 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork
 }
 
 void ppe_c16_free(PpeWork& w) {
-    if (w.c16_shared) w.c16_cells = w.c16_nbr = nullptr;
-    w.c16_shared = false;
-    void* ps[] = {w.c16_cells, w.c16_nbr, w.c16_base, w.cpos, w.clen, w.c16_off, w.c16_ent, w.c16_tile,
-                  w.c16_collist, w.c16_stats, w.cb64, w.cx64, w.cdiag64, w.cdiag32, w.cinv_diag, w.cdsq, w.cr, w.cp,
-                  w.cpub[0], w.cpub[1], w.c16_slots, w.c16_epoch, w.c16_dense, w.c16_sfirst, w.c16_srow, w.c16_tb,
-                  w.c16_rowlist, w.c16_nrows, w.c16_tsum, w.c16_spfirst, w.c16_spent, w.c16_spside};
-    for (void* p : ps)
+    for (void* p : {(void*)w.c16_block, (void*)w.c16_spfirst, (void*)w.c16_spent, (void*)w.c16_spside})
         if (p) cudaFree(p);
+    w.c16_block = nullptr;
     w.c16_cells = w.c16_nbr = w.c16_base = w.cpos = w.clen = w.c16_off = w.c16_tile = nullptr;
     w.c16_collist = w.c16_stats = nullptr;
     w.c16_ent = nullptr;
@@ -2349,6 +2374,7 @@ void ppe_c16_free(PpeWork& w) {
     w.c16_tsum = nullptr;
     w.c16_epoch = nullptr;
     w.c16_spfirst = w.c16_spent = w.c16_spside = nullptr;
+    w.c16_shared = false;
     w.c16_ready = false;
     w.c16 = false;
     w.c16_learned = false;
