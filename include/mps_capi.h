@@ -108,8 +108,9 @@ typedef struct {
                             give the same stable order.                       */
     int ppe_layout;      /* PPE matrix in the solver: 0 = compact (tiles of
                             neighbouring rows, 16-bit codes into each tile's
-                            list of columns, 6 bytes per entry); -1 = always
-                            the 8-byte layout.  Same matrix either way;
+                            list of columns, 6 bytes per entry), or the
+                            8-byte layout in grids with more than 4 linked
+                            cells a particle; -1 = always the 8-byte layout.  Same matrix either way;
                             mps_autotune may change a single scene's.         */
     int ppe_smem_chunks; /* 128-entry chunks of the matrix kept in shared
                             memory across CG iterations, per each of an SM's

@@ -594,7 +594,7 @@ static mps_status setup(mps_handle* h, const mps_params& prm, uint32_t np, uint3
         h->ppe.c16_smem_chunks = h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
         h->ppe.precond_every = h->opt.precond_every > 0 ? h->opt.precond_every : 40;
         h->ppe.index_of_id = h->index_of_id;
-        if (h->opt.ppe_layout == 0 && ppe_c16_takes(h->cap, &h->g, 1)) {
+        if (h->opt.ppe_layout == 0 && ppe_c16_prefers(h->cap, &h->g, 1)) {
             e = ppe_c16_enable(h->ppe, &h->g, 1, nullptr, h->stream, &h->err);
             if (e == MPS_OK && h->opt.precond == MPS_PRECOND_LEARNED) e = ppe_c16_learned_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
@@ -909,7 +909,7 @@ static mps_status setup_batch(mps_handle* h, const std::vector<mps_params>& prms
             if (e == MPS_OK) e = ppe_sp_enable(h->ppe, &h->err);
             if (e != MPS_OK) return (mps_status)e;
         }
-        if (h->opt.ppe_layout == 0 && ppe_c16_takes(cap, h->scene_grid.data(), S)) {
+        if (h->opt.ppe_layout == 0 && ppe_c16_prefers(cap, h->scene_grid.data(), S)) {
             h->ppe.c16_smem_chunks =
                 h->opt.ppe_smem_chunks == 0 ? 8 : (h->opt.ppe_smem_chunks < 0 ? 0 : h->opt.ppe_smem_chunks);
             e = ppe_c16_enable(h->ppe, h->scene_grid.data(), S, nullptr, h->stream, &h->err);

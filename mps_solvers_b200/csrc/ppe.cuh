@@ -184,9 +184,11 @@ void ppe_free(PpeWork& w);
 int ppe_export_stencil(const PpeWork& w, uint32_t np, uint32_t* row_start, uint32_t* cols, float* wts,
                        uint64_t max_entries, uint64_t* nnz, cudaStream_t st);
 // The compact 16-bit layout and its persistent solver (ppe_compact.cu):
-// whether it takes a grid and capacity, buffers, the pack after the assembly, the solve with p = max(x, 0), the
+// whether it takes a grid and capacity, and is the faster one for them,
+// buffers, the pack after the assembly, the solve with p = max(x, 0), the
 // escaped-entry count of the last pack, and the stencil export.
 bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids);
+bool ppe_c16_prefers(uint32_t cap, const Grid* grids, uint32_t ngrids);
 // same: a work of the same grids whose linked cells are used (it is freed with or after w), or null
 int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, cudaStream_t st,
                    std::string* err);

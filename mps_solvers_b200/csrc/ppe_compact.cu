@@ -2260,11 +2260,29 @@ static bool c16_solver_smem() {
     return true;
 }
 
-// the pack's page table is in shared memory: 20 M particles
+static uint64_t c16_cells(const Grid* grids, uint32_t ngrids) {
+    uint64_t n = 0;
+    for (uint32_t s = 0; s < ngrids; s++) n += C16Cells(grids[s]).count();
+    return n;
+}
+
+// the pack's page table is in shared memory: 20 M particles; a warp a linked
+// cell in 32-bit thread numbers
 bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
     for (uint32_t s = 0; s < ngrids; s++)
         if (grids[s].reach > 2) return false;
-    return c16_page_bytes(ppe_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
+    return c16_cells(grids, ngrids) < (1u << 26) &&
+           c16_page_bytes(ppe_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
+}
+
+// Every step counts and scans the linked cells, empty ones too (0.6 ms a
+// million), and a cell's links take 128 bytes: in a grid that is nearly empty
+// (a particle far from the others) the 8-byte layout is faster.  70,912
+// particles, ms a step over tiles and in the 8-byte layout: 4.05 cells a
+// particle 0.68 and 0.78 (learned 0.86 and 0.99), 5.95 0.77 and 0.79, 8.4 0.89
+// and 0.80, 19 1.37 and 0.86.  A tank full of water has 0.02, half full 0.04.
+bool ppe_c16_prefers(uint32_t cap, const Grid* grids, uint32_t ngrids) {
+    return ppe_c16_takes(cap, grids, ngrids) && c16_cells(grids, ngrids) <= 4ull * cap;
 }
 
 int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, cudaStream_t st,
