@@ -268,6 +268,31 @@ __device__ __forceinline__ CellNear cell_near(const Grid& g, uint32_t c, float x
     return n;
 }
 
+// A Crank-Nicolson component's reach: components after the first see positions
+// that the earlier ones moved since the particles were sorted, by at most
+// moved[0] (and moved[1]) along their axes.  A neighbour is then up to that
+// much nearer than its cell, and the particle itself up to that much outside
+// its own, so the cells are culled at twice the distance more.  Both rows of a
+// pair find each other again: the matrix is symmetric.
+__device__ __forceinline__ float cn_reach(float re, const uint32_t* __restrict__ moved, int c) {
+    float m = 0.f;
+    for (int k = 0; k < c; k++) m += __uint_as_float(moved[k]);
+    return re + 2.f * m;
+}
+
+// The largest |m| of a block of 256 threads into *most (its bits; all threads call it)
+__device__ __forceinline__ void block_max_abs(float m, uint32_t* __restrict__ most) {
+    __shared__ uint32_t part[8];
+    uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(m)));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = b;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; w++) b = max(b, part[w]);
+        if (b) atomicMax(most, b);
+    }
+}
+
 // link_row restricted to the cells that can hold a particle within re
 // row (dz, dy) of the walk
 __device__ __forceinline__ RowRange link_row_near_at(const Grid& g, const uint32_t* __restrict__ cell_start,

@@ -1438,6 +1438,7 @@ int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid&, const Phy
     ok &= al((void**)&w.n_snap, (size_t)cap * sizeof(float));
     ok &= al((void**)&w.id_snap, (size_t)cap * sizeof(uint32_t));
     ok &= al((void**)&w.nrows, sizeof(uint32_t));
+    ok &= al((void**)&w.moved, 3 * sizeof(uint32_t));
     if (!ok) {
         *err = "cudaMalloc failed for the PPE matrix";
         return MPS_ERR_CUDA;
@@ -1875,10 +1876,8 @@ int ppe_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt, ui
 // over every neighbour j != i within rlap (all types; w = rlap/r - 1), with
 // 1/R = lambda n0 / (dim niu dt) and g the step's body force; other rows are
 // Dirichlet (the reference's identity rows, x = u).  x starts at u.  One warp
-// per particle walks the linked cells, culled as for the other stages.
-// Components after the first see positions the earlier ones moved since the
-// last cell rebuild: a neighbour that crossed a cell face since then can be
-// missed at the very edge of rlap, where its weight is almost 0.
+// per particle walks the linked cells, culled for what the earlier components
+// moved (cn_reach).
 struct CnArgs {
     StageArgs a;
     int c;
@@ -1891,6 +1890,7 @@ struct CnArgs {
     double* b64;
     double* x64;
     unsigned* bar;
+    uint32_t* moved;                // by component
     double lambda_n0_over_dim_niu;  // lambda n0 / (dim niu): 1/R = this / dt
 };
 
@@ -1903,7 +1903,10 @@ __global__ void __launch_bounds__(256) k_cn_assemble(CnArgs A) {
     const uint32_t n = a.sc->np;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) A.bar[0] = 0u;  // the solver's barrier starts empty
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.bar[0] = 0u;  // the solver's barrier starts empty
+        A.moved[A.c] = 0u;
+    }
     if (i >= n) return;
     const float4* __restrict__ pos = a.cur.pos;
     const float4* __restrict__ vel = a.cur.vel;
@@ -1927,7 +1930,7 @@ __global__ void __launch_bounds__(256) k_cn_assemble(CnArgs A) {
     uint32_t count = 0;
     double diag = 0.0, bi = 0.0;
     const uint32_t lt = (1u << lane) - 1u;
-    const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
+    const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, cn_reach(re, A.moved, A.c));
     walk_cells<!EX>(L.g, L.cs, L.c, nr, lane, [&](uint32_t j, bool in) {
         {
             bool app = false;
@@ -1976,19 +1979,23 @@ __global__ void __launch_bounds__(256) k_cn_assemble(CnArgs A) {
 
 // MPS_CPU_IMPL::updatePosVel<dir> (MPS_CAL_v4.0/MPS_CPU_IMPL.cpp:129-190):
 // fluid u_c = x, x_c += dt u_c.
-__global__ void k_cn_finish(const double* __restrict__ x64, const uint32_t* __restrict__ rlen, State s, int c,
-                            const Scalars* sc) {
+__global__ void __launch_bounds__(256) k_cn_finish(const double* __restrict__ x64, const uint32_t* __restrict__ rlen,
+                                                   State s, int c, const Scalars* sc, uint32_t* __restrict__ moved) {
     after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= sc->np || rlen[i] == PPE_DIRICHLET) return;
-    const float x = (float)x64[i];
-    float4 u = s.vel[i], p = s.pos[i];
-    const float np_ = __fadd_rn(comp(p, c), __fmul_rn(sc->dt, x));
-    if (c == 0) { u.x = x; p.x = np_; }
-    else if (c == 1) { u.y = x; p.y = np_; }
-    else { u.z = x; p.z = np_; }
-    s.vel[i] = u;
-    s.pos[i] = p;
+    float step = 0.f;
+    if (i < sc->np && rlen[i] != PPE_DIRICHLET) {
+        const float x = (float)x64[i];
+        float4 u = s.vel[i], p = s.pos[i];
+        step = __fmul_rn(sc->dt, x);
+        const float np_ = __fadd_rn(comp(p, c), step);
+        if (c == 0) { u.x = x; p.x = np_; }
+        else if (c == 1) { u.y = x; p.y = np_; }
+        else { u.z = x; p.z = np_; }
+        s.vel[i] = u;
+        s.pos[i] = p;
+    }
+    block_max_abs(step, moved + c);
 }
 
 int ppe_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c, double n0, double lambda,
@@ -2007,13 +2014,14 @@ int ppe_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, int c
     A.b64 = w.b64;
     A.x64 = w.x64;
     A.bar = w.bar;
+    A.moved = w.moved;
     A.lambda_n0_over_dim_niu = lambda_n0_over_dim_niu;
     const uint32_t warps_blocks = blocks_for(cap * 32u, 256);
     if (a.exact) launch(k_cn_assemble<true>, warps_blocks, 256, 0, st, A);
     else launch(k_cn_assemble<false>, warps_blocks, 256, 0, st, A);
     int launched = 1 + enqueue_rows_pack(w, a, cap, st);
     launched += ppe_enqueue_solve(w, a, opt, cap, st);
-    launch(k_cn_finish, blocks_for(cap, 256), 256, 0, st, w.x64, w.rlen, a.cur, c, a.sc);
+    launch(k_cn_finish, blocks_for(cap, 256), 256, 0, st, w.x64, w.rlen, a.cur, c, a.sc, w.moved);
     return launched + 1;
 }
 
@@ -2063,7 +2071,7 @@ int ppe_setup_batch(PpeWork& w, const PpeScene* scenes, uint32_t nscenes, cudaSt
 void ppe_free(PpeWork& w) {
     void* ps[] = {w.cols, w.wrm, w.rlen, w.diag64, w.diag32, w.inv_diag, w.b64, w.x64,
                   w.r,    w.zp[0], w.zp[1], w.q,    w.qp,   w.part,     w.result, w.bar,
-                  w.rowlist, w.tilecnt, w.nrows, w.sell_off, w.sell_cols, w.sell_w, w.pos_snap, w.n_snap,
+                  w.rowlist, w.tilecnt, w.nrows, w.moved, w.sell_off, w.sell_cols, w.sell_w, w.pos_snap, w.n_snap,
                   w.id_snap, w.pu, w.pw, w.pz, w.pq, w.ps, w.pp, w.pm[0], w.pm[1], w.scenes, w.row_scene, w.bpart, w.bresult, w.scene_iters, w.scene_outer,
                   w.scene_relres, w.sp_off, w.sp_ent, w.sp_diag, w.rq[0], w.rq[1]};
     lp_free(w.lp);

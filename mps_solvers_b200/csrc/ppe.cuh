@@ -37,6 +37,7 @@ struct PpeScene {
 };
 
 struct PpeWork {
+    uint32_t* moved = nullptr;  // the viscosity's solves: the farthest each component moved a particle (float bits)
     bool ready = false;
     uint32_t cap = 0;
     int blocks = 0;                    // co-resident blocks of the persistent solver

@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(256) k_c16_rowend(C16AsmArgs A) {
 struct C16CnArgs {
     C16AsmArgs A;
     int c;                          // velocity component
+    uint32_t* moved;                // by component (cn_reach)
     double lambda_n0_over_dim_niu;  // 1/R = this / dt
 };
 
@@ -403,6 +404,7 @@ __global__ void __launch_bounds__(256) k_c16_cn_assemble(C16CnArgs C) {
     const StageArgs& a = A.a;
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
     const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) C.moved[C.c] = 0u;
     if (k >= *A.nrows) return;
     const uint32_t i = __ldg(A.rowlist + k);
     HitRing hits(rings[threadIdx.x >> 5]);
@@ -437,7 +439,7 @@ __global__ void __launch_bounds__(256) k_c16_cn_assemble(C16CnArgs C) {
         }
         count += __popc(ma);
     };
-    const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, re);
+    const CellNear nr = cell_near(L.g, L.c, pi.x, pi.y, pi.z, cn_reach(re, C.moved, C.c));
     flat_batches(flat_walk(L.g, L.cs, L.c, nr, lane), lane, [&](uint32_t j, bool in) {
         const float4 pj = __ldg(pos + j);
         const float dx = fsub<EX>(pj.x, pi.x), dy = fsub<EX>(pj.y, pi.y), dz = fsub<EX>(pj.z, pi.z);
@@ -479,20 +481,24 @@ __global__ void __launch_bounds__(256) k_c16_cn_rowend(C16CnArgs C) {
 // MPS_CPU_IMPL::updatePosVel<dir> (MPS_CAL_v4.0/MPS_CPU_IMPL.cpp:129-190):
 // fluid u_c = x, x_c += dt u_c.
 __global__ void __launch_bounds__(256) k_c16_cn_finish(const double* __restrict__ cx64, const uint32_t* __restrict__ cpos,
-                                                       State s, int c, const Scalars* __restrict__ sc) {
+                                                       State s, int c, const Scalars* __restrict__ sc,
+                                                       uint32_t* __restrict__ moved) {
     after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= sc->np) return;
-    const uint32_t k = cpos[i];
-    if (k == C16_NONE) return;
-    const float x = (float)cx64[k];
-    float4 u = s.vel[i], p = s.pos[i];
-    const float at = __fadd_rn(c16_comp(p, c), __fmul_rn(sc->dt, x));
-    if (c == 0) { u.x = x; p.x = at; }
-    else if (c == 1) { u.y = x; p.y = at; }
-    else { u.z = x; p.z = at; }
-    s.vel[i] = u;
-    s.pos[i] = p;
+    const uint32_t k = i < sc->np ? cpos[i] : C16_NONE;
+    float step = 0.f;
+    if (k != C16_NONE) {
+        const float x = (float)cx64[k];
+        float4 u = s.vel[i], p = s.pos[i];
+        step = __fmul_rn(sc->dt, x);
+        const float at = __fadd_rn(c16_comp(p, c), step);
+        if (c == 0) { u.x = x; p.x = at; }
+        else if (c == 1) { u.y = x; p.y = at; }
+        else { u.z = x; p.z = at; }
+        s.vel[i] = u;
+        s.pos[i] = p;
+    }
+    block_max_abs(step, moved + c);
 }
 
 // Weight of the slices before s when tiles are cut.
@@ -2604,6 +2610,7 @@ int ppe_c16_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, i
     C16CnArgs C;
     C.A = c16_asm_args(w, a, cap);
     C.c = c;
+    C.moved = w.moved;
     C.lambda_n0_over_dim_niu = lambda_n0_over_dim_niu;
     const uint32_t blocks = cblocks(a.cap_fluid * 32u, 256);
     if (a.exact) launch(k_c16_cn_assemble<true>, blocks, 256, 0, st, C);
@@ -2611,7 +2618,7 @@ int ppe_c16_enqueue_cn(PpeWork& w, const StageArgs& a, const mps_options& opt, i
     launch(k_c16_cn_rowend, cblocks(C16_ROWS * (C.A.maxslices + 1), 256), 256, 0, st, C);
     launched += 2 + ppe_c16_enqueue_pack(w, a, cap, st);
     launched += ppe_c16_enqueue_solve(w, a, opt, cap, st);
-    launch(k_c16_cn_finish, cblocks(cap, 256), 256, 0, st, w.cx64, w.cpos, a.cur, c, a.sc);
+    launch(k_c16_cn_finish, cblocks(cap, 256), 256, 0, st, w.cx64, w.cpos, a.cur, c, a.sc, w.moved);
     return launched + 1;
 }
 
