@@ -1447,6 +1447,7 @@ int ppe_setup(PpeWork& w, uint32_t cap, uint32_t nscenes, const Grid&, const Phy
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaDeviceGetAttribute(&w.l2_bytes, cudaDevAttrL2CacheSize, dev);
     {
         per_sm = 1 << 30;
         for (const void* f : solve_kernels()) {

@@ -94,6 +94,7 @@ struct PpeWork {
     bool c16 = false;                  // the solve uses this layout
     bool c16_ready = false;            // its buffers exist
     bool c16_shared = false;           // c16_cells and c16_nbr are another work's
+    int l2_bytes = 0;                  // of the device
     int c16_smem_chunks = 8;           // chunks per warp held in shared memory across iterations
     unsigned char* c16_block = nullptr;  // the allocation of the arrays from here to c16_epoch
     uint32_t c16_nsuper = 0;           // linked cells, in curve order

@@ -75,14 +75,17 @@ constexpr int C16_PACK_THREADS = 1024;
 constexpr int C16_BATCH = 4;                // chunks a warp loads at a time, twice buffered
 constexpr int C16_BATCH64 = 3;              // (6 of them: 5 % slower; 768 threads with 3: 2 to 10 % slower)
 // A matrix of several L2s comes from memory: every warp has the batch after
-// the next fetched into L2, 3 KB at a time, before it loads it.  A solve of
-// 1,088,346 rows with S' 16.7 -> 15.5 ms, without S' 851,839 rows 13.0 -> 12.2
-// and 507,178 rows 7.43 -> 7.22; where L2 holds a good part of the matrix the
-// fetches are in its way (311,747 rows 4.43 -> 4.52 ms, 189,647 2.37 -> 3.19).
-// 8, 16 and 24 chunks ahead: 15.8, 15.9 and 16.1 ms; none (the loaded batch
-// itself) 15.8.
+// the next fetched into L2, 3 KB at a time, before it loads it.  Where L2 holds
+// a good part of the matrix the fetches are in its way; with S', which L2
+// holds too, up to a larger one.  ms a solve without and with them, by rows
+// (1.45 KB of entries each): 303,860 4.46 and 4.56 (S' 4.54, 4.78), 374,952
+// 5.49 and 5.57 (5.53, 5.85), 419,968 6.15 and 6.10 (6.20, 6.44), 468,160 7.03
+// and 6.86 (7.05, 7.08), 531,196 8.12 and 7.88 (8.43, 8.17), 689,132 10.34 and
+// 10.06 (10.89, 10.45): they cross at 4.5 and 5 times the L2.
+// 8, 16 and 24 chunks ahead: 15.8, 15.9 and 16.1 ms at 1,088,346 rows with S',
+// 4 15.5; none (the loaded batch itself) 15.8.
 constexpr uint32_t C16_AHEAD = 4;
-constexpr uint32_t C16_AHEAD_FROM = 700000;  // chunks: 540 MB, some 400,000 rows
+constexpr uint32_t C16_AHEAD_FROM = 9, C16_AHEAD_FROM_SP = 10;  // half L2s of entries
 constexpr uint32_t C16_STATS = 4;
 constexpr uint32_t C16_SP_SLICES = C16_COLS / 32 + 1;  // S' slices (32 rows) a tile can have, and one
 
@@ -1096,6 +1099,7 @@ struct C16Args {
     Scalars* sc;
     double tol, eta_min;
     uint32_t keep;              // chunks read as evict_last, over all tiles
+    uint32_t ahead_from;        // chunks of the smallest matrix fetched ahead (C16_AHEAD_FROM)
     int max_iter, inner_cap, max_outer;
     uint32_t smem_chunks;       // most chunks a block holds in shared memory
     uint32_t smem_bytes;        // its dynamic shared memory
@@ -1235,7 +1239,7 @@ __device__ __forceinline__ C16View c16_view(const C16Args& S, uint32_t t, uint32
     v.nseg = ti.wmax ? (ti.wmax + v.cpw - 2) / v.cpw + 1 : 1u;
     v.resw = 0;
     v.keepw = keep == 0xffffffffu ? keep : (uint32_t)((uint64_t)v.cpw * min(keep, C) / C);
-    v.ahead = C >= C16_AHEAD_FROM ? C16_AHEAD : 0x7fffffffu;
+    v.ahead = C >= S.ahead_from ? C16_AHEAD : 0x7fffffffu;
     v.cl = S.collist + (size_t)t * C16_COLS;
     v.spf = S.sp_first + (size_t)t * C16_SP_SLICES;
     v.tile = t;
@@ -2585,6 +2589,8 @@ int ppe_c16_enqueue_solve(PpeWork& w, const StageArgs& a, const mps_options& opt
     // the share of the matrix kept in L2: the same byte budget as the 8-byte layout
     S.keep = w.l2_keep_entries == 0xFFFFFFFFu ? 0xFFFFFFFFu
                                                : (uint32_t)((size_t)w.l2_keep_entries * 8 / C16_CHUNK_BYTES);
+    S.ahead_from = (uint32_t)((size_t)w.l2_bytes / 2 *
+                            (w.c16_learned ? C16_AHEAD_FROM_SP : C16_AHEAD_FROM) / C16_CHUNK_BYTES);
     const int chunks = w.c16_smem_chunks < 0 ? 0 : (w.c16_smem_chunks > 8 ? 8 : w.c16_smem_chunks);
     S.smem_chunks = (uint32_t)chunks * 32;  // of the 32 warps an SM's share is counted in
     S.smem_bytes = (uint32_t)C16_SMEM;
