@@ -10,6 +10,7 @@
 // global gradient with atomics.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -1254,6 +1255,10 @@ __global__ void __launch_bounds__(TW_THREADS) k_lp_wgrad_tc(const float* __restr
 // ---------------------------------------------------------------- host side
 int lp_setup(LearnedWork& L, uint32_t cap, std::string* err) {
     L.cap = cap;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    L.sms = (uint32_t)sms;
     bool ok = true;
     auto al = [&](void** p, size_t bytes) {
         if (cudaMalloc(p, bytes + 64) != cudaSuccess) { ok = false; return; }
@@ -1404,7 +1409,7 @@ void lp_forward(LearnedWork& L, const LpSystem& S, bool exact, uint32_t cap, cud
     (void)exact;
     const uint32_t wb = blocks_for(cap * 32u, 256);   // warp per row
     const uint32_t db = blocks_for(cap, DT);          // tiles of the dense layers
-    const uint32_t dgrid = db < 148u * 4u ? db : 148u * 4u;
+    const uint32_t dgrid = std::min(db, L.sms * 4u);
     const uint32_t tgrid = tensor_cores ? tc_grids(cap).dense : 0u;
     uint32_t* err = const_cast<uint32_t*>(&S.sc->err);
     auto dense = [&](const float* x, int woff, int boff, const float* resid, float* pre, float* out, int act) {
@@ -1492,9 +1497,9 @@ int lp_loss_grad(LearnedWork& L, const LpSystem& S, bool exact, uint64_t seed, u
     const bool tc = L.train_tensor_cores;
     lp_forward(L, S, exact, cap, st, tc, true);
     const uint32_t tb = blocks_for(cap, 256), wb = blocks_for(cap * 32u, 256);
-    const uint32_t gb = wb < 148u * 3u ? wb : 148u * 3u;  // the kernels with weight gradients: three blocks an SM
+    const uint32_t gb = std::min(wb, L.sms * 3u);  // the kernels with weight gradients: three blocks an SM
     const uint32_t db = blocks_for(cap, DT);
-    const uint32_t dgrid = db < 148u * 3u ? db : 148u * 3u;
+    const uint32_t dgrid = std::min(db, L.sms * 3u);
     const TcGrids tg = tc ? tc_grids(cap) : TcGrids{0u, 0u};
     uint32_t* err = const_cast<uint32_t*>(&S.sc->err);
     // dx (+)= W^T dy, grad(W) += dy x^T, grad(b) += dy (boff >= 0)

@@ -72,6 +72,7 @@ struct LearnedWork {
     bool tensor_cores = false;       // inference forward on tcgen05 (set after a self-check)
     bool train_tensor_cores = false; // training's 64 -> 64 products on tcgen05 (BF16 operands)
     uint32_t cap = 0;
+    uint32_t sms = 0;                // of the device
     // parameters
     float* w32 = nullptr;            // FP32 master
     __nv_bfloat16* w16 = nullptr;    // BF16 copy used by the kernels
