@@ -109,9 +109,10 @@ typedef struct {
     int ppe_layout;      /* PPE matrix in the solver: 0 = compact (tiles of
                             neighbouring rows, 16-bit codes into each tile's
                             list of columns, 6 bytes per entry), or the
-                            8-byte layout in grids with more than 4 linked
-                            cells a particle; -1 = always the 8-byte layout.  Same matrix either way;
-                            mps_autotune may change a single scene's.         */
+                            8-byte layout in grids of more than 65,536 linked
+                            cells and 4 a particle; -1 = always the 8-byte
+                            layout.  Same matrix either way; mps_autotune may
+                            change a single scene's.                          */
     int ppe_smem_chunks; /* 128-entry chunks of the matrix kept in shared
                             memory across CG iterations, per each of an SM's
                             32 warps (0: 8; -1: none; at most 8 in the

@@ -2290,9 +2290,14 @@ bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
 // (a particle far from the others) the 8-byte layout is faster.  70,912
 // particles, ms a step over tiles and in the 8-byte layout: 4.05 cells a
 // particle 0.68 and 0.78 (learned 0.86 and 0.99), 5.95 0.77 and 0.79, 8.4 0.89
-// and 0.80, 19 1.37 and 0.86.  A tank full of water has 0.02, half full 0.04.
+// and 0.80, 19 1.37 and 0.86.  The tiles gain 0.06 ms and more in the smallest
+// scenes, so few cells are always taken: 5,312 particles in 68,921 cells 0.26
+// and 0.30, in 140,608 0.305 and 0.308, in 262,144 0.38 and 0.32.  A tank full
+// of water has 0.02 cells a particle, one half full 0.04.
+constexpr uint64_t C16_FEW_CELLS = 65536;
 bool ppe_c16_prefers(uint32_t cap, const Grid* grids, uint32_t ngrids) {
-    return ppe_c16_takes(cap, grids, ngrids) && c16_cells(grids, ngrids) <= 4ull * cap;
+    return ppe_c16_takes(cap, grids, ngrids) &&
+           c16_cells(grids, ngrids) <= std::max<uint64_t>(4ull * cap, C16_FEW_CELLS);
 }
 
 int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, cudaStream_t st,

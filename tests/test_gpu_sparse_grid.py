@@ -1,6 +1,6 @@
 """Grids with many more linked cells than particles (one particle far from
-the others): past 4 cells a particle the default is the 8-byte layout; the
-compact one can still be asked for, and both give the same step."""
+the others): past 65,536 cells and 4 a particle the default is the 8-byte
+layout; the compact one can still be asked for, and both give the same step."""
 import numpy as np
 import pytest
 
@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 def test_layout_by_cells(capi, cells, compact):
     pos, vel, nb2, nb1 = _flow((14, 8, 13), (9, 6, 10), 0.01)
     edge = 0.04 * (cells * (len(pos) + 1)) ** (1 / 3)
+    assert cells < 4 or cells * len(pos) > 65536
     pos = np.concatenate([pos.min(0)[None] + np.float32(edge), pos]).astype(np.float32)  # a dummy
     vel = np.concatenate([np.zeros((1, 3), np.float32), vel])
     args = (_params(capi, 0.01, 5e-4), pos, nb2 + 1, nb1, vel)
