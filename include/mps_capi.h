@@ -110,7 +110,7 @@ typedef struct {
                             neighbouring rows, 16-bit codes into each tile's
                             list of columns, 6 bytes per entry), or the
                             8-byte layout in grids of more than 65,536 linked
-                            cells and 4 a particle; -1 = always the 8-byte
+                            cells and 64 a particle; -1 = always the 8-byte
                             layout.  Same matrix either way; mps_autotune may
                             change a single scene's.                          */
     int ppe_smem_chunks; /* 128-entry chunks of the matrix kept in shared

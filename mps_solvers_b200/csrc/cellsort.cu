@@ -156,74 +156,99 @@ __global__ void __launch_bounds__(256) k_radix_scan(uint32_t* __restrict__ hist,
     if (lane == 0) hist[(size_t)SORT_RADIX * tiles + d] = carry;
 }
 
-// Exclusive scan of `total` counters by one block: chunks of 16384 entries,
-// each thread loading 16 consecutive counters as four 16-byte vectors (the
-// array starts 16-byte aligned), a block scan of the thread sums, and a
-// running carry between chunks.
+// Exclusive scan of the counters [c0, c0 + 16384) below total by a block of 1024
+// threads, from carry: each thread loads 16 consecutive counters as four
+// 16-byte vectors (the array starts 16-byte aligned), then a block scan of the
+// thread sums.  Returns the chunk's sum.
+constexpr uint32_t SCAN_CHUNK = 16384;
+__device__ __forceinline__ uint32_t scan_chunk(uint32_t* __restrict__ a, uint32_t c0, uint32_t total, uint32_t carry,
+                                               uint32_t* warp_sums) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t b0 = c0 + 16 * threadIdx.x;
+    const bool full = b0 + 16 <= total;
+    uint32_t v[16];
+    if (full) {
+        const uint4* p = reinterpret_cast<const uint4*>(a + b0);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint4 t = p[u];
+            v[4 * u] = t.x;
+            v[4 * u + 1] = t.y;
+            v[4 * u + 2] = t.z;
+            v[4 * u + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 16; u++) v[u] = (b0 + u < total) ? a[b0 + u] : 0u;
+    }
+    uint32_t s = 0;
+#pragma unroll
+    for (int u = 0; u < 16; u++) s += v[u];
+    uint32_t x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += t;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = warp_sums[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += t;
+        }
+        warp_sums[lane] = w;
+    }
+    __syncthreads();
+    uint32_t run = carry + (x - s) + (warp > 0 ? warp_sums[warp - 1] : 0u);
+    const uint32_t chunk_total = warp_sums[31];
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+        const uint32_t e = run;
+        run += v[u];
+        v[u] = e;
+    }
+    if (full) {
+        uint4* p = reinterpret_cast<uint4*>(a + b0);
+#pragma unroll
+        for (int u = 0; u < 4; u++) p[u] = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            if (b0 + u < total) a[b0 + u] = v[u];
+    }
+    return chunk_total;
+}
+
+// Exclusive scan of `total` counters by one block, chunk after chunk.
 __global__ void __launch_bounds__(1024) k_scan_exclusive(uint32_t* __restrict__ a, uint32_t total) {
     after_previous();
     __shared__ uint32_t warp_sums[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t carry = 0;
-    for (uint32_t c0 = 0; c0 < total; c0 += 16384) {
-        const uint32_t b0 = c0 + 16 * threadIdx.x;
-        const bool full = b0 + 16 <= total;
-        uint32_t v[16];
-        if (full) {
-            const uint4* p = reinterpret_cast<const uint4*>(a + b0);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const uint4 t = p[u];
-                v[4 * u] = t.x;
-                v[4 * u + 1] = t.y;
-                v[4 * u + 2] = t.z;
-                v[4 * u + 3] = t.w;
-            }
-        } else {
-#pragma unroll
-            for (int u = 0; u < 16; u++) v[u] = (b0 + u < total) ? a[b0 + u] : 0u;
-        }
-        uint32_t s = 0;
-#pragma unroll
-        for (int u = 0; u < 16; u++) s += v[u];
-        uint32_t x = s;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += t;
-        }
-        if (lane == 31) warp_sums[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t w = warp_sums[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += t;
-            }
-            warp_sums[lane] = w;
-        }
-        __syncthreads();
-        uint32_t run = carry + (x - s) + (warp > 0 ? warp_sums[warp - 1] : 0u);
-        const uint32_t chunk_total = warp_sums[31];
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const uint32_t e = run;
-            run += v[u];
-            v[u] = e;
-        }
-        if (full) {
-            uint4* p = reinterpret_cast<uint4*>(a + b0);
-#pragma unroll
-            for (int u = 0; u < 4; u++) p[u] = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-        } else {
-#pragma unroll
-            for (int u = 0; u < 16; u++)
-                if (b0 + u < total) a[b0 + u] = v[u];
-        }
-        carry += chunk_total;
+    for (uint32_t c0 = 0; c0 < total; c0 += SCAN_CHUNK) {
+        carry += scan_chunk(a, c0, total, carry, warp_sums);
         __syncthreads();  // warp_sums is rewritten by the next chunk
     }
+}
+
+// The same for many counters: a block a chunk, the chunks' sums scanned, then
+// added.  1.2 million counters in 20 us for the 150 of one block.
+__global__ void __launch_bounds__(1024) k_scan_chunks(uint32_t* __restrict__ a, uint32_t total,
+                                                      uint32_t* __restrict__ sums) {
+    after_previous();
+    __shared__ uint32_t warp_sums[32];
+    const uint32_t t = scan_chunk(a, blockIdx.x * SCAN_CHUNK, total, 0u, warp_sums);
+    if (threadIdx.x == 0) sums[blockIdx.x] = t;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_add(uint32_t* __restrict__ a, uint32_t total,
+                                                   const uint32_t* __restrict__ sums) {
+    after_previous();
+    const uint32_t add = sums[blockIdx.x];
+    const uint32_t end = min(blockIdx.x * SCAN_CHUNK + SCAN_CHUNK, total);
+    for (uint32_t i = blockIdx.x * SCAN_CHUNK + threadIdx.x; i < end; i += 1024) a[i] += add;
 }
 
 // Downsweep: stable rank of every key inside its tile and scatter.
@@ -503,6 +528,15 @@ int launch_keys_and_sort(const float4* pos, const float4* tmp, int apply, const 
 
 void launch_scan_exclusive(uint32_t* a, uint32_t total, cudaStream_t st) {
     launch(k_scan_exclusive, 1, 1024, 0, st, a, total);
+}
+
+uint32_t scan_sums(uint32_t total) { return blocks_for(total, SCAN_CHUNK); }
+
+void launch_scan_exclusive_many(uint32_t* a, uint32_t total, uint32_t* sums, cudaStream_t st) {
+    const uint32_t nb = scan_sums(total);
+    launch(k_scan_chunks, nb, 1024, 0, st, a, total, sums);
+    launch(k_scan_exclusive, 1, 1024, 0, st, sums, nb);
+    launch(k_scan_add, nb, 1024, 0, st, a, total, sums);
 }
 
 

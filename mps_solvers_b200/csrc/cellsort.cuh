@@ -94,6 +94,9 @@ void launch_cell_start_plain(const uint32_t* keys_sorted, uint32_t n, const Grid
                              uint32_t* n_in_grid, cudaStream_t st);
 // exclusive scan of `total` uint32 counters in place (one block)
 void launch_scan_exclusive(uint32_t* a, uint32_t total, cudaStream_t st);
+// the same by many blocks, with sums of scan_sums(total) words
+uint32_t scan_sums(uint32_t total);
+void launch_scan_exclusive_many(uint32_t* a, uint32_t total, uint32_t* sums, cudaStream_t st);
 void launch_cell_end_from_start(const uint32_t* cell_start, uint32_t ncells, uint32_t* start_out,
                                 uint32_t* end_out, cudaStream_t st);
 

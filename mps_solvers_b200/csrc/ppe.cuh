@@ -101,6 +101,10 @@ struct PpeWork {
     uint32_t* c16_cells = nullptr;     // the up to 4 cells of the sorted grid of each
     uint32_t* c16_nbr = nullptr;       // the 27 linked cells around each
     uint32_t* c16_base = nullptr;      // its rows (counts, then scanned: its first row)
+    uint32_t* c16_list = nullptr;      // many linked cells: the occupied ones,
+    uint32_t* c16_list_n = nullptr;    // their number, and the scan's sums
+    uint32_t* c16_sums = nullptr;
+    uint32_t* c16_rowcell = nullptr;   // linked cell of each row
     uint32_t* cpos = nullptr;          // compact row of each particle (rows only)
     uint32_t* clen = nullptr;          // off-diagonal entries of each compact row
     uint32_t* c16_off = nullptr;       // chunks per slice, then (scanned) the slices' first chunk

@@ -128,28 +128,61 @@ __device__ __forceinline__ bool c16_is_row(const C16Flag& F, uint32_t i) {
     return ptype(F.pos[i]) != T_DUMMY && !((double)F.n[i] < b);
 }
 
-// Rows of linked cell h (its up to 4 cells of the sorted grid).
-__global__ void __launch_bounds__(256) k_c16_count(C16Flag F, const uint32_t* __restrict__ cells, uint32_t nsuper,
-                                                   const uint32_t* __restrict__ cs, uint32_t* __restrict__ base,
-                                                   uint32_t* __restrict__ stats) {
+// Grids of many linked cells, most of them empty (c16_lists): the ones that hold
+// particles as a list, in any order (the counts of the others are 0).
+__global__ void __launch_bounds__(256) k_c16_occupied(const uint32_t* __restrict__ cells, uint32_t nsuper,
+                                                      const uint32_t* __restrict__ cs, uint32_t* __restrict__ base,
+                                                      uint32_t* __restrict__ list, uint32_t* __restrict__ list_n) {
     after_previous();
-    const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31;
-    if (blockIdx.x == 0 && threadIdx.x < C16_STATS) stats[threadIdx.x] = 0u;
-    if (h > nsuper) return;
-    uint32_t n = 0;
+    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    bool some = false;
     if (h < nsuper) {
         const uint4 c4 = *reinterpret_cast<const uint4*>(cells + 4 * (size_t)h);
         const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            if (c[u] == C16_NONE) continue;
-            const uint32_t lo = cs[c[u]], hi = cs[c[u] + 1];
-            for (uint32_t i = lo + lane; i < hi; i += 32) n += c16_is_row(F, i) ? 1u : 0u;
-        }
-        n = __reduce_add_sync(0xffffffffu, n);
+        for (int u = 0; u < 4; u++)
+            if (c[u] != C16_NONE) some |= cs[c[u]] != cs[c[u] + 1];
     }
-    if (lane == 0) base[h] = n;  // base[nsuper] = 0: the scan leaves R there
+    if (h <= nsuper) base[h] = 0u;
+    const uint32_t m = __ballot_sync(0xffffffffu, some);
+    uint32_t at = 0;
+    if (lane == 0 && m) at = atomicAdd(list_n, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (some) list[at + __popc(m & ((1u << lane) - 1u))] = h;
+}
+
+// The linked cell of a warp: its own number, or its place in the list of
+// occupied ones (list not null; C16_NONE past the end of either).
+__device__ __forceinline__ uint32_t c16_cell_of(uint32_t warp, uint32_t nsuper, const uint32_t* __restrict__ list,
+                                                const uint32_t* __restrict__ list_n) {
+    if (!list) return warp < nsuper ? warp : C16_NONE;
+    return warp < *list_n ? list[warp] : C16_NONE;
+}
+
+// Rows of linked cell h (its up to 4 cells of the sorted grid).
+__global__ void __launch_bounds__(256) k_c16_count(C16Flag F, const uint32_t* __restrict__ cells, uint32_t nsuper,
+                                                   const uint32_t* __restrict__ list,
+                                                   const uint32_t* __restrict__ list_n,
+                                                   const uint32_t* __restrict__ cs, uint32_t* __restrict__ base,
+                                                   uint32_t* __restrict__ stats) {
+    after_previous();
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x < C16_STATS) stats[threadIdx.x] = 0u;
+    if (warp == nsuper && !list && lane == 0) base[nsuper] = 0u;  // the scan leaves R there
+    const uint32_t h = c16_cell_of(warp, nsuper, list, list_n);
+    if (h == C16_NONE) return;
+    uint32_t n = 0;
+    const uint4 c4 = *reinterpret_cast<const uint4*>(cells + 4 * (size_t)h);
+    const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        if (c[u] == C16_NONE) continue;
+        const uint32_t lo = cs[c[u]], hi = cs[c[u] + 1];
+        for (uint32_t i = lo + lane; i < hi; i += 32) n += c16_is_row(F, i) ? 1u : 0u;
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) base[h] = n;
 }
 
 // A batch: the scenes' rows start at multiples of 8, so that no slice (and no
@@ -160,7 +193,8 @@ __global__ void __launch_bounds__(256) k_c16_count(C16Flag F, const uint32_t* __
 __global__ void __launch_bounds__(256) k_c16_shift(const uint32_t* __restrict__ dense, uint32_t nsuper,
                                                    const uint32_t* __restrict__ sfirst, uint32_t ns,
                                                    uint32_t* __restrict__ base, uint32_t* __restrict__ srow,
-                                                   uint32_t* __restrict__ rowlist, uint32_t* __restrict__ nrows) {
+                                                   uint32_t* __restrict__ rowlist, uint32_t* __restrict__ rowcell,
+                                                   uint32_t* __restrict__ nrows) {
     after_previous();
     __shared__ uint32_t first[PPE_MAX_SCENES + 1], at[PPE_MAX_SCENES + 1];
     for (uint32_t x = threadIdx.x; x <= ns; x += blockDim.x) first[x] = sfirst[x];
@@ -195,7 +229,8 @@ __global__ void __launch_bounds__(256) k_c16_shift(const uint32_t* __restrict__ 
         for (uint32_t s = threadIdx.x; s <= ns; s += blockDim.x) {
             srow[s] = at[s];
             if (s < ns)
-                for (uint32_t k = at[s] + dense[first[s + 1]] - dense[first[s]]; k < at[s + 1]; k++) rowlist[k] = C16_NONE;
+                for (uint32_t k = at[s] + dense[first[s + 1]] - dense[first[s]]; k < at[s + 1]; k++)
+                    rowlist[k] = rowcell[k] = C16_NONE;
         }
         if (threadIdx.x == 0) *nrows = at[ns];
     }
@@ -207,24 +242,26 @@ __global__ void __launch_bounds__(256) k_c16_shift(const uint32_t* __restrict__ 
 struct C16RowArgs {
     const uint32_t *cells, *cs, *base;
     uint32_t nsuper;
+    const uint32_t *list, *list_n;  // occupied linked cells (k_c16_occupied), or null
     const uint32_t* dense;  // batch: first row of every linked cell without the gaps
+    uint32_t* rowcell;      // linked cell of every row
     uint32_t *cpos, *rowlist, *nrows, *dense_list, *dense_n, *rlen;
     double* diag64;
 };
 
 __global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, C16RowArgs A) {
     after_previous();
-    const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
-    if (h >= A.nsuper) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (A.dense) *A.dense_n = A.dense[A.nsuper];
+        else *A.nrows = A.base[A.nsuper];
+    }
+    const uint32_t h = c16_cell_of((blockIdx.x * blockDim.x + threadIdx.x) >> 5, A.nsuper, A.list, A.list_n);
+    if (h == C16_NONE) return;
     uint32_t at = A.base[h];
     const uint32_t dd = A.dense ? at - A.dense[h] : 0u;  // gaps before this cell
     const uint4 c4 = *reinterpret_cast<const uint4*>(A.cells + 4 * (size_t)h);
     const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
-    if (h == A.nsuper - 1 && lane == 0) {
-        if (A.dense) *A.dense_n = A.dense[A.nsuper];
-        else *A.nrows = A.base[A.nsuper];
-    }
 #pragma unroll
     for (int u = 0; u < 4; u++) {
         if (c[u] == C16_NONE) continue;
@@ -237,6 +274,7 @@ __global__ void __launch_bounds__(256) k_c16_rows(C16Flag F, C16RowArgs A) {
                 const uint32_t k = at + __popc(m & lt);
                 A.cpos[i] = k;
                 A.rowlist[k] = i;
+                A.rowcell[k] = h;
                 if (A.dense) A.dense_list[k - dd] = i;
             } else if (i < hi) {
                 A.cpos[i] = C16_NONE;
@@ -588,7 +626,8 @@ struct C16PackArgs {
     const uint32_t* off;
     const uint32_t* base;     // first row of every linked cell
     const uint32_t* nbr;      // 27 linked cells around each (C16_NONE: outside)
-    uint32_t nsuper, blocks;
+    const uint32_t* rowcell;  // linked cell of every row
+    uint32_t blocks;
     uint32_t ns;              // scenes of a batch (0: a single scene)
     const uint32_t* srow;     // their first rows
     const uint32_t* tb;       // and first tiles
@@ -656,7 +695,7 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
     extern __shared__ uint16_t page_slot[];  // slot of every page of rows (0xffff: none)
     __shared__ uint2 bits[C16_PAGES * 8];    // columns in use, and those before the word
     __shared__ uint32_t slot_page[C16_PAGES];
-    __shared__ uint32_t ws[32], found[4];
+    __shared__ uint32_t ws[32], found[2], cell[C16_PACK_THREADS], ncell;
     const uint32_t R = *A.nrows;
     const uint32_t nsl = (R + C16_ROWS - 1) / C16_ROWS;
     const uint32_t T = c16_tiles(R, A.blocks, A.ns);
@@ -688,21 +727,23 @@ __global__ void __launch_bounds__(C16_PACK_THREADS) k_c16_pack(C16PackArgs A) {
         return;
     }
     const uint32_t r0 = s0 * C16_ROWS, r1 = min(s1 * C16_ROWS, R), rows = r1 - r0;
-    if (warp < 2) {  // the linked cells of the first and the last row
-        const uint32_t k = warp ? r1 - 1 : r0;
-        const uint32_t h = warp_lower(A.nsuper, (uint64_t)k + 1, [&](uint32_t x) { return (uint64_t)__ldg(A.base + x); });
-        if (lane == 0) found[2 + warp] = h - 1;
+    // the linked cells of its rows, a thread a row, and what is around each
+    for (uint32_t k0 = r0; k0 < r1; k0 += nthr) {
+        if (tid == 0) ncell = 0u;
+        __syncthreads();
+        const uint32_t k = k0 + tid;
+        const uint32_t h = k < r1 ? __ldg(A.rowcell + k) : C16_NONE;
+        if (h != C16_NONE && (k == r0 || __ldg(A.rowcell + k - 1) != h)) cell[atomicAdd(&ncell, 1u)] = h;
+        __syncthreads();
+        for (uint32_t x = tid; x < ncell * 27u; x += nthr) {
+            const uint32_t nb = __ldg(A.nbr + (size_t)cell[x / 27u] * 27 + x % 27u);
+            if (nb == C16_NONE) continue;
+            const uint32_t lo = __ldg(A.base + nb), hi = __ldg(A.base + nb + 1);
+            if (lo < hi)
+                for (uint32_t p = lo / C16_PAGE; p <= (hi - 1) / C16_PAGE; p++) page_slot[p] = 1;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    const uint32_t h0 = found[2], h1 = found[3];
-    for (uint32_t x = tid; x < (h1 - h0 + 1) * 27u; x += nthr) {
-        const uint32_t nb = __ldg(A.nbr + (size_t)h0 * 27 + x);
-        if (nb == C16_NONE) continue;
-        const uint32_t lo = __ldg(A.base + nb), hi = __ldg(A.base + nb + 1);
-        if (lo < hi)
-            for (uint32_t p = lo / C16_PAGE; p <= (hi - 1) / C16_PAGE; p++) page_slot[p] = 1;
-    }
-    __syncthreads();
     // slots in page order
     uint32_t nslots;
     {
@@ -2285,20 +2326,24 @@ bool ppe_c16_takes(uint32_t cap, const Grid* grids, uint32_t ngrids) {
            c16_page_bytes(ppe_rows_cap(cap, ngrids)) <= C16_PAGE_BYTES_MAX;
 }
 
-// Every step counts and scans the linked cells, empty ones too (0.6 ms a
-// million), and a cell's links take 128 bytes: in a grid that is nearly empty
-// (a particle far from the others) the 8-byte layout is faster.  70,912
-// particles, ms a step over tiles and in the 8-byte layout: 4.05 cells a
-// particle 0.68 and 0.78 (learned 0.86 and 0.99), 5.95 0.77 and 0.79, 8.4 0.89
-// and 0.80, 19 1.37 and 0.86.  The tiles gain 0.06 ms and more in the smallest
-// scenes, so few cells are always taken: 5,312 particles in 68,921 cells 0.26
-// and 0.30, in 140,608 0.305 and 0.308, in 262,144 0.38 and 0.32.  A tank full
-// of water has 0.02 cells a particle, one half full 0.04.
+// The links of a linked cell take 132 bytes.  The tiles are the faster layout in
+// nearly empty grids too (70,912 particles with one far away, ms a step over
+// tiles and in the 8-byte layout: 2 cells a particle 0.52 and 0.78, 16 0.63 and
+// 0.87, 64 0.99 and 1.16; with S' at 64 1.17 and 1.38), but past 64 cells a
+// particle the links are more than both layouts' matrices.  A tank full of
+// water has 0.02 cells a particle, one half full 0.04.
 constexpr uint64_t C16_FEW_CELLS = 65536;
 bool ppe_c16_prefers(uint32_t cap, const Grid* grids, uint32_t ngrids) {
     return ppe_c16_takes(cap, grids, ngrids) &&
-           c16_cells(grids, ngrids) <= std::max<uint64_t>(4ull * cap, C16_FEW_CELLS);
+           c16_cells(grids, ngrids) <= std::max<uint64_t>(64ull * cap, C16_FEW_CELLS);
 }
+
+// Whether the numbering lists the occupied cells first (k_c16_occupied): three
+// launches more and a scan by many blocks, 16 us, where a warp for every cell
+// costs 0.6 us a thousand: 27,700 particles in 19,683 cells 0.424 ms a step with
+// and 0.42 without, in 59,319 0.428 and 0.437; of 70,913 in 287,496 0.54 and
+// 0.68.  Not where most cells are full.
+static bool c16_lists(const PpeWork& w) { return w.c16_nsuper > 32768u && w.c16_nsuper > w.cap / 8u; }
 
 int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork* same, cudaStream_t st,
                    std::string* err) {
@@ -2326,6 +2371,12 @@ int ppe_c16_enable(PpeWork& w, const Grid* grids, uint32_t ngrids, const PpeWork
         A.add(&w.c16_nbr, 27 * (size_t)w.c16_nsuper);
     }
     A.add(&w.c16_base, (size_t)w.c16_nsuper + 2);
+    if (c16_lists(w)) {
+        A.add(&w.c16_list, std::min<size_t>(w.c16_nsuper, w.cap));
+        A.add(&w.c16_list_n, 1);
+        A.add(&w.c16_sums, scan_sums(w.c16_nsuper + 1));
+    }
+    A.add(&w.c16_rowcell, vec);
     if (ns) {
         A.add(&w.c16_dense, (size_t)w.c16_nsuper + 2);
         A.add(&w.c16_sfirst, ns + 1);
@@ -2397,6 +2448,7 @@ void ppe_c16_free(PpeWork& w) {
         if (p) cudaFree(p);
     w.c16_block = nullptr;
     w.c16_cells = w.c16_nbr = w.c16_base = w.cpos = w.clen = w.c16_off = w.c16_tile = nullptr;
+    w.c16_list = w.c16_list_n = w.c16_sums = w.c16_rowcell = nullptr;
     w.c16_collist = w.c16_stats = nullptr;
     w.c16_ent = nullptr;
     w.cb64 = w.cx64 = w.cdiag64 = nullptr;
@@ -2448,14 +2500,26 @@ static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, boo
     F.scenes = a.batch.n ? w.scenes : nullptr;
     F.bthr = bthr;
     uint32_t* counts = a.batch.n ? w.c16_dense : w.c16_base;
-    launch(k_c16_count, cblocks((w.c16_nsuper + 1) * 32u, 256), 256, 0, st, F, w.c16_cells, w.c16_nsuper, a.cell_start,
-           counts, w.c16_stats);
-    launch_scan_exclusive(counts, w.c16_nsuper + 1, st);
+    uint32_t warps = w.c16_nsuper + 1, launched = 0;
+    if (w.c16_list) {
+        cudaMemsetAsync(w.c16_list_n, 0, sizeof(uint32_t), st);
+        launch(k_c16_occupied, cblocks(w.c16_nsuper + 1, 256), 256, 0, st, w.c16_cells, w.c16_nsuper, a.cell_start,
+               counts, w.c16_list, w.c16_list_n);
+        warps = std::min(w.c16_nsuper, w.cap);  // an occupied cell holds a particle
+        launched = 3;
+    }
+    launch(k_c16_count, cblocks(warps * 32u, 256), 256, 0, st, F, w.c16_cells, w.c16_nsuper, w.c16_list, w.c16_list_n,
+           a.cell_start, counts, w.c16_stats);
+    if (w.c16_list) launch_scan_exclusive_many(counts, w.c16_nsuper + 1, w.c16_sums, st);
+    else launch_scan_exclusive(counts, w.c16_nsuper + 1, st);
     C16RowArgs A;
     A.cells = w.c16_cells;
     A.cs = a.cell_start;
     A.base = w.c16_base;
     A.nsuper = w.c16_nsuper;
+    A.list = w.c16_list;
+    A.list_n = w.c16_list_n;
+    A.rowcell = w.c16_rowcell;
     A.dense = a.batch.n ? w.c16_dense : nullptr;
     A.cpos = w.cpos;
     A.rowlist = c16_rowlist(w);
@@ -2466,9 +2530,9 @@ static int ppe_c16_enqueue_rows(PpeWork& w, const StageArgs& a, double bthr, boo
     A.diag64 = w.diag64;
     if (a.batch.n)
         launch(k_c16_shift, cblocks(w.c16_nsuper + 1, 256), 256, 0, st, w.c16_dense, w.c16_nsuper, w.c16_sfirst,
-               w.nscenes, w.c16_base, w.c16_srow, A.rowlist, A.nrows);
-    launch(k_c16_rows, cblocks(w.c16_nsuper * 32u, 256), 256, 0, st, F, A);
-    return a.batch.n ? 4 : 3;
+               w.nscenes, w.c16_base, w.c16_srow, A.rowlist, A.rowcell, A.nrows);
+    launch(k_c16_rows, cblocks(warps * 32u, 256), 256, 0, st, F, A);
+    return launched + (a.batch.n ? 4 : 3);
 }
 
 static uint32_t c16_maxslices(const PpeWork& w, uint32_t cap) {
@@ -2533,7 +2597,7 @@ int ppe_c16_enqueue_pack(PpeWork& w, const StageArgs& a, uint32_t cap, cudaStrea
     P.off = w.c16_off;
     P.base = w.c16_base;
     P.nbr = w.c16_nbr;
-    P.nsuper = w.c16_nsuper;
+    P.rowcell = w.c16_rowcell;
     P.blocks = (uint32_t)w.sms;
     P.tiles = reinterpret_cast<C16Tile*>(w.c16_tile);
     P.collist = w.c16_collist;
